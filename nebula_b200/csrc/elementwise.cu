@@ -520,31 +520,6 @@ __global__ void lstm_cell_kernel(const float *z, const float *c_prev, float *c_o
     }
 }
 
-// ------------------------------------------------------------ generic SGEMM
-// _gemm_ (common/gemm.h:21-25) with the CPU path's meaning of every argument
-// (row-major, leading dimensions honoured, all four transpose cases), unlike the
-// reference's CUDA stand-in (common/gemm.cu:38-153) which ignores lda/ldb/ldc.
-__global__ void sgemm_kernel(int ta, int tb, int M, int N, int K, float alpha, const float *A, int lda, const float *B,
-                             int ldb, float beta, float *C, int ldc) {
-    __shared__ float As[16][17], Bs[16][17];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int row = blockIdx.y * 16 + ty, col = blockIdx.x * 16 + tx;
-    float acc = 0.0f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        const int ka = k0 + tx, kb = k0 + ty;
-        As[ty][tx] = (row < M && ka < K) ? (ta ? A[(size_t)ka * lda + row] : A[(size_t)row * lda + ka]) : 0.0f;
-        Bs[ty][tx] = (col < N && kb < K) ? (tb ? B[(size_t)col * ldb + kb] : B[(size_t)kb * ldb + col]) : 0.0f;
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < 16; k++) acc = fmaf(As[ty][k], Bs[k][tx], acc);
-        __syncthreads();
-    }
-    if (row < M && col < N) {
-        float *c = C + (size_t)row * ldc + col;
-        *c = alpha * acc + (beta == 0.0f ? 0.0f : beta * *c);
-    }
-}
-
 }  // namespace
 
 // Loads the code of every kernel of this file on the current device (a kernel's code is otherwise loaded by its
@@ -558,20 +533,12 @@ void elementwise_prepare_device() {
         (const void *)pool_kernel<false>, (const void *)pool_nhwc4_kernel, (const void *)shortcut_kernel<true>,
         (const void *)shortcut_kernel<false>, (const void *)weight_pack_kernel, (const void *)weight_rowwin_kernel,
         (const void *)rowwin_input_kernel, (const void *)weight_relayout_kernel, (const void *)fc_permute_kernel,
-        (const void *)splitk_reduce_kernel, (const void *)lstm_cell_kernel, (const void *)sgemm_kernel,
+        (const void *)splitk_reduce_kernel, (const void *)lstm_cell_kernel,
         (const void *)u8_pack_kernel, (const void *)splitk_reduce4_kernel, (const void *)shortcut_nhwc4_kernel};
     for (const void *k : kernels) NB_CHECK_CUDA(cudaFuncGetAttributes(&fa, k));
 }
 
 // ---------------------------------------------------------------- launchers
-void launch_sgemm(nb_handle_s *h, bool ta, bool tb, int M, int N, int K, float alpha, const float *A, int lda,
-                  const float *B, int ldb, float beta, float *C, int ldc) {
-    dim3 grid((N + 15) / 16, (M + 15) / 16), block(16, 16);
-    if (grid.y > 65535) throw Error(NB_ERR_UNSUPPORTED, "gemm: M too large for this operator");
-    sgemm_kernel<<<grid, block, 0, h->stream>>>(ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
-    check_launch("sgemm_kernel");
-    count_launch(h);
-}
 void launch_activation(nb_handle_s *h, int act, float *data, size_t n) {
     if (act == NB_ACT_LINEAR || n == 0) return;
     activation_kernel<<<grid_for(n, h, 4), TPB, 0, h->stream>>>(data, n, act);

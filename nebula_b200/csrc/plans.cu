@@ -141,7 +141,7 @@ size_t ConvPlan::reserve(const ForwardOpts &o) {
     const size_t yout = (size_t)d.batch * d.filters * OH * OW;
     const bool tc_mode = h->math_mode != NB_MATH_FP32;
     if (!o.y_nhwc) y_scratch.reserve(yout);
-    if (pth == PATH_SIMT && rowwin_ok && tc_mode) {
+    if (pth == PATH_SIMT && rowwin_ok) {
         x_rowwin.reserve((size_t)d.batch * d.height * rw_wp * 4);
     } else if (pth == PATH_SIMT && pack_ok && tc_mode && h->encode_tiled) {
         // the kernel gathers x in place
@@ -165,12 +165,14 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
     g.batch = d.batch; g.C = d.channels; g.H = d.height; g.W = d.width; g.OH = OH; g.OW = OW;
     g.ksize = d.size; g.stride = d.stride; g.pad = d.padding;
 
-    if (pth == PATH_SIMT && rowwin_ok && h->math_mode != NB_MATH_FP32) {
-        // tensor-core route for 1-4 input channels: one TMA-fetched K slice per filter row
-        const bool three = h->math_mode == NB_MATH_TF32X3;
+    if (pth == PATH_SIMT && rowwin_ok) {
+        // 1-4 input channels: one K slice per filter row (fetched by TMA on the tensor-core routes; on the CUDA cores a
+        // slice of 4*size aligned floats per row instead of `size` taps of 1-4 scattered ones)
+        const bool three = h->math_mode == NB_MATH_TF32X3, cuda_cores = h->math_mode == NB_MATH_FP32;
         float *xw = x_rowwin.p;
         if (o.x_rowwin) xw = const_cast<float *>(x);       // the caller already holds the input in this layout
-        else launch_rowwin_input(h, x, xw, d.batch, d.channels, d.height, d.width, rw_wp, d.padding, o.x_nhwc, !three);
+        else launch_rowwin_input(h, x, xw, d.batch, d.channels, d.height, d.width, rw_wp, d.padding, o.x_nhwc,
+                                 h->math_mode == NB_MATH_TF32);
         GemmArgs ra;
         ra.a = xw; ra.a_is_conv = true;
         ConvGeom &rg = ra.g;
@@ -188,6 +190,13 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         ra.y = yo; ra.ldy = d.filters;
         ra.algo_flops = 2.0 * (double)ra.M * d.filters * d.channels * d.size * d.size;
         ra.b = wr.hi.p; ra.b_lo = wr.lo.p;
+        if (cuda_cores) {
+            ra.Kc = 4 * d.size;             // without the zero columns that fill up a tensor-core K block
+            ra.b = wr.exact.p;
+            gemm_simt(h, ra);
+            if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
+            return;
+        }
         if (gemm_tc_supported(h, ra)) {
             gemm_tc(h, ra, three);
             if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
