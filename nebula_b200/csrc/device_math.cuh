@@ -8,6 +8,17 @@
 
 namespace nb {
 
+// Programmatic dependent launch.  The first call of every kernel lets the next one on the stream become resident while
+// this one runs (its set-up, its first weight tiles); grid_dependency_wait returns when every earlier kernel is
+// complete and its writes are visible.  A kernel waits before its first access to anything an earlier kernel
+// writes or reads, its own stores included; every thread block passes the wait, so completion is transitive.
+__device__ __forceinline__ void grid_dependents_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_begin() {
+    grid_dependents_start();
+    grid_dependency_wait();
+}
+
 // Round-to-nearest conversion of an fp32 value to TF32 (10-bit mantissa), kept
 // in fp32 storage with the low 13 mantissa bits cleared.  The tensor core reads
 // only the upper 19 bits of each operand, so pre-rounded data makes its result

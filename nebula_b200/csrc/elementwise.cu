@@ -78,6 +78,7 @@ inline unsigned grid_for(size_t n, const nb_handle_s *h, int per_thread = 1) {
 // ------------------------------------------------------------- activations
 // _<name>_activation_ (common/activations.cu:8-141) with the CPU formulas.
 __global__ void activation_kernel(float *data, size_t n, int act) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if ((((uintptr_t)data) & 15) == 0) {
@@ -97,6 +98,7 @@ __global__ void activation_kernel(float *data, size_t n, int act) {
 
 // _add_bias_ (common/utils.cu:118-134): y[b,c,s] += bias[c]
 __global__ void bias_kernel(float *out, const float *bias, unsigned channel, unsigned size, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride)
         out[i] += bias[(i / size) % channel];
@@ -105,6 +107,7 @@ __global__ void bias_kernel(float *out, const float *bias, unsigned channel, uns
 // float subtraction, double divisor sqrt(var)+0.00001, stored as float.
 __global__ void bn_normalize_kernel(float *out, const float *mean, const float *var, unsigned channel, unsigned size,
                                     size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const unsigned c = (i / size) % channel;
@@ -113,6 +116,7 @@ __global__ void bn_normalize_kernel(float *out, const float *mean, const float *
 }
 // _scale_ (common/batchnorm.cu:86-104)
 __global__ void bn_scale_kernel(float *out, const float *scale, unsigned channel, unsigned size, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride)
         out[i] *= scale[(i / size) % channel];
@@ -131,6 +135,7 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 __global__ void softmax_kernel(const float *x, float *y, int rows, int classes) {
+    grid_begin();
     __shared__ float red[32];
     __shared__ float bcast;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -174,6 +179,7 @@ __global__ void softmax_kernel(const float *x, float *y, int rows, int classes) 
 // ------------------------------------------------------------------ layouts
 // [B][C][HW] <-> [B][HW][C] through a 32x32 shared-memory tile.
 __global__ void transpose_kernel(const float *src, float *dst, int rows, int cols, int round) {
+    grid_begin();
     // src is [batch][rows][cols], dst is [batch][cols][rows]
     __shared__ float tile[32][33];
     const size_t img = (size_t)blockIdx.z * rows * cols;
@@ -194,6 +200,7 @@ __global__ void transpose_kernel(const float *src, float *dst, int rows, int col
 
 // 128-bit accesses when both pointers are 16-byte aligned (every buffer of the library is); scalar tail / fallback.
 __global__ void round_tf32_kernel(const float *src, float *dst, size_t n) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x, tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t done = 0;
     if (((((uintptr_t)src) | ((uintptr_t)dst)) & 15) == 0) {
@@ -240,6 +247,7 @@ __global__ void split_tf32_kernel(const float *src, float *hi, float *lo, size_t
 template <bool NHWC>
 __global__ void pool_kernel(const float *x, float *y, int B, int C, int H, int W, int OH, int OW, int k, int s, int p,
                             int is_max, int round, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         int c, ow, oh, b;
@@ -265,6 +273,7 @@ __global__ void pool_kernel(const float *x, float *y, int B, int C, int H, int W
 // NHWC with C % 4 == 0: one thread per 4 channels
 __global__ void pool_nhwc4_kernel(const float4 *x, float4 *y, int B, int C4, int H, int W, int OH, int OW, int k, int s,
                                   int p, int is_max, int round, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         size_t t = i;
@@ -298,6 +307,7 @@ __global__ void pool_nhwc4_kernel(const float4 *x, float4 *y, int B, int C4, int
 template <bool NHWC>
 __global__ void shortcut_kernel(const float *prev, const float *conn, float *y, int B, int Ci, int Hi, int Wi, int Co,
                                 int Ho, int Wo, int stride, int sample, int act, int round, size_t total) {
+    grid_begin();
     const int mw = Wi < Wo ? Wi : Wo, mh = Hi < Ho ? Hi : Ho, mc = Ci < Co ? Ci : Co;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
@@ -321,6 +331,7 @@ __global__ void shortcut_kernel(const float *prev, const float *conn, float *y, 
 // NHWC with both channel counts divisible by 4: one thread per 4 channels, 128-bit accesses
 __global__ void shortcut_nhwc4_kernel(const float4 *prev, const float4 *conn, float4 *y, int B, int Ci4, int Hi, int Wi, int Co4,
                                       int Ho, int Wo, int stride, int sample, int act, int round, size_t total) {
+    grid_begin();
     const int mw = Wi < Wo ? Wi : Wo, mh = Hi < Ho ? Hi : Ho, mc = Ci4 < Co4 ? Ci4 : Co4;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
@@ -379,6 +390,7 @@ __global__ void weight_rowwin_kernel(const float *w, float *dst, int F, int C, i
 }
 __global__ void rowwin_input_kernel(const float *x, float4 *dst, int N, int C, int H, int W, int Wp, int pad, int nhwc_in,
                                     int round, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         const int pcol = (int)(i % Wp);
@@ -403,6 +415,7 @@ __global__ void rowwin_input_kernel(const float *x, float4 *dst, int N, int C, i
 // first convolution's row-window tensor [N][H][Wp][4] directly (zero pixels left and right, zero in channels >= C).
 __global__ void u8_pack_kernel(const unsigned char *img, float *dst, int N, int C, int H, int W, int rowwin, int Wp, int pad,
                                int round, size_t total) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         if (rowwin) {       // one thread per padded pixel
@@ -460,6 +473,7 @@ __global__ void fc_permute_kernel(const float *w, float *dst, int out, int C, in
 // N % 4 == 0 (what the split-K path requires) and 16-byte aligned tensors: four columns per thread, 128-bit accesses
 __global__ void splitk_reduce4_kernel(const float4 *ws, int S, size_t MN4, int N4, const float4 *scale, const float4 *shift,
                                       int act, int round, float4 *y) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < MN4; i += stride) {
         float4 acc = ws[i];
@@ -484,6 +498,7 @@ __global__ void splitk_reduce4_kernel(const float4 *ws, int S, size_t MN4, int N
 }
 __global__ void splitk_reduce_kernel(const float *ws, int S, size_t MN, int N, const float *scale, const float *shift,
                                      int act, int round, float *y) {
+    grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < MN; i += stride) {
         float acc = ws[i];
@@ -502,6 +517,7 @@ __global__ void splitk_reduce_kernel(const float *ws, int S, size_t MN, int N, c
 // fp32 roundings as on the CPU path (no fused multiply-add).
 __global__ void lstm_cell_kernel(const float *z, const float *c_prev, float *c_out, float *h_out, float *h_round,
                                  int B, int H) {
+    grid_begin();
     const size_t total = (size_t)B * H;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
@@ -541,14 +557,14 @@ void elementwise_prepare_device() {
 // ---------------------------------------------------------------- launchers
 void launch_activation(nb_handle_s *h, int act, float *data, size_t n) {
     if (act == NB_ACT_LINEAR || n == 0) return;
-    activation_kernel<<<grid_for(n, h, 4), TPB, 0, h->stream>>>(data, n, act);
+    launch_overlapped(h, activation_kernel, grid_for(n, h, 4), TPB, 0, data, n, act);
     check_launch("activation_kernel");
     count_launch(h);
 }
 void launch_bias(nb_handle_s *h, float *out, const float *bias, unsigned channel, unsigned size, unsigned batch) {
     const size_t total = (size_t)channel * size * batch;
     if (!total) return;
-    bias_kernel<<<grid_for(total, h), TPB, 0, h->stream>>>(out, bias, channel, size, total);
+    launch_overlapped(h, bias_kernel, grid_for(total, h), TPB, 0, out, bias, channel, size, total);
     check_launch("bias_kernel");
     count_launch(h);
 }
@@ -556,21 +572,21 @@ void launch_bn_normalize(nb_handle_s *h, float *out, const float *mean, const fl
                          unsigned size, unsigned batch) {
     const size_t total = (size_t)channel * size * batch;
     if (!total) return;
-    bn_normalize_kernel<<<grid_for(total, h), TPB, 0, h->stream>>>(out, mean, var, channel, size, total);
+    launch_overlapped(h, bn_normalize_kernel, grid_for(total, h), TPB, 0, out, mean, var, channel, size, total);
     check_launch("bn_normalize_kernel");
     count_launch(h);
 }
 void launch_bn_scale(nb_handle_s *h, float *out, const float *scale, unsigned channel, unsigned size, unsigned batch) {
     const size_t total = (size_t)channel * size * batch;
     if (!total) return;
-    bn_scale_kernel<<<grid_for(total, h), TPB, 0, h->stream>>>(out, scale, channel, size, total);
+    launch_overlapped(h, bn_scale_kernel, grid_for(total, h), TPB, 0, out, scale, channel, size, total);
     check_launch("bn_scale_kernel");
     count_launch(h);
 }
 void launch_softmax(nb_handle_s *h, const float *x, float *y, int rows, int classes) {
     if (rows <= 0 || classes <= 0) return;
     const int threads = classes >= 1024 ? 256 : (classes >= 128 ? 128 : 32);
-    softmax_kernel<<<std::min(rows, h->sm_count * 16), threads, 0, h->stream>>>(x, y, rows, classes);
+    launch_overlapped(h, softmax_kernel, std::min(rows, h->sm_count * 16), threads, 0, x, y, rows, classes);
     check_launch("softmax_kernel");
     count_launch(h);
 }
@@ -583,7 +599,7 @@ void launch_layout(nb_handle_s *h, const float *src, float *dst, int B, int C, i
         const int nb_ = std::min(65535, B - b0);
         dim3 grid((cols + 31) / 32, (rows + 31) / 32, nb_), block(32, 8);
         if (grid.y > 65535) throw Error(NB_ERR_UNSUPPORTED, "layout conversion: extent too large");
-        transpose_kernel<<<grid, block, 0, h->stream>>>(src + (size_t)b0 * C * HW, dst + (size_t)b0 * C * HW, rows, cols,
+        launch_overlapped(h, transpose_kernel, grid, block, 0, src + (size_t)b0 * C * HW, dst + (size_t)b0 * C * HW, rows, cols,
                                                        round ? 1 : 0);
         check_launch("transpose_kernel");
         count_launch(h);
@@ -591,7 +607,7 @@ void launch_layout(nb_handle_s *h, const float *src, float *dst, int B, int C, i
 }
 void launch_round_tf32(nb_handle_s *h, const float *src, float *dst, size_t n) {
     if (!n) return;
-    round_tf32_kernel<<<grid_for(n, h), TPB, 0, h->stream>>>(src, dst, n);
+    launch_overlapped(h, round_tf32_kernel, grid_for(n, h), TPB, 0, src, dst, n);
     check_launch("round_tf32_kernel");
     count_launch(h);
 }
@@ -608,15 +624,15 @@ void launch_pool(nb_handle_s *h, const nb_pool_desc_t &d, const float *x, float 
     const int is_max = d.mode == NB_POOL_MAX;
     if (d.layout == NB_LAYOUT_NHWC && (d.channels % 4) == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
         const size_t t4 = total / 4;
-        pool_nhwc4_kernel<<<grid_for(t4, h), TPB, 0, h->stream>>>((const float4 *)x, (float4 *)y, d.batch, d.channels / 4,
+        launch_overlapped(h, pool_nhwc4_kernel, grid_for(t4, h), TPB, 0, (const float4 *)x, (float4 *)y, d.batch, d.channels / 4,
                                                                    d.height, d.width, OH, OW, d.size, d.stride, d.padding,
                                                                    is_max, round ? 1 : 0, t4);
     } else if (d.layout == NB_LAYOUT_NHWC) {
-        pool_kernel<true><<<grid_for(total, h), TPB, 0, h->stream>>>(x, y, d.batch, d.channels, d.height, d.width, OH, OW,
+        launch_overlapped(h, pool_kernel<true>, grid_for(total, h), TPB, 0, x, y, d.batch, d.channels, d.height, d.width, OH, OW,
                                                                       d.size, d.stride, d.padding, is_max, round ? 1 : 0,
                                                                       total);
     } else {
-        pool_kernel<false><<<grid_for(total, h), TPB, 0, h->stream>>>(x, y, d.batch, d.channels, d.height, d.width, OH,
+        launch_overlapped(h, pool_kernel<false>, grid_for(total, h), TPB, 0, x, y, d.batch, d.channels, d.height, d.width, OH,
                                                                        OW, d.size, d.stride, d.padding, is_max,
                                                                        round ? 1 : 0, total);
     }
@@ -631,15 +647,15 @@ void launch_shortcut(nb_handle_s *h, const nb_shortcut_desc_t &d, const float *p
     const int sample = d.out_width / d.conn_width > 1 ? d.out_width / d.conn_width : 1;
     if (d.layout == NB_LAYOUT_NHWC && (d.conn_channels % 4) == 0 && (d.out_channels % 4) == 0 &&
         ((((uintptr_t)prev) | ((uintptr_t)conn) | ((uintptr_t)y)) & 15) == 0)
-        shortcut_nhwc4_kernel<<<grid_for(total / 4, h), TPB, 0, h->stream>>>(
+        launch_overlapped(h, shortcut_nhwc4_kernel, grid_for(total / 4, h), TPB, 0, 
             (const float4 *)prev, (const float4 *)conn, (float4 *)y, d.batch, d.conn_channels / 4, d.conn_height, d.conn_width,
             d.out_channels / 4, d.out_height, d.out_width, stride, sample, d.activation, round ? 1 : 0, total / 4);
     else if (d.layout == NB_LAYOUT_NHWC)
-        shortcut_kernel<true><<<grid_for(total, h), TPB, 0, h->stream>>>(
+        launch_overlapped(h, shortcut_kernel<true>, grid_for(total, h), TPB, 0, 
             prev, conn, y, d.batch, d.conn_channels, d.conn_height, d.conn_width, d.out_channels, d.out_height,
             d.out_width, stride, sample, d.activation, round ? 1 : 0, total);
     else
-        shortcut_kernel<false><<<grid_for(total, h), TPB, 0, h->stream>>>(
+        launch_overlapped(h, shortcut_kernel<false>, grid_for(total, h), TPB, 0, 
             prev, conn, y, d.batch, d.conn_channels, d.conn_height, d.conn_width, d.out_channels, d.out_height,
             d.out_width, stride, sample, d.activation, round ? 1 : 0, total);
     check_launch("shortcut_kernel");
@@ -660,7 +676,7 @@ void launch_weight_rowwin(nb_handle_s *h, const float *w, float *dst, int F, int
 void launch_rowwin_input(nb_handle_s *h, const float *x, float *dst, int N, int C, int H, int W, int Wp, int pad, bool nhwc_in,
                          bool round) {
     const size_t total = (size_t)N * H * Wp;
-    rowwin_input_kernel<<<grid_for(total, h), TPB, 0, h->stream>>>(x, reinterpret_cast<float4 *>(dst), N, C, H, W, Wp, pad,
+    launch_overlapped(h, rowwin_input_kernel, grid_for(total, h), TPB, 0, x, reinterpret_cast<float4 *>(dst), N, C, H, W, Wp, pad,
                                                                   nhwc_in ? 1 : 0, round ? 1 : 0, total);
     check_launch("rowwin_input_kernel");
     count_launch(h);
@@ -669,7 +685,7 @@ void launch_u8_pack(nb_handle_s *h, const unsigned char *img, float *dst, int N,
                     int pad, bool round) {
     const size_t total = rowwin ? (size_t)N * H * Wp : (size_t)N * C * H * W;
     if (!total) return;
-    u8_pack_kernel<<<grid_for(total, h), TPB, 0, h->stream>>>(img, dst, N, C, H, W, rowwin ? 1 : 0, Wp, pad, round ? 1 : 0, total);
+    launch_overlapped(h, u8_pack_kernel, grid_for(total, h), TPB, 0, img, dst, N, C, H, W, rowwin ? 1 : 0, Wp, pad, round ? 1 : 0, total);
     check_launch("u8_pack_kernel");
     count_launch(h);
 }
@@ -690,16 +706,16 @@ void launch_splitk_reduce(nb_handle_s *h, const float *ws, int S, int M, int N, 
     const size_t MN = (size_t)M * N;
     const bool vec = (N % 4) == 0 && ((((uintptr_t)ws) | ((uintptr_t)y) | ((uintptr_t)scale) | ((uintptr_t)shift)) & 15) == 0;
     if (vec)
-        splitk_reduce4_kernel<<<grid_for(MN / 4, h), TPB, 0, h->stream>>>((const float4 *)ws, S, MN / 4, N / 4, (const float4 *)scale,
+        launch_overlapped(h, splitk_reduce4_kernel, grid_for(MN / 4, h), TPB, 0, (const float4 *)ws, S, MN / 4, N / 4, (const float4 *)scale,
                                                                          (const float4 *)shift, act, round ? 1 : 0, (float4 *)y);
     else
-        splitk_reduce_kernel<<<grid_for(MN, h), TPB, 0, h->stream>>>(ws, S, MN, N, scale, shift, act, round ? 1 : 0, y);
+        launch_overlapped(h, splitk_reduce_kernel, grid_for(MN, h), TPB, 0, ws, S, MN, N, scale, shift, act, round ? 1 : 0, y);
     check_launch("splitk_reduce_kernel");
     count_launch(h);
 }
 void launch_lstm_cell(nb_handle_s *h, const float *z, const float *c_prev, float *c_out, float *h_out, float *h_round,
                       int B, int H) {
-    lstm_cell_kernel<<<grid_for((size_t)B * H, h), TPB, 0, h->stream>>>(z, c_prev, c_out, h_out, h_round, B, H);
+    launch_overlapped(h, lstm_cell_kernel, grid_for((size_t)B * H, h), TPB, 0, z, c_prev, c_out, h_out, h_round, B, H);
     check_launch("lstm_cell_kernel");
     count_launch(h);
 }

@@ -91,17 +91,24 @@ struct TcParams {
     // two buffers and lets one store read while the next slab is staged.
     int slab2_offset;
     EpiParams e;                // fused epilogue
-    // gather mode: warps 6-9 build the A tile in shared memory from a strided activation tensor
+    int b_static;               // B is a plan's weights: its first tiles may be fetched before the kernels in front are done
+    int *status;
+};
+
+// The gather variants' parameters: the offset table is three quarters of them, and the other variants' launches do not
+// carry it.
+struct TcGatherParams : TcParams {
+    // gather mode: warps 10-13 build the A tile in shared memory from a strided activation tensor
     // (channel counts TMA cannot address, e.g. the 3-channel input layer); rows are output pixels
-    int gather;
     const float *gx;
     long gsn, gsh, gsw;         // element strides of the gathered tensor
     int gks, gpad, gK;          // filter size, padding, k*k*C: column kk = (kh, kw, c), c fastest
     int gH, gW, gOH, gOW, gstride, gM, ground;
     // per column: {element offset of (c, kh-pad, kw-pad) from the pixel's origin, (kh-pad) & 0xffff | (kw-pad) << 16}
     int2 gtab[GATHER_MAX_K];
-    int *status;
 };
+template <bool GATHER> struct ParamsOf { typedef TcParams type; };
+template <> struct ParamsOf<true> { typedef TcGatherParams type; };
 
 // The digits (split, n_tile, tw, th, tn) of a CTA's current tile.  Decoding a tile index costs seven integer
 // divisions (over a thousand cycles of dependent instructions on a role's critical path), so the index is decoded
@@ -164,7 +171,7 @@ struct Cfg {
 // held to the register budget of fourteen).
 template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
 __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
-gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
+gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
     using C = Cfg<BLOCK_N, THREE>;
     constexpr int STAGES = C::STAGES;                   // barrier slots; the ring uses the first p.stages of them
     extern __shared__ uint8_t smem_raw[];
@@ -201,7 +208,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
     const int lane = threadIdx.x & 31;
     const int total_tiles = p.m_tiles * p.n_tiles * p.k_splits;
 
+    grid_dependents_start();
     if (threadIdx.x == 0) {
+        if (!GATHER) prefetch_tensor_map(&p.tm_a);
+        prefetch_tensor_map(&p.tm_b);
         for (int s = 0; s < STAGES; s++) {
             mbar_init(&full[s], GATHER ? 129 : 1);
             mbar_init(&empty[s], 1);
@@ -250,6 +260,36 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
         uint32_t phase = 0;
         bool ok = true;
         TileIter ti(p, blockIdx.x, gridDim.x);
+        const uint32_t tx_bytes = (!THREE && p.col3)
+            ? (uint32_t)(p.a_box_bytes + 3 * C::B_STAGE_BYTES)
+            : (uint32_t)(((GATHER ? 0 : p.tx_bytes_a) + C::B_STAGE_BYTES * (THREE ? 2 : 1)) * cbs);
+        // The first tile's weights fill the ring while the kernels in front still run; only the activations wait for them.
+        int primed = 0;
+        if (p.b_static) {
+            const int kb0 = ti.split * p.kb_per_split, kb_end = min(kb0 + p.kb_per_split, p.num_k_blocks);
+            const bool cols = !THREE && p.col3;
+            const int loads = cols ? p.ksize_w * p.c_blocks : (kb_end - kb0 + cbs - 1) / cbs;
+            primed = min(stages, loads);
+            for (int i = 0; i < primed; i++) {
+                uint8_t *sa = smem + i * stage_bytes;
+                mbar_expect_tx(&full[i], tx_bytes);
+                if (cols) {
+                    const int cb3 = i / p.ksize_w;
+                    tma_load_4d(sa + p.a_box_bytes, &p.tm_b, &full[i], cb3 * BLOCK_K, ti.n_tile * BLOCK_N, i - cb3 * p.ksize_w, 0);
+                    continue;
+                }
+                const int kb = kb0 + i * cbs, tap = kb / p.c_blocks, cb = kb - tap * p.c_blocks;
+                uint8_t *sb = sa + A_STAGE_BYTES * cbs;
+                if (cbs == 2) {
+                    tma_load_4d(sb, &p.tm_b, &full[i], 0, ti.n_tile * BLOCK_N, cb, tap);
+                } else {
+                    tma_load_3d(sb, &p.tm_b, &full[i], cb * BLOCK_K, ti.n_tile * BLOCK_N, tap);
+                    if (THREE)
+                        tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, &full[i], cb * BLOCK_K, ti.n_tile * BLOCK_N, tap);
+                }
+            }
+        }
+        grid_dependency_wait();
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ti.next(p)) {
             const int split = ti.split, n_tile = ti.n_tile, tw = ti.tw, th = ti.th, tn = ti.tn;
             const int w0 = tw * p.bw * p.stride - p.pad_w;
@@ -260,16 +300,16 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
             if (!THREE && p.col3) {
                 // two requests per stage: the activation box and the three weight tiles of this filter column
                 // (tm_b is 4-D here, {C, N, kw, kh}: a box of one kw and all three kh)
-                const uint32_t tx3 = (uint32_t)(p.a_box_bytes + 3 * C::B_STAGE_BYTES);
                 for (int cb3 = 0; cb3 < p.c_blocks && ok; cb3++) {       // kw fastest, then the channel slice
                     for (int kw3 = 0; kw3 < p.ksize_w; kw3++) {
                         if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status))) break;
                         uint8_t *sa = smem + stage * stage_bytes;
-                        if (leader) {
-                            mbar_expect_tx(&full[stage], tx3);
-                            tma_load_4d(sa, &p.tm_a, &full[stage], cb3 * BLOCK_K, w0 + kw3, h0, n0);
+                        const bool b_there = primed > 0;
+                        if (b_there) primed--;
+                        else mbar_expect_tx(&full[stage], tx_bytes);
+                        tma_load_4d(sa, &p.tm_a, &full[stage], cb3 * BLOCK_K, w0 + kw3, h0, n0);
+                        if (!b_there)
                             tma_load_4d(sa + p.a_box_bytes, &p.tm_b, &full[stage], cb3 * BLOCK_K, n_tile * BLOCK_N, kw3, 0);
-                        }
                         if (++stage == stages) { stage = 0; phase ^= 1; }
                     }
                 }
@@ -280,18 +320,19 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
                 tap = kb0 / p.c_blocks; cb = kb0 - tap * p.c_blocks;
                 kh = tap / p.ksize_w; kw = tap - kh * p.ksize_w;
             }
-            const uint32_t tx_bytes = (uint32_t)(((GATHER ? 0 : p.tx_bytes_a) + C::B_STAGE_BYTES * (THREE ? 2 : 1)) * cbs);
             for (int kb = kb0; kb < kb_end; kb += cbs) {
                 if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status))) break;
                 uint8_t *sa = smem + stage * stage_bytes;
                 uint8_t *sb = sa + A_STAGE_BYTES * cbs;
-                if (leader) {
-                    mbar_expect_tx(&full[stage], tx_bytes);
-                    if (cbs == 2) {
-                        tma_load_5d(sa, &p.tm_a, &full[stage], 0, w0 + kw, h0 + kh, n0, cb);
-                        tma_load_4d(sb, &p.tm_b, &full[stage], 0, n_tile * BLOCK_N, cb, tap);
-                    } else {
-                        if (!GATHER) tma_load_4d(sa, &p.tm_a, &full[stage], cb * BLOCK_K, w0 + kw, h0 + kh, n0);
+                const bool b_there = primed > 0;
+                if (b_there) primed--;
+                else mbar_expect_tx(&full[stage], tx_bytes);
+                if (cbs == 2) {
+                    tma_load_5d(sa, &p.tm_a, &full[stage], 0, w0 + kw, h0 + kh, n0, cb);
+                    if (!b_there) tma_load_4d(sb, &p.tm_b, &full[stage], 0, n_tile * BLOCK_N, cb, tap);
+                } else {
+                    if (!GATHER) tma_load_4d(sa, &p.tm_a, &full[stage], cb * BLOCK_K, w0 + kw, h0 + kh, n0);
+                    if (!b_there) {
                         tma_load_3d(sb, &p.tm_b, &full[stage], cb * BLOCK_K, n_tile * BLOCK_N, tap);
                         if (THREE)
                             tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, &full[stage], cb * BLOCK_K,
@@ -327,6 +368,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
         uint32_t acc_phase = 0;
         int tile_parity = 0;
         bool ok = true;
+        grid_dependency_wait();         // the bounded waits below must not count the kernels in front
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             if (!(ok = mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status))) break;
             tc_fence_after();
@@ -432,6 +474,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
         uint32_t acc_phase = 0;
         bool ok = true;
         TileIter ti(p, blockIdx.x, gridDim.x);
+        grid_dependency_wait();                 // (addends, cell states; the outputs may still be read)
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ti.next(p)) {
             const int split = ti.split, n_tile = ti.n_tile, tw = ti.tw, th = ti.th, tn = ti.tn;
             const int ow = tw * p.bw + rw, oh = th * p.bh * halves + rh, n = tn * p.bn + rn;
@@ -551,11 +594,12 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
             }
         }
         if (store_thread) tma_store_wait_all();     // staged tiles must have left shared memory
-    } else if (GATHER) {
+    } else if constexpr (GATHER) {
         // ------------------------------------------------- in-kernel patch gather
         // One thread per tile row (output pixel): 32 columns (kh,kw,c) of this K block are read
         // through the cache (neighbouring threads read neighbouring pixels) and written as one
         // 128-byte swizzled row, TF32-rounded (or split into hi/lo for the three-pass kernel).
+        grid_dependency_wait();
         const int t = threadIdx.x - 320;
         int stage = 0;
         uint32_t phase = 0;
@@ -620,6 +664,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ TcParams p) {
         // values, so the tensor core's truncation of its operands changes nothing and the split has no bias.
         // Element positions are kept, so the swizzled tile layout written by TMA is preserved.
         const int t = threadIdx.x - 320;        // 0..127
+        grid_dependency_wait();
         int stage = 0;
         uint32_t phase = 0;
         bool ok = true;
@@ -694,12 +739,10 @@ void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const c
     encode_tensor_map(h, tm, base, rank, dims, strides_bytes, box, elem_strides);
 }
 
-typedef void (*TcKernel)(const TcParams);
-
-struct Variant { TcKernel kernel; int smem; };
+struct Variant { const void *kernel; int smem; };      // takes a TcParams, or a TcGatherParams
 
 template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
-Variant variant() { return {gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER>, Cfg<BLOCK_N, THREE>::SMEM_BYTES}; }
+Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER>, Cfg<BLOCK_N, THREE>::SMEM_BYTES}; }
 
 // index: [gather][three][promote][block_n: 0 = 64, 1 = 128, 2 = 256]; absent combinations are null
 const Variant VARIANTS[2][2][2][3] = {
@@ -715,7 +758,7 @@ const Variant VARIANTS[2][2][2][3] = {
 
 // One worked-out launch: kernel parameters (tile geometry, tensor maps), kernel variant, grid.
 struct TcLaunch : LaunchRecord {
-    TcParams p;
+    TcGatherParams p;       // the other variants take the TcParams it starts with
     Variant v;
     int grid = 1, threads = 320;
     double flops = 0;
@@ -759,6 +802,7 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra) {
     key_add(k, a.res_stride); key_add(k, a.res_c); key_add(k, a.res_h); key_add(k, a.res_w);
     key_add(k, a.act); key_add(k, a.round_out_tf32); key_add(k, a.y); key_add(k, a.ldy); key_add(k, a.y_pool);
     key_add(k, a.lstm_H); key_add(k, a.lstm_c_prev); key_add(k, a.lstm_c); key_add(k, a.lstm_h); key_add(k, a.lstm_h_round);
+    key_add(k, a.b_static);
     key_add(k, a.split_k); key_add(k, a.block_n_hint); key_add(k, a.algo_flops);
     return k;
 }
@@ -787,8 +831,8 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     if (a.y_pool && a.a_gather) throw Error(NB_ERR_UNSUPPORTED, "fused pooling is not available with the gathered A operand");
     if (three_pass && !a.b_lo) throw Error(NB_ERR_INVALID_ARG, "three-pass GEMM needs the low-order weight split");
     std::unique_ptr<TcLaunch> L(new TcLaunch());
-    TcParams &p = L->p;
-    std::memset(&p, 0, sizeof p);
+    TcGatherParams &p = L->p;
+    std::memset((void *)&p, 0, sizeof p);
 
     ConvGeom g;
     const bool gather = a.a_gather;
@@ -864,6 +908,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         throw Error(NB_ERR_INVALID_ARG, "GEMM without an output tensor");
     }
     p.status = h->d_status;
+    p.b_static = a.b_static ? 1 : 0;
 
     // tile width in filters: widest tile that still gives every SM work
     // Promoted accumulation: always for 3xTF32 (its point is fp32-level agreement); in TF32 mode only for
@@ -918,7 +963,6 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         const int used = p.stages * p.stage_bytes;
         p.slab2_offset = (!three_pass && !promote && !gather && ring_cap - used >= 2 * BLOCK_M * 32 * 4) ? used : 0;
     }
-    p.gather = gather ? 1 : 0;
     if (gather) {
         p.gx = a.a;
         p.gsn = a.g.sn; p.gsh = a.g.sh; p.gsw = a.g.sw;
@@ -1063,7 +1107,18 @@ void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass) {
     }
     const TcLaunch &L = static_cast<const TcLaunch &>(*it->second);
     ProfileScope prof(h, 0, L.flops);
-    L.v.kernel<<<L.grid, L.threads, L.v.smem, h->stream>>>(L.p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)L.grid);
+    cfg.blockDim = dim3((unsigned)L.threads);
+    cfg.dynamicSmemBytes = (size_t)L.v.smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    void *args[1] = {const_cast<TcGatherParams *>(&L.p)};
+    (void)cudaLaunchKernelExC(&cfg, L.v.kernel, args);
     try {
         check_launch("gemm_tf32_tcgen05_kernel");
     } catch (const Error &err) {

@@ -181,6 +181,9 @@ struct GemmArgs {
     const float *b = nullptr;       // operand used by the TF32 / FP32 paths
     const float *b_lo = nullptr;    // low-order split of B for the 3xTF32 path
     long ldb = 0;
+    // b and b_lo are a plan's weights, written and synchronised with when they were set: no kernel in front of this one on
+    // the stream writes them, so they may be fetched before those are complete
+    bool b_static = false;
     int M = 0, N = 0;           // logical output extents
     int Kc = 0;                 // contraction length per tap (channels or FC inputs)
     // epilogue
@@ -313,6 +316,24 @@ std::string trace_report(nb_handle_s *h);
 // Fails with NB_ERR_INVALID_ARG when [p + lo_bytes, p + hi_bytes) is not inside ONE device allocation (as the driver
 // reports it for p).  Pointers the driver does not know as an allocation (module globals, host memory) pass.
 void check_extent(nb_handle_s *h, const void *p, long long lo_bytes, long long hi_bytes, const char *what);
+
+// Launches `kernel` so that it may become resident while the kernel before it on the stream still runs (programmatic
+// dependent launch): the kernel executes grid_dependency_wait() before it touches memory that an earlier kernel may
+// have written or may still read, and nothing before it but constants, weights and its own set-up.
+template <class... P, class... A>
+inline void launch_overlapped(nb_handle_s *h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // a failure is sticky: check_launch reports it
+}
 
 // Appends the raw bytes of a value to a cache key.
 template <class T>

@@ -189,7 +189,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         }
         ra.y = yo; ra.ldy = d.filters;
         ra.algo_flops = 2.0 * (double)ra.M * d.filters * d.channels * d.size * d.size;
-        ra.b = wr.hi.p; ra.b_lo = wr.lo.p;
+        ra.b = wr.hi.p; ra.b_lo = wr.lo.p; ra.b_static = true;
         if (cuda_cores) {
             ra.Kc = 4 * d.size;             // without the zero columns that fill up a tensor-core K block
             ra.b = wr.exact.p;
@@ -224,8 +224,9 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         }
         pa.y = yo; pa.ldy = d.filters;
         pa.algo_flops = 2.0 * (double)M * d.filters * d.channels * d.size * d.size;
+        const bool split_now = !wp.split_ready;
         wp.ensure_split(h);
-        pa.b = wp.hi.p; pa.b_lo = wp.lo.p;
+        pa.b = wp.hi.p; pa.b_lo = wp.lo.p; pa.b_static = !split_now;
         gemm_tc(h, pa, three);
         if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
         return;
@@ -288,6 +289,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         a.b = w.exact.p;
         gemm_simt(h, a);
     } else {
+        a.b_static = w.split_ready;
         w.ensure_split(h);
         a.b = w.hi.p;
         a.b_lo = w.lo.p;
@@ -417,6 +419,7 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
         gemm_simt(h, a);
         return;
     }
+    a.b_static = w.split_ready;
     w.ensure_split(h);
     a.b = w.hi.p; a.b_lo = w.lo.p;
     int S, block_n;
@@ -549,6 +552,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         a.a = xa; a.lda = in; a.ldb = in; a.M = (int)rows; a.N = 4 * H; a.Kc = in;
         a.shift = shift.p; a.act = d.activation; a.y = pre.p; a.ldy = 4 * H;
         if (tc_u) {
+            a.b_static = wu.split_ready;
             wu.ensure_split(h);
             a.b = wu.hi.p; a.b_lo = wu.lo.p;
             gemm_tc(h, a, three);
@@ -584,6 +588,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
             if (!linear) { a.shift = shift_w.p; a.addend_after_act = true; }
             if (tc_w) {
                 // the cell update runs in the GEMM epilogue: one launch per time step
+                a.b_static = ww.split_ready;
                 ww.ensure_split(h);
                 a.b = ww.hi.p; a.b_lo = ww.lo.p;
                 a.lstm_H = H; a.lstm_c_prev = c_prev; a.lstm_c = ct; a.lstm_h = ht; a.lstm_h_round = hrt;
