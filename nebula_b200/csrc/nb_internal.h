@@ -63,6 +63,7 @@ struct nb_handle_s {
     std::string last_error;
     int *d_status = nullptr;            // device status word (nb::DEV_*)
     unsigned int *d_grid_sync = nullptr; // arrival counter of the persistent LSTM kernel's grid barrier
+    int clusters_of_16 = 0;             // 16-CTA clusters with full shared memory that the device holds at once
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
     nb_encode_tiled_fn encode_tiled = nullptr;
     nb_get_address_range_fn get_address_range = nullptr;   // cuMemGetAddressRange: the allocation a pointer lies in
@@ -348,6 +349,21 @@ void lstm_persistent_prepare_device();
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B,
                      int H, int t_first);
+// The recurrence of an LSTM (gates = 4) or RNN (gates = 1) layer over all steps, exact fp32, for layers whose recurrent
+// weights fit the shared memory of one cluster (recurrent_cluster.cu).
+struct RecurrentArgs {
+    const float *w;             // [gates*H][H] recurrent weights as loaded, LSTM rows interleaved [unit][i,f,g,o]
+    const float *pre;           // [T][B][gates*H] input-side values
+    const float *scale, *shift; // RNN: folded batch-norm of the hidden gate; LSTM with an activation: recurrent-side shift [4H]
+    float *cell, *out, *out_round;      // LSTM: c_t, h_t and (may be null) the TF32-rounded h_t
+                                        // RNN: out = what the output gate reads (h_0, s_1, s_2, ...), the others unused
+    int T, B, H, gates, lstm, act;
+    int cell_f32;               // LSTM: gate activations in fp32 instead of the double formulas
+    int round_out;              // RNN: store TF32-rounded values
+};
+void recurrent_cluster_prepare_device(nb_handle_s *h);
+bool recurrent_cluster_supported(const nb_handle_s *h, int gates, int H, int B);
+void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a);
 void conv_halo_prepare_device();
 void elementwise_prepare_device();
 

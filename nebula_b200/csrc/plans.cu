@@ -575,6 +575,17 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H, 1);
         return;
     }
+    // Everything else (the modes that promise fp32 agreement, widths off 32, gate layers with an activation) runs all
+    // steps in one kernel of exact fp32 products while the weights fit a cluster's shared memory.
+    if (!(lp_env && *lp_env == '0') && recurrent_cluster_supported(h, 4, H, B)) {
+        RecurrentArgs r{};
+        r.w = ww.exact.p; r.pre = pre.p; r.shift = linear ? nullptr : shift_w.p;
+        r.cell = cell; r.out = out; r.out_round = hr;
+        r.T = T; r.B = B; r.H = H; r.gates = 4; r.lstm = 1; r.act = d.activation;
+        r.cell_f32 = tc_w && !three;
+        recurrent_cluster(h, r);
+        return;
+    }
     for (int t = 0; t < T; t++) {
         const float *zt = pre.p + (size_t)t * B * 4 * H;
         float *ct = cell + (size_t)t * B * H, *ht = out + (size_t)t * B * H, *hrt = hr ? hr + (size_t)t * B * H : nullptr;
@@ -653,7 +664,7 @@ size_t RnnPlan::reserve(bool x_rounded, bool x_foreign) {
     o.x_rounded = false; o.x_foreign = false;
     hid_gate->reserve(o, (int)B);                   // step 0 reads the (unrounded) input-gate output
     o.x_rounded = tf32;
-    out_gate->reserve(o, (int)((T > 1 ? T - 1 : 1) * B));
+    out_gate->reserve(o, (int)(T * B));
     return workspace_bytes();
 }
 
@@ -668,6 +679,22 @@ void RnnPlan::forward(const float *x, float *out, bool x_rounded, bool round_out
     // a_t for every step at once: the input gate does not depend on the state
     o.x_rounded = x_rounded; o.x_foreign = x_foreign;
     in_gate->forward(x, a_all.p, o, T * B);
+    // all steps in one kernel while the hidden gate's weights fit a cluster's shared memory: its state buffer holds what
+    // the output gate reads, h_0 in the place of s_0
+    if (recurrent_cluster_supported(h, 1, d.hidden, B)) {
+        RecurrentArgs r{};
+        r.w = hid_gate->w.exact.p; r.pre = a_all.p;
+        r.scale = hid_gate->has_scale ? hid_gate->scale.p : nullptr; r.shift = hid_gate->shift.p;
+        r.out = state.p;
+        r.T = T; r.B = B; r.H = d.hidden; r.gates = 1; r.act = d.activation;
+        const bool out_tc = out_gate->path() == PATH_TC;
+        r.round_out = out_tc;
+        recurrent_cluster(h, r);
+        ForwardOpts q;
+        q.x_rounded = out_tc; q.round_out = round_out;
+        out_gate->forward(state.p, out, q, T * B);
+        return;
+    }
     // step 0: the hidden gate reads the input gate's output, the output gate reads the hidden gate's
     o = ForwardOpts();
     o.round_out = tf32;
