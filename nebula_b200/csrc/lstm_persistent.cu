@@ -10,8 +10,8 @@
 // the steps: step t + 1 of every CTA reads what all CTAs wrote in step t.
 //
 // h_{t-1} was written by other SMs' ordinary stores earlier in this same kernel and is read here by TMA, i.e. through
-// the async proxy: the writers release (fence + release-add on the barrier counter), the reader acquires the counter and
-// then issues fence.proxy.async before its first copy of the step.  (A first version read h with ld.global.cg from
+// the async proxy: the writers release (a release-add on the barrier counter), the thread that issues the copies acquires
+// the counter itself and then issues fence.proxy.async before its first copy of the step.  (A first version read h with ld.global.cg from
 // 128 threads: correct, but 63 us per step, three times slower than a launch per step.)  The results are bit-identical
 // to the per-step path (same K order, same fp32 cell arithmetic).
 #include <cstring>
@@ -26,7 +26,7 @@ namespace {
 
 constexpr int LP_N = 32;                    // gate columns per CTA
 constexpr int LP_STAGES = 4;                // most ring stages (barrier slots)
-constexpr int LP_THREADS = 192;             // warps 0-3: epilogue and grid barrier; warp 4: MMA issue; warp 5: TMA
+constexpr int LP_THREADS = 192;             // warps 0-3: epilogue; warp 4: MMA issue; warp 5: grid barrier and TMA
 constexpr int LP_W_TILE = LP_N * 128;       // one K block of the weight slice: 32 rows x 128 bytes
 
 struct LstmPParams {
@@ -64,8 +64,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
     uint64_t *empty = bars + LP_STAGES;     // MMA -> loaders   [LP_STAGES]
     uint64_t *w_full = bars + 2 * LP_STAGES;
     uint64_t *acc_full = w_full + 1;
-    uint64_t *step_go = acc_full + 1;       // grid barrier passed: h of the previous step is complete
-    uint32_t *tmem_slot = (uint32_t *)(step_go + 1);
+    uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5;
@@ -76,7 +75,6 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
         }
         mbar_init(w_full, 1);
         mbar_init(acc_full, 1);
-        mbar_init(step_go, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -133,14 +131,23 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
         // ------------------------------------------------ h_{t-1} of every step, one K block per ring stage
         if (elect_one()) {
             int stage = 0;
-            uint32_t phase = 0, go_phase = 0;
+            uint32_t phase = 0;
             const uint32_t tx = (uint32_t)(p.B * BLOCK_K * 4 * cbs);
             for (int t = p.t_first; t < p.T && ok; t++) {
                 if (t > p.t_first) {
-                    // the other CTAs' stores of h_{t-1} (generic proxy) are ordered before the acquire that opened the
-                    // barrier; this fence orders the copies below (async proxy) behind it
-                    if (!(ok = mbar_wait(step_go, go_phase, abort_flag, p.status))) break;
-                    go_phase ^= 1;
+                    // grid barrier: all CTAs have arrived with h_{t-1}.  Their stores (generic proxy) are ordered before this
+                    // acquire; the fence orders the copies below (async proxy) behind it
+                    const unsigned int target = ctas * (unsigned int)(t - p.t_first);
+                    const long long t0 = clock64();
+                    while (ld_acquire_u32(p.sync) < target) {
+                        if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
+                            *abort_flag = 1;
+                            atomicExch(p.status, (int)DEV_TIMEOUT);
+                            ok = false;
+                            break;
+                        }
+                    }
+                    if (!ok) break;
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
                 for (int kb = 0; kb < KB; kb += cbs) {
@@ -189,8 +196,9 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
             tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
             tmem_ld_wait();
             tc_fence_before();
+            float hn[8];
+            const size_t o = row * p.H + unit0;
             if (row_ok) {
-                float hn[8];
 #pragma unroll
                 for (int u = 0; u < 8; u++) {
                     const float zi = __uint_as_float(v[4 * u]) + z4[u].x, zf = __uint_as_float(v[4 * u + 1]) + z4[u].y;
@@ -198,36 +206,24 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
                     const float2 ch = lstm_cell_unit_f32_inline(zi, zf, zg, zo, c[u]);
                     c[u] = ch.x; hn[u] = ch.y;
                 }
-                const size_t o = row * p.H + unit0;
 #pragma unroll
                 for (int q = 0; q < 2; q++) {
-                    *reinterpret_cast<float4 *>(p.cell + o + 4 * q) = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
-                    *reinterpret_cast<float4 *>(p.out + o + 4 * q) = make_float4(hn[4 * q], hn[4 * q + 1], hn[4 * q + 2], hn[4 * q + 3]);
                     *reinterpret_cast<float4 *>(p.hr_w + o + 4 * q) = make_float4(round_tf32(hn[4 * q]), round_tf32(hn[4 * q + 1]),
                                                                                    round_tf32(hn[4 * q + 2]), round_tf32(hn[4 * q + 3]));
                 }
             }
-            // ---- grid barrier: every CTA's h_t is written before any CTA reads it
+            // ---- grid barrier, this CTA's arrival: its rounded h_t is written (the barrier orders the group's stores before
+            // the release).  What the next step does not read leaves behind it, so that the release does not wait for it
             if (t + 1 < p.T) {
-                __threadfence();
                 epilogue_bar_sync(1);
-                bool arrived = true;
-                if (tid == 0) {
-                    red_release_add(p.sync, 1u);
-                    const unsigned int target = ctas * (unsigned int)(t - p.t_first + 1);
-                    const long long t0 = clock64();
-                    while (ld_acquire_u32(p.sync) < target) {
-                        if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                            *abort_flag = 1;
-                            atomicExch(p.status, (int)DEV_TIMEOUT);
-                            arrived = false;
-                            break;
-                        }
-                    }
-                    __threadfence();
-                    if (arrived) mbar_arrive(step_go);
+                if (tid == 0) red_release_add(p.sync, 1u);
+            }
+            if (row_ok) {
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    *reinterpret_cast<float4 *>(p.cell + o + 4 * q) = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
+                    *reinterpret_cast<float4 *>(p.out + o + 4 * q) = make_float4(hn[4 * q], hn[4 * q + 1], hn[4 * q + 2], hn[4 * q + 3]);
                 }
-                ok = epilogue_all(arrived, 1);
             }
         }
         if (!ok) *abort_flag = 1;

@@ -63,7 +63,7 @@ struct nb_handle_s {
     std::string last_error;
     int *d_status = nullptr;            // device status word (nb::DEV_*)
     unsigned int *d_grid_sync = nullptr; // arrival counter of the persistent LSTM kernel's grid barrier
-    int clusters_of_16 = 0;             // 16-CTA clusters with full shared memory that the device holds at once
+    int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
     nb_encode_tiled_fn encode_tiled = nullptr;
     nb_get_address_range_fn get_address_range = nullptr;   // cuMemGetAddressRange: the allocation a pointer lies in
@@ -357,7 +357,7 @@ struct RecurrentArgs {
     const float *scale, *shift; // RNN: folded batch-norm of the hidden gate; LSTM with an activation: recurrent-side shift [4H]
     float *cell, *out, *out_round;      // LSTM: c_t, h_t and (may be null) the TF32-rounded h_t
                                         // RNN: out = what the output gate reads (h_0, s_1, s_2, ...), the others unused
-    int T, B, H, gates, lstm, act;
+    int T, B, H, gates, act;
     int cell_f32;               // LSTM: gate activations in fp32 instead of the double formulas
     int round_out;              // RNN: store TF32-rounded values
 };

@@ -581,7 +581,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         RecurrentArgs r{};
         r.w = ww.exact.p; r.pre = pre.p; r.shift = linear ? nullptr : shift_w.p;
         r.cell = cell; r.out = out; r.out_round = hr;
-        r.T = T; r.B = B; r.H = H; r.gates = 4; r.lstm = 1; r.act = d.activation;
+        r.T = T; r.B = B; r.H = H; r.gates = 4; r.act = d.activation;
         r.cell_f32 = tc_w && !three;
         recurrent_cluster(h, r);
         return;

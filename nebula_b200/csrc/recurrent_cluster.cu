@@ -9,6 +9,8 @@
 // for the RB states (both from shared memory, packed FMAs along K), four K lanes are added by shuffles, the warps' partial
 // sums through shared memory; one thread per (unit, batch row) then adds the input-side values fetched a step ahead,
 // runs the cell update and stores the new state into the shared memory of all CS CTAs; a cluster barrier ends the step.
+// The step's results leave for HBM between the barrier's arrive and its wait: an arrive releases what was stored in front
+// of it, so there it would wait for HBM on every step (T35 B20 H300: 4.1 us a step in front, 2.8 us behind).
 // CS depends on the layer only, so a batch and its slices add in the same order.
 #include <cooperative_groups.h>
 
@@ -45,14 +47,14 @@ __device__ __forceinline__ void ffma2(unsigned long long &c, unsigned long long 
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
-template <int RB>
+template <int RB, int G>            // G: gates, 4 (LSTM) or 1 (RNN)
 __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const RecParams p) {
     extern __shared__ __align__(16) float smem[];
     const RecurrentArgs &a = p.a;
-    const int H = a.H, G = a.gates, Hs = p.s.Hs, rows2 = 2 * p.s.RP;
+    const int H = a.H, Hs = p.s.Hs, rows2 = 2 * p.s.RP;
     float *w_s = smem;                              // [2 RP][Hs]
     float *h_s = w_s + rows2 * Hs;                  // [2][RB][Hs]: the state read by this step and written by it
-    float *part = h_s + 2 * RB * Hs;                // [kg][2 RP][RB]
+    float *part = h_s + 2 * RB * Hs;                // [kg][RB][2 RP]
     cg::cluster_group cluster = cg::this_cluster();
     const int CS = p.s.CS, rank = CS > 1 ? (int)cluster.block_rank() : 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -67,7 +69,7 @@ __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const 
     }
     for (int i = tid; i < 2 * RB * Hs; i += RC_THREADS) h_s[i] = 0.0f;
     grid_dependency_wait();
-    if (!a.lstm) {                                  // step 0 of an RNN multiplies the input gate's output
+    if (G == 1) {                                   // step 0 of an RNN multiplies the input gate's output
         __syncthreads();
         for (int i = tid; i < RB * H; i += RC_THREADS) {
             const int b = i / H, k = i - b * H;
@@ -77,10 +79,10 @@ __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const 
 
     // the (unit, batch row) pairs this thread finishes
     int item_u[RC_ITEMS], item_b[RC_ITEMS];
-    float c[RC_ITEMS], z[RC_ITEMS][4], scale[RC_ITEMS], shift[RC_ITEMS][4];
-    auto fetch_pre = [&](int t, int i, float (&v)[4]) {
+    float c[RC_ITEMS], z[RC_ITEMS][G], scale[RC_ITEMS], shift[RC_ITEMS][G];
+    auto fetch_pre = [&](int t, int i, float (&v)[G]) {
         const float *src = a.pre + ((long)t * a.B + b0 + item_b[i]) * G * H + (long)G * (unit0 + item_u[i]);
-        if (G == 4) {
+        if constexpr (G == 4) {
             const float4 q = *reinterpret_cast<const float4 *>(src);
             v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
         } else {
@@ -95,13 +97,13 @@ __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const 
         if (item_b[i] >= RB || b0 + item_b[i] >= a.B) item_b[i] = -1;
         c[i] = 0.0f; scale[i] = 1.0f;
 #pragma unroll
-        for (int g = 0; g < 4; g++) { z[i][g] = 0.0f; shift[i][g] = 0.0f; }
+        for (int g = 0; g < G; g++) { z[i][g] = 0.0f; shift[i][g] = 0.0f; }
         if (item_b[i] >= 0) {
             fetch_pre(0, i, z[i]);
             if (a.scale) scale[i] = a.scale[unit0 + item_u[i]];
 #pragma unroll
-            for (int g = 0; g < 4; g++)
-                if (a.shift && g < G) shift[i][g] = a.shift[(long)G * (unit0 + item_u[i]) + g];
+            for (int g = 0; g < G; g++)
+                if (a.shift) shift[i][g] = a.shift[(long)G * (unit0 + item_u[i]) + g];
         }
     }
     if (CS > 1) cluster.sync();
@@ -114,13 +116,6 @@ __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const 
     for (int t = 0; t < a.T; t++) {
         const float *h_cur = h_s + (t & 1) * RB * Hs;
         const int next_off = ((t + 1) & 1) * RB * Hs;
-        float zn[RC_ITEMS][4];
-#pragma unroll
-        for (int i = 0; i < RC_ITEMS; i++) {
-#pragma unroll
-            for (int g = 0; g < 4; g++) zn[i][g] = 0.0f;
-            if (item_b[i] >= 0 && t + 1 < a.T) fetch_pre(t + 1, i, zn[i]);
-        }
         if (multiplies) {
             unsigned long long acc[2][RB];
 #pragma unroll
@@ -135,64 +130,97 @@ __global__ void __launch_bounds__(RC_THREADS, 1) recurrent_cluster_kernel(const 
                     ffma2(acc[1][b], v1.x, hv.x); ffma2(acc[1][b], v1.y, hv.y);
                 }
             }
+            // The 2 RB sums of eight rows' pairs lie in four lanes: two exchanges halve the values and the lanes' shares (each
+            // lane ends with RB / 2 of them)
+            constexpr int N = 2 * RB;
+            float v[N];
 #pragma unroll
-            for (int j = 0; j < 2; j++)
+            for (int i = 0; i < N; i++) {
+                const unsigned long long s = acc[i / RB][i % RB];
+                v[i] = __uint_as_float((unsigned)s) + __uint_as_float((unsigned)(s >> 32));
+            }
+            const bool hi = lane & 16, odd = lane & 8;
 #pragma unroll
-                for (int b = 0; b < RB; b++) {
-                    float v = __uint_as_float((unsigned)acc[j][b]) + __uint_as_float((unsigned)(acc[j][b] >> 32));
-                    v += __shfl_xor_sync(0xffffffffu, v, 8);
-                    v += __shfl_xor_sync(0xffffffffu, v, 16);
-                    if (lane < 8) part[(kg * rows2 + rp + j * p.s.RP) * RB + b] = v;
+            for (int i = 0; i < N / 2; i++) {
+                const float mine = hi ? v[i + N / 2] : v[i], theirs = hi ? v[i] : v[i + N / 2];
+                v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, 16);
+            }
+            if constexpr (N == 2) {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], 8);
+                if (!odd) part[kg * rows2 + rp + (hi ? p.s.RP : 0)] = v[0];
+            } else {
+#pragma unroll
+                for (int i = 0; i < N / 4; i++) {
+                    const float mine = odd ? v[i + N / 4] : v[i], theirs = odd ? v[i] : v[i + N / 4];
+                    v[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, 8);
                 }
+#pragma unroll
+                for (int i = 0; i < N / 4; i++)         // row half `hi`, batch row (odd ? RB / 2 : 0) + i
+                    part[(kg * RB + (odd ? N / 4 : 0) + i) * rows2 + rp + (hi ? p.s.RP : 0)] = v[i];
+            }
         }
         __syncthreads();
+        const bool more = t + 1 < a.T;
+        float y[RC_ITEMS];
 #pragma unroll
         for (int i = 0; i < RC_ITEMS; i++) {
             if (item_b[i] < 0) continue;
             const int u = item_u[i], b = item_b[i];
-            float v[4];
-            for (int g = 0; g < G; g++) {
-                float s = 0.0f;
-                for (int q = 0; q < p.s.kg; q++) s += part[(q * rows2 + G * u + g) * RB + b];
-                v[g] = s;
+            float v[G], state;
+#pragma unroll
+            for (int g = 0; g < G; g++) v[g] = 0.0f;
+#pragma unroll 4
+            for (int q = 0; q < p.s.kg; q++) {
+                const float *src = part + (q * RB + b) * rows2 + G * u;
+                if constexpr (G == 4) {
+                    const float4 w = *reinterpret_cast<const float4 *>(src);
+                    v[0] += w.x; v[1] += w.y; v[2] += w.z; v[3] += w.w;
+                } else {
+                    v[0] += *src;
+                }
             }
-            const long o = ((long)t * a.B + b0 + b) * H + unit0 + u;
-            float state;
-            if (a.lstm) {
-                float zg[4];
+            if constexpr (G == 4) {
 #pragma unroll
                 for (int g = 0; g < 4; g++)         // linear gate layers: their shifts are in `pre` already
-                    zg[g] = a.act == NB_ACT_LINEAR ? z[i][g] + v[g] : z[i][g] + apply_activation_call(v[g] + shift[i][g], a.act);
-                const float2 ch = a.cell_f32 ? lstm_cell_unit_f32(zg[0], zg[1], zg[2], zg[3], c[i])
-                                             : lstm_cell_unit(zg[0], zg[1], zg[2], zg[3], c[i]);
-                c[i] = ch.x; state = ch.y;
-                a.cell[o] = c[i];
-                a.out[o] = state;
-                if (a.out_round) a.out_round[o] = round_tf32(state);
+                    v[g] = z[i][g] + (a.act == NB_ACT_LINEAR ? v[g] : apply_activation_call(v[g] + shift[i][g], a.act));
+                const float2 ch = a.cell_f32 ? lstm_cell_unit_f32_inline(v[0], v[1], v[2], v[3], c[i])
+                                             : lstm_cell_unit(v[0], v[1], v[2], v[3], c[i]);
+                c[i] = ch.x; state = y[i] = ch.y;
             } else {
-                const float x = a.scale ? fmaf(v[0], scale[i], shift[i][0]) : v[0] + shift[i][0];
-                const float hv = apply_activation_fast(x, a.act);
+                const float hv = apply_activation_fast(a.scale ? fmaf(v[0], scale[i], shift[i][0]) : v[0] + shift[i][0], a.act);
                 state = z[i][0] + hv;
-                const float y = t == 0 ? hv : state;        // what the output gate reads: h_0, then the states
-                a.out[o] = a.round_out ? round_tf32(y) : y;
+                y[i] = t == 0 ? hv : state;         // what the output gate reads: h_0, then the states
             }
-            if (t + 1 < a.T) {
+            if (more) {
                 float *dst = h_s + next_off + b * Hs + unit0 + u;
                 for (int q = 0; q < CS; q++) *(CS > 1 ? cluster.map_shared_rank(dst, q) : dst) = state;
             }
-#pragma unroll
-            for (int g = 0; g < 4; g++) z[i][g] = zn[i][g];
         }
-        if (t + 1 < a.T) {
-            if (CS > 1) cluster.sync();             // (the last step sends nothing: no CTA leaves before its peers' stores)
+        if (more && CS > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < RC_ITEMS; i++) {
+            if (item_b[i] < 0) continue;
+            const long o = ((long)t * a.B + b0 + item_b[i]) * H + unit0 + item_u[i];
+            if constexpr (G == 4) {
+                a.cell[o] = c[i];
+                a.out[o] = y[i];
+                if (a.out_round) a.out_round[o] = round_tf32(y[i]);
+            } else {
+                a.out[o] = a.round_out ? round_tf32(y[i]) : y[i];
+            }
+            if (more) fetch_pre(t + 1, i, z[i]);
+        }
+        if (more) {         // (the last step sends nothing: no CTA leaves before its peers' stores)
+            if (CS > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
             else __syncthreads();
         }
     }
 }
 
 typedef void (*RecKernel)(const RecParams);
-const RecKernel KERNELS[4] = {recurrent_cluster_kernel<1>, recurrent_cluster_kernel<2>, recurrent_cluster_kernel<4>,
-                              recurrent_cluster_kernel<8>};
+const RecKernel KERNELS[2][4] = {       // [LSTM][rows per cluster: 1, 2, 4, 8]
+    {recurrent_cluster_kernel<1, 1>, recurrent_cluster_kernel<2, 1>, recurrent_cluster_kernel<4, 1>, recurrent_cluster_kernel<8, 1>},
+    {recurrent_cluster_kernel<1, 4>, recurrent_cluster_kernel<2, 4>, recurrent_cluster_kernel<4, 4>, recurrent_cluster_kernel<8, 4>}};
 constexpr int MAX_SMEM = 227 * 1024;
 
 bool shape_of(int gates, int H, int CS, int RB, Shape *s) {
@@ -207,19 +235,20 @@ bool shape_of(int gates, int H, int CS, int RB, Shape *s) {
     return s->smem <= MAX_SMEM;
 }
 
-// Clock cycles of a step: every warp row-group reads its 16 weight rows and RB states (8 + RB wavefronts per K quad and
-// eight rows), plus the fixed chain of a step (measured: about 1000 cycles with a cluster barrier, 500 without).
-double step_cost(const Shape &s, int H) { return (double)s.rg * H / 16 * (8 + s.RB) + (s.CS > 1 ? 1000.0 : 500.0); }
-
-// Clusters that run at once: 148 SMs in groups of 16 to 18 that a cluster cannot span.
-int clusters_at_once(const nb_handle_s *h, int CS) { return CS == 16 ? h->clusters_of_16 : (h->sm_count / 18) * (18 / CS); }
+// Clock cycles of a step, fitted to measurements of RNN and LSTM layers of 40 to 600 units: every warp row-group reads its
+// 16 weight rows (8 wavefronts per K quad and eight rows) and multiplies RB states with them; the rest of a step is the
+// chain of reductions, cell and exchange (RNN H256, clusters of 8: 1.0 / 1.1 / 1.4 / 1.9 us at RB = 1 / 2 / 4 / 8; H40 in a
+// single CTA: 0.7 us).
+double step_cost(const Shape &s, int H) {
+    return (double)s.rg * H / 16 * (8 + 2.5 * s.RB) + (s.CS > 1 ? 1600.0 : 1150.0) + 130.0 * s.RB;
+}
 
 // Cluster size from the layer alone (at a batch of 32); rows per cluster from the batch.
 bool choose(const nb_handle_s *h, int gates, int H, int B, Shape *best) {
     auto pick = [&](int batch, int cs_lo, int cs_hi) {
         double best_cost = -1;
         for (int CS = cs_lo; CS <= cs_hi; CS *= 2) {
-            const int at_once = clusters_at_once(h, CS);
+            const int at_once = CS == 1 ? h->sm_count : h->clusters_at_once[CS];
             if (at_once < 1) continue;
             for (int RB = 1; RB <= 8; RB *= 2) {
                 Shape s;
@@ -237,23 +266,27 @@ bool choose(const nb_handle_s *h, int gates, int H, int B, Shape *best) {
 }  // namespace
 
 void recurrent_cluster_prepare_device(nb_handle_s *h) {
-    for (RecKernel k : KERNELS) {
-        NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
-        NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    for (auto &kind : KERNELS)
+        for (RecKernel k : kind) {
+            NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
+            NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        }
+    // how many clusters of each size run at once (they do not span the groups of SMs the part is made of, and 16 CTAs
+    // are beyond the portable size)
+    for (int CS = 2; CS <= 16; CS *= 2) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)CS);
+        cfg.blockDim = dim3(RC_THREADS);
+        cfg.dynamicSmemBytes = MAX_SMEM;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)CS; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, KERNELS[1][0], &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+        h->clusters_at_once[CS] = n;
     }
-    // clusters of 16 are beyond the portable size: ask how many of them the device holds
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(16);
-    cfg.blockDim = dim3(RC_THREADS);
-    cfg.dynamicSmemBytes = MAX_SMEM;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = 16; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, KERNELS[0], &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
-    h->clusters_of_16 = n;
 }
 
 bool recurrent_cluster_supported(const nb_handle_s *h, int gates, int H, int B) {
@@ -277,7 +310,7 @@ void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a) {
     at[1].val.clusterDim.x = (unsigned)p.s.CS; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    const RecKernel k = KERNELS[p.s.RB == 1 ? 0 : (p.s.RB == 2 ? 1 : (p.s.RB == 4 ? 2 : 3))];
+    const RecKernel k = KERNELS[a.gates == 4][p.s.RB == 1 ? 0 : (p.s.RB == 2 ? 1 : (p.s.RB == 4 ? 2 : 3))];
     ProfileScope prof(h, 1, 2.0 * (double)a.T * a.B * a.gates * a.H * a.H);
     (void)cudaLaunchKernelEx(&cfg, k, p);
     check_launch("recurrent_cluster_kernel");
