@@ -66,6 +66,23 @@ __device__ __forceinline__ float apply_activation(float x, int act) {
 // instruction stream of loops that almost always run relu / leaky / linear.
 static __device__ __noinline__ float apply_activation_call(float x, int act) { return apply_activation(x, act); }
 
+// Four values at once: a double exponential is a chain of some two hundred cycles, and the four chains overlap.
+__device__ __forceinline__ float4 apply_activation4(float4 x, int act) {
+    if (act == NB_ACT_LOGISTIC || act == NB_ACT_LOGGY || act == NB_ACT_TANH) {
+        const double m = act == NB_ACT_TANH ? 2.0 : -1.0;
+        const double e0 = exp(m * (double)x.x), e1 = exp(m * (double)x.y), e2 = exp(m * (double)x.z), e3 = exp(m * (double)x.w);
+        if (act == NB_ACT_TANH)
+            return make_float4((float)((e0 - 1.0) / (e0 + 1.0)), (float)((e1 - 1.0) / (e1 + 1.0)), (float)((e2 - 1.0) / (e2 + 1.0)),
+                               (float)((e3 - 1.0) / (e3 + 1.0)));
+        const double q0 = 1.0 + e0, q1 = 1.0 + e1, q2 = 1.0 + e2, q3 = 1.0 + e3;
+        if (act == NB_ACT_LOGISTIC) return make_float4((float)(1.0 / q0), (float)(1.0 / q1), (float)(1.0 / q2), (float)(1.0 / q3));
+        return make_float4((float)(2.0 / q0 - 1.0), (float)(2.0 / q1 - 1.0), (float)(2.0 / q2 - 1.0), (float)(2.0 / q3 - 1.0));
+    }
+    return make_float4(apply_activation(x.x, act), apply_activation(x.y, act), apply_activation(x.z, act), apply_activation(x.w, act));
+}
+
+static __device__ __noinline__ float4 apply_activation4_call(float4 x, int act) { return apply_activation4(x, act); }
+
 // One LSTM cell update (lstm_layer.cc:286-311) from the four gate pre-activations of a hidden unit: out of line to
 // keep the GEMM epilogue small, with the four gate activations inline so that their exp chains overlap. The
 // products and the sum round to fp32 separately, as the CPU path's loops do.
@@ -105,6 +122,13 @@ __device__ __forceinline__ float apply_activation_fast(float x, int act) {
     if (act == NB_ACT_LINEAR) return x;
     if (act == NB_ACT_LEAKY) return x > 0.0f ? x : (float)(0.1 * (double)x);
     return apply_activation_call(x, act);
+}
+
+__device__ __forceinline__ float4 apply_activation4_fast(float4 x, int act) {
+    if (act == NB_ACT_RELU || act == NB_ACT_LINEAR || act == NB_ACT_LEAKY)
+        return make_float4(apply_activation_fast(x.x, act), apply_activation_fast(x.y, act), apply_activation_fast(x.z, act),
+                           apply_activation_fast(x.w, act));
+    return apply_activation4_call(x, act);
 }
 
 }  // namespace nb

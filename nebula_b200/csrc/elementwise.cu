@@ -85,10 +85,7 @@ __global__ void activation_kernel(float *data, size_t n, int act) {
         const size_t n4 = n / 4;
         float4 *d4 = reinterpret_cast<float4 *>(data);
         for (size_t j = i; j < n4; j += stride) {
-            float4 v = d4[j];
-            v.x = apply_activation(v.x, act); v.y = apply_activation(v.y, act);
-            v.z = apply_activation(v.z, act); v.w = apply_activation(v.w, act);
-            d4[j] = v;
+            d4[j] = apply_activation4_fast(d4[j], act);
         }
         for (size_t j = n4 * 4 + i; j < n; j += stride) data[j] = apply_activation(data[j], act);
     } else {
@@ -349,8 +346,7 @@ __global__ void shortcut_nhwc4_kernel(const float4 *prev, const float4 *conn, fl
                 v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
             }
         }
-        v.x = apply_activation_fast(v.x, act); v.y = apply_activation_fast(v.y, act);
-        v.z = apply_activation_fast(v.z, act); v.w = apply_activation_fast(v.w, act);
+        v = apply_activation4_fast(v, act);
         if (round) { v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w); }
         y[i] = v;
     }
@@ -470,30 +466,64 @@ __global__ void fc_permute_kernel(const float *w, float *dst, int out, int C, in
 // -------------------------------------------------------------- split-K tail
 // y[m][n] = act(scale[n] * sum_s ws[s][m][n] + shift[n]): the epilogue of a split-K contraction
 // (slices are added in a fixed order, so the result does not depend on scheduling).
-// N % 4 == 0 (what the split-K path requires) and 16-byte aligned tensors: four columns per thread, 128-bit accesses
-__global__ void splitk_reduce4_kernel(const float4 *ws, int S, size_t MN4, int N4, const float4 *scale, const float4 *shift,
-                                      int act, int round, float4 *y) {
+// N % 4 == 0 (what the split-K path requires) and 16-byte aligned tensors: four columns per thread, 128-bit accesses.  For a
+// convolution the layer behind it may be folded in: a residual tensor added before the activation (the rule of
+// addend_row in tc_common.cuh), or the 2x2/2 max-pool, whose windows lie in four rows of the slices.
+__global__ void splitk_reduce4_kernel(const SplitReduce p) {
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < MN4; i += stride) {
+    const int N4 = p.N / 4;
+    const float4 *ws = reinterpret_cast<const float4 *>(p.ws);
+    auto value = [&](size_t i, int n, size_t row) {
         float4 acc = ws[i];
-        for (int s = 1; s < S; s++) {       // slices in a fixed order: the sum does not depend on scheduling
-            const float4 v = ws[(size_t)s * MN4 + i];
+#pragma unroll 4
+        for (int s = 1; s < p.S; s++) {     // slices in a fixed order: the sum does not depend on scheduling
+            const float4 v = ws[(size_t)s * p.M * N4 + i];
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
-        const int n = (int)(i % N4);
-        if (scale) {
-            const float4 sc = scale[n], sh = shift[n];
+        if (p.scale) {
+            const float4 sc = reinterpret_cast<const float4 *>(p.scale)[n], sh = reinterpret_cast<const float4 *>(p.shift)[n];
             acc.x = fmaf(acc.x, sc.x, sh.x); acc.y = fmaf(acc.y, sc.y, sh.y);
             acc.z = fmaf(acc.z, sc.z, sh.z); acc.w = fmaf(acc.w, sc.w, sh.w);
-        } else if (shift) {
-            const float4 sh = shift[n];
+        } else if (p.shift) {
+            const float4 sh = reinterpret_cast<const float4 *>(p.shift)[n];
             acc.x += sh.x; acc.y += sh.y; acc.z += sh.z; acc.w += sh.w;
         }
-        acc.x = apply_activation_fast(acc.x, act); acc.y = apply_activation_fast(acc.y, act);
-        acc.z = apply_activation_fast(acc.z, act); acc.w = apply_activation_fast(acc.w, act);
-        if (round) { acc.x = round_tf32(acc.x); acc.y = round_tf32(acc.y); acc.z = round_tf32(acc.z); acc.w = round_tf32(acc.w); }
-        y[i] = acc;
+        if (p.res && 4 * n < p.res_c) {
+            const int ow = (int)(row % p.OW), oh = (int)(row / p.OW % p.OH);
+            const int ih = oh * p.res_stride, iw = ow * p.res_stride;
+            if (ih < p.res_h && iw < p.res_w) {
+                const size_t img = row / ((size_t)p.OW * p.OH);
+                const float4 r = *reinterpret_cast<const float4 *>(p.res + ((img * p.res_h + ih) * p.res_w + iw) * p.res_ld + 4 * n);
+                acc.x += r.x; acc.y += r.y; acc.z += r.z; acc.w += r.w;
+            }
+        }
+        acc = apply_activation4_fast(acc, p.act);
+        if (p.round) { acc.x = round_tf32(acc.x); acc.y = round_tf32(acc.y); acc.z = round_tf32(acc.z); acc.w = round_tf32(acc.w); }
+        return acc;
+    };
+    const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!p.pool) {
+        for (size_t i = first; i < (size_t)p.M * N4; i += stride)
+            reinterpret_cast<float4 *>(p.y)[i] = value(i, (int)(i % N4), i / N4);
+        return;
+    }
+    const int PW = p.OW / 2, PH = p.OH / 2;
+    for (size_t i = first; i < (size_t)p.M / 4 * N4; i += stride) {
+        const int n = (int)(i % N4);
+        size_t t = i / N4;
+        const int pw = (int)(t % PW); t /= PW;
+        const int ph = (int)(t % PH); t /= PH;
+        const size_t r0 = (t * p.OH + 2 * ph) * p.OW + 2 * pw;
+        float4 m = make_float4(-1e8f, -1e8f, -1e8f, -1e8f);         // the reference's identity
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const size_t row = r0 + (k >> 1) * p.OW + (k & 1);
+            const float4 x = value(row * N4 + n, n, row);
+            m.x = x.x > m.x ? x.x : m.x; m.y = x.y > m.y ? x.y : m.y;
+            m.z = x.z > m.z ? x.z : m.z; m.w = x.w > m.w ? x.w : m.w;
+        }
+        reinterpret_cast<float4 *>(p.y)[i] = m;
     }
 }
 __global__ void splitk_reduce_kernel(const float *ws, int S, size_t MN, int N, const float *scale, const float *shift,
@@ -701,15 +731,19 @@ void launch_fc_permute(nb_handle_s *h, const float *w, float *dst, int out, int 
     check_launch("fc_permute_kernel");
     count_launch(h);
 }
-void launch_splitk_reduce(nb_handle_s *h, const float *ws, int S, int M, int N, const float *scale, const float *shift,
-                          int act, bool round, float *y) {
-    const size_t MN = (size_t)M * N;
-    const bool vec = (N % 4) == 0 && ((((uintptr_t)ws) | ((uintptr_t)y) | ((uintptr_t)scale) | ((uintptr_t)shift)) & 15) == 0;
-    if (vec)
-        launch_overlapped(h, splitk_reduce4_kernel, grid_for(MN / 4, h), TPB, 0, (const float4 *)ws, S, MN / 4, N / 4, (const float4 *)scale,
-                                                                         (const float4 *)shift, act, round ? 1 : 0, (float4 *)y);
-    else
-        launch_overlapped(h, splitk_reduce_kernel, grid_for(MN, h), TPB, 0, ws, S, MN, N, scale, shift, act, round ? 1 : 0, y);
+void launch_splitk_reduce(nb_handle_s *h, const SplitReduce &p) {
+    const size_t MN = (size_t)p.M * p.N;
+    const bool vec = (p.N % 4) == 0 && ((((uintptr_t)p.ws) | ((uintptr_t)p.y) | ((uintptr_t)p.scale) | ((uintptr_t)p.shift)) & 15) == 0;
+    if (vec) {
+        // a few thousand outputs: small blocks, so that every SM adds some
+        const unsigned threads = MN / 4 < (size_t)h->sm_count * TPB ? 64 : TPB;
+        const size_t work = MN / 4 / (p.pool ? 4 : 1);
+        const unsigned grid = (unsigned)std::max<size_t>(1, std::min((work + threads - 1) / threads, (size_t)h->sm_count * 32));
+        launch_overlapped(h, splitk_reduce4_kernel, grid, threads, 0, p);
+    } else {
+        if (p.res || p.pool) throw Error(NB_ERR_UNSUPPORTED, "split-K: a folded layer needs 16-byte aligned rows");
+        launch_overlapped(h, splitk_reduce_kernel, grid_for(MN, h), TPB, 0, p.ws, p.S, MN, p.N, p.scale, p.shift, p.act, p.round, p.y);
+    }
     check_launch("splitk_reduce_kernel");
     count_launch(h);
 }

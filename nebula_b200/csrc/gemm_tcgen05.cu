@@ -669,7 +669,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         uint32_t phase = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            for (int kb = 0; kb < p.kb_per_split; kb++) {
+            const int tile_kb = min(p.kb_per_split, p.num_k_blocks - (tile % p.k_splits) * p.kb_per_split);
+            for (int kb = 0; kb < tile_kb; kb++) {
                 if (!(ok = mbar_wait(&full[stage], phase, abort_flag, p.status))) break;
                 float4 *a = reinterpret_cast<float4 *>(smem + stage * C::STAGE_BYTES);
                 float4 *a_lo = reinterpret_cast<float4 *>(smem + stage * C::STAGE_BYTES + A_STAGE_BYTES + C::B_STAGE_BYTES);
@@ -873,7 +874,8 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.c_blocks = (kc + BLOCK_K - 1) / BLOCK_K;
     p.num_k_blocks = taps * p.c_blocks;
     p.kb_per_split = (p.num_k_blocks + S - 1) / S;
-    if (S > 1 && ((long)(S - 1) * p.kb_per_split >= p.num_k_blocks || a.y_pool || a.addend || three_pass || a.scale || a.shift || a.act != NB_ACT_LINEAR))
+    if (S > 1 && a.a_is_conv && p.c_blocks % 2 == 0) p.kb_per_split += p.kb_per_split & 1;     // (see conv_tc_split)
+    if (S > 1 && ((long)(S - 1) * p.kb_per_split >= p.num_k_blocks || a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
         throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks and a plain epilogue");
     p.k_splits = S;
     p.m_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
@@ -947,7 +949,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.col3 = (col3 && !promote && block_n <= 128) ? 1 : 0;
     p.halves = p.col3 ? halves : 1;
     if (halves == 2 && !p.col3) throw Error(NB_ERR_UNSUPPORTED, "two-box tiles need the filter-column mode");
-    p.cbs = (!p.col3 && !three_pass && !gather && !promote && S == 1 && a.a_is_conv && block_n <= 128 &&
+    p.cbs = (!p.col3 && !three_pass && !gather && !promote && (S == 1 || p.kb_per_split % 2 == 0) && a.a_is_conv && block_n <= 128 &&
              (kc % (2 * BLOCK_K)) == 0 && box.bw * box.bh * box.bn == BLOCK_M) ? 2 : 1;
     {
         const int b_stage = block_n * BLOCK_K * 4;
@@ -1097,6 +1099,24 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
 }
 
 }  // namespace
+
+// A convolution of one or a few small images has fewer tiles than SMs, and its tiles run their whole K alone: at about 0.15 us
+// per 32-column block (two TMA requests of one thread) the 3x3 layers of a single ResNet-50 image (8 tiles, 72 and 144
+// blocks) took 29 and 47 us.  Such layers are cut along K until they occupy the SMs, four blocks per slice at least; the
+// slices are added by splitk_reduce4_kernel (2-3 us), so layers of fewer than 32 blocks stay whole.  Layers with more
+// tiles than half the SMs are never cut: their results do not depend on the batch.
+int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
+    const int c_blocks = (Kc + BLOCK_K - 1) / BLOCK_K, blocks = g.ksize * (g.ksize_w > 0 ? g.ksize_w : g.ksize) * c_blocks;
+    if (blocks < 32 || (N % 4) != 0) return 1;
+    const Box box = choose_box(g.OW, g.OH, g.batch, g.stride, false, true, (double)g.C * g.H * g.W * 4.0);
+    const long tiles = (long)((g.OW + box.bw - 1) / box.bw) * ((g.OH + box.bh - 1) / box.bh) * ((g.batch + box.bn - 1) / box.bn) *
+                       ((N + 63) / 64);
+    if (2 * tiles > h->sm_count) return 1;
+    const int S = (int)std::min<long>({h->sm_count / tiles, blocks / 4, 16});
+    int per = (blocks + S - 1) / S;
+    if (c_blocks % 2 == 0) per += per & 1;      // whole pairs of slices: two-block ring stages stay possible
+    return (blocks + per - 1) / per;
+}
 
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass) {
     std::string key = gemm_args_key(a, 'G', three_pass ? 1 : 0);

@@ -208,7 +208,7 @@ struct GemmArgs {
     int lstm_H = 0;
     const float *lstm_c_prev = nullptr;
     float *lstm_c = nullptr, *lstm_h = nullptr, *lstm_h_round = nullptr;
-    // plain matrices only: contract K in `split_k` slices of ceil(K blocks / split_k) 32-wide blocks (the last may be
+    // contract K in `split_k` slices of ceil(K blocks / split_k) 32-wide blocks (the last may be
     // shorter, none empty); slice s writes y + s*M*ldy
     // (y must hold split_k * M * ldy floats; the caller reduces the slices and applies the epilogue)
     int split_k = 1;
@@ -221,6 +221,8 @@ struct GemmArgs {
 // operands do not meet TMA's layout rules; callers then use gemm_simt.
 bool gemm_tc_supported(const nb_handle_s *h, const GemmArgs &a);
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
+// How many K slices (GemmArgs::split_k) an NHWC convolution should be cut into on the tensor cores; 1: none.
+int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
 // 3x3 stride-1 convolutions with 32..128 input channels: one halo load per channel slice serves all nine taps.
 bool conv_halo_supported(const nb_handle_s *h, const GemmArgs &a);
 void conv_halo_tc(nb_handle_s *h, const GemmArgs &a);
@@ -259,9 +261,21 @@ void launch_weight_relayout(nb_handle_s *h, const float *w_oihw, float *dst, int
 void launch_weight_pack(nb_handle_s *h, const float *w_oihw, float *dst, int F, int C, int k, int Kpad);
 // FC weights whose columns index (c,h,w) -> columns indexing (h,w,c)
 void launch_fc_permute(nb_handle_s *h, const float *w, float *dst, int out, int C, int H, int W);
-// sum of S slices [S][M][N] + folded scale/shift + activation (+ TF32 rounding) -> y [M][N]
-void launch_splitk_reduce(nb_handle_s *h, const float *ws, int S, int M, int N, const float *scale, const float *shift,
-                          int act, bool round_tf32, float *y);
+// sum of S slices [S][M][N] + folded scale/shift + activation (+ TF32 rounding) -> y [M][N]; for a convolution (rows are
+// pixels of OH x OW images) optionally with the shortcut or the 2x2/2 max-pool behind it
+struct SplitReduce {
+    const float *ws;
+    int S, M, N;
+    const float *scale, *shift;
+    int act, round;
+    float *y;
+    int OH, OW;
+    const float *res;                           // as GemmArgs' residual addend: NHWC [batch][res_h][res_w][res_ld], channels [0, res_c)
+    long res_ld;
+    int res_stride, res_c, res_h, res_w;
+    int pool;
+};
+void launch_splitk_reduce(nb_handle_s *h, const SplitReduce &p);
 // LSTM cell: z [B,4H] laid out [hidden unit][i,f,g,o] -> c_t, h_t (+ TF32-rounded copy of h_t)
 void launch_lstm_cell(nb_handle_s *h, const float *z, const float *c_prev, float *c_out, float *h_out,
                       float *h_round, int B, int H);

@@ -134,6 +134,15 @@ bool ConvPlan::can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const {
            (conn_c % 4) == 0 && (d.filters % 4) == 0;
 }
 
+int ConvPlan::splits(const ForwardOpts &o) const {
+    if (path(o) == PATH_SIMT || o.addend) return 1;
+    if (o.residual && ((o.res_c % 4) != 0 || ((uintptr_t)o.residual & 15))) return 1;     // (the reduction reads it in quads)
+    ConvGeom g;
+    g.batch = d.batch; g.C = d.channels; g.H = d.height; g.W = d.width; g.OH = OH; g.OW = OW;
+    g.ksize = d.size; g.stride = d.stride; g.pad = d.padding;
+    return conv_tc_split(h, g, d.channels, d.filters);
+}
+
 // Which of the three routes forward() takes, and the scratch each needs.
 size_t ConvPlan::reserve(const ForwardOpts &o) {
     const GemmPath pth = path(o);
@@ -148,6 +157,8 @@ size_t ConvPlan::reserve(const ForwardOpts &o) {
     } else if (pth != PATH_SIMT) {
         const bool need_round = (pth == PATH_TC) && !o.x_rounded;
         if (!o.x_nhwc || need_round || o.x_foreign) x_scratch.reserve(xin);
+        const int S = splits(o);
+        if (S > 1) split_ws.reserve((size_t)S * yout);
     }
     return workspace_bytes();
 }
@@ -307,7 +318,23 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
             const double eff = ((double)OW / ((OW + 13) / 14 * 14)) * ((double)OH / ((OH + bh - 1) / bh * bh));
             halo = eff >= 0.6;
         }
-        if (halo) conv_halo_tc(h, a);
+        const int S = splits(o);
+        if (S > 1 && !halo) {
+            GemmArgs sa = a;
+            sa.split_k = S;
+            sa.scale = sa.shift = sa.addend = nullptr; sa.res_stride = 0; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;
+            sa.y = split_ws.p; sa.y_pool = nullptr;
+            sa.algo_flops = 2.0 * (double)a.M * d.filters * d.channels * d.size * d.size;
+            gemm_tc(h, sa, pth == PATH_TC3);
+            SplitReduce r{};
+            r.ws = split_ws.p; r.S = S; r.M = a.M; r.N = d.filters; r.scale = a.scale; r.shift = a.shift; r.act = a.act;
+            r.round = o.round_out; r.y = o.pool_out ? o.pool_out : yo; r.OH = OH; r.OW = OW; r.pool = o.pool_out != nullptr;
+            if (o.residual) {
+                r.res = a.addend; r.res_ld = a.ld_addend; r.res_stride = a.res_stride;
+                r.res_c = a.res_c; r.res_h = a.res_h; r.res_w = a.res_w;
+            }
+            launch_splitk_reduce(h, r);
+        } else if (halo) conv_halo_tc(h, a);
         else gemm_tc(h, a, pth == PATH_TC3);
     }
     if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
@@ -356,16 +383,18 @@ GemmPath FcPlan::path() const {
     return h->math_mode == NB_MATH_TF32X3 ? PATH_TC3 : PATH_TC;
 }
 
-// Few rows and a long contraction (weight streaming): split K so that every SM pulls weights.  Chosen from K, N
-// and the SM count only, never from the batch: a batch and its slices add in the same order.  Wide tiles keep the
-// most weight bytes in flight per SM; the split count then fills the SMs, and of the three tile widths the one
-// that leaves the fewest SMs idle in the last wave wins.
-void FcPlan::split_choice(bool tc, bool has_addend, int *S_out, int *block_n_out) const {
+// Few rows and a long contraction (weight streaming): split K so that every SM pulls weights.  From 2048 columns on the
+// choice depends on K, N and the SM count only, never from the batch: a batch and its slices add in the same order.  Wide
+// tiles keep the most weight bytes in flight per SM; the split count then fills the SMs, and of the tile widths the one
+// that leaves the fewest SMs idle in the last wave wins.  Shorter contractions are split only for a single row of tiles that
+// leaves three quarters of the SMs idle (DBN at 32 images, 2000 -> 1000: 16 tiles of 63 K blocks took 36 us).
+void FcPlan::split_choice(GemmPath pth, bool has_addend, int rows, int *S_out, int *block_n_out) const {
     int S = 1, block_n = 0;
-    if (tc && !has_addend && (d.outputs % 4) == 0 && d.inputs >= 2048) {
-        const int kblocks = (d.inputs + 31) / 32;
+    const int kblocks = (d.inputs + 31) / 32;
+    if (pth == PATH_SIMT || has_addend || (d.outputs % 4) != 0) {
+    } else if (d.inputs >= 2048) {
         double best = 0.0;
-        for (int bn = 256; bn >= 64; bn /= 2) {
+        for (int bn = pth == PATH_TC3 ? 128 : 256; bn >= 64; bn /= 2) {
             const int nt = (d.outputs + bn - 1) / bn;
             int s = std::max(1, std::min({32, h->sm_count / nt, kblocks / 8}));
             const int per = (kblocks + s - 1) / s;
@@ -375,6 +404,14 @@ void FcPlan::split_choice(bool tc, bool has_addend, int *S_out, int *block_n_out
             if (fill > best + 0.05) { best = fill; S = s; block_n = bn; }
         }
         if (S == 1) block_n = 0;
+    } else if (rows <= 128 && kblocks >= 16) {
+        const int nt = (d.outputs + 63) / 64;
+        if (4 * nt <= h->sm_count) {
+            S = std::min({8, h->sm_count / nt, kblocks / 4});
+            const int per = (kblocks + S - 1) / S;
+            S = (kblocks + per - 1) / per;
+            block_n = 64;
+        }
     }
     *S_out = S; *block_n_out = block_n;
 }
@@ -384,7 +421,7 @@ size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
     const GemmPath pth = path();
     if ((pth == PATH_TC && !o.x_rounded) || (pth == PATH_TC3 && o.x_foreign)) x_scratch.reserve((size_t)M * d.inputs);
     int S, bn;
-    split_choice(pth == PATH_TC, o.addend != nullptr, &S, &bn);
+    split_choice(pth, o.addend != nullptr, M, &S, &bn);
     if (S > 1) split_ws.reserve((size_t)S * M * d.outputs);
     return workspace_bytes();
 }
@@ -423,15 +460,18 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
     w.ensure_split(h);
     a.b = w.hi.p; a.b_lo = w.lo.p;
     int S, block_n;
-    split_choice(pth == PATH_TC, o.addend != nullptr, &S, &block_n);
+    split_choice(pth, o.addend != nullptr, M, &S, &block_n);
     if (S > 1) {
         GemmArgs sa = a;
         sa.split_k = S; sa.block_n_hint = block_n;
         sa.scale = nullptr; sa.shift = nullptr; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;
         sa.y = split_ws.p; sa.ldy = d.outputs;
         sa.algo_flops = 2.0 * (double)M * d.outputs * d.inputs;
-        gemm_tc(h, sa, false);
-        launch_splitk_reduce(h, split_ws.p, S, M, d.outputs, a.scale, a.shift, d.activation, o.round_out, y);
+        gemm_tc(h, sa, pth == PATH_TC3);
+        SplitReduce r{};
+        r.ws = split_ws.p; r.S = S; r.M = M; r.N = d.outputs; r.scale = a.scale; r.shift = a.shift; r.act = d.activation;
+        r.round = o.round_out; r.y = y;
+        launch_splitk_reduce(h, r);
     } else {
         gemm_tc(h, a, pth == PATH_TC3);
     }

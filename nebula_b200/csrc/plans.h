@@ -78,16 +78,18 @@ struct ConvPlan : nb_plan_s {
     DeviceBuffer x_rowwin;
     DeviceBuffer scale, shift;
     bool has_scale = false, ready = false;
-    DeviceBuffer x_scratch, y_scratch;
+    DeviceBuffer x_scratch, y_scratch, split_ws;
     ConvPlan(nb_handle_s *h, const nb_conv2d_desc_t &desc);
     void set_weights(const float *weight, const float *bias, const float *g, const float *m, const float *v, int mem);
     void forward(const float *x, float *y, const ForwardOpts &o);
     // allocates the scratch tensors forward() would need with these options in the handle's current math mode
     // (forward() calls it too: a pass that was prepared allocates nothing); returns their total size in bytes
     size_t reserve(const ForwardOpts &o);
-    size_t workspace_bytes() const override { return (x_rowwin.n + x_scratch.n + y_scratch.n) * sizeof(float); }
+    size_t workspace_bytes() const override { return (x_rowwin.n + x_scratch.n + y_scratch.n + split_ws.n) * sizeof(float); }
     void output_dims(int dims[3]) const override { dims[0] = d.filters; dims[1] = OH; dims[2] = OW; }
     GemmPath path(const ForwardOpts &o) const;
+    // K slices of the tensor-core path with these options (1: none)
+    int splits(const ForwardOpts &o) const;
     // can the following 2x2 stride-2 max-pool be done in this layer's epilogue?
     bool can_fuse_pool() const;
     bool can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const;
@@ -107,7 +109,7 @@ struct FcPlan : nb_plan_s {
     size_t reserve(const ForwardOpts &o, int rows = -1);
     size_t workspace_bytes() const override { return (x_scratch.n + split_ws.n) * sizeof(float); }
     // split-K choice for `rows` input rows: number of K slices (1: none) and the tile width that goes with it
-    void split_choice(bool tc, bool has_addend, int *S, int *block_n) const;
+    void split_choice(GemmPath pth, bool has_addend, int rows, int *S, int *block_n) const;
     void output_dims(int dims[3]) const override { dims[0] = d.outputs; dims[1] = 1; dims[2] = 1; }
     GemmPath path() const;
 };

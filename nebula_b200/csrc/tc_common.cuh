@@ -258,6 +258,14 @@ __device__ __forceinline__ void tmem_ld_wait() {
 }
 
 
+static __device__ __noinline__ void activate_slab(float *x, int act) {
+#pragma unroll 1
+    for (int j = 0; j < 32; j += 4) {
+        float4 *q = reinterpret_cast<float4 *>(x + j);
+        *q = apply_activation4(*q, act);
+    }
+}
+
 // One 128-row x 32-column slab of accumulators (already in registers): folded batch-norm
 // scale/shift + bias, optional addend, activation, optional TF32 rounding, then either a swizzled
 // staging slab that leaves by TMA (optionally 2x2/2 max-pooled first) or plain global stores.
@@ -336,7 +344,7 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &e, const CUtenso
         }
     };
     auto activate = [&]() {
-        // the common ones inline, the rest through one out-of-line call per value
+        // the common ones inline, the rest through one out-of-line call
         if (e.act == NB_ACT_RELU) {
 #pragma unroll
             for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));   // NaN and -0 give +0, as x > 0 ? x : 0 does
@@ -346,9 +354,14 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &e, const CUtenso
                 const float x = __uint_as_float(v[j]);
                 v[j] = __float_as_uint(x > 0.0f ? x : (float)(0.1 * (double)x));
             }
-        } else if (e.act != NB_ACT_LINEAR) {
+        } else if (e.act != NB_ACT_LINEAR && rw.row_ok) {       // (rows without a pixel are never stored: the double formulas cost too much)
+            // through memory: with the slab's values passed in registers, those live across the call cost every mode registers
+            __align__(16) float x[32];
 #pragma unroll
-            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(apply_activation_call(__uint_as_float(v[j]), e.act));
+            for (int j = 0; j < 32; j++) x[j] = __uint_as_float(v[j]);
+            activate_slab(x, e.act);
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = __float_as_uint(x[j]);
         }
     };
     const bool has_addend = rw.arow && col0 < e.addend_cols;
