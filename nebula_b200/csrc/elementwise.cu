@@ -93,12 +93,16 @@ __global__ void activation_kernel(float *data, size_t n, int act) {
     }
 }
 
+// channel of element i of [batch][channel][size]; a 64-bit division only where the index needs one
+__device__ __forceinline__ unsigned channel_of(size_t i, unsigned size, unsigned channel) {
+    return (i >> 32) ? (unsigned)((i / size) % channel) : ((unsigned)i / size) % channel;
+}
 // _add_bias_ (common/utils.cu:118-134): y[b,c,s] += bias[c]
 __global__ void bias_kernel(float *out, const float *bias, unsigned channel, unsigned size, size_t total) {
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride)
-        out[i] += bias[(i / size) % channel];
+        out[i] += bias[channel_of(i, size, channel)];
 }
 // _normalize_ (common/batchnorm.cu:77-84) with the CPU formula (batchnorm.cc:70):
 // float subtraction, double divisor sqrt(var)+0.00001, stored as float.
@@ -107,7 +111,7 @@ __global__ void bn_normalize_kernel(float *out, const float *mean, const float *
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const unsigned c = (i / size) % channel;
+        const unsigned c = channel_of(i, size, channel);
         out[i] = (float)((double)(out[i] - mean[c]) / (sqrt((double)var[c]) + 0.00001));
     }
 }
@@ -116,7 +120,7 @@ __global__ void bn_scale_kernel(float *out, const float *scale, unsigned channel
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride)
-        out[i] *= scale[(i / size) % channel];
+        out[i] *= scale[channel_of(i, size, channel)];
 }
 
 // ----------------------------------------------------------------- softmax
@@ -174,23 +178,57 @@ __global__ void softmax_kernel(const float *x, float *y, int rows, int classes) 
 }
 
 // ------------------------------------------------------------------ layouts
-// [B][C][HW] <-> [B][HW][C] through a 32x32 shared-memory tile.
-__global__ void transpose_kernel(const float *src, float *dst, int rows, int cols, int round) {
+// [B][C][HW] <-> [B][HW][C]: src is [batch][rows][cols], dst is [batch][cols][rows], through a 64 x 64 tile in shared
+// memory.  Bound by HBM: 16-byte accesses on both sides where extent and alignment allow (VEC_IN: cols, VEC_OUT: rows
+// a multiple of 4), four in flight per thread; the 32 x 32 tile of single floats before it reached 3.4 TB/s.
+template <bool VEC_IN, bool VEC_OUT>
+__global__ void __launch_bounds__(256) transpose_kernel(const float *src, float *dst, int rows, int cols, int round) {
     grid_begin();
-    // src is [batch][rows][cols], dst is [batch][cols][rows]
-    __shared__ float tile[32][33];
+    __shared__ float tile[64][65];
     const size_t img = (size_t)blockIdx.z * rows * cols;
-    const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int r = r0 + j, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) tile[j][threadIdx.x] = src[img + (size_t)r * cols + c];
+    const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64, t = threadIdx.x;
+    if (VEC_IN) {
+        float4 v[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int r = r0 + (t >> 4) + 16 * i, c = c0 + 4 * (t & 15);
+            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < rows && c < cols) v[i] = *reinterpret_cast<const float4 *>(src + img + (size_t)r * cols + c);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            float *q = &tile[(t >> 4) + 16 * i][4 * (t & 15)];
+            q[0] = v[i].x; q[1] = v[i].y; q[2] = v[i].z; q[3] = v[i].w;
+        }
+    } else {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const int r = r0 + (t >> 6) + 4 * i, c = c0 + (t & 63);
+            v[i] = (r < rows && c < cols) ? src[img + (size_t)r * cols + c] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) tile[(t >> 6) + 4 * i][t & 63] = v[i];
     }
     __syncthreads();
-    for (int j = threadIdx.y; j < 32; j += blockDim.y) {
-        const int c = c0 + j, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) {
-            const float v = tile[threadIdx.x][j];
-            dst[img + (size_t)c * rows + r] = round ? round_tf32(v) : v;
+    if (VEC_OUT) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int c = (t >> 4) + 16 * i, r = 4 * (t & 15);
+            if (c0 + c < cols && r0 + r < rows) {
+                float4 v = make_float4(tile[r][c], tile[r + 1][c], tile[r + 2][c], tile[r + 3][c]);
+                if (round) { v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w); }
+                *reinterpret_cast<float4 *>(dst + img + (size_t)(c0 + c) * rows + r0 + r) = v;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const int c = (t >> 6) + 4 * i, r = t & 63;
+            if (c0 + c < cols && r0 + r < rows) {
+                const float v = tile[r][c];
+                dst[img + (size_t)(c0 + c) * rows + r0 + r] = round ? round_tf32(v) : v;
+            }
         }
     }
 }
@@ -241,14 +279,16 @@ __global__ void split_tf32_kernel(const float *src, float *hi, float *lo, size_t
 // ------------------------------------------------------------------ pooling
 // pooling_layer_t::forward (pooling_layer.cc:109-182): window origin oh*s-p,
 // max identity -1e8, average divisor k*k (padding included).
-template <bool NHWC>
+// (Index: unsigned while the tensor allows it.  The digits of an output index take six divisions, and as 64-bit ones they
+// were most of these kernels' time.)
+template <bool NHWC, class Index>
 __global__ void pool_kernel(const float *x, float *y, int B, int C, int H, int W, int OH, int OW, int k, int s, int p,
                             int is_max, int round, size_t total) {
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
         int c, ow, oh, b;
-        size_t t = i;
+        Index t = (Index)i;
         if (NHWC) { c = t % C; t /= C; ow = t % OW; t /= OW; oh = t % OH; b = (int)(t / OH); }
         else { ow = t % OW; t /= OW; oh = t % OH; t /= OH; c = t % C; b = (int)(t / C); }
         float mx = -1e8f, sum = 0.0f;
@@ -268,12 +308,13 @@ __global__ void pool_kernel(const float *x, float *y, int B, int C, int H, int W
     }
 }
 // NHWC with C % 4 == 0: one thread per 4 channels
+template <class Index>
 __global__ void pool_nhwc4_kernel(const float4 *x, float4 *y, int B, int C4, int H, int W, int OH, int OW, int k, int s,
                                   int p, int is_max, int round, size_t total) {
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        size_t t = i;
+        Index t = (Index)i;
         const int c = t % C4; t /= C4;
         const int ow = t % OW; t /= OW;
         const int oh = t % OH;
@@ -299,9 +340,34 @@ __global__ void pool_nhwc4_kernel(const float4 *x, float4 *y, int B, int C4, int
     }
 }
 
+// NCHW, 2x2 windows of stride 2 without padding, rows of whole quads: a thread reads a quad of two rows and writes two
+// outputs (b32 c256 56x56: 57 -> 25 us against pool_kernel with 64-bit index arithmetic).
+template <class Index>
+__global__ void pool_nchw_2x2_kernel(const float4 *x, float2 *y, int OH, int OW2, int is_max, int round, size_t total) {
+    grid_begin();
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        Index t = (Index)i;
+        const int q = (int)(t % OW2);
+        const size_t row = t / OW2;                 // (plane, oh); its input rows are 2 row and 2 row + 1
+        const float4 a = x[2 * row * OW2 + q], b = x[(2 * row + 1) * OW2 + q];
+        float2 o;
+        if (is_max) {
+            o.x = o.y = -1e8f;
+            o.x = a.x > o.x ? a.x : o.x; o.x = a.y > o.x ? a.y : o.x; o.x = b.x > o.x ? b.x : o.x; o.x = b.y > o.x ? b.y : o.x;
+            o.y = a.z > o.y ? a.z : o.y; o.y = a.w > o.y ? a.w : o.y; o.y = b.z > o.y ? b.z : o.y; o.y = b.w > o.y ? b.w : o.y;
+        } else {
+            o.x = (((0.0f + a.x) + a.y) + b.x + b.y) / 4.0f;
+            o.y = (((0.0f + a.z) + a.w) + b.z + b.w) / 4.0f;
+        }
+        if (round) { o.x = round_tf32(o.x); o.y = round_tf32(o.y); }
+        y[i] = o;
+    }
+}
+
 // ----------------------------------------------------------------- shortcut
 // shortcut() (common/utils.cc:28-60) + activation, as one pass over the output.
-template <bool NHWC>
+template <bool NHWC, class Index>
 __global__ void shortcut_kernel(const float *prev, const float *conn, float *y, int B, int Ci, int Hi, int Wi, int Co,
                                 int Ho, int Wo, int stride, int sample, int act, int round, size_t total) {
     grid_begin();
@@ -309,7 +375,7 @@ __global__ void shortcut_kernel(const float *prev, const float *conn, float *y, 
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
         int c, w, h, b;
-        size_t t = i;
+        Index t = (Index)i;
         if (NHWC) { c = t % Co; t /= Co; w = t % Wo; t /= Wo; h = t % Ho; b = (int)(t / Ho); }
         else { w = t % Wo; t /= Wo; h = t % Ho; t /= Ho; c = t % Co; b = (int)(t / Co); }
         float v = prev[i];
@@ -326,13 +392,14 @@ __global__ void shortcut_kernel(const float *prev, const float *conn, float *y, 
 }
 
 // NHWC with both channel counts divisible by 4: one thread per 4 channels, 128-bit accesses
+template <class Index>
 __global__ void shortcut_nhwc4_kernel(const float4 *prev, const float4 *conn, float4 *y, int B, int Ci4, int Hi, int Wi, int Co4,
                                       int Ho, int Wo, int stride, int sample, int act, int round, size_t total) {
     grid_begin();
     const int mw = Wi < Wo ? Wi : Wo, mh = Hi < Ho ? Hi : Ho, mc = Ci4 < Co4 ? Ci4 : Co4;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
-        size_t t = i;
+        Index t = (Index)i;
         const int c = (int)(t % Co4); t /= Co4;
         const int w = (int)(t % Wo); t /= Wo;
         const int h = (int)(t % Ho);
@@ -349,6 +416,24 @@ __global__ void shortcut_nhwc4_kernel(const float4 *prev, const float4 *conn, fl
         v = apply_activation4_fast(v, act);
         if (round) { v.x = round_tf32(v.x); v.y = round_tf32(v.y); v.z = round_tf32(v.z); v.w = round_tf32(v.w); }
         y[i] = v;
+    }
+}
+
+// NCHW, the connection as large as the output and planes of whole quads: the sum is over the leading channels of each image
+template <class Index>
+__global__ void shortcut_nchw4_kernel(const float4 *prev, const float4 *conn, float4 *y, int Ci, int Co, int plane4, int act, size_t total) {
+    grid_begin();
+    const size_t gstride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gstride) {
+        Index t = (Index)i;
+        const int px = (int)(t % plane4); t /= plane4;
+        const int c = (int)(t % Co);
+        float4 v = prev[i];
+        if (c < Ci) {
+            const float4 r = conn[((size_t)(t / Co) * Ci + c) * plane4 + px];
+            v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w;
+        }
+        y[i] = apply_activation4_fast(v, act);
     }
 }
 
@@ -389,10 +474,9 @@ __global__ void rowwin_input_kernel(const float *x, float4 *dst, int N, int C, i
     grid_begin();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
-        const int pcol = (int)(i % Wp);
-        const size_t nh = i / Wp;
-        const int hrow = (int)(nh % H);
-        const size_t n = nh / H;
+        const unsigned row = (unsigned)(i / Wp);        // (image, row): fits 32 bits, the pixel index need not
+        const int pcol = (int)(i - (size_t)row * Wp), hrow = (int)(row % H);
+        const size_t n = row / H;
         const int iw = pcol - pad;
         float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (iw >= 0 && iw < W) {
@@ -574,13 +658,14 @@ void elementwise_prepare_device() {
     cudaFuncAttributes fa;
     const void *kernels[] = {
         (const void *)activation_kernel, (const void *)bias_kernel, (const void *)bn_normalize_kernel,
-        (const void *)bn_scale_kernel, (const void *)softmax_kernel, (const void *)transpose_kernel,
-        (const void *)round_tf32_kernel, (const void *)split_tf32_kernel, (const void *)pool_kernel<true>,
-        (const void *)pool_kernel<false>, (const void *)pool_nhwc4_kernel, (const void *)shortcut_kernel<true>,
-        (const void *)shortcut_kernel<false>, (const void *)weight_pack_kernel, (const void *)weight_rowwin_kernel,
+        (const void *)bn_scale_kernel, (const void *)softmax_kernel, (const void *)transpose_kernel<true, true>, (const void *)transpose_kernel<true, false>,
+        (const void *)transpose_kernel<false, true>, (const void *)transpose_kernel<false, false>,
+        (const void *)round_tf32_kernel, (const void *)split_tf32_kernel, (const void *)pool_kernel<true, unsigned>,
+        (const void *)pool_kernel<false, unsigned>, (const void *)pool_nhwc4_kernel<unsigned>, (const void *)pool_nchw_2x2_kernel<unsigned>,
+        (const void *)shortcut_kernel<true, unsigned>, (const void *)shortcut_kernel<false, unsigned>, (const void *)shortcut_nchw4_kernel<unsigned>, (const void *)weight_pack_kernel, (const void *)weight_rowwin_kernel,
         (const void *)rowwin_input_kernel, (const void *)weight_relayout_kernel, (const void *)fc_permute_kernel,
         (const void *)splitk_reduce_kernel, (const void *)lstm_cell_kernel,
-        (const void *)u8_pack_kernel, (const void *)splitk_reduce4_kernel, (const void *)shortcut_nhwc4_kernel};
+        (const void *)u8_pack_kernel, (const void *)splitk_reduce4_kernel, (const void *)shortcut_nhwc4_kernel<unsigned>};
     for (const void *k : kernels) NB_CHECK_CUDA(cudaFuncGetAttributes(&fa, k));
 }
 
@@ -627,10 +712,14 @@ void launch_layout(nb_handle_s *h, const float *src, float *dst, int B, int C, i
     const int rows = to_nhwc ? C : HW, cols = to_nhwc ? HW : C;
     for (int b0 = 0; b0 < B; b0 += 65535) {
         const int nb_ = std::min(65535, B - b0);
-        dim3 grid((cols + 31) / 32, (rows + 31) / 32, nb_), block(32, 8);
-        if (grid.y > 65535) throw Error(NB_ERR_UNSUPPORTED, "layout conversion: extent too large");
-        launch_overlapped(h, transpose_kernel, grid, block, 0, src + (size_t)b0 * C * HW, dst + (size_t)b0 * C * HW, rows, cols,
-                                                       round ? 1 : 0);
+        if ((rows + 31) / 32 > 65535) throw Error(NB_ERR_UNSUPPORTED, "layout conversion: extent too large");
+        const dim3 grid((cols + 63) / 64, (rows + 63) / 64, nb_);
+        const float *sp = src + (size_t)b0 * C * HW;
+        float *dp = dst + (size_t)b0 * C * HW;
+        const bool vi = (cols % 4) == 0 && (((uintptr_t)sp) & 15) == 0, vo = (rows % 4) == 0 && (((uintptr_t)dp) & 15) == 0;
+        const auto kernel = vi ? (vo ? transpose_kernel<true, true> : transpose_kernel<true, false>)
+                               : (vo ? transpose_kernel<false, true> : transpose_kernel<false, false>);
+        launch_overlapped(h, kernel, grid, TPB, 0, sp, dp, rows, cols, round ? 1 : 0);
         check_launch("transpose_kernel");
         count_launch(h);
     }
@@ -651,20 +740,21 @@ void launch_pool(nb_handle_s *h, const nb_pool_desc_t &d, const float *x, float 
     const int OH = (d.height + 2 * d.padding) / d.stride, OW = (d.width + 2 * d.padding) / d.stride;
     const size_t total = (size_t)d.batch * d.channels * OH * OW;
     if (!total) return;
-    const int is_max = d.mode == NB_POOL_MAX;
-    if (d.layout == NB_LAYOUT_NHWC && (d.channels % 4) == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) {
+    const int is_max = d.mode == NB_POOL_MAX, rnd = round ? 1 : 0;
+    const bool small = total < (1ull << 32), aligned = (((uintptr_t)x | (uintptr_t)y) & 15) == 0;
+    if (d.layout == NB_LAYOUT_NHWC && (d.channels % 4) == 0 && aligned) {
         const size_t t4 = total / 4;
-        launch_overlapped(h, pool_nhwc4_kernel, grid_for(t4, h), TPB, 0, (const float4 *)x, (float4 *)y, d.batch, d.channels / 4,
-                                                                   d.height, d.width, OH, OW, d.size, d.stride, d.padding,
-                                                                   is_max, round ? 1 : 0, t4);
-    } else if (d.layout == NB_LAYOUT_NHWC) {
-        launch_overlapped(h, pool_kernel<true>, grid_for(total, h), TPB, 0, x, y, d.batch, d.channels, d.height, d.width, OH, OW,
-                                                                      d.size, d.stride, d.padding, is_max, round ? 1 : 0,
-                                                                      total);
+        launch_overlapped(h, small ? pool_nhwc4_kernel<unsigned> : pool_nhwc4_kernel<size_t>, grid_for(t4, h), TPB, 0, (const float4 *)x,
+                          (float4 *)y, d.batch, d.channels / 4, d.height, d.width, OH, OW, d.size, d.stride, d.padding, is_max, rnd, t4);
+    } else if (d.layout == NB_LAYOUT_NCHW && d.size == 2 && d.stride == 2 && d.padding == 0 && (d.width % 4) == 0 &&
+               (d.height % 2) == 0 && aligned) {
+        launch_overlapped(h, small ? pool_nchw_2x2_kernel<unsigned> : pool_nchw_2x2_kernel<size_t>, grid_for(total / 2, h), TPB, 0,
+                          (const float4 *)x, (float2 *)y, OH, d.width / 4, is_max, rnd, total / 2);
     } else {
-        launch_overlapped(h, pool_kernel<false>, grid_for(total, h), TPB, 0, x, y, d.batch, d.channels, d.height, d.width, OH,
-                                                                       OW, d.size, d.stride, d.padding, is_max,
-                                                                       round ? 1 : 0, total);
+        const auto kernel = d.layout == NB_LAYOUT_NHWC ? (small ? pool_kernel<true, unsigned> : pool_kernel<true, size_t>)
+                                                       : (small ? pool_kernel<false, unsigned> : pool_kernel<false, size_t>);
+        launch_overlapped(h, kernel, grid_for(total, h), TPB, 0, x, y, d.batch, d.channels, d.height, d.width, OH, OW, d.size, d.stride,
+                          d.padding, is_max, rnd, total);
     }
     check_launch("pool_kernel");
     count_launch(h);
@@ -675,19 +765,24 @@ void launch_shortcut(nb_handle_s *h, const nb_shortcut_desc_t &d, const float *p
     if (!total) return;
     const int stride = d.conn_width / d.out_width > 1 ? d.conn_width / d.out_width : 1;
     const int sample = d.out_width / d.conn_width > 1 ? d.out_width / d.conn_width : 1;
-    if (d.layout == NB_LAYOUT_NHWC && (d.conn_channels % 4) == 0 && (d.out_channels % 4) == 0 &&
-        ((((uintptr_t)prev) | ((uintptr_t)conn) | ((uintptr_t)y)) & 15) == 0)
-        launch_overlapped(h, shortcut_nhwc4_kernel, grid_for(total / 4, h), TPB, 0, 
-            (const float4 *)prev, (const float4 *)conn, (float4 *)y, d.batch, d.conn_channels / 4, d.conn_height, d.conn_width,
-            d.out_channels / 4, d.out_height, d.out_width, stride, sample, d.activation, round ? 1 : 0, total / 4);
-    else if (d.layout == NB_LAYOUT_NHWC)
-        launch_overlapped(h, shortcut_kernel<true>, grid_for(total, h), TPB, 0, 
-            prev, conn, y, d.batch, d.conn_channels, d.conn_height, d.conn_width, d.out_channels, d.out_height,
-            d.out_width, stride, sample, d.activation, round ? 1 : 0, total);
-    else
-        launch_overlapped(h, shortcut_kernel<false>, grid_for(total, h), TPB, 0, 
-            prev, conn, y, d.batch, d.conn_channels, d.conn_height, d.conn_width, d.out_channels, d.out_height,
-            d.out_width, stride, sample, d.activation, round ? 1 : 0, total);
+    const bool small = total < (1ull << 32);
+    const bool aligned = ((((uintptr_t)prev) | ((uintptr_t)conn) | ((uintptr_t)y)) & 15) == 0;
+    const int plane = d.out_height * d.out_width;
+    if (d.layout == NB_LAYOUT_NHWC && (d.conn_channels % 4) == 0 && (d.out_channels % 4) == 0 && aligned) {
+        launch_overlapped(h, small ? shortcut_nhwc4_kernel<unsigned> : shortcut_nhwc4_kernel<size_t>, grid_for(total / 4, h), TPB, 0,
+                          (const float4 *)prev, (const float4 *)conn, (float4 *)y, d.batch, d.conn_channels / 4, d.conn_height, d.conn_width,
+                          d.out_channels / 4, d.out_height, d.out_width, stride, sample, d.activation, round ? 1 : 0, total / 4);
+    } else if (d.layout == NB_LAYOUT_NCHW && !round && aligned && (plane % 4) == 0 && d.conn_height == d.out_height &&
+               d.conn_width == d.out_width) {
+        launch_overlapped(h, small ? shortcut_nchw4_kernel<unsigned> : shortcut_nchw4_kernel<size_t>, grid_for(total / 4, h), TPB, 0,
+                          (const float4 *)prev, (const float4 *)conn, (float4 *)y, d.conn_channels, d.out_channels, plane / 4, d.activation,
+                          total / 4);
+    } else {
+        const auto kernel = d.layout == NB_LAYOUT_NHWC ? (small ? shortcut_kernel<true, unsigned> : shortcut_kernel<true, size_t>)
+                                                       : (small ? shortcut_kernel<false, unsigned> : shortcut_kernel<false, size_t>);
+        launch_overlapped(h, kernel, grid_for(total, h), TPB, 0, prev, conn, y, d.batch, d.conn_channels, d.conn_height, d.conn_width,
+                          d.out_channels, d.out_height, d.out_width, stride, sample, d.activation, round ? 1 : 0, total);
+    }
     check_launch("shortcut_kernel");
     count_launch(h);
 }

@@ -801,7 +801,7 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra) {
     key_add(k, a.M); key_add(k, a.N); key_add(k, a.Kc);
     key_add(k, a.scale); key_add(k, a.shift); key_add(k, a.addend); key_add(k, a.ld_addend); key_add(k, a.addend_after_act);
     key_add(k, a.res_stride); key_add(k, a.res_c); key_add(k, a.res_h); key_add(k, a.res_w);
-    key_add(k, a.act); key_add(k, a.round_out_tf32); key_add(k, a.y); key_add(k, a.ldy); key_add(k, a.y_pool);
+    key_add(k, a.act); key_add(k, a.round_out_tf32); key_add(k, a.y); key_add(k, a.ldy); key_add(k, a.y_nchw); key_add(k, a.y_pool);
     key_add(k, a.lstm_H); key_add(k, a.lstm_c_prev); key_add(k, a.lstm_c); key_add(k, a.lstm_h); key_add(k, a.lstm_h_round);
     key_add(k, a.b_static);
     key_add(k, a.split_k); key_add(k, a.block_n_hint); key_add(k, a.algo_flops);
@@ -890,7 +890,12 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     if (a.lstm_H > 0 && a.act != NB_ACT_LINEAR && !p.e.addend_post)
         throw Error(NB_ERR_INVALID_ARG, "LSTM epilogue: a non-linear gate activation needs the addend added after it");
     p.e.y = a.y; p.e.ldy = a.ldy;
-    p.e.tma_store = a.y && aligned16(a.y) && (a.ldy % 4) == 0;
+    p.e.tma_store = a.y && aligned16(a.y) && (a.ldy % 4) == 0 && !a.y_nchw;
+    if (a.y_nchw) {
+        if (!a.a_is_conv || gather || S > 1 || pool || a.lstm_H > 0)
+            throw Error(NB_ERR_INVALID_ARG, "NCHW output needs a whole convolution whose rows are pixels");
+        p.e.plane = g.OH * g.OW;
+    }
     if (S > 1 && !p.e.tma_store) throw Error(NB_ERR_INVALID_ARG, "split-K needs a 16-byte aligned output with ldy % 4 == 0");
     p.e.pool = pool ? 1 : 0;
     if (pool) {

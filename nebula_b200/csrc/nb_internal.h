@@ -200,6 +200,7 @@ struct GemmArgs {
     bool round_out_tf32 = false;    // store RN(TF32) values (the consumer is a TF32 contraction)
     float *y = nullptr;
     long ldy = 0;
+    bool y_nchw = false;            // tensor-core conv only (whole K, TMA-fed): y is NCHW [batch][N][OH][OW]
     // tensor-core conv only: write the 2x2 stride-2 max-pooled output [B][OH/2][OW/2][N] here INSTEAD of y
     float *y_pool = nullptr;
     // tensor-core kernel, plain matrices: the N = 4*lstm_H columns are gate pre-activations laid out

@@ -143,13 +143,21 @@ int ConvPlan::splits(const ForwardOpts &o) const {
     return conv_tc_split(h, g, d.channels, d.filters);
 }
 
+// The TMA-fed tensor-core routes write NCHW themselves; the others (CUDA cores, in-kernel gather, K slices) go through
+// a layout pass.
+bool ConvPlan::writes_nchw(const ForwardOpts &o) const {
+    if (o.y_nhwc || h->math_mode == NB_MATH_FP32) return false;
+    if (path(o) == PATH_SIMT) return rowwin_ok;
+    return splits(o) == 1;
+}
+
 // Which of the three routes forward() takes, and the scratch each needs.
 size_t ConvPlan::reserve(const ForwardOpts &o) {
     const GemmPath pth = path(o);
     const size_t xin = (size_t)d.batch * d.channels * d.height * d.width;
     const size_t yout = (size_t)d.batch * d.filters * OH * OW;
     const bool tc_mode = h->math_mode != NB_MATH_FP32;
-    if (!o.y_nhwc) y_scratch.reserve(yout);
+    if (!o.y_nhwc) y_scratch.reserve(yout);         // (also where this route writes NCHW itself: a later math mode may not)
     if (pth == PATH_SIMT && rowwin_ok) {
         x_rowwin.reserve((size_t)d.batch * d.height * rw_wp * 4);
     } else if (pth == PATH_SIMT && pack_ok && tc_mode && h->encode_tiled) {
@@ -194,9 +202,10 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         ra.scale = has_scale ? scale.p : nullptr; ra.shift = shift.p; ra.act = d.activation;
         ra.round_out_tf32 = o.round_out; ra.addend = o.addend; ra.ld_addend = d.filters;
         float *yo = y;
+        ra.y_nchw = writes_nchw(o);
         if (!o.y_nhwc) {
             NB_REQUIRE(o.addend == nullptr, "conv: addend needs NHWC output");
-            yo = y_scratch.p;
+            if (!ra.y_nchw) yo = y_scratch.p;
         }
         ra.y = yo; ra.ldy = d.filters;
         ra.algo_flops = 2.0 * (double)ra.M * d.filters * d.channels * d.size * d.size;
@@ -210,7 +219,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         }
         if (gemm_tc_supported(h, ra)) {
             gemm_tc(h, ra, three);
-            if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
+            if (yo != y) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
             return;
         }
     }
@@ -276,9 +285,10 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
     a.addend = o.addend;
     a.ld_addend = d.filters;
     float *yo = y;
+    a.y_nchw = writes_nchw(o);
     if (!o.y_nhwc) {
         NB_REQUIRE(o.addend == nullptr, "conv: addend needs NHWC output");
-        yo = y_scratch.p;
+        if (!a.y_nchw) yo = y_scratch.p;
     }
     a.y = yo;
     a.ldy = d.filters;
@@ -311,7 +321,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
             const char *v = std::getenv("NEBULA_B200_HALO");
             return v && *v == '1';
         }();
-        bool halo = halo_on && pth == PATH_TC && (d.channels <= 64 || (d.channels <= 128 && d.filters <= 128)) &&
+        bool halo = halo_on && pth == PATH_TC && !a.y_nchw && (d.channels <= 64 || (d.channels <= 128 && d.filters <= 128)) &&
                     conv_halo_supported(h, a);
         if (halo) {
             const int bh = OH >= 16 ? 16 : 8;
@@ -337,7 +347,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         } else if (halo) conv_halo_tc(h, a);
         else gemm_tc(h, a, pth == PATH_TC3);
     }
-    if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
+    if (!o.y_nhwc && yo != y) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
 }
 
 // ---------------------------------------------------------------------- fc

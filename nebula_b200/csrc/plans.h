@@ -90,6 +90,7 @@ struct ConvPlan : nb_plan_s {
     GemmPath path(const ForwardOpts &o) const;
     // K slices of the tensor-core path with these options (1: none)
     int splits(const ForwardOpts &o) const;
+    bool writes_nchw(const ForwardOpts &o) const;
     // can the following 2x2 stride-2 max-pool be done in this layer's epilogue?
     bool can_fuse_pool() const;
     bool can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const;

@@ -34,6 +34,8 @@ struct EpiParams {
     float *y;
     long ldy;
     int tma_store;              // y meets TMA's rules: slabs leave through a tensor map; else plain stores
+    int plane;                  // > 0: y is NCHW, `plane` pixels per channel; a lane owns a pixel, so a warp's store of a column is
+                                // one contiguous run, and no layout pass follows
     int pool;                   // fuse the following 2x2 stride-2 max-pool: only the pooled tensor is written
     int N;                      // valid output columns
     // LSTM mode (lstm_H > 0): columns are gate pre-activations laid out [hidden unit][i,f,g,o]; instead of
@@ -485,6 +487,14 @@ __device__ __forceinline__ void epilogue_chunk(const EpiParams &e, const CUtenso
                 tma_store_4d(tm_yp, slab, col0, bx.ow0 >> 1, bx.oh0 >> 1, bx.n0);
                 tma_store_commit();
             }
+        }
+    } else if (e.plane) {
+        if (rw.row_ok) {
+            const int n = (int)rw.grow / e.plane;           // (the image: worked out here so that other modes do not carry it)
+            float *yp = e.y + ((long)n * e.N + col0) * e.plane + ((int)rw.grow - n * e.plane);
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (full_cols || col0 + j < e.N) yp[(long)j * e.plane] = __uint_as_float(v[j]);
         }
     } else if (rw.row_ok) {
         float *yrow = e.y + rw.grow * e.ldy + col0;
