@@ -72,10 +72,12 @@ struct TcParams {
     // and the TMEM accumulator restarts; parts = number of such partial sums per tile (1: no promotion).
     int kb_per_part, parts;
     // Ring stages of `cbs` K blocks (1 or 2).  One TMA request costs its issuing thread a few hundred cycles whatever
-    // its size, and a narrow tile's K block is only 180-350 cycles of MMAs, so convolutions with 64-128 input
-    // channels fetch two 32-channel slices of a tap per request: the A map then has the slice index as a fifth
-    // dimension (tm_a is 5-D, tm_b 4-D), a stage is [A0 | A1 | B0 | B1], `stages` of them fit the ring.
-    int cbs, stages;
+    // its size, and a narrow tile's K block is only 180-350 cycles of MMAs, so tiles of up to 128 columns whose 32-column
+    // slices pair up fetch two slices per request: the A map then has the slice index as a fifth dimension (tm_a is 5-D,
+    // tm_b 4-D), a stage is [A0 | A1 | B0 | B1], `stages` of them fit the ring.  A slice of the A box is a_slice_bytes (a
+    // whole number of 1024-byte swizzle repeats); the MMA reads 128 rows from its start, so A takes a_region bytes, and what
+    // it reads past a box of fewer rows only feeds accumulator rows that are never stored.
+    int cbs, stages, a_slice_bytes, a_region;
     // Filter-column stages (col3 = 1): 3x3 stride-1 convolutions with few input channels are bound by the L2 -> shared
     // memory traffic of re-loading the activation tile once per tap.  Here a stage is one filter COLUMN kw of one channel
     // slice: ONE activation box of bh + 2 image rows (a_box_bytes) and the three weight tiles kh = 0..2.  Tap (kh, kw)
@@ -179,6 +181,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
     // per stage: [A | B | (A_lo | B_lo)], or [A0 | A1 | B0 | B1] with two K blocks per stage
     const int cbs = THREE ? 1 : p.cbs;
     const int stages = p.stages;
+    const int a_region = (THREE || cbs == 1) ? A_STAGE_BYTES : p.a_region, a_slice = (THREE || cbs == 1) ? A_STAGE_BYTES : p.a_slice_bytes;
     const int stage_bytes = p.stage_bytes;
     const int halves = (THREE || PROMOTE || BLOCK_N > 128) ? 1 : p.halves;
     const int acc_cols = halves * BLOCK_N;              // TMEM columns of one accumulator set
@@ -237,9 +240,9 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         const int box_rows = (GATHER || p.col3) ? BLOCK_M : p.bw * p.bh * p.bn;
         if (box_rows < BLOCK_M) {
             const int tail16 = (BLOCK_M - box_rows) * 8;          // 16-byte chunks per stage tail
-            for (int i = threadIdx.x; i < stages * tail16; i += blockDim.x) {      // (two-block stages only take full boxes)
+            for (int i = threadIdx.x; i < stages * tail16; i += blockDim.x) {
                 const int s = i / tail16, c = i - s * tail16;
-                reinterpret_cast<float4 *>(smem + s * stage_bytes + box_rows * 128)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+                reinterpret_cast<float4 *>(smem + s * stage_bytes + cbs * box_rows * 128)[c] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
@@ -260,6 +263,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         uint32_t phase = 0;
         bool ok = true;
         TileIter ti(p, blockIdx.x, gridDim.x);
+        const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), ring0 = smem_u32(smem);
+        uint32_t sa = ring0;            // the current stage
         const uint32_t tx_bytes = (!THREE && p.col3)
             ? (uint32_t)(p.a_box_bytes + 3 * C::B_STAGE_BYTES)
             : (uint32_t)(((GATHER ? 0 : p.tx_bytes_a) + C::B_STAGE_BYTES * (THREE ? 2 : 1)) * cbs);
@@ -279,7 +284,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     continue;
                 }
                 const int kb = kb0 + i * cbs, tap = kb / p.c_blocks, cb = kb - tap * p.c_blocks;
-                uint8_t *sb = sa + A_STAGE_BYTES * cbs;
+                uint8_t *sb = sa + a_region;
                 if (cbs == 2) {
                     tma_load_4d(sb, &p.tm_b, &full[i], 0, ti.n_tile * BLOCK_N, cb, tap);
                 } else {
@@ -302,15 +307,16 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 // (tm_b is 4-D here, {C, N, kw, kh}: a box of one kw and all three kh)
                 for (int cb3 = 0; cb3 < p.c_blocks && ok; cb3++) {       // kw fastest, then the channel slice
                     for (int kw3 = 0; kw3 < p.ksize_w; kw3++) {
-                        if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status))) break;
-                        uint8_t *sa = smem + stage * stage_bytes;
+                        if (!(ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, p.status))) break;
+                        const uint32_t bar = full0 + 8 * stage;
                         const bool b_there = primed > 0;
                         if (b_there) primed--;
-                        else mbar_expect_tx(&full[stage], tx_bytes);
-                        tma_load_4d(sa, &p.tm_a, &full[stage], cb3 * BLOCK_K, w0 + kw3, h0, n0);
+                        else mbar_expect_tx(bar, tx_bytes);
+                        tma_load_4d(sa, &p.tm_a, bar, cb3 * BLOCK_K, w0 + kw3, h0, n0);
                         if (!b_there)
-                            tma_load_4d(sa + p.a_box_bytes, &p.tm_b, &full[stage], cb3 * BLOCK_K, n_tile * BLOCK_N, kw3, 0);
-                        if (++stage == stages) { stage = 0; phase ^= 1; }
+                            tma_load_4d(sa + p.a_box_bytes, &p.tm_b, bar, cb3 * BLOCK_K, n_tile * BLOCK_N, kw3, 0);
+                        sa += stage_bytes;
+                        if (++stage == stages) { stage = 0; phase ^= 1; sa = ring0; }
                     }
                 }
                 continue;
@@ -321,21 +327,20 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 kh = tap / p.ksize_w; kw = tap - kh * p.ksize_w;
             }
             for (int kb = kb0; kb < kb_end; kb += cbs) {
-                if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status))) break;
-                uint8_t *sa = smem + stage * stage_bytes;
-                uint8_t *sb = sa + A_STAGE_BYTES * cbs;
+                if (!(ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, p.status))) break;
+                const uint32_t bar = full0 + 8 * stage, sb = sa + a_region;
                 const bool b_there = primed > 0;
                 if (b_there) primed--;
-                else mbar_expect_tx(&full[stage], tx_bytes);
+                else mbar_expect_tx(bar, tx_bytes);
                 if (cbs == 2) {
-                    tma_load_5d(sa, &p.tm_a, &full[stage], 0, w0 + kw, h0 + kh, n0, cb);
-                    if (!b_there) tma_load_4d(sb, &p.tm_b, &full[stage], 0, n_tile * BLOCK_N, cb, tap);
+                    tma_load_5d(sa, &p.tm_a, bar, 0, w0 + kw, h0 + kh, n0, cb);
+                    if (!b_there) tma_load_4d(sb, &p.tm_b, bar, 0, n_tile * BLOCK_N, cb, tap);
                 } else {
-                    if (!GATHER) tma_load_4d(sa, &p.tm_a, &full[stage], cb * BLOCK_K, w0 + kw, h0 + kh, n0);
+                    if (!GATHER) tma_load_4d(sa, &p.tm_a, bar, cb * BLOCK_K, w0 + kw, h0 + kh, n0);
                     if (!b_there) {
-                        tma_load_3d(sb, &p.tm_b, &full[stage], cb * BLOCK_K, n_tile * BLOCK_N, tap);
+                        tma_load_3d(sb, &p.tm_b, bar, cb * BLOCK_K, n_tile * BLOCK_N, tap);
                         if (THREE)
-                            tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, &full[stage], cb * BLOCK_K,
+                            tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, bar, cb * BLOCK_K,
                                         n_tile * BLOCK_N, tap);
                     }
                 }
@@ -343,7 +348,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     cb = 0; tap++;
                     if (++kw == p.ksize_w) { kw = 0; kh++; }
                 }
-                if (++stage == stages) { stage = 0; phase ^= 1; }
+                sa += stage_bytes;
+                if (++stage == stages) { stage = 0; phase ^= 1; sa = ring0; }
             }
         }
         // Tail: the MMA warp's last release of every stage (an mbarrier arrive that the tensor core performs
@@ -368,6 +374,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         uint32_t acc_phase = 0;
         int tile_parity = 0;
         bool ok = true;
+        // this lane's instructions between two MMAs are on the critical path of narrow tiles: addresses advance by increments
+        const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), ring0 = smem_desc_lo(smem_u32(smem));
+        const uint32_t ring_step = (uint32_t)stage_bytes >> 4;
+        uint32_t ring = ring0;          // the current stage's descriptor word
         grid_dependency_wait();         // the bounded waits below must not count the kernels in front
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             if (!(ok = mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status))) break;
@@ -376,24 +386,23 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
             int kb_in_part = 0;
             if (!THREE && p.col3) {
                 for (int it = 0; it < p.ksize_w * p.c_blocks; it++) {
-                    if (!(ok = mbar_wait(&full[stage], phase, abort_flag, p.status))) break;
+                    if (!(ok = mbar_wait(full0 + 8 * stage, phase, abort_flag, p.status))) break;
                     tc_fence_after();
-                    const uint32_t sa = smem_u32(smem + stage * stage_bytes);
-                    if (leader) {
+                    const uint32_t b_base = ring + ((uint32_t)p.a_box_bytes >> 4);
 #pragma unroll
-                        for (int kh3 = 0; kh3 < 3; kh3++) {
-                            const uint32_t b_lo = smem_desc_lo(sa + (uint32_t)p.a_box_bytes + kh3 * C::B_STAGE_BYTES);
-                            for (int hf = 0; hf < halves; hf++) {       // image row kh3 (+ bh for the second half) of the box
-                                const uint32_t a_lo = smem_desc_lo(sa + (uint32_t)((hf * p.bh + kh3) * p.bw * 128));
+                    for (int kh3 = 0; kh3 < 3; kh3++) {
+                        const uint32_t b_lo = b_base + kh3 * (C::B_STAGE_BYTES >> 4);
+                        for (int hf = 0; hf < halves; hf++) {       // image row kh3 (+ 8 for the second half) of the 16 pixels wide box
+                            const uint32_t a_lo = ring + (hf * 8 + kh3) * (16 * 128 >> 4);
 #pragma unroll
-                                for (int k = 0; k < BLOCK_K / UMMA_K; k++)
-                                    umma_tf32(d_tmem + (uint32_t)(hf * BLOCK_N), smem_desc(a_lo + 2 * k), smem_desc(b_lo + 2 * k),
-                                              idesc, (it | kh3 | k) != 0);
-                            }
+                            for (int k = 0; k < BLOCK_K / UMMA_K; k++)
+                                umma_tf32(d_tmem + (uint32_t)(hf * BLOCK_N), smem_desc(a_lo + 2 * k), smem_desc(b_lo + 2 * k),
+                                          idesc, (it | kh3 | k) != 0);
                         }
-                        umma_commit(&empty[stage]);
                     }
-                    if (++stage == stages) { stage = 0; phase ^= 1; }
+                    umma_commit(empty0 + 8 * stage);
+                    ring += ring_step;
+                    if (++stage == stages) { stage = 0; phase ^= 1; ring = ring0; }
                 }
                 if (ok && leader) umma_commit(&acc_full[acc]);
                 if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -413,37 +422,35 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     d_tmem = tmem_base + (uint32_t)(acc * acc_cols);
                     kb_in_part = 0;
                 }
-                uint64_t *ready = (THREE && !GATHER) ? &split[stage] : &full[stage];
+                const uint32_t ready = (THREE && !GATHER) ? full0 + 8 * (2 * STAGES + stage) : full0 + 8 * stage;
                 if (!(ok = mbar_wait(ready, phase, abort_flag, p.status))) break;
                 tc_fence_after();
-                const uint32_t sa = smem_u32(smem + stage * stage_bytes);
-                if (leader) {
-                    for (int c = 0; c < cbs; c++) {
-                        const uint32_t a_lo = smem_desc_lo(sa + c * A_STAGE_BYTES);
-                        const uint32_t b_lo = smem_desc_lo(sa + cbs * A_STAGE_BYTES + c * C::B_STAGE_BYTES);
+                uint32_t a_lo = ring, b_lo = ring + ((uint32_t)a_region >> 4);
+#pragma unroll 1
+                for (int c = 0; c < cbs; c++, a_lo += (uint32_t)a_slice >> 4, b_lo += C::B_STAGE_BYTES >> 4) {
 #pragma unroll
-                        for (int k = 0; k < BLOCK_K / UMMA_K; k++) {        // +32 bytes per K step = +2 in the descriptor
-                            const uint64_t da = smem_desc(a_lo + 2 * k), db = smem_desc(b_lo + 2 * k);
-                            if (THREE) {
-                                const uint64_t da_lo = smem_desc(b_lo + (C::B_STAGE_BYTES >> 4) + 2 * k);
-                                const uint64_t db_lo = smem_desc(b_lo + ((C::B_STAGE_BYTES + A_STAGE_BYTES) >> 4) + 2 * k);
-                                if (cross_cols) {
-                                    umma_tf32(x_tmem, da_lo, db, idesc, (kb | k) != 0);
-                                    umma_tf32(x_tmem, da, db_lo, idesc, 1);
-                                    umma_tf32(d_tmem, da, db, idesc, (kb_in_part | k) != 0);
-                                } else {
-                                    umma_tf32(d_tmem, da_lo, db, idesc, (kb_in_part | k) != 0);
-                                    umma_tf32(d_tmem, da, db_lo, idesc, 1);
-                                    umma_tf32(d_tmem, da, db, idesc, 1);
-                                }
+                    for (int k = 0; k < BLOCK_K / UMMA_K; k++) {        // +32 bytes per K step = +2 in the descriptor
+                        const uint64_t da = smem_desc(a_lo + 2 * k), db = smem_desc(b_lo + 2 * k);
+                        if (THREE) {
+                            const uint64_t da_lo = smem_desc(b_lo + (C::B_STAGE_BYTES >> 4) + 2 * k);
+                            const uint64_t db_lo = smem_desc(b_lo + ((C::B_STAGE_BYTES + A_STAGE_BYTES) >> 4) + 2 * k);
+                            if (cross_cols) {
+                                umma_tf32(x_tmem, da_lo, db, idesc, (kb | k) != 0);
+                                umma_tf32(x_tmem, da, db_lo, idesc, 1);
+                                umma_tf32(d_tmem, da, db, idesc, (kb_in_part | k) != 0);
                             } else {
-                                umma_tf32(d_tmem, da, db, idesc, (kb_in_part | c | k) != 0);
+                                umma_tf32(d_tmem, da_lo, db, idesc, (kb_in_part | k) != 0);
+                                umma_tf32(d_tmem, da, db_lo, idesc, 1);
+                                umma_tf32(d_tmem, da, db, idesc, 1);
                             }
+                        } else {
+                            umma_tf32(d_tmem, da, db, idesc, (kb_in_part | c | k) != 0);
                         }
                     }
-                    umma_commit(&empty[stage]);     // frees the stage once these MMAs have read it
                 }
-                if (++stage == stages) { stage = 0; phase ^= 1; }
+                umma_commit(empty0 + 8 * stage);     // frees the stage once these MMAs have read it
+                ring += ring_step;
+                if (++stage == stages) { stage = 0; phase ^= 1; ring = ring0; }
             }
             if (ok && leader) umma_commit(&acc_full[acc]);
             if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -735,6 +742,22 @@ Box choose_box(int OW, int OH, int NB, int stride, bool even, bool bn_divides, d
     return best;
 }
 
+// A box of whole 8-row groups that covers the plane with no more tiles, where there is one: its K slices can then be
+// fetched in pairs.  Rows of the box past the plane are zero-filled loads and clipped stores.
+Box whole_groups(Box box, int OW, int OH, bool even) {
+    if ((box.bw * box.bh * box.bn) % 8 == 0) return box;
+    if (OH == 1) {                      // a plain matrix: its rows lie along w
+        const int bw = (box.bw + 7) / 8 * 8;
+        return bw * box.bn <= BLOCK_M && (OW + bw - 1) / bw <= (OW + box.bw - 1) / box.bw ? Box{bw, 1, box.bn} : box;
+    }
+    const int tiles = (OH + box.bh - 1) / box.bh;
+    for (int d = 1; d < 8; d++)
+        for (int bh : {box.bh + d, box.bh - d})
+            if (bh >= 1 && box.bw * bh * box.bn <= BLOCK_M && (box.bw * bh * box.bn) % 8 == 0 && (OH + bh - 1) / bh <= tiles && !(even && (bh & 1)))
+                return Box{box.bw, bh, box.bn};
+    return box;
+}
+
 void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const cuuint64_t *dims,
             const cuuint64_t *strides_bytes, const cuuint32_t *box, const cuuint32_t *elem_strides) {
     encode_tensor_map(h, tm, base, rank, dims, strides_bytes, box, elem_strides);
@@ -861,6 +884,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
                       ((ksize_w == 3 && (g.pad_w < 0 || g.pad_w == g.pad)) || (ksize_w == 1 && g.pad_w == 0)) &&
                       kc <= 128 && a.N <= 128 && g.OW >= 16 && g.OH >= 8 &&
                       ((double)g.OW / ((g.OW + 15) / 16 * 16)) * ((double)g.OH / ((g.OH + 7) / 8 * 8)) >= 0.8;
+    const bool pairs = !col3 && !gather && !three_pass && kc % (2 * BLOCK_K) == 0;      // K slices may be fetched in pairs
     if (col3) box = Box{16, 8, 1};
     // two boxes per tile when the plane is tall enough for 16-row tiles not to waste much of it
     const int halves = (col3 && g.OH >= 16 && ((double)g.OW / ((g.OW + 15) / 16 * 16)) * ((double)g.OH / ((g.OH + 15) / 16 * 16)) >= 0.8)
@@ -874,7 +898,9 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.c_blocks = (kc + BLOCK_K - 1) / BLOCK_K;
     p.num_k_blocks = taps * p.c_blocks;
     p.kb_per_split = (p.num_k_blocks + S - 1) / S;
-    if (S > 1 && a.a_is_conv && p.c_blocks % 2 == 0) p.kb_per_split += p.kb_per_split & 1;     // (see conv_tc_split)
+    // whole pairs of K slices per split where that leaves none empty (256-wide tiles do not fetch pairs)
+    if (S > 1 && p.c_blocks % 2 == 0 && (p.kb_per_split & 1) && a.block_n_hint <= 128 && (long)(S - 1) * (p.kb_per_split + 1) < p.num_k_blocks)
+        p.kb_per_split++;
     if (S > 1 && ((long)(S - 1) * p.kb_per_split >= p.num_k_blocks || a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
         throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks and a plain epilogue");
     p.k_splits = S;
@@ -949,19 +975,33 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.kb_per_part = !promote ? p.kb_per_split : (three_pass ? 3 : 16);
     p.parts = (p.kb_per_split + p.kb_per_part - 1) / p.kb_per_part;
 
-    // two K blocks per ring stage: narrow tiles (<= 128 filters) of a convolution whose channel slices pair up, a
-    // full 128-row pixel box (the second slice's tile must start on a swizzle-pattern boundary), one K split
+    // two K blocks per ring stage: tiles of up to 128 columns whose K slices pair up, a box of whole 8-row groups (the
+    // second slice must start on a swizzle-pattern boundary), whole pairs per split.  A box of fewer than 128 rows only
+    // where a tile steps through a short K alone (64 wide, one wave, up to 16 blocks: a ResNet-50 image 504 -> 487 us); with
+    // longer K the shallower ring costs more (AlexNet b16 282 -> 291 us, ResNet-50 b64 2318 -> 2348 us)
     p.col3 = (col3 && !promote && block_n <= 128) ? 1 : 0;
     p.halves = p.col3 ? halves : 1;
     if (halves == 2 && !p.col3) throw Error(NB_ERR_UNSUPPORTED, "two-box tiles need the filter-column mode");
-    p.cbs = (!p.col3 && !three_pass && !gather && !promote && (S == 1 || p.kb_per_split % 2 == 0) && a.a_is_conv && block_n <= 128 &&
-             (kc % (2 * BLOCK_K)) == 0 && box.bw * box.bh * box.bn == BLOCK_M) ? 2 : 1;
+    const bool alone = block_n == 64 && a.a_is_conv && (long)p.m_tiles * p.n_tiles * S <= h->sm_count && p.kb_per_split <= 16;
+    if (pairs && alone) {
+        box = whole_groups(box, g.OW, g.OH, pool);
+        p.bw = box.bw; p.bh = box.bh; p.bn = box.bn;
+        p.tiles_w = (g.OW + box.bw - 1) / box.bw;
+        p.tiles_h = (g.OH + box.bh - 1) / box.bh;
+        p.m_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
+        p.tx_bytes_a = BLOCK_K * 4 * box.bw * box.bh * box.bn;
+    }
+    const int box_rows = box.bw * box.bh * box.bn;
+    p.cbs = (pairs && !promote && (S == 1 || p.kb_per_split % 2 == 0) && block_n <= 128 &&
+             (box_rows == BLOCK_M ? a.a_is_conv : alone && box_rows % 8 == 0)) ? 2 : 1;
+    p.a_slice_bytes = box_rows * 128;
+    p.a_region = A_STAGE_BYTES + (p.cbs - 1) * p.a_slice_bytes;
     {
         const int b_stage = block_n * BLOCK_K * 4;
         const int stage1 = (A_STAGE_BYTES + b_stage) * (three_pass ? 2 : 1);
         const int ring = std::min(8, (196 * 1024) / stage1) * stage1;       // bytes the variant's ring holds
         p.a_box_bytes = BLOCK_K * 4 * box.bw * (box.bh * halves + 2);
-        p.stage_bytes = p.col3 ? p.a_box_bytes + 3 * b_stage : stage1 * p.cbs;
+        p.stage_bytes = p.col3 ? p.a_box_bytes + 3 * b_stage : (p.cbs == 2 ? p.a_region + 2 * b_stage : stage1);
         p.stages = std::min(8, ring / p.stage_bytes);
         // a second staging buffer per epilogue group in what the ring leaves unused; a one-column filter (row windows:
         // one stage per tile, bound by its epilogue) gives up its third stage for it
