@@ -24,7 +24,7 @@
 //   warp 0      TMA producer (one elected lane)
 //   warp 1      TMEM allocation + MMA issue (one elected lane)
 //   warps 2-9   epilogue, two groups of four (TMEM -> registers -> shared-memory slab -> TMA store)
-//   warps 10-13 three-pass mode: split each A tile into hi/lo TF32 terms; gather mode: build the
+//   warps 10-13 three-pass mode: split each A tile into hi/lo TF32 terms in tensor memory; gather mode: build the
 //               A tile in shared memory from a strided tensor (3-channel input layers)
 //
 // Every wait is bounded: a wait that runs out sets the CTA's abort flag and the
@@ -155,10 +155,19 @@ struct TileIter {
     }
 };
 
-template <int BLOCK_N, bool THREE>
+// 3xTF32 multiplies every K block three times, and with both operands in shared memory the port is the bound: at N = 128
+// twelve MMAs read 96 KB, the splitter reads 16 KB and writes 32, TMA writes 48: 1536 cycles of port per 768 of MMAs (1450
+// measured).  So the splitter writes the two terms of A to tensor memory instead (TS): the MMAs then read only B from
+// shared memory, 48 + 16 + 48 KB.  Tensor memory holds two accumulators, the cross terms of one tile (two at N = 64) and
+// A_BUFS pairs of A terms, 64 columns each.
+template <int BLOCK_N, bool THREE, bool GATHER>
 struct Cfg {
+    static constexpr bool TS = THREE && !GATHER;
+    static constexpr int A_BUFS = BLOCK_N == 64 ? 4 : 2, X_BUFS = TS && BLOCK_N != 64 ? 1 : 2;
+    static constexpr int A_COL = (2 + X_BUFS) * BLOCK_N;
     static constexpr int B_STAGE_BYTES = BLOCK_N * BLOCK_K * 4;
-    static constexpr int STAGE_BYTES = (A_STAGE_BYTES + B_STAGE_BYTES) * (THREE ? 2 : 1);
+    static constexpr int STAGE_BYTES = TS ? A_STAGE_BYTES + 2 * B_STAGE_BYTES : (A_STAGE_BYTES + B_STAGE_BYTES) * (THREE ? 2 : 1);
+    static constexpr int B_LO_OFFSET = TS ? B_STAGE_BYTES : B_STAGE_BYTES + A_STAGE_BYTES;      // from B's high-order terms
     static constexpr int STAGES = (196 * 1024) / STAGE_BYTES < 8 ? (196 * 1024) / STAGE_BYTES : 8;
     static constexpr int TMEM_COLS = 2 * BLOCK_N;
     static constexpr int OUT_STAGE_BYTES = BLOCK_M * 32 * 4;     // one 128 x 32 output slab
@@ -174,11 +183,11 @@ struct Cfg {
 template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
 __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
-    using C = Cfg<BLOCK_N, THREE>;
+    using C = Cfg<BLOCK_N, THREE, GATHER>;
     constexpr int STAGES = C::STAGES;                   // barrier slots; the ring uses the first p.stages of them
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    // per stage: [A | B | (A_lo | B_lo)], or [A0 | A1 | B0 | B1] with two K blocks per stage
+    // per stage: [A | B], 3xTF32 [A | B | B_lo] (gathered: [A | B | A_lo | B_lo]), or [A0 | A1 | B0 | B1] with two K blocks per stage
     const int cbs = THREE ? 1 : p.cbs;
     const int stages = p.stages;
     const int a_region = (THREE || cbs == 1) ? A_STAGE_BYTES : p.a_region, a_slice = (THREE || cbs == 1) ? A_STAGE_BYTES : p.a_slice_bytes;
@@ -191,7 +200,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
     // Only the hi*hi chain is then promoted, and a K block adds 4 MMAs to it instead of 12: a third of the promotions
     // for the same chain length.
     const bool cross_cols = THREE && p.parts > 1;
-    const uint32_t tmem_cols = (uint32_t)(C::TMEM_COLS * (THREE ? 2 : halves));
+    const uint32_t tmem_cols = C::TS ? 512u : (uint32_t)(C::TMEM_COLS * (THREE ? 2 : halves));
     uint8_t *out_stage = smem + STAGES * C::STAGE_BYTES;      // 2 x [128 rows][32 floats], 128B-swizzled
     uint64_t *bars = (uint64_t *)(out_stage + 2 * C::OUT_STAGE_BYTES);
     uint64_t *full = bars;                    // TMA -> (splitter or MMA)
@@ -199,7 +208,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
     uint64_t *split = bars + 2 * STAGES;      // splitter -> MMA (three-pass only)
     uint64_t *acc_full = bars + 3 * STAGES;   // MMA -> epilogue   [2]
     uint64_t *acc_empty = acc_full + 2;       // epilogue -> MMA   [2]
-    uint32_t *tmem_slot = (uint32_t *)(acc_empty + 2);
+    uint64_t *x_empty = acc_empty + 2;        // epilogue -> MMA: the cross terms have been read (where there is one set)
+    uint32_t *tmem_slot = (uint32_t *)(x_empty + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
     // per epilogue group: scale [BLOCK_N / 2] then shift [BLOCK_N / 2] of the columns of its slabs, if the alignment of
     // the dynamic shared memory left room behind the barriers (it does when the base is 1024-byte aligned already)
@@ -224,6 +234,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
             mbar_init(&acc_full[a], 1);
             mbar_init(&acc_empty[a], 256);
         }
+        mbar_init(x_empty, 256);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -290,7 +301,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 } else {
                     tma_load_3d(sb, &p.tm_b, &full[i], cb * BLOCK_K, ti.n_tile * BLOCK_N, tap);
                     if (THREE)
-                        tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, &full[i], cb * BLOCK_K, ti.n_tile * BLOCK_N, tap);
+                        tma_load_3d(sb + C::B_LO_OFFSET, &p.tm_b_lo, &full[i], cb * BLOCK_K, ti.n_tile * BLOCK_N, tap);
                 }
             }
         }
@@ -340,7 +351,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     if (!b_there) {
                         tma_load_3d(sb, &p.tm_b, bar, cb * BLOCK_K, n_tile * BLOCK_N, tap);
                         if (THREE)
-                            tma_load_3d(sb + C::B_STAGE_BYTES + A_STAGE_BYTES, &p.tm_b_lo, bar, cb * BLOCK_K,
+                            tma_load_3d(sb + C::B_LO_OFFSET, &p.tm_b_lo, bar, cb * BLOCK_K,
                                         n_tile * BLOCK_N, tap);
                     }
                 }
@@ -378,6 +389,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         const uint32_t full0 = smem_u32(full), empty0 = smem_u32(empty), ring0 = smem_desc_lo(smem_u32(smem));
         const uint32_t ring_step = (uint32_t)stage_bytes >> 4;
         uint32_t ring = ring0;          // the current stage's descriptor word
+        int a_buf = 0;                  // tensor-memory buffer of the next K block's A terms
+        uint32_t x_phase = 0;
         grid_dependency_wait();         // the bounded waits below must not count the kernels in front
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             if (!(ok = mbar_wait(&acc_empty[acc], acc_phase ^ 1, abort_flag, p.status))) break;
@@ -410,8 +423,13 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
             }
             const int ksplit = p.k_splits > 1 ? tile % p.k_splits : 0;
             const int tile_kb = min(p.kb_per_split, p.num_k_blocks - ksplit * p.kb_per_split);
-            const uint32_t x_tmem = tmem_base + (uint32_t)(2 * BLOCK_N + tile_parity * BLOCK_N);    // cross terms of this tile
+            const uint32_t x_tmem = tmem_base + (uint32_t)(2 * BLOCK_N + (C::X_BUFS == 2 ? tile_parity : 0) * BLOCK_N);    // cross terms of this tile
             tile_parity ^= 1;
+            if (C::X_BUFS == 1 && cross_cols) {
+                if (!(ok = mbar_wait(x_empty, x_phase ^ 1, abort_flag, p.status))) break;
+                x_phase ^= 1;
+                tc_fence_after();
+            }
             for (int kb = 0; kb < tile_kb; kb += cbs, kb_in_part += cbs) {
                 if (kb_in_part == p.kb_per_part) {
                     // hand this partial sum to the epilogue warps and restart in the other accumulator
@@ -431,9 +449,16 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
 #pragma unroll
                     for (int k = 0; k < BLOCK_K / UMMA_K; k++) {        // +32 bytes per K step = +2 in the descriptor
                         const uint64_t da = smem_desc(a_lo + 2 * k), db = smem_desc(b_lo + 2 * k);
-                        if (THREE) {
+                        if constexpr (C::TS) {
+                            const uint64_t db_lo = smem_desc(b_lo + (C::B_LO_OFFSET >> 4) + 2 * k);
+                            const uint32_t ta = tmem_base + (uint32_t)(C::A_COL + a_buf * 64 + k * UMMA_K), ta_lo = ta + 32;
+                            const uint32_t xd = cross_cols ? x_tmem : d_tmem;
+                            umma_tf32_ts(xd, ta_lo, db, idesc, ((cross_cols ? kb : kb_in_part) | k) != 0);
+                            umma_tf32_ts(xd, ta, db_lo, idesc, 1);
+                            umma_tf32_ts(d_tmem, ta, db, idesc, cross_cols ? (kb_in_part | k) != 0 : 1);
+                        } else if (THREE) {
                             const uint64_t da_lo = smem_desc(b_lo + (C::B_STAGE_BYTES >> 4) + 2 * k);
-                            const uint64_t db_lo = smem_desc(b_lo + ((C::B_STAGE_BYTES + A_STAGE_BYTES) >> 4) + 2 * k);
+                            const uint64_t db_lo = smem_desc(b_lo + (C::B_LO_OFFSET >> 4) + 2 * k);
                             if (cross_cols) {
                                 umma_tf32(x_tmem, da_lo, db, idesc, (kb | k) != 0);
                                 umma_tf32(x_tmem, da, db_lo, idesc, 1);
@@ -448,7 +473,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                         }
                     }
                 }
-                umma_commit(empty0 + 8 * stage);     // frees the stage once these MMAs have read it
+                umma_commit(empty0 + 8 * stage);     // frees the stage (and A's buffer) once these MMAs have read it
+                if (C::TS && ++a_buf == C::A_BUFS) a_buf = 0;
                 ring += ring_step;
                 if (++stage == stages) { stage = 0; phase ^= 1; ring = ring0; }
             }
@@ -557,7 +583,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 uint32_t sum[CH][32];
                 const int tile_kb = min(p.kb_per_split, p.num_k_blocks - split * p.kb_per_split);
                 const int parts = (tile_kb + p.kb_per_part - 1) / p.kb_per_part;
-                const uint32_t x_cols = (uint32_t)(2 * BLOCK_N + epi_tile_parity * BLOCK_N);
+                const uint32_t x_cols = (uint32_t)(2 * BLOCK_N + (C::X_BUFS == 2 ? epi_tile_parity : 0) * BLOCK_N);
                 epi_tile_parity ^= 1;
                 for (int part = 0; part < parts && ok; part++) {
                     if (!(ok = epilogue_all(mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status), bar_id))) break;
@@ -588,6 +614,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     }
                     tc_fence_before();
                     mbar_arrive(&acc_empty[acc]);
+                    if (C::X_BUFS == 1 && cross_cols && part == parts - 1) mbar_arrive(x_empty);
                     if (++acc == 2) { acc = 0; acc_phase ^= 1; }
                 }
                 if (!ok) break;
@@ -665,36 +692,50 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 if (++stage == STAGES) { stage = 0; phase ^= 1; }
             }
         }
-    } else if (THREE) {
+    } else if constexpr (THREE) {
         // ---------------------------------------------- hi/lo operand splitter
         // hi = RN_tf32(x), lo = RN_tf32(x - hi), the same split the weights get at load: both terms are exact TF32
         // values, so the tensor core's truncation of its operands changes nothing and the split has no bias.
-        // Element positions are kept, so the swizzled tile layout written by TMA is preserved.
-        const int t = threadIdx.x - 320;        // 0..127
+        // A thread owns a row: it reads the row's eight 16-byte chunks at their swizzled places (eight rows of a read fall into
+        // different banks) and writes the two terms as 32 columns each of its tensor-memory lane.
+        const int q = warp & 3, r = q * 32 + lane;      // TMEM lane quarter this warp may write
         grid_dependency_wait();
-        int stage = 0;
+        int stage = 0, buf = 0;
         uint32_t phase = 0;
+        int back = stages - C::A_BUFS;          // stage and phase of the K block A_BUFS before this one
+        uint32_t back_phase = 1;
+        long seen = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             const int tile_kb = min(p.kb_per_split, p.num_k_blocks - (tile % p.k_splits) * p.kb_per_split);
-            for (int kb = 0; kb < tile_kb; kb++) {
-                if (!(ok = mbar_wait(&full[stage], phase, abort_flag, p.status))) break;
-                float4 *a = reinterpret_cast<float4 *>(smem + stage * C::STAGE_BYTES);
-                float4 *a_lo = reinterpret_cast<float4 *>(smem + stage * C::STAGE_BYTES + A_STAGE_BYTES + C::B_STAGE_BYTES);
+            for (int kb = 0; kb < tile_kb; kb++, seen++) {
+                // the buffer is free when the MMAs of the K block that used it last have retired (they also freed its stage)
+                bool mine = mbar_wait(&full[stage], phase, abort_flag, p.status);
+                if (seen >= C::A_BUFS) mine = mine && mbar_wait(&empty[back], back_phase, abort_flag, p.status);
+                if (!(ok = __all_sync(0xffffffffu, mine))) break;
+                tc_fence_after();
+                const float4 *a = reinterpret_cast<const float4 *>(smem + stage * C::STAGE_BYTES + r * 128);
+                uint32_t hi[32], lo[32];
 #pragma unroll
-                for (int i = 0; i < A_STAGE_BYTES / 16 / 128; i++) {
-                    float4 x = a[i * 128 + t], h, l;
-                    h.x = round_tf32(x.x); l.x = round_tf32(x.x - h.x);
-                    h.y = round_tf32(x.y); l.y = round_tf32(x.y - h.y);
-                    h.z = round_tf32(x.z); l.z = round_tf32(x.z - h.z);
-                    h.w = round_tf32(x.w); l.w = round_tf32(x.w - h.w);
-                    a[i * 128 + t] = h;
-                    a_lo[i * 128 + t] = l;
+                for (int j = 0; j < 8; j++) {
+                    const float4 x = a[j ^ (r & 7)];
+                    const float v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const float h = round_tf32(v[e]);
+                        hi[4 * j + e] = __float_as_uint(h);
+                        lo[4 * j + e] = __float_as_uint(round_tf32(v[e] - h));
+                    }
                 }
-                // make the generic-proxy writes visible to the tensor core (async proxy)
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(C::A_COL + buf * 64);
+                tmem_st_32x32(ta, hi);
+                tmem_st_32x32(ta + 32, lo);
+                tmem_st_wait();
+                tc_fence_before();
                 mbar_arrive(&split[stage]);
-                if (++stage == STAGES) { stage = 0; phase ^= 1; }
+                if (++stage == stages) { stage = 0; phase ^= 1; }
+                if (++back == stages) { back = 0; back_phase ^= 1; }
+                if (++buf == C::A_BUFS) buf = 0;
             }
         }
     }
@@ -766,7 +807,7 @@ void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const c
 struct Variant { const void *kernel; int smem; };      // takes a TcParams, or a TcGatherParams
 
 template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
-Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER>, Cfg<BLOCK_N, THREE>::SMEM_BYTES}; }
+Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
 
 // index: [gather][three][promote][block_n: 0 = 64, 1 = 128, 2 = 256]; absent combinations are null
 const Variant VARIANTS[2][2][2][3] = {
@@ -998,7 +1039,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.a_region = A_STAGE_BYTES + (p.cbs - 1) * p.a_slice_bytes;
     {
         const int b_stage = block_n * BLOCK_K * 4;
-        const int stage1 = (A_STAGE_BYTES + b_stage) * (three_pass ? 2 : 1);
+        const int stage1 = three_pass && !gather ? A_STAGE_BYTES + 2 * b_stage : (A_STAGE_BYTES + b_stage) * (three_pass ? 2 : 1);
         const int ring = std::min(8, (196 * 1024) / stage1) * stage1;       // bytes the variant's ring holds
         p.a_box_bytes = BLOCK_K * 4 * box.bw * (box.bh * halves + 2);
         p.stage_bytes = p.col3 ? p.a_box_bytes + 3 * b_stage : (p.cbs == 2 ? p.a_region + 2 * b_stage : stage1);
