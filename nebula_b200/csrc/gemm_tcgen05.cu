@@ -694,8 +694,11 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         }
     } else if constexpr (THREE) {
         // ---------------------------------------------- hi/lo operand splitter
-        // hi = RN_tf32(x), lo = RN_tf32(x - hi), the same split the weights get at load: both terms are exact TF32
-        // values, so the tensor core's truncation of its operands changes nothing and the split has no bias.
+        // hi = RN_tf32(x) in integer arithmetic (cvt.rna runs at a quarter of that rate and was the pace of this kernel:
+        // VGG-16 b8 1951 us with two of them per value, 1871 with one, 1756 with none); lo = x - hi, exact.  With ulp the
+        // spacing of x, lo is a whole number of ulp up to 2^12, so its 11 leading bits lose the last bit of some odd numbers
+        // above 2^11: one ulp(x), whether the tensor core's truncation drops it or a rounding moves that tie, and lo's
+        // sign does not depend on x, so there is no bias.  A NaN whose payload overflows the addition survives in lo.
         // A thread owns a row: it reads the row's eight 16-byte chunks at their swizzled places (eight rows of a read fall into
         // different banks) and writes the two terms as 32 columns each of its tensor-memory lane.
         const int q = warp & 3, r = q * 32 + lane;      // TMEM lane quarter this warp may write
@@ -709,11 +712,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
             const int tile_kb = min(p.kb_per_split, p.num_k_blocks - (tile % p.k_splits) * p.kb_per_split);
             for (int kb = 0; kb < tile_kb; kb++, seen++) {
-                // the buffer is free when the MMAs of the K block that used it last have retired (they also freed its stage)
-                bool mine = mbar_wait(&full[stage], phase, abort_flag, p.status);
-                if (seen >= C::A_BUFS) mine = mine && mbar_wait(&empty[back], back_phase, abort_flag, p.status);
-                if (!(ok = __all_sync(0xffffffffu, mine))) break;
-                tc_fence_after();
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, p.status)))) break;
                 const float4 *a = reinterpret_cast<const float4 *>(smem + stage * C::STAGE_BYTES + r * 128);
                 uint32_t hi[32], lo[32];
 #pragma unroll
@@ -722,11 +721,13 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                     const float v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        const float h = round_tf32(v[e]);
-                        hi[4 * j + e] = __float_as_uint(h);
-                        lo[4 * j + e] = __float_as_uint(round_tf32(v[e] - h));
+                        hi[4 * j + e] = (__float_as_uint(v[e]) + 0x1000u) & 0xFFFFE000u;
+                        lo[4 * j + e] = __float_as_uint(v[e] - __uint_as_float(hi[4 * j + e]));
                     }
                 }
+                // the buffer is free when the MMAs of the K block that used it last have retired (they also freed its stage)
+                if (seen >= C::A_BUFS && !(ok = __all_sync(0xffffffffu, mbar_wait(&empty[back], back_phase, abort_flag, p.status)))) break;
+                tc_fence_after();
                 const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(C::A_COL + buf * 64);
                 tmem_st_32x32(ta, hi);
                 tmem_st_32x32(ta + 32, lo);
