@@ -64,6 +64,7 @@ struct nb_handle_s {
     int *d_status = nullptr;            // device status word (nb::DEV_*)
     unsigned int *d_grid_sync = nullptr; // arrival counter of the persistent LSTM kernel's grid barrier
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
+    bool recurrent_ready = false;       // recurrent_cluster_prepare_device has run
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
     nb_encode_tiled_fn encode_tiled = nullptr;
     nb_get_address_range_fn get_address_range = nullptr;   // cuMemGetAddressRange: the allocation a pointer lies in

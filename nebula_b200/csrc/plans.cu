@@ -491,6 +491,7 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
 LstmPlan::LstmPlan(nb_handle_s *hh, const nb_lstm_desc_t &desc) : nb_plan_s(NB_PLAN_LSTM, hh), d(desc) {
     NB_REQUIRE(d.time_steps > 0 && d.batch > 0 && d.inputs > 0 && d.hidden > 0, "lstm: non-positive extent");
     NB_REQUIRE(d.activation > NB_ACT_UNDEFINED && d.activation < NB_ACT_COUNT, "lstm: undefined activation");
+    recurrent_cluster_prepare_device(h);
 }
 
 size_t LstmPlan::weight_count() const {
@@ -669,6 +670,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
 RnnPlan::RnnPlan(nb_handle_s *hh, const nb_rnn_desc_t &desc) : nb_plan_s(NB_PLAN_RNN, hh), d(desc) {
     NB_REQUIRE(d.time_steps > 0 && d.batch > 0 && d.inputs > 0 && d.hidden > 0, "rnn: non-positive extent");
     NB_REQUIRE(d.activation > NB_ACT_UNDEFINED && d.activation < NB_ACT_COUNT, "rnn: undefined activation");
+    recurrent_cluster_prepare_device(h);
     // the three gates are connected layers built from the same section (rnn_layer.cc:47-54)
     nb_fc_desc_t g{};
     g.batch = d.batch; g.outputs = d.hidden; g.batch_normalize = d.batch_normalize; g.activation = d.activation;

@@ -265,7 +265,10 @@ bool choose(const nb_handle_s *h, int gates, int H, int B, Shape *best) {
 
 }  // namespace
 
+// Once per handle, when its first recurrent plan is created (the queries cost a handle that has none a millisecond).
 void recurrent_cluster_prepare_device(nb_handle_s *h) {
+    if (h->cc_major != 10 || h->recurrent_ready) return;
+    h->recurrent_ready = true;
     for (auto &kind : KERNELS)
         for (RecKernel k : kind) {
             NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
