@@ -221,7 +221,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
     const int lane = threadIdx.x & 31;
     const int total_tiles = p.m_tiles * p.n_tiles * p.k_splits;
 
-    grid_dependents_start();
+    if (!GATHER) grid_dependents_start();       // (the gather variants run in stream order on both sides: gemm_tc)
     if (threadIdx.x == 0) {
         if (!GATHER) prefetch_tensor_map(&p.tm_a);
         prefetch_tensor_map(&p.tm_b);
@@ -826,6 +826,7 @@ const Variant VARIANTS[2][2][2][3] = {
 struct TcLaunch : LaunchRecord {
     TcGatherParams p;       // the other variants take the TcParams it starts with
     Variant v;
+    bool gather = false;
     int grid = 1, threads = 320;
     double flops = 0;
     std::string desc;       // names the launch in error messages
@@ -983,7 +984,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         throw Error(NB_ERR_INVALID_ARG, "GEMM without an output tensor");
     }
     p.status = h->d_status;
-    p.b_static = a.b_static ? 1 : 0;
+    p.b_static = a.b_static && !gather ? 1 : 0;
 
     // tile width in filters: widest tile that still gives every SM work
     // Promoted accumulation: always for 3xTF32 (its point is fp32-level agreement); in TF32 mode only for
@@ -1174,6 +1175,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     const int tiles = p.m_tiles * p.n_tiles * p.k_splits;
     L->grid = std::max(1, std::min(tiles, h->sm_count));
     L->threads = (three_pass || gather) ? 448 : 320;
+    L->gather = gather;
     L->flops = a.algo_flops > 0 ? a.algo_flops : 2.0 * (double)a.M * a.N * a.Kc * taps;
     L->desc = " [M=" + std::to_string(a.M) + " N=" + std::to_string(a.N) + " K=" + std::to_string(a.Kc) + " taps=" +
               std::to_string(taps) + " stride=" + std::to_string(g.stride) + " out=" + std::to_string(g.OW) + "x" +
@@ -1223,7 +1225,11 @@ void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass) {
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    // The gather variants are not launched ahead.  Launched ahead, every second of two queued calls (30 channels, 3x3, 8
+    // images of 33 x 33: 9 K blocks, 69 CTAs) left about ten CTAs whose accumulators never completed, so that the wait for them
+    // ran out and the output kept the call's before; alone the same call is right.  They are the only launches with more than
+    // 4096 bytes of parameters (TcGatherParams: 4160), the one thing that sets them apart; the cause is not proven.
+    cfg.numAttrs = L.gather ? 0 : 1;
     void *args[1] = {const_cast<TcGatherParams *>(&L.p)};
     (void)cudaLaunchKernelExC(&cfg, L.v.kernel, args);
     try {
