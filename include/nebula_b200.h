@@ -82,7 +82,7 @@ typedef struct {
     unsigned long long tc_launches;
     double simt_ms, simt_flops;
     unsigned long long simt_launches;
-    double halo_ms, halo_flops;             /* the 3x3 halo convolution kernel (few input channels) */
+    double halo_ms, halo_flops;             /* always 0: the kernel these counted is gone */
     unsigned long long halo_launches;
 } nb_profile_t;
 int nb_profile_begin(nb_handle_t handle);

@@ -108,7 +108,6 @@ int nb_create(int device_id, nb_handle_t *handle) {
         gemm_tc_prepare_device();
         gemm_simt_prepare_device();
         lstm_persistent_prepare_device();
-        conv_halo_prepare_device();
         elementwise_prepare_device();
     });
     if (rc != NB_OK) {
@@ -193,7 +192,6 @@ int nb_profile_end(nb_handle_t h, nb_profile_t *r) {
             float ms = 0;
             NB_CHECK_CUDA(cudaEventElapsedTime(&ms, t.start, t.stop));
             if (t.kind == 0) { r->tc_ms += ms; r->tc_flops += t.flops; r->tc_launches++; }
-            else if (t.kind == 2) { r->halo_ms += ms; r->halo_flops += t.flops; r->halo_launches++; }
             else { r->simt_ms += ms; r->simt_flops += t.flops; r->simt_launches++; }
             h->event_pool.push_back(t.start); h->event_pool.push_back(t.stop);
         }

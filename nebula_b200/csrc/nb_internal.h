@@ -225,9 +225,6 @@ bool gemm_tc_supported(const nb_handle_s *h, const GemmArgs &a);
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
 // How many K slices (GemmArgs::split_k) an NHWC convolution should be cut into on the tensor cores; 1: none.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
-// 3x3 stride-1 convolutions with 32..128 input channels: one halo load per channel slice serves all nine taps.
-bool conv_halo_supported(const nb_handle_s *h, const GemmArgs &a);
-void conv_halo_tc(nb_handle_s *h, const GemmArgs &a);
 // CUDA-core fp32 path: any extents, strides and alignments.
 void gemm_simt(nb_handle_s *h, const GemmArgs &a);
 // Dispatch on the handle's math mode.
@@ -287,7 +284,7 @@ void launch_sgemm(nb_handle_s *h, bool ta, bool tb, int M, int N, int K, float a
                   const float *B, int ldb, float beta, float *C, int ldc);
 
 // Brackets one contraction launch with events while profiling is on
-// (kind 0 = generic tensor-core kernel, 1 = CUDA-core kernel, 2 = 3x3 halo tensor-core kernel).
+// (kind 0 = tensor-core kernel, 1 = CUDA-core kernel).
 struct ProfileScope {
     nb_handle_s *h;
     nb_handle_s::Timed t;
@@ -380,7 +377,6 @@ struct RecurrentArgs {
 void recurrent_cluster_prepare_device(nb_handle_s *h);
 bool recurrent_cluster_supported(const nb_handle_s *h, int gates, int H, int B);
 void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a);
-void conv_halo_prepare_device();
 void elementwise_prepare_device();
 
 }  // namespace nb

@@ -314,22 +314,8 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         w.ensure_split(h);
         a.b = w.hi.p;
         a.b_lo = w.lo.p;
-        // few input channels: the generic kernel would re-load the activations once per tap from L2
-        // The halo kernel is routed off: a kernel launched right behind it has faulted (illegal address) in a few
-        // runs out of many and the cause is not known.  NEBULA_B200_HALO=1 turns it on for investigation only.
-        static const bool halo_on = [] {
-            const char *v = std::getenv("NEBULA_B200_HALO");
-            return v && *v == '1';
-        }();
-        bool halo = halo_on && pth == PATH_TC && !a.y_nchw && (d.channels <= 64 || (d.channels <= 128 && d.filters <= 128)) &&
-                    conv_halo_supported(h, a);
-        if (halo) {
-            const int bh = OH >= 16 ? 16 : 8;
-            const double eff = ((double)OW / ((OW + 13) / 14 * 14)) * ((double)OH / ((OH + bh - 1) / bh * bh));
-            halo = eff >= 0.6;
-        }
         const int S = splits(o);
-        if (S > 1 && !halo) {
+        if (S > 1) {
             GemmArgs sa = a;
             sa.split_k = S;
             sa.scale = sa.shift = sa.addend = nullptr; sa.res_stride = 0; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;
@@ -344,8 +330,9 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
                 r.res_c = a.res_c; r.res_h = a.res_h; r.res_w = a.res_w;
             }
             launch_splitk_reduce(h, r);
-        } else if (halo) conv_halo_tc(h, a);
-        else gemm_tc(h, a, pth == PATH_TC3);
+        } else {
+            gemm_tc(h, a, pth == PATH_TC3);
+        }
     }
     if (!o.y_nhwc && yo != y) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
 }

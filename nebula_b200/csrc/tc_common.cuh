@@ -1,6 +1,6 @@
 // Shared device code of the tcgen05 kernels: PTX wrappers (mbarrier, TMA, tcgen05),
-// descriptor builders, and the fused epilogue that both the generic GEMM kernel and
-// the 3x3 halo convolution kernel run on every 128-row x 32-column slab.
+// descriptor builders, and the fused epilogue that the contraction kernel runs on
+// every 128-row x 32-column slab.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -19,7 +19,7 @@ constexpr int A_STAGE_BYTES = BLOCK_M * BLOCK_K * 4;   // 16 KiB
 constexpr long long WAIT_LIMIT_CYCLES = 4000000000LL;  // ~2 s at 2 GHz
 
 
-// What the epilogue needs to know, common to both kernels.
+// What the epilogue needs to know.
 struct EpiParams {
     const float *scale, *shift, *addend;    // scale/shift readable up to the next multiple of 32 columns
     long ld_addend;
@@ -148,12 +148,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *tm,
         : "memory");
 }
 __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *tm, uint64_t *bar, int c0, int c1, int c2, int c3, int c4) { tma_load_5d(smem_u32(dst), tm, smem_u32(bar), c0, c1, c2, c3, c4); }
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tm, uint64_t *bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(smem_u32(dst)), "l"(tm), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
-        : "memory");
-}
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *tm, uint32_t bar, int c0, int c1, int c2) {
     asm volatile(
         "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -199,22 +193,10 @@ __device__ __forceinline__ bool epilogue_all(bool pred, int id) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows 128 B
-// apart, 8-row groups 1024 B apart (bits: start>>4 [0,14), LBO>>4 [16,30),
-// SBO>>4 [32,46), version=1 [46,48), layout=SWIZZLE_128B(2) [61,64)).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-    d |= (uint64_t)1 << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-// The same descriptor split in halves, for the MMA issue loop: the upper word is a constant, the lower
-// word is (start >> 4) | LBO, so stepping the start address by b bytes is `lo += b >> 4` (shared-memory
-// addresses stay below 2^18, so the 14-bit field never carries).
+// Shared-memory matrix descriptor: K-major operand, 128-byte swizzle, rows 128 B apart, 8-row groups 1024 B apart (bits:
+// start>>4 [0,14), LBO>>4 [16,30), SBO>>4 [32,46), version=1 [46,48), layout=SWIZZLE_128B(2) [61,64)), in halves for the
+// MMA issue loop: the upper word is a constant, the lower word is (start >> 4) | LBO, so stepping the start address by b
+// bytes is `lo += b >> 4` (shared-memory addresses stay below 2^18, so the 14-bit field never carries).
 constexpr uint32_t SMEM_DESC_HI = (uint32_t)(1024 >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t smem_desc_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFF) | (1u << 16); }
 __device__ __forceinline__ uint64_t smem_desc(uint32_t lo) { return ((uint64_t)SMEM_DESC_HI << 32) | lo; }
