@@ -785,18 +785,22 @@ Box choose_box(int OW, int OH, int NB, int stride, bool even, bool bn_divides, d
 }
 
 // A box of whole 8-row groups that covers the plane with no more tiles, where there is one: its K slices can then be
-// fetched in pairs.  Rows of the box past the plane are zero-filled loads and clipped stores.
-Box whole_groups(Box box, int OW, int OH, bool even) {
+// fetched in pairs.  Rows of the box past the plane are zero-filled loads and clipped stores.  The limits are choose_box's: a
+// TMA box traverses at most 256 elements per dimension, and what it reads behind the tensor stays under 4 MB.
+Box whole_groups(Box box, int OW, int OH, int stride, bool even, double row_bytes) {
     if ((box.bw * box.bh * box.bn) % 8 == 0) return box;
+    const int max_dim = 256 / std::max(1, stride);
     if (OH == 1) {                      // a plain matrix: its rows lie along w
         const int bw = (box.bw + 7) / 8 * 8;
-        return bw * box.bn <= BLOCK_M && (OW + bw - 1) / bw <= (OW + box.bw - 1) / box.bw ? Box{bw, 1, box.bn} : box;
+        return bw <= max_dim && bw * box.bn <= BLOCK_M && (OW + bw - 1) / bw <= (OW + box.bw - 1) / box.bw ? Box{bw, 1, box.bn} : box;
     }
     const int tiles = (OH + box.bh - 1) / box.bh;
     for (int d = 1; d < 8; d++)
-        for (int bh : {box.bh + d, box.bh - d})
-            if (bh >= 1 && box.bw * bh * box.bn <= BLOCK_M && (box.bw * bh * box.bn) % 8 == 0 && (OH + bh - 1) / bh <= tiles && !(even && (bh & 1)))
-                return Box{box.bw, bh, box.bn};
+        for (int bh : {box.bh + d, box.bh - d}) {
+            if (bh < 1 || bh > max_dim || (even && (bh & 1)) || (box.bw * bh * box.bn) % 8 || box.bw * bh * box.bn > BLOCK_M) continue;
+            const int t = (OH + bh - 1) / bh;
+            if (t <= tiles && (double)(t * bh - OH) * stride * row_bytes <= 4e6) return Box{box.bw, bh, box.bn};
+        }
     return box;
 }
 
@@ -1027,7 +1031,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     if (halves == 2 && !p.col3) throw Error(NB_ERR_UNSUPPORTED, "two-box tiles need the filter-column mode");
     const bool alone = block_n == 64 && a.a_is_conv && (long)p.m_tiles * p.n_tiles * S <= h->sm_count && p.kb_per_split <= 16;
     if (pairs && alone) {
-        box = whole_groups(box, g.OW, g.OH, pool);
+        box = whole_groups(box, g.OW, g.OH, g.stride, pool, (double)g.sh * 4.0);
         p.bw = box.bw; p.bh = box.bh; p.bn = box.bn;
         p.tiles_w = (g.OW + box.bw - 1) / box.bw;
         p.tiles_h = (g.OH + box.bh - 1) / box.bh;

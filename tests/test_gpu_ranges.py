@@ -1,0 +1,33 @@
+"""Calls at the edges of what the routes accept, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from tests.util import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+
+
+# (OH, OW, stride, k): planes one to three pixels thin whose pixel box, grown to whole 8-row groups, would traverse more than
+# the 256 elements a TMA box may (85 -> 88 at stride 3, 51 -> 56 at stride 5, 36 -> 40 at stride 7 ...)
+@pytest.mark.parametrize("case", [(1, 85, 3, 1), (51, 1, 5, 1), (52, 2, 5, 1), (1, 42, 6, 1), (1, 36, 7, 1), (36, 3, 7, 1), (36, 3, 7, 3)], ids=str)
+def test_thin_strided_planes(handle, case):
+    from nebula_b200 import api
+    from oracle import oracle as O
+    OH, OW, s, k = case
+    C, F, H, W = 64, 48, (OH - 1) * s + k, (OW - 1) * s + k
+    rng = np.random.default_rng(OH * OW)
+    x = rng.standard_normal((1, C, H, W), dtype=np.float32)
+    w = (rng.standard_normal((F, C, k, k)) * np.sqrt(2.0 / (C * k * k))).astype(np.float32)
+    b = (0.1 * rng.standard_normal(F)).astype(np.float32)
+    handle.set_math("tf32")
+    plan = api.Conv2d(handle, 1, C, H, W, F, k, s, 0, False, "relu", api.LAYOUT_NHWC)
+    plan.set_weights(w, b)
+    y = plan.forward(_t(x.transpose(0, 2, 3, 1))).cpu().numpy().transpose(0, 3, 1, 2)
+    handle.synchronize()
+    plan.close()
+    assert_close(y, O.conv_forward(x, w, b, k, s, 0, "relu"), "tf32", f"{case}")
