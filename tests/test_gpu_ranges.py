@@ -31,3 +31,32 @@ def test_thin_strided_planes(handle, case):
     handle.synchronize()
     plan.close()
     assert_close(y, O.conv_forward(x, w, b, k, s, 0, "relu"), "tf32", f"{case}")
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+def test_folded_shortcut_of_a_split_layer_to_any_address(handle, mode):
+    """Few tiles and a long contraction (cut along K where the output allows), the output 4 bytes off a 16-byte boundary."""
+    import ctypes
+    import torch
+    from nebula_b200 import api
+    from oracle import oracle as O
+    rng = np.random.default_rng(2)
+    x = rng.standard_normal((1, 256, 7, 7), dtype=np.float32)
+    w = (rng.standard_normal((96, 256, 3, 3)) * np.sqrt(2.0 / (256 * 9))).astype(np.float32)
+    b = (0.1 * rng.standard_normal(96)).astype(np.float32)
+    r = rng.standard_normal((1, 96, 7, 7), dtype=np.float32)
+    handle.set_math(mode)
+    plan = api.Conv2d(handle, 1, 256, 7, 7, 96, 3, 1, 1, False, "linear", api.LAYOUT_NHWC)
+    plan.set_weights(w, b)
+    xd, rd = _t(x.transpose(0, 2, 3, 1)), _t(r.transpose(0, 2, 3, 1))
+    f = api.ConvFusion(rd.data_ptr(), 96, 7, 7, api.ACT["relu"], None)
+    outs = []
+    for off in (0, 1):
+        y = torch.empty(7 * 7 * 96 + 4, device="cuda")[off:off + 7 * 7 * 96]
+        handle.check(handle.lib.nb_conv2d_forward_fused(plan.p, xd.data_ptr(), y.data_ptr(), ctypes.byref(f)))
+        outs.append(y.cpu().numpy().reshape(7, 7, 96).transpose(2, 0, 1)[None])
+    handle.synchronize()
+    plan.close()
+    ref = np.maximum(O.conv_forward(x, w, b, 3, 1, 1, "linear") + r, 0)
+    for y in outs:
+        assert_close(y, ref, mode)
