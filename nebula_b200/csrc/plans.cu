@@ -696,15 +696,20 @@ size_t RnnPlan::reserve(bool x_rounded, bool x_foreign) {
     const size_t T = d.time_steps, B = d.batch, H = d.hidden;
     a_all.reserve(T * B * H);
     state.reserve(T * B * H);
-    h0.reserve(B * H);
     const bool tf32 = h->math_mode == NB_MATH_TF32;
     ForwardOpts o;
     o.x_rounded = x_rounded; o.x_foreign = x_foreign;
     in_gate->reserve(o, (int)(T * B));
-    o.x_rounded = false; o.x_foreign = false;
-    hid_gate->reserve(o, (int)B);                   // step 0 reads the (unrounded) input-gate output
-    o.x_rounded = tf32;
-    out_gate->reserve(o, (int)(T * B));
+    o.x_rounded = tf32; o.x_foreign = false;
+    if (recurrent_cluster_supported(h, 1, d.hidden, (int)B)) {
+        out_gate->reserve(o, (int)(T * B));
+    } else {                                            // a launch per step; the output gate runs step 0 by itself
+        h0.reserve(B * H);
+        out_gate->reserve(o, (int)B);
+        if (T > 1) out_gate->reserve(o, (int)((T - 1) * B));
+        o.x_rounded = false;
+        hid_gate->reserve(o, (int)B);                   // step 0 reads the (unrounded) input-gate output
+    }
     return workspace_bytes();
 }
 

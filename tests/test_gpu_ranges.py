@@ -60,3 +60,27 @@ def test_folded_shortcut_of_a_split_layer_to_any_address(handle, mode):
     ref = np.maximum(O.conv_forward(x, w, b, 3, 1, 1, "linear") + r, 0)
     for y in outs:
         assert_close(y, ref, mode)
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3", "fp32"])
+@pytest.mark.parametrize("case", [(16, 32, 1024), (5, 32, 1024), (1, 3, 900), (3, 130, 1000)], ids=str)
+def test_rnn_wider_than_a_cluster(handle, mode, case):
+    """One launch per step: the output gate sees the rows of step 0 and those of the other steps; a prepared plan has the
+    scratch of both."""
+    import torch
+    from nebula_b200 import api
+    from oracle import oracle as O
+    T, B, H = case
+    rng = np.random.default_rng(H)
+    blobs = [{"bias": (0.1 * rng.standard_normal(H)).astype(np.float32), "w": (rng.uniform(-1, 1, (H, n)) / np.sqrt(n)).astype(np.float32)}
+             for n in (64, H, H)]
+    x = rng.standard_normal((T, B, 64), dtype=np.float32)
+    handle.set_math(mode)
+    plan = api.Rnn(handle, T, B, 64, H, False, "tanh")
+    plan.set_weights(np.concatenate([a.ravel() for b in blobs for a in (b["bias"], b["w"])]))
+    prepared = plan.prepare()
+    y = plan.forward(_t(x))
+    assert plan.workspace_size() == prepared
+    handle.synchronize()
+    plan.close()
+    assert_close(y.cpu().numpy(), O.rnn_forward(x, blobs, H, "tanh"), mode, f"rnn {case}", factor=3.0)
