@@ -362,6 +362,8 @@ void lstm_persistent_prepare_device();
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B,
                      int H, int t_first);
+// what a contraction runs on: the tensor cores in TF32 or 3xTF32, or the CUDA cores
+enum GemmPath { PATH_TC = 0, PATH_TC3 = 1, PATH_SIMT = 2 };
 // The recurrence of an LSTM (gates = 4) or RNN (gates = 1) layer over all steps, exact fp32, for layers whose recurrent
 // weights fit the shared memory of one cluster (recurrent_cluster.cu).
 struct RecurrentArgs {
@@ -375,7 +377,8 @@ struct RecurrentArgs {
     int round_out;              // RNN: store TF32-rounded values
 };
 void recurrent_cluster_prepare_device(nb_handle_s *h);
-bool recurrent_cluster_supported(const nb_handle_s *h, int gates, int H, int B);
+// step_path: what a launch per step would run on
+bool recurrent_cluster_pays(const nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path);
 void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a);
 void elementwise_prepare_device();
 

@@ -614,9 +614,13 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H, 1);
         return;
     }
-    // Everything else (the modes that promise fp32 agreement, widths off 32, gate layers with an activation) runs all
-    // steps in one kernel of exact fp32 products while the weights fit a cluster's shared memory.
-    if (!(lp_env && *lp_env == '0') && recurrent_cluster_supported(h, 4, H, B)) {
+    // The modes that promise fp32 agreement, widths off 32 and gate layers with an activation run all steps in one kernel of
+    // exact fp32 products where that is the faster way.  The layers whose batches up to 128 run above take the same TF32
+    // products a launch per step beyond (bit-identical), whatever the cluster would cost; a single step of linear gate
+    // layers has no product.
+    const bool tf32_width = tc_w && !three && linear && (H % 32) == 0;
+    if (!(lp_env && *lp_env == '0') && !tf32_width && (T > 1 || !linear) &&
+        recurrent_cluster_pays(h, 4, H, B, T, linear, !tc_w ? PATH_SIMT : (three ? PATH_TC3 : PATH_TC))) {
         RecurrentArgs r{};
         r.w = ww.exact.p; r.pre = pre.p; r.shift = linear ? nullptr : shift_w.p;
         r.cell = cell; r.out = out; r.out_round = hr;
@@ -692,6 +696,10 @@ void RnnPlan::set_weights(const float *stream, size_t count, int mem) {
     ready = true;
 }
 
+bool RnnPlan::one_kernel() const {
+    return recurrent_cluster_pays(h, 1, d.hidden, d.batch, d.time_steps, true, hid_gate->path());
+}
+
 size_t RnnPlan::reserve(bool x_rounded, bool x_foreign) {
     const size_t T = d.time_steps, B = d.batch, H = d.hidden;
     a_all.reserve(T * B * H);
@@ -701,7 +709,7 @@ size_t RnnPlan::reserve(bool x_rounded, bool x_foreign) {
     o.x_rounded = x_rounded; o.x_foreign = x_foreign;
     in_gate->reserve(o, (int)(T * B));
     o.x_rounded = tf32; o.x_foreign = false;
-    if (recurrent_cluster_supported(h, 1, d.hidden, (int)B)) {
+    if (one_kernel()) {
         out_gate->reserve(o, (int)(T * B));
     } else {                                            // a launch per step; the output gate runs step 0 by itself
         h0.reserve(B * H);
@@ -724,9 +732,9 @@ void RnnPlan::forward(const float *x, float *out, bool x_rounded, bool round_out
     // a_t for every step at once: the input gate does not depend on the state
     o.x_rounded = x_rounded; o.x_foreign = x_foreign;
     in_gate->forward(x, a_all.p, o, T * B);
-    // all steps in one kernel while the hidden gate's weights fit a cluster's shared memory: its state buffer holds what
-    // the output gate reads, h_0 in the place of s_0
-    if (recurrent_cluster_supported(h, 1, d.hidden, B)) {
+    // all steps in one kernel where that is the faster way: its state buffer holds what the output gate reads, h_0 in the
+    // place of s_0
+    if (one_kernel()) {
         RecurrentArgs r{};
         r.w = hid_gate->w.exact.p; r.pre = a_all.p;
         r.scale = hid_gate->has_scale ? hid_gate->scale.p : nullptr; r.shift = hid_gate->shift.p;

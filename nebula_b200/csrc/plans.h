@@ -19,7 +19,6 @@ struct nb_plan_s {
 
 namespace nb {
 
-enum GemmPath { PATH_TC = 0, PATH_TC3 = 1, PATH_SIMT = 2 };
 
 // Weights of one contraction in the three forms the math modes need.
 struct WeightSet {
@@ -157,6 +156,7 @@ struct RnnPlan : nb_plan_s {
     size_t weight_count() const;
     void set_weights(const float *stream, size_t count, int mem);
     void forward(const float *x, float *out, bool x_rounded, bool round_out, bool x_foreign = true);
+    bool one_kernel() const;        // the recurrence as one kernel on clusters, in the handle's math mode
     size_t reserve(bool x_rounded, bool x_foreign = true);
     size_t workspace_bytes() const override {
         return (a_all.n + state.n + h0.n) * sizeof(float) + in_gate->workspace_bytes() + hid_gate->workspace_bytes() +

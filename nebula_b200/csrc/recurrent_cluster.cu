@@ -11,7 +11,8 @@
 // runs the cell update and stores the new state into the shared memory of all CS CTAs; a cluster barrier ends the step.
 // The step's results leave for HBM between the barrier's arrive and its wait: an arrive releases what was stored in front
 // of it, so there it would wait for HBM on every step (T35 B20 H300: 4.1 us a step in front, 2.8 us behind).
-// CS depends on the layer only, so a batch and its slices add in the same order.
+// CS depends on the layer only, so batches that run here add in the same order as their slices; how large a batch runs
+// here at all, and not a launch per step, depends on the batch too (recurrent_cluster_pays).
 #include <cooperative_groups.h>
 
 #include "device_math.cuh"
@@ -292,9 +293,38 @@ void recurrent_cluster_prepare_device(nb_handle_s *h) {
     }
 }
 
-bool recurrent_cluster_supported(const nb_handle_s *h, int gates, int H, int B) {
+// Fits, and beats a launch per step.  A cluster runs at most 8 rows, so large batches go through it in waves, each of which
+// loads the weights again; a launch per step takes its batch at once.  Fitted in microseconds to LSTM and RNN layers of 33 to
+// 864 units, batches of 1 to 2048, 4 and 36 steps; the better of the two is missed by 26 % at most, seldom by 10 %:
+//   cluster   waves * (2 + 0.03 per KB of shared memory + T * step_cost * 1.4, 1.2 more for gate layers with an activation)
+//   per step  T * step, without the first product where the state is zero, and two launches more for the RNN.  A TF32 step
+//             takes 12.5 (LSTM), 17 (LSTM with an activation) or 15 us (RNN), a 3xTF32 one 17.5, 24 or 20, on the CUDA cores
+//             16 + 0.02 H + 45 per GFLOP (LSTM), 14 + 0.005 H + 50 per GFLOP (RNN).
+// T = 36, TF32: LSTM H = 300 at B = 128 / 256: 12.4 / 20.7 us a step in the cluster, 16.0 / 16.0 launched; RNN H = 800 at
+// B = 32 / 128: 8.7 / 29.2 and 17.0 / 19.9.
+static bool pays(const nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path) {
     Shape s;
-    return h->cc_major == 10 && choose(h, gates, H, B, &s);
+    if (!choose(h, gates, H, B, &s)) return false;
+    const int at_once = s.CS == 1 ? h->sm_count : h->clusters_at_once[s.CS];
+    const int waves = ((B + s.RB - 1) / s.RB + at_once - 1) / at_once;
+    const bool lstm = gates == 4, activated = lstm && !linear;
+    const double in_cluster = waves * (2.0 + 0.03 * (double)s.smem / 1024 + T * (1.4 * step_cost(s, H) / 1900 + (activated ? 1.2 : 0.0)));
+    double step;
+    if (step_path == PATH_SIMT) {
+        const double gflop = 2e-9 * B * gates * H * H;
+        step = lstm ? 16 + 0.02 * H + 45 * gflop : 14 + 0.005 * H + 50 * gflop;
+    } else {
+        const bool three = step_path == PATH_TC3;
+        step = activated ? (three ? 24 : 17) : (lstm ? (three ? 17.5 : 12.5) : (three ? 20 : 15));
+    }
+    return in_cluster <= (activated ? T * step : (lstm ? 2 + (T - 1) * step : (T + 2) * step));
+}
+
+// On the CUDA cores, whose results do not depend on the batch otherwise, the layer and its steps decide up to 256 rows.
+bool recurrent_cluster_pays(const nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path) {
+    if (h->cc_major != 10) return false;
+    if (step_path != PATH_SIMT) return pays(h, gates, H, B, T, linear, step_path);
+    return pays(h, gates, H, 32, T, linear, step_path) && (B <= 256 || pays(h, gates, H, B, T, linear, step_path));
 }
 
 void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a) {

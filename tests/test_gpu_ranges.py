@@ -84,3 +84,55 @@ def test_rnn_wider_than_a_cluster(handle, mode, case):
     handle.synchronize()
     plan.close()
     assert_close(y.cpu().numpy(), O.rnn_forward(x, blobs, H, "tanh"), mode, f"rnn {case}", factor=3.0)
+
+
+# (kind, T, B, hidden, activation, mode, all steps in one launch): batches that go through a cluster in waves
+RECURRENT_CASES = [("lstm", 6, 20, 300, "linear", "tf32", True), ("lstm", 6, 512, 300, "linear", "tf32", False), ("lstm", 5, 400, 420, "linear", "tf32x3", False),
+                   ("lstm", 6, 300, 100, "linear", "tf32", True), ("lstm", 4, 1024, 416, "tanh", "tf32", False), ("lstm", 3, 900, 300, "linear", "fp32", False),
+                   ("lstm", 3, 700, 301, "linear", "tf32", False), ("lstm", 1, 5, 40, "linear", "tf32", False), ("rnn", 6, 32, 256, "tanh", "tf32", True),
+                   ("rnn", 5, 300, 800, "tanh", "tf32", False), ("rnn", 4, 260, 800, "relu", "tf32x3", False), ("rnn", 3, 600, 864, "tanh", "fp32", False)]
+
+
+@pytest.mark.parametrize("case", RECURRENT_CASES, ids=lambda c: "-".join(map(str, c)))
+def test_recurrence_of_large_batches(handle, case):
+    from nebula_b200 import api
+    from nebula_b200.workloads import NetBuilder
+    from oracle import oracle as O
+    kind, T, B, H, act, mode, one_launch = case
+    nb = NetBuilder("r", B, input_size=32, time_steps=T, bias_init="bias_n01")
+    getattr(nb, kind)(H, act, bound=1.0 / np.sqrt(H))
+    wl = nb.build("normal")
+    w, x = wl.make_weights(H), wl.make_input(B)
+    handle.set_math(mode)
+    plan = (api.Lstm if kind == "lstm" else api.Rnn)(handle, T, B, 32, H, False, act)
+    plan.set_weights(w)
+    prepared = plan.prepare()
+    n0 = handle.launch_count()
+    y = plan.forward(_t(x))
+    n = handle.launch_count() - n0
+    # per step: a launch per step, behind the input side's; an LSTM's single step of linear gates is one cell update
+    assert (n <= 5) == (one_launch or T == 1), n
+    assert plan.workspace_size() == prepared
+    handle.synchronize()
+    plan.close()
+    assert_close(y.cpu().numpy(), O.forward_network(wl.cfg, w, x)[0], mode, f"{case}", factor=1.0 if act in ("linear", "relu") else 3.0)
+
+
+@pytest.mark.parametrize("H", [64, 416])
+def test_tf32_lstm_of_any_batch_equals_its_slices(handle, H):
+    """Widths that are multiples of 32: TF32 products in one kernel up to 128 rows, launched per step beyond, bit for bit alike."""
+    import torch
+    from nebula_b200 import api
+    T, B = 4, 200
+    g = torch.Generator(device="cuda").manual_seed(1)
+    w = torch.randn(8 * (H + H * H), device="cuda", generator=g) / H ** 0.5
+    x = torch.randn(T, B, H, device="cuda", generator=g)
+    handle.set_math("tf32")
+    outs = []
+    for lo, hi in ((0, 200), (0, 100), (100, 129), (129, 200)):
+        plan = api.Lstm(handle, T, hi - lo, H, H, False, "linear")
+        plan.set_weights(w)
+        outs.append(plan.forward(x[:, lo:hi].contiguous()))
+        handle.synchronize()
+        plan.close()
+    assert torch.equal(outs[0], torch.cat(outs[1:], 1))
