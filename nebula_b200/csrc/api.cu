@@ -106,7 +106,6 @@ int nb_create(int device_id, nb_handle_t *handle) {
             }
         }
         gemm_tc_prepare_device();
-        gemm_simt_prepare_device();
         lstm_persistent_prepare_device();
         elementwise_prepare_device();
     });

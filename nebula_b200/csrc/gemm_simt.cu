@@ -283,15 +283,31 @@ int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks) {
     return S;
 }
 
-void launch(nb_handle_s *h, SimtParams &p, int amode, int bmode, int S) {
+// The tile shape with the cheapest last wave, and its kernel for these copy modes, loaded and with its shared-memory limit set.
+// The 36 kernels are not loaded with the handle: that was 19 ms for a process's first one (29 instead of 10), while a handle
+// uses a few of them at most.  A plan asks for its own when it reserves its scratch (gemm_simt_load); a kernel first met by a
+// launch, captured ones included, is loaded there.
+int ready_variant(nb_handle_s *h, long M, int N, int S, int amode, int bmode) {
     int best = 0;
     double best_cost = 0;
     for (int v = 0; v < 4; v++) {
-        const long ctas = ((p.M + VARIANTS[v].bm - 1L) / VARIANTS[v].bm) * ((p.N + VARIANTS[v].bn - 1L) / VARIANTS[v].bn) * S;
+        const long ctas = ((M + VARIANTS[v].bm - 1L) / VARIANTS[v].bm) * ((N + VARIANTS[v].bn - 1L) / VARIANTS[v].bn) * S;
         const double cost = (double)((ctas + h->sm_count - 1) / h->sm_count) * VARIANTS[v].bm * VARIANTS[v].bn / RATE[v];
         if (v == 0 || cost < best_cost) { best_cost = cost; best = v; }
     }
-    const SimtVariant &v = VARIANTS[best];
+    const unsigned long long bit = 1ull << (9 * best + 3 * amode + bmode);
+    if (!(h->simt_ready & bit)) {
+        const SimtVariant &v = VARIANTS[best];
+        cudaFuncAttributes fa;          // (loads the code)
+        if (v.smem > 48 * 1024) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel[amode][bmode], cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+        else NB_CHECK_CUDA(cudaFuncGetAttributes(&fa, v.kernel[amode][bmode]));
+        h->simt_ready |= bit;
+    }
+    return best;
+}
+
+void launch(nb_handle_s *h, SimtParams &p, int amode, int bmode, int S) {
+    const SimtVariant &v = VARIANTS[ready_variant(h, p.M, p.N, S, amode, bmode)];
     p.n_tiles = (p.N + v.bn - 1) / v.bn;
     p.kb_per_split = (p.k_blocks + S - 1) / S;
     cudaLaunchConfig_t cfg = {};
@@ -319,19 +335,8 @@ inline bool vec_ok(const float *p, long s0, long s1, long s2) {
 
 }  // namespace
 
-void gemm_simt_prepare_device() {
-    for (const SimtVariant &v : VARIANTS)
-        for (auto &row : v.kernel)
-            for (SimtKernel k : row) {
-                cudaFuncAttributes fa;          // (loads the code)
-                if (v.smem > 48 * 1024) NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
-                else NB_CHECK_CUDA(cudaFuncGetAttributes(&fa, k));
-            }
-}
-
-void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
-    if (a.addend && a.res_stride > 0) throw Error(NB_ERR_UNSUPPORTED, "the CUDA-core path takes no fused residual");
-    SimtParams p{};
+static void simt_params(const nb_handle_s *h, const GemmArgs &a, SimtParams *out, int *amode, int *bmode, int *S) {
+    SimtParams &p = *out;
     p.a = a.a; p.b = a.b;
     if (a.a_is_conv) {
         p.g = a.g;
@@ -350,9 +355,24 @@ void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
     p.y = a.y; p.ldy = a.ldy;
     // 16-byte copies need whole quads of columns on 16-byte boundaries; a tensor whose pixels are contiguous per
     // channel (NCHW) is read with lanes along the pixels
-    const int amode = p.g.sc == 1 ? (a.Kc % 4 == 0 && vec_ok(p.a, p.g.sn, p.g.sh, p.g.sw) ? VEC_K : ONE_K) : ONE_ROW;
-    const int bmode = a.Kc % 4 == 0 && vec_ok(p.b, a.ldb, p.b_tap, 0) ? VEC_K : ONE_K;
-    launch(h, p, amode, bmode, split_of(h, a.a_is_conv ? (long)p.g.OH * p.g.OW : 1, a.N, p.k_blocks));
+    *amode = p.g.sc == 1 ? (a.Kc % 4 == 0 && vec_ok(p.a, p.g.sn, p.g.sh, p.g.sw) ? VEC_K : ONE_K) : ONE_ROW;
+    *bmode = a.Kc % 4 == 0 && vec_ok(p.b, a.ldb, p.b_tap, 0) ? VEC_K : ONE_K;
+    *S = split_of(h, a.a_is_conv ? (long)p.g.OH * p.g.OW : 1, a.N, p.k_blocks);
+}
+
+void gemm_simt_load(nb_handle_s *h, const GemmArgs &a) {
+    SimtParams p{};
+    int amode, bmode, S;
+    simt_params(h, a, &p, &amode, &bmode, &S);
+    ready_variant(h, p.M, p.N, S, amode, bmode);
+}
+
+void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
+    if (a.addend && a.res_stride > 0) throw Error(NB_ERR_UNSUPPORTED, "the CUDA-core path takes no fused residual");
+    SimtParams p{};
+    int amode, bmode, S;
+    simt_params(h, a, &p, &amode, &bmode, &S);
+    launch(h, p, amode, bmode, S);
 }
 
 // _gemm_ (common/gemm.h:21-25) with the CPU path's meaning of every argument (row-major, leading dimensions honoured, all

@@ -64,7 +64,8 @@ struct nb_handle_s {
     int *d_status = nullptr;            // device status word (nb::DEV_*)
     unsigned int *d_grid_sync = nullptr; // arrival counter of the persistent LSTM kernel's grid barrier
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
-    bool recurrent_ready = false;       // recurrent_cluster_prepare_device has run
+    bool recurrent_ready = false;       // recurrent_cluster.cu: limits set, clusters_at_once filled
+    unsigned long long simt_ready = 0;  // gemm_simt.cu: kernels loaded and with their limits set, by variant and copy modes
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
     nb_encode_tiled_fn encode_tiled = nullptr;
     nb_get_address_range_fn get_address_range = nullptr;   // cuMemGetAddressRange: the allocation a pointer lies in
@@ -227,6 +228,8 @@ void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
 // CUDA-core fp32 path: any extents, strides and alignments.
 void gemm_simt(nb_handle_s *h, const GemmArgs &a);
+// Loads the kernel that gemm_simt takes for these extents (null operands: aligned ones), so that no pass has to.
+void gemm_simt_load(nb_handle_s *h, const GemmArgs &a);
 // Dispatch on the handle's math mode.
 void gemm(nb_handle_s *h, const GemmArgs &a);
 
@@ -357,7 +360,6 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra);
 
 // Per-device set-up of the tensor-core kernels (shared-memory limits; also loads their code), once per handle.
 void gemm_tc_prepare_device();
-void gemm_simt_prepare_device();
 void lstm_persistent_prepare_device();
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B,
@@ -376,9 +378,8 @@ struct RecurrentArgs {
     int cell_f32;               // LSTM: gate activations in fp32 instead of the double formulas
     int round_out;              // RNN: store TF32-rounded values
 };
-void recurrent_cluster_prepare_device(nb_handle_s *h);
 // step_path: what a launch per step would run on
-bool recurrent_cluster_pays(const nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path);
+bool recurrent_cluster_pays(nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path);
 void recurrent_cluster(nb_handle_s *h, const RecurrentArgs &a);
 void elementwise_prepare_device();
 

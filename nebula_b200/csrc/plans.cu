@@ -151,6 +151,32 @@ bool ConvPlan::writes_nchw(const ForwardOpts &o) const {
     return splits(o) == 1;
 }
 
+// The product of this layer: x as it lies, and as row windows (without the zero columns that fill up a tensor-core K block).
+GemmArgs ConvPlan::conv_args(const float *x, bool nhwc) const {
+    GemmArgs a;
+    a.a = x; a.a_is_conv = true;
+    ConvGeom &g = a.g;
+    g.batch = d.batch; g.C = d.channels; g.H = d.height; g.W = d.width; g.OH = OH; g.OW = OW;
+    g.ksize = d.size; g.stride = d.stride; g.pad = d.padding;
+    if (nhwc) {
+        g.sc = 1; g.sw = d.channels; g.sh = (long)d.width * d.channels; g.sn = (long)d.height * d.width * d.channels;
+    } else {
+        g.sw = 1; g.sh = d.width; g.sc = (long)d.height * d.width; g.sn = (long)d.channels * d.height * d.width;
+    }
+    a.ldb = Cp; a.M = d.batch * OH * OW; a.N = d.filters; a.Kc = d.channels;
+    return a;
+}
+GemmArgs ConvPlan::rowwin_args(const float *xw, const float *weights, bool cuda_cores) const {
+    GemmArgs a;
+    a.a = xw; a.b = weights; a.a_is_conv = true;
+    ConvGeom &g = a.g;
+    g.batch = d.batch; g.C = rw_inner; g.H = d.height; g.W = rw_wp - rw_inner / 4 + 1; g.OH = OH; g.OW = OW;
+    g.ksize = d.size; g.ksize_w = 1; g.stride = d.stride; g.pad = d.padding; g.pad_w = 0;
+    g.sc = 1; g.sw = 4; g.sh = (long)rw_wp * 4; g.sn = (long)d.height * rw_wp * 4;
+    a.ldb = rw_inner; a.M = d.batch * OH * OW; a.N = d.filters; a.Kc = cuda_cores ? 4 * d.size : rw_inner;
+    return a;
+}
+
 // Which of the three routes forward() takes, and the scratch each needs.
 size_t ConvPlan::reserve(const ForwardOpts &o) {
     const GemmPath pth = path(o);
@@ -160,9 +186,12 @@ size_t ConvPlan::reserve(const ForwardOpts &o) {
     if (!o.y_nhwc) y_scratch.reserve(yout);         // (also where this route writes NCHW itself: a later math mode may not)
     if (pth == PATH_SIMT && rowwin_ok) {
         x_rowwin.reserve((size_t)d.batch * d.height * rw_wp * 4);
+        if (!tc_mode) gemm_simt_load(h, rowwin_args(nullptr, nullptr, true));
     } else if (pth == PATH_SIMT && pack_ok && tc_mode && h->encode_tiled) {
         // the kernel gathers x in place
-    } else if (pth != PATH_SIMT) {
+    } else if (pth == PATH_SIMT) {
+        gemm_simt_load(h, conv_args(nullptr, o.x_nhwc));
+    } else {
         const bool need_round = (pth == PATH_TC) && !o.x_rounded;
         if (!o.x_nhwc || need_round || o.x_foreign) x_scratch.reserve(xin);
         const int S = splits(o);
@@ -178,12 +207,6 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
     const size_t xin = (size_t)d.batch * d.channels * d.height * d.width;
     reserve(o);
 
-    GemmArgs a;
-    a.a_is_conv = true;
-    ConvGeom &g = a.g;
-    g.batch = d.batch; g.C = d.channels; g.H = d.height; g.W = d.width; g.OH = OH; g.OW = OW;
-    g.ksize = d.size; g.stride = d.stride; g.pad = d.padding;
-
     if (pth == PATH_SIMT && rowwin_ok) {
         // 1-4 input channels: one K slice per filter row (fetched by TMA on the tensor-core routes; on the CUDA cores a
         // slice of 4*size aligned floats per row instead of `size` taps of 1-4 scattered ones)
@@ -192,13 +215,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         if (o.x_rowwin) xw = const_cast<float *>(x);       // the caller already holds the input in this layout
         else launch_rowwin_input(h, x, xw, d.batch, d.channels, d.height, d.width, rw_wp, d.padding, o.x_nhwc,
                                  h->math_mode == NB_MATH_TF32);
-        GemmArgs ra;
-        ra.a = xw; ra.a_is_conv = true;
-        ConvGeom &rg = ra.g;
-        rg.batch = d.batch; rg.C = rw_inner; rg.H = d.height; rg.W = rw_wp - rw_inner / 4 + 1; rg.OH = OH; rg.OW = OW;
-        rg.ksize = d.size; rg.ksize_w = 1; rg.stride = d.stride; rg.pad = d.padding; rg.pad_w = 0;
-        rg.sc = 1; rg.sw = 4; rg.sh = (long)rw_wp * 4; rg.sn = (long)d.height * rw_wp * 4;
-        ra.ldb = rw_inner; ra.M = d.batch * OH * OW; ra.N = d.filters; ra.Kc = rw_inner;
+        GemmArgs ra = rowwin_args(xw, cuda_cores ? wr.exact.p : wr.hi.p, cuda_cores);
         ra.scale = has_scale ? scale.p : nullptr; ra.shift = shift.p; ra.act = d.activation;
         ra.round_out_tf32 = o.round_out; ra.addend = o.addend; ra.ld_addend = d.filters;
         float *yo = y;
@@ -209,10 +226,8 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         }
         ra.y = yo; ra.ldy = d.filters;
         ra.algo_flops = 2.0 * (double)ra.M * d.filters * d.channels * d.size * d.size;
-        ra.b = wr.hi.p; ra.b_lo = wr.lo.p; ra.b_static = true;
+        ra.b_lo = wr.lo.p; ra.b_static = true;
         if (cuda_cores) {
-            ra.Kc = 4 * d.size;             // without the zero columns that fill up a tensor-core K block
-            ra.b = wr.exact.p;
             gemm_simt(h, ra);
             if (!o.y_nhwc) launch_layout(h, yo, y, d.batch, d.filters, OH, OW, false, false);
             return;
@@ -226,15 +241,9 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
     if (pth == PATH_SIMT && pack_ok && h->math_mode != NB_MATH_FP32 && h->encode_tiled) {
         // tensor-core route for small channel counts: the kernel gathers the patches itself
         const bool three = h->math_mode == NB_MATH_TF32X3;
-        const size_t M = (size_t)d.batch * OH * OW;
-        if (o.x_nhwc) {
-            g.sc = 1; g.sw = d.channels; g.sh = (long)d.width * d.channels; g.sn = (long)d.height * d.width * d.channels;
-        } else {
-            g.sw = 1; g.sh = d.width; g.sc = (long)d.height * d.width; g.sn = (long)d.channels * d.height * d.width;
-        }
-        GemmArgs pa;
-        pa.a = x; pa.a_is_conv = true; pa.g = g; pa.a_gather = true;
-        pa.ldb = Kpad; pa.M = (int)M; pa.N = d.filters; pa.Kc = Kpad;
+        GemmArgs pa = conv_args(x, o.x_nhwc);
+        pa.a_gather = true;
+        pa.ldb = Kpad; pa.Kc = Kpad;
         pa.scale = has_scale ? scale.p : nullptr; pa.shift = shift.p; pa.act = d.activation;
         pa.round_out_tf32 = o.round_out; pa.addend = o.addend; pa.ld_addend = d.filters;
         float *yo = y;
@@ -243,7 +252,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
             yo = y_scratch.p;
         }
         pa.y = yo; pa.ldy = d.filters;
-        pa.algo_flops = 2.0 * (double)M * d.filters * d.channels * d.size * d.size;
+        pa.algo_flops = 2.0 * (double)pa.M * d.filters * d.channels * d.size * d.size;
         const bool split_now = !wp.split_ready;
         wp.ensure_split(h);
         pa.b = wp.hi.p; pa.b_lo = wp.lo.p; pa.b_static = !split_now;
@@ -268,16 +277,7 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
             xa = x_scratch.p;
         }
     }
-    if (nhwc) {
-        g.sc = 1; g.sw = d.channels; g.sh = (long)d.width * d.channels; g.sn = (long)d.height * d.width * d.channels;
-    } else {
-        g.sw = 1; g.sh = d.width; g.sc = (long)d.height * d.width; g.sn = (long)d.channels * d.height * d.width;
-    }
-    a.a = xa;
-    a.ldb = Cp;
-    a.M = d.batch * OH * OW;
-    a.N = d.filters;
-    a.Kc = d.channels;
+    GemmArgs a = conv_args(xa, nhwc);
     a.scale = has_scale ? scale.p : nullptr;
     a.shift = shift.p;
     a.act = d.activation;
@@ -418,6 +418,11 @@ size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
     const int M = rows > 0 ? rows : d.batch;
     const GemmPath pth = path();
     if ((pth == PATH_TC && !o.x_rounded) || (pth == PATH_TC3 && o.x_foreign)) x_scratch.reserve((size_t)M * d.inputs);
+    if (pth == PATH_SIMT) {
+        GemmArgs a;
+        a.lda = a.ldb = a.Kc = d.inputs; a.M = M; a.N = d.outputs;
+        gemm_simt_load(h, a);
+    }
     int S, bn;
     split_choice(pth, o.addend != nullptr, M, &S, &bn);
     if (S > 1) split_ws.reserve((size_t)S * M * d.outputs);
@@ -479,7 +484,6 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
 LstmPlan::LstmPlan(nb_handle_s *hh, const nb_lstm_desc_t &desc) : nb_plan_s(NB_PLAN_LSTM, hh), d(desc) {
     NB_REQUIRE(d.time_steps > 0 && d.batch > 0 && d.inputs > 0 && d.hidden > 0, "lstm: non-positive extent");
     NB_REQUIRE(d.activation > NB_ACT_UNDEFINED && d.activation < NB_ACT_COUNT, "lstm: undefined activation");
-    recurrent_cluster_prepare_device(h);
 }
 
 size_t LstmPlan::weight_count() const {
@@ -546,6 +550,20 @@ void LstmPlan::set_weights(const float *stream, size_t count, int mem) {
     ready = true;
 }
 
+// The modes that promise fp32 agreement, widths off 32 and gate layers with an activation run all steps in one kernel of exact
+// fp32 products where that is the faster way.  The layers whose batches up to 128 run on the tensor cores in one kernel
+// (lstm_persistent.cu) take the same TF32 products a launch per step beyond (bit-identical), whatever the cluster would cost; a
+// single step of linear gate layers has no product.  NEBULA_B200_LSTM_PERSISTENT=0: a launch per step in every case.
+bool LstmPlan::one_kernel() const {
+    const char *env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
+    if (env && *env == '0') return false;
+    const int H = d.hidden;
+    const bool linear = d.activation == NB_ACT_LINEAR, three = h->math_mode == NB_MATH_TF32X3;
+    const bool tc_w = h->math_mode != NB_MATH_FP32 && h->encode_tiled && h->cc_major == 10 && (H % 4) == 0 && H >= 32;
+    if ((tc_w && !three && linear && (H % 32) == 0) || (d.time_steps == 1 && linear)) return false;
+    return recurrent_cluster_pays(h, 4, H, d.batch, d.time_steps, linear, !tc_w ? PATH_SIMT : (three ? PATH_TC3 : PATH_TC));
+}
+
 size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, bool x_foreign) {
     const int T = d.time_steps, B = d.batch, H = d.hidden, in = d.inputs;
     const size_t rows = (size_t)T * B;
@@ -555,6 +573,16 @@ size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, boo
     const bool three = h->math_mode == NB_MATH_TF32X3;
     pre.reserve(rows * 4 * H);
     if (!tc_w) z.reserve((size_t)B * 4 * H);
+    GemmArgs a;
+    a.N = 4 * H;
+    if (!tc_u) {
+        a.lda = a.ldb = a.Kc = in; a.M = (int)rows;
+        gemm_simt_load(h, a);
+    }
+    if (!one_kernel() && !tc_w) {
+        a.lda = a.ldb = a.Kc = H; a.M = B;
+        gemm_simt_load(h, a);
+    }
     if (own_cell) cell_own.reserve(rows * H);
     if (!have_out_round && tc_w && !three) h_round.reserve(rows * H);
     if (tc_u && ((!three && !x_rounded) || (three && x_foreign))) x_round.reserve(rows * in);
@@ -614,13 +642,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H, 1);
         return;
     }
-    // The modes that promise fp32 agreement, widths off 32 and gate layers with an activation run all steps in one kernel of
-    // exact fp32 products where that is the faster way.  The layers whose batches up to 128 run above take the same TF32
-    // products a launch per step beyond (bit-identical), whatever the cluster would cost; a single step of linear gate
-    // layers has no product.
-    const bool tf32_width = tc_w && !three && linear && (H % 32) == 0;
-    if (!(lp_env && *lp_env == '0') && !tf32_width && (T > 1 || !linear) &&
-        recurrent_cluster_pays(h, 4, H, B, T, linear, !tc_w ? PATH_SIMT : (three ? PATH_TC3 : PATH_TC))) {
+    if (one_kernel()) {
         RecurrentArgs r{};
         r.w = ww.exact.p; r.pre = pre.p; r.shift = linear ? nullptr : shift_w.p;
         r.cell = cell; r.out = out; r.out_round = hr;
@@ -662,7 +684,6 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
 RnnPlan::RnnPlan(nb_handle_s *hh, const nb_rnn_desc_t &desc) : nb_plan_s(NB_PLAN_RNN, hh), d(desc) {
     NB_REQUIRE(d.time_steps > 0 && d.batch > 0 && d.inputs > 0 && d.hidden > 0, "rnn: non-positive extent");
     NB_REQUIRE(d.activation > NB_ACT_UNDEFINED && d.activation < NB_ACT_COUNT, "rnn: undefined activation");
-    recurrent_cluster_prepare_device(h);
     // the three gates are connected layers built from the same section (rnn_layer.cc:47-54)
     nb_fc_desc_t g{};
     g.batch = d.batch; g.outputs = d.hidden; g.batch_normalize = d.batch_normalize; g.activation = d.activation;

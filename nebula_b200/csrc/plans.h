@@ -87,6 +87,8 @@ struct ConvPlan : nb_plan_s {
     size_t workspace_bytes() const override { return (x_rowwin.n + x_scratch.n + y_scratch.n + split_ws.n) * sizeof(float); }
     void output_dims(int dims[3]) const override { dims[0] = d.filters; dims[1] = OH; dims[2] = OW; }
     GemmPath path(const ForwardOpts &o) const;
+    GemmArgs conv_args(const float *x, bool nhwc) const;
+    GemmArgs rowwin_args(const float *xw, const float *weights, bool cuda_cores) const;
     // K slices of the tensor-core path with these options (1: none)
     int splits(const ForwardOpts &o) const;
     bool writes_nchw(const ForwardOpts &o) const;
@@ -132,6 +134,7 @@ struct LstmPlan : nb_plan_s {
     LstmPlan(nb_handle_s *h, const nb_lstm_desc_t &desc);
     void set_weights(const float *stream, size_t count, int mem);
     size_t weight_count() const;
+    bool one_kernel() const;        // the recurrence as one kernel on clusters, in the handle's math mode
     // out_round (optional): receives a TF32-rounded copy of out
     void forward(const float *x, float *out, float *cell, bool x_rounded, float *out_round, bool x_foreign = true);
     size_t reserve(bool own_cell, bool x_rounded, bool have_out_round, bool x_foreign = true);

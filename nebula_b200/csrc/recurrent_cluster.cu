@@ -266,10 +266,10 @@ bool choose(const nb_handle_s *h, int gates, int H, int B, Shape *best) {
 
 }  // namespace
 
-// Once per handle, when its first recurrent plan is created (the queries cost a handle that has none a millisecond).
-void recurrent_cluster_prepare_device(nb_handle_s *h) {
-    if (h->cc_major != 10 || h->recurrent_ready) return;
-    h->recurrent_ready = true;
+// Once per handle, when a plan first asks whether its layer runs here (a millisecond for the first handle of a process that
+// has such a plan, 0.03 ms for the others).
+static void prepare_device(nb_handle_s *h) {
+    if (h->recurrent_ready) return;
     for (auto &kind : KERNELS)
         for (RecKernel k : kind) {
             NB_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM));
@@ -291,6 +291,7 @@ void recurrent_cluster_prepare_device(nb_handle_s *h) {
         if (cudaOccupancyMaxActiveClusters(&n, KERNELS[1][0], &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
         h->clusters_at_once[CS] = n;
     }
+    h->recurrent_ready = true;
 }
 
 // Fits, and beats a launch per step.  A cluster runs at most 8 rows, so large batches go through it in waves, each of which
@@ -321,8 +322,10 @@ static bool pays(const nb_handle_s *h, int gates, int H, int B, int T, bool line
 }
 
 // On the CUDA cores, whose results do not depend on the batch otherwise, the layer and its steps decide up to 256 rows.
-bool recurrent_cluster_pays(const nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path) {
-    if (h->cc_major != 10) return false;
+bool recurrent_cluster_pays(nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path) {
+    Shape s;
+    if (h->cc_major != 10 || !shape_of(gates, H, 16, 1, &s)) return false;      // (the largest cluster holds the most)
+    prepare_device(h);
     if (step_path != PATH_SIMT) return pays(h, gates, H, B, T, linear, step_path);
     return pays(h, gates, H, 32, T, linear, step_path) && (B <= 256 || pays(h, gates, H, B, T, linear, step_path));
 }
