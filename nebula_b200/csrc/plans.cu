@@ -73,6 +73,7 @@ ConvPlan::ConvPlan(nb_handle_s *hh, const nb_conv2d_desc_t &desc) : nb_plan_s(NB
     rw_wp = std::max((OW - 1) * d.stride + rw_inner / 4, d.width + 2 * d.padding);
     // NEBULA_B200_ROW_WINDOWS=0 (read when the plan is created) sends these layers through the in-kernel gather instead
     const char *rw_env = std::getenv("NEBULA_B200_ROW_WINDOWS");
+    tc_split = conv_tc_split(h, conv_args(nullptr, true).g, d.channels, d.filters);
     rowwin_ok = !(rw_env && *rw_env == '0') && d.channels <= 4 && rw_inner <= 256 && d.stride <= 8 && h->encode_tiled &&
                 h->cc_major == 10;
 }
@@ -137,10 +138,7 @@ bool ConvPlan::can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const {
 int ConvPlan::splits(const ForwardOpts &o) const {
     if (path(o) == PATH_SIMT || o.addend) return 1;
     if (o.residual && ((o.res_c % 4) != 0 || ((uintptr_t)o.residual & 15))) return 1;     // (the reduction reads it in quads)
-    ConvGeom g;
-    g.batch = d.batch; g.C = d.channels; g.H = d.height; g.W = d.width; g.OH = OH; g.OW = OW;
-    g.ksize = d.size; g.stride = d.stride; g.pad = d.padding;
-    return conv_tc_split(h, g, d.channels, d.filters);
+    return tc_split;
 }
 
 // The TMA-fed tensor-core routes write NCHW themselves; the others (CUDA cores, in-kernel gather, K slices) go through

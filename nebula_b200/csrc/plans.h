@@ -77,6 +77,7 @@ struct ConvPlan : nb_plan_s {
     DeviceBuffer x_rowwin;
     DeviceBuffer scale, shift;
     bool has_scale = false, ready = false;
+    int tc_split = 1;           // K slices on the tensor cores: a search over pixel boxes, so done once
     DeviceBuffer x_scratch, y_scratch, split_ws;
     ConvPlan(nb_handle_s *h, const nb_conv2d_desc_t &desc);
     void set_weights(const float *weight, const float *bias, const float *g, const float *m, const float *v, int mem);
