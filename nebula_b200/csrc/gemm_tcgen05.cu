@@ -804,6 +804,18 @@ Box whole_groups(Box box, int OW, int OH, int stride, bool even, double row_byte
     return box;
 }
 
+// filter-column stages: 3x3 / stride 1, at most 128 input channels and filters (the layers that are bound by
+// re-loading activations from L2), a fixed 16 x 8 pixel box; not worth it when the box wastes much of the plane
+// (the row-window layout of a layer with <= 4 input channels has the filter columns folded into its "channels":
+// three filter rows, one column, no padding in w)
+bool column_stages(const ConvGeom &g, int kc, int N) {
+    const int ksize_w = g.ksize_w > 0 ? g.ksize_w : g.ksize;
+    return g.ksize == 3 && g.stride == 1 && g.pad <= 1 &&
+           ((ksize_w == 3 && (g.pad_w < 0 || g.pad_w == g.pad)) || (ksize_w == 1 && g.pad_w == 0)) &&
+           kc <= 128 && N <= 128 && g.OW >= 16 && g.OH >= 8 &&
+           ((double)g.OW / ((g.OW + 15) / 16 * 16)) * ((double)g.OH / ((g.OH + 7) / 8 * 8)) >= 0.8;
+}
+
 void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const cuuint64_t *dims,
             const cuuint64_t *strides_bytes, const cuuint32_t *box, const cuuint32_t *elem_strides) {
     encode_tensor_map(h, tm, base, rank, dims, strides_bytes, box, elem_strides);
@@ -923,14 +935,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     const int taps = g.ksize * ksize_w;
     const bool pool = a.y_pool != nullptr;
     Box box = choose_box(g.OW, g.OH, g.batch, g.stride, pool, S > 1, (double)g.sn * 4.0);
-    // filter-column stages: 3x3 / stride 1, at most 128 input channels and filters (the layers that are bound by
-    // re-loading activations from L2), a fixed 16 x 8 pixel box; not worth it when the box wastes much of the plane
-    // (the row-window layout of a layer with <= 4 input channels has the filter columns folded into its "channels":
-    // three filter rows, one column, no padding in w)
-    const bool col3 = a.a_is_conv && !gather && !three_pass && S == 1 && g.ksize == 3 && g.stride == 1 && g.pad <= 1 &&
-                      ((ksize_w == 3 && (g.pad_w < 0 || g.pad_w == g.pad)) || (ksize_w == 1 && g.pad_w == 0)) &&
-                      kc <= 128 && a.N <= 128 && g.OW >= 16 && g.OH >= 8 &&
-                      ((double)g.OW / ((g.OW + 15) / 16 * 16)) * ((double)g.OH / ((g.OH + 7) / 8 * 8)) >= 0.8;
+    const bool col3 = a.a_is_conv && !gather && !three_pass && S == 1 && column_stages(g, kc, a.N);
     const bool pairs = !col3 && !gather && !three_pass && kc % (2 * BLOCK_K) == 0;      // K slices may be fetched in pairs
     if (col3) box = Box{16, 8, 1};
     // two boxes per tile when the plane is tall enough for 16-row tiles not to waste much of it
@@ -1209,6 +1214,19 @@ int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
     int per = (blocks + S - 1) / S;
     if (c_blocks % 2 == 0) per += per & 1;      // whole pairs of slices: two-block ring stages stay possible
     return (blocks + per - 1) / per;
+}
+
+// A lane of the epilogue owns a pixel, so in NCHW a warp's stores of a column are as contiguous as its box's pixels.  Boxes
+// of many images and few pixels of each (13 x 13 at 128 images: one pixel of 128 images) scatter them: 512 -> 2048 1x1 there
+// 558 us against 175 with a layout pass behind.  Of 360 layers measured, runs of 7 pixels and more and whole planes are the
+// faster for it in all but five (7 x 7 at 32 images, 256 -> 1024: 12.7 against 18.3 us), single pixels never; in between while
+// L2 holds the partial sectors until their neighbours arrive (runs of 2: 10 MB, of 4: 40 MB of output).
+bool conv_tc_writes_nchw(const GemmArgs &a, bool three_pass) {
+    const ConvGeom &g = a.g;
+    if (!three_pass && column_stages(g, a.Kc, a.N)) return true;
+    const Box b = choose_box(g.OW, g.OH, g.batch, g.stride, false, false, (double)g.sn * 4.0);
+    const int run = b.bw == g.OW ? b.bw * b.bh : b.bw;
+    return run >= 7 || (b.bw == g.OW && b.bh == g.OH) || (run >= 2 && 4.0 * a.M * a.N <= 2.5e6 * run * run);
 }
 
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass) {

@@ -226,6 +226,8 @@ bool gemm_tc_supported(const nb_handle_s *h, const GemmArgs &a);
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
 // How many K slices (GemmArgs::split_k) an NHWC convolution should be cut into on the tensor cores; 1: none.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
+// Is an NCHW output (GemmArgs::y_nchw) the faster way for this convolution, against a layout pass behind it?
+bool conv_tc_writes_nchw(const GemmArgs &a, bool three_pass);
 // CUDA-core fp32 path: any extents, strides and alignments.
 void gemm_simt(nb_handle_s *h, const GemmArgs &a);
 // Loads the kernel that gemm_simt takes for these extents (null operands: aligned ones), so that no pass has to.

@@ -141,12 +141,15 @@ int ConvPlan::splits(const ForwardOpts &o) const {
     return tc_split;
 }
 
-// The TMA-fed tensor-core routes write NCHW themselves; the others (CUDA cores, in-kernel gather, K slices) go through
-// a layout pass.
-bool ConvPlan::writes_nchw(const ForwardOpts &o) const {
+// The TMA-fed tensor-core routes write NCHW themselves where their pixel boxes suit it; the others (CUDA cores, in-kernel
+// gather, K slices) go through a layout pass.
+bool ConvPlan::writes_nchw(const ForwardOpts &o) {
     if (o.y_nhwc || h->math_mode == NB_MATH_FP32) return false;
-    if (path(o) == PATH_SIMT) return rowwin_ok;
-    return splits(o) == 1;
+    const bool simt = path(o) == PATH_SIMT, three = h->math_mode == NB_MATH_TF32X3;
+    if (simt ? !rowwin_ok : splits(o) > 1) return false;
+    if (nchw_direct[three] < 0)
+        nchw_direct[three] = conv_tc_writes_nchw(simt ? rowwin_args(nullptr, nullptr, false) : conv_args(nullptr, true), three);
+    return nchw_direct[three] > 0;
 }
 
 // The product of this layer: x as it lies, and as row windows (without the zero columns that fill up a tensor-core K block).

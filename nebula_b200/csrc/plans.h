@@ -78,6 +78,7 @@ struct ConvPlan : nb_plan_s {
     DeviceBuffer scale, shift;
     bool has_scale = false, ready = false;
     int tc_split = 1;           // K slices on the tensor cores: a search over pixel boxes, so done once
+    int nchw_direct[2] = {-1, -1};      // TF32, 3xTF32: does the epilogue write NCHW?  (-1: not asked yet)
     DeviceBuffer x_scratch, y_scratch, split_ws;
     ConvPlan(nb_handle_s *h, const nb_conv2d_desc_t &desc);
     void set_weights(const float *weight, const float *bias, const float *g, const float *m, const float *v, int mem);
@@ -92,7 +93,7 @@ struct ConvPlan : nb_plan_s {
     GemmArgs rowwin_args(const float *xw, const float *weights, bool cuda_cores) const;
     // K slices of the tensor-core path with these options (1: none)
     int splits(const ForwardOpts &o) const;
-    bool writes_nchw(const ForwardOpts &o) const;
+    bool writes_nchw(const ForwardOpts &o);
     // can the following 2x2 stride-2 max-pool be done in this layer's epilogue?
     bool can_fuse_pool() const;
     bool can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const;

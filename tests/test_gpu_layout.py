@@ -51,3 +51,24 @@ def test_shortcut_nchw_quads(handle, shapes, act):
     prev, conn = _x(shapes[0], 1), _x(shapes[1], 2)
     y = handle.shortcut(prev, conn, act)
     assert torch.equal(y, handle.shortcut(_shifted(prev), conn, act))
+
+
+# (B, C, H, F, k): whole planes, long runs of pixels per image, single pixels of many images, runs of two and four
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+@pytest.mark.parametrize("case", [(40, 64, 1, 48, 1), (8, 32, 7, 64, 1), (128, 32, 7, 40, 1), (128, 32, 13, 36, 1), (32, 32, 14, 64, 1), (130, 32, 14, 260, 1),
+                                  (5, 64, 28, 33, 3), (16, 3, 28, 32, 3)], ids=str)
+def test_convolution_to_nchw(handle, case, mode):
+    """NCHW written by the epilogue or by a pass behind it: the NHWC result, bit for bit."""
+    import torch
+    from nebula_b200 import api
+    B, C, H, F, k = case
+    x, w, b = _x((B, C, H, H), 1), _x((F, C, k, k), 2) / (C * k * k) ** 0.5, _x((F,), 3)
+    handle.set_math(mode)
+    ys = []
+    for layout, xi in ((api.LAYOUT_NCHW, x), (api.LAYOUT_NHWC, x.permute(0, 2, 3, 1).contiguous())):
+        plan = api.Conv2d(handle, B, C, H, H, F, k, 1, k // 2, False, "leaky", layout)
+        plan.set_weights(w, b)
+        ys.append(plan.forward(xi))
+        handle.synchronize()
+        plan.close()
+    assert torch.equal(ys[0], ys[1].permute(0, 3, 1, 2))
