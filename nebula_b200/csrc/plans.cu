@@ -382,15 +382,20 @@ GemmPath FcPlan::path() const {
     return h->math_mode == NB_MATH_TF32X3 ? PATH_TC3 : PATH_TC;
 }
 
-// Few rows and a long contraction (weight streaming): split K so that every SM pulls weights.  From 2048 columns on the
-// choice depends on K, N and the SM count only, never from the batch: a batch and its slices add in the same order.  Wide
-// tiles keep the most weight bytes in flight per SM; the split count then fills the SMs, and of the tile widths the one
-// that leaves the fewest SMs idle in the last wave wins.  Shorter contractions are split only for a single row of tiles that
-// leaves three quarters of the SMs idle (DBN at 32 images, 2000 -> 1000: 16 tiles of 63 K blocks took 36 us).
+// Few rows and a long contraction (weight streaming): split K so that every SM pulls weights.  Wide tiles keep the most weight
+// bytes in flight per SM; the split count then fills the SMs, and of the tile widths the one that leaves the fewest SMs idle in
+// the last wave wins.  In TF32 from 2048 columns on all of that depends on K, N and the SM count only: a batch and its slices
+// add in the same order.  The rest depends on the rows as well, so that slices of a batch may differ from it in the last bits:
+// 3xTF32, whose slices cost more to add than they gain once the 128 x 128 tiles of the batch fill a quarter of the SMs, half of
+// them from 8192 columns on (2048 -> 1000 at 512 / 2048 rows: 33 / 90 us split, 36 / 48 us whole; 9216 -> 4096 at 256 / 512:
+// 142 / 234 and 159 / 200); and shorter contractions, split only for a single row of tiles that leaves three quarters of the SMs
+// idle (DBN at 32 images, 2000 -> 1000: 16 tiles of 63 K blocks took 36 us).
 void FcPlan::split_choice(GemmPath pth, bool has_addend, int rows, int *S_out, int *block_n_out) const {
     int S = 1, block_n = 0;
     const int kblocks = (d.inputs + 31) / 32;
+    const long tiles128 = (rows + 127L) / 128 * ((d.outputs + 127) / 128);
     if (pth == PATH_SIMT || has_addend || (d.outputs % 4) != 0) {
+    } else if (pth == PATH_TC3 && d.inputs >= 2048 && 4 * tiles128 > h->sm_count * (d.inputs >= 8192 ? 2L : 1L)) {
     } else if (d.inputs >= 2048) {
         double best = 0.0;
         for (int bn = pth == PATH_TC3 ? 128 : 256; bn >= 64; bn /= 2) {

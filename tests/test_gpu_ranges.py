@@ -86,6 +86,29 @@ def test_rnn_wider_than_a_cluster(handle, mode, case):
     assert_close(y.cpu().numpy(), O.rnn_forward(x, blobs, H, "tanh"), mode, f"rnn {case}", factor=3.0)
 
 
+# (rows, inputs, outputs, launches): a quarter of the SMs filled or not, half of them from 8192 inputs on
+@pytest.mark.parametrize("case", [(600, 2048, 512, 3), (1300, 2048, 512, 2), (130, 8192, 2100, 3), (400, 8192, 3000, 2)], ids=str)
+def test_split_connected_by_rows(handle, case):
+    from nebula_b200 import api
+    from oracle import oracle as O
+    B, inp, out, launches = case
+    rng = np.random.default_rng(inp)
+    x = rng.standard_normal((B, inp), dtype=np.float32)
+    w = (rng.standard_normal((out, inp), dtype=np.float32) / np.sqrt(inp)).astype(np.float32)
+    b = (0.1 * rng.standard_normal(out)).astype(np.float32)
+    handle.set_math("tf32x3")
+    plan = api.Connected(handle, B, inp, out, False, "relu")
+    plan.set_weights(w, b)
+    prepared = plan.prepare()
+    n0 = handle.launch_count()
+    y = plan.forward(_t(x))
+    assert handle.launch_count() - n0 == launches - 1 and plan.workspace_size() == prepared
+    handle.synchronize()
+    plan.close()
+    rows = np.r_[0:40, B - 40:B]
+    assert_close(y.cpu().numpy()[rows], O.connected_forward(x[rows], w, b, "relu"), "tf32x3", f"{case}")
+
+
 # (kind, T, B, hidden, activation, mode, all steps in one launch): batches that go through a cluster in waves
 RECURRENT_CASES = [("lstm", 6, 20, 300, "linear", "tf32", True), ("lstm", 6, 512, 300, "linear", "tf32", False), ("lstm", 5, 400, 420, "linear", "tf32x3", False),
                    ("lstm", 6, 300, 100, "linear", "tf32", True), ("lstm", 4, 1024, 416, "tanh", "tf32", False), ("lstm", 3, 900, 300, "linear", "fp32", False),
