@@ -15,8 +15,8 @@
 //     reads for 128 packed FMAs; the read port is idle three quarters of the time.
 //   * A long contraction with few output tiles is cut into S = 2..8 ranges of K, one CTA each, joined as a cluster:
 //     the partial tiles stay in shared memory, every CTA adds a slice of the tile over the cluster's shared memory in
-//     rank order and writes it.  No workspace, no second launch, no atomics.  S depends on N, K and the pixels of ONE
-//     image, never on the batch, so a batch and its slices add in the same order.
+//     rank order and writes it.  No workspace, no second launch, no atomics.  In layers S depends on N, K and the pixels of
+//     ONE image, never on the batch, so a batch and its slices add in the same order; in _gemm_ it depends on M as well.
 // Measured against the 64 x 64 tile with scalar loads and two barriers per 16 columns (and a 16 x 16 tile for _gemm_)
 // before it: AlexNet b4 in fp32 2938 -> 642 us, 256 x 1024 x 1024 _gemm_ + bias + relu 183 -> 30 us.
 #include <cooperative_groups.h>
@@ -257,6 +257,42 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
     cluster.sync();                     // no CTA may exit while another still reads its partial tile
 }
 
+// _gemm_ with few columns of K and few tiles, where a product is a handful of dependent steps whatever its tiles: 16 x 16
+// outputs per CTA, one per thread, operands loaded straight into both tiles.  Nothing is set up per copy and thread, which is
+// what the kernel above spends such a call on (64 x 64 x 64: 4.3 us here, 6.6 there; 200 x 48 x 16: 2.0 and 3.7).
+__global__ void __launch_bounds__(256) gemm_small_kernel(int ta, int tb, int M, int N, int K, float alpha, const float *A, int lda,
+                                                         const float *B, int ldb, float beta, float *C, int ldc) {
+    __shared__ float As[16][17], Bs[16][17];
+    grid_dependents_start();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int row = blockIdx.y * 16 + ty, col = blockIdx.x * 16 + tx;
+    float acc = 0.0f;
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        const int ka = k0 + tx, kb = k0 + ty;
+        As[ty][tx] = (row < M && ka < K) ? (ta ? A[(size_t)ka * lda + row] : A[(size_t)row * lda + ka]) : 0.0f;
+        Bs[ty][tx] = (col < N && kb < K) ? (tb ? B[(size_t)col * ldb + kb] : B[(size_t)kb * ldb + col]) : 0.0f;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc = fmaf(As[ty][k], Bs[k][tx], acc);
+        __syncthreads();
+    }
+    if (row < M && col < N) {
+        float *c = C + (size_t)row * ldc + col;
+        *c = alpha * acc + (beta == 0.0f ? 0.0f : beta * *c);
+    }
+}
+
+// Fitted to 1101 products of 1 to 2048 rows, 16 to 4096 columns, K of 16 to 1024, timed without host time: what this kernel
+// loses on more tiles than the SMs take at once against what it gains per call, more the fewer 16-byte copies the other can make.
+bool small_gemm(bool ta, bool tb, int M, int N, int K) {
+    const double tiles = (double)((M + 15) / 16) * ((N + 15) / 16);
+    if (K <= 32) return tiles <= 2500;
+    const bool quads = !ta && tb;               // both operands K-contiguous
+    if (K > (quads ? 128 : 256)) return false;
+    const double gain_us = quads ? 1.2 : (ta ? 2.2 + 0.008 * K : (K <= 128 ? 2.4 : 0.9));
+    return (tiles - 230) * 1.2e-4 * K <= gain_us;
+}
+
 typedef void (*SimtKernel)(const SimtParams);
 struct SimtVariant { SimtKernel kernel[3][3]; int bm, bn, threads, smem; };
 
@@ -275,7 +311,7 @@ const SimtVariant VARIANTS[] = {variant<128, 128, 8, 8, 3>(), variant<64, 64, 8,
 const double RATE[] = {1.0, 0.85, 0.7, 0.6};
 
 // Ranges of K: none shorter than 256 columns, and only as many as it takes to occupy the SMs with 64 x 64 tiles of
-// one image (one row of a plain matrix).
+// one image (one row of a connected layer, all rows of _gemm_).
 int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks) {
     const long tiles = ((unit_rows + 63) / 64) * ((N + 63) / 64);
     int S = 1;
@@ -380,6 +416,12 @@ void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
 void launch_sgemm(nb_handle_s *h, bool ta, bool tb, int M, int N, int K, float alpha, const float *A, int lda,
                   const float *B, int ldb, float beta, float *C, int ldc) {
     if ((M + 15) / 16 > 65535) throw Error(NB_ERR_UNSUPPORTED, "gemm: M too large for this operator");
+    if (small_gemm(ta, tb, M, N, K)) {
+        gemm_small_kernel<<<dim3((N + 15) / 16, (M + 15) / 16), 256, 0, h->stream>>>(ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+        check_launch("gemm_small_kernel");
+        count_launch(h);
+        return;
+    }
     SimtParams p{};
     p.a = A; p.b = B;
     p.g = ConvGeom();

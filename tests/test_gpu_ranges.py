@@ -159,3 +159,22 @@ def test_tf32_lstm_of_any_batch_equals_its_slices(handle, H):
         handle.synchronize()
         plan.close()
     assert torch.equal(outs[0], torch.cat(outs[1:], 1))
+
+
+# around the products that _gemm_ runs in 16 x 16 tiles: the last and the first K of either kernel, many tiles, one element
+@pytest.mark.parametrize("ta,tb", [(0, 0), (0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("shape", [(70, 90, 32), (70, 90, 33), (33, 17, 128), (33, 17, 129), (70, 90, 256), (70, 90, 257), (800, 810, 32), (530, 900, 33), (1, 1, 3)], ids=str)
+def test_small_products(handle, shape, ta, tb):
+    """Bound: (K + 4) * 2^-24 * sum|a||b| per element, whatever the order of the additions."""
+    M, N, K = shape
+    rng = np.random.default_rng(K)
+    A = rng.standard_normal((K, M + 1) if ta else (M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K) if tb else (K, N + 1)).astype(np.float32)
+    Cm = rng.standard_normal((M, N + 1)).astype(np.float32)
+    a64 = (A[:, :M].T if ta else A).astype(np.float64)
+    b64 = (B.T if tb else B[:, :N]).astype(np.float64)
+    got = handle.gemm(ta, tb, M, N, K, -0.5, _t(A), A.shape[1], _t(B), B.shape[1], 1.5, _t(Cm), N + 1).cpu().numpy()
+    want = -0.5 * (a64 @ b64) + 1.5 * Cm[:, :N]
+    bound = 2.0 ** -24 * ((K + 4) * 0.5 * (np.abs(a64) @ np.abs(b64)) + 4 * np.abs(Cm[:, :N]) + 4 * np.abs(want))
+    assert (np.abs(got[:, :N] - want) <= bound).all()
+    assert np.array_equal(got[:, N:], Cm[:, N:])
