@@ -85,7 +85,12 @@ __global__ void activation_kernel(float *data, size_t n, int act) {
         const size_t n4 = n / 4;
         float4 *d4 = reinterpret_cast<float4 *>(data);
         for (size_t j = i; j < n4; j += stride) {
-            d4[j] = apply_activation4_fast(d4[j], act);
+            // (four values one by one, inline: with an out-of-line call for the four, or for one, the loads of the next rounds
+            // wait for it; 25.7 M values, relu 33.5 us inline, 40.1 with the call, elu 55 and 73)
+            float4 v = d4[j];
+            v.x = apply_activation(v.x, act); v.y = apply_activation(v.y, act);
+            v.z = apply_activation(v.z, act); v.w = apply_activation(v.w, act);
+            d4[j] = v;
         }
         for (size_t j = n4 * 4 + i; j < n; j += stride) data[j] = apply_activation(data[j], act);
     } else {
