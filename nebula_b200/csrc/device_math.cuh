@@ -124,10 +124,16 @@ __device__ __forceinline__ float apply_activation_fast(float x, int act) {
     return apply_activation_call(x, act);
 }
 
+// relu, leaky and linear only
+__device__ __forceinline__ float4 apply_activation4_cheap(float4 x, int act) {
+    if (act == NB_ACT_LINEAR) return x;
+    if (act == NB_ACT_RELU) return make_float4(x.x > 0.0f ? x.x : 0.0f, x.y > 0.0f ? x.y : 0.0f, x.z > 0.0f ? x.z : 0.0f, x.w > 0.0f ? x.w : 0.0f);
+    auto leaky = [](float v) { return v > 0.0f ? v : (float)(0.1 * (double)v); };
+    return make_float4(leaky(x.x), leaky(x.y), leaky(x.z), leaky(x.w));
+}
+
 __device__ __forceinline__ float4 apply_activation4_fast(float4 x, int act) {
-    if (act == NB_ACT_RELU || act == NB_ACT_LINEAR || act == NB_ACT_LEAKY)
-        return make_float4(apply_activation_fast(x.x, act), apply_activation_fast(x.y, act), apply_activation_fast(x.z, act),
-                           apply_activation_fast(x.w, act));
+    if (act == NB_ACT_RELU || act == NB_ACT_LINEAR || act == NB_ACT_LEAKY) return apply_activation4_cheap(x, act);
     return apply_activation4_call(x, act);
 }
 
