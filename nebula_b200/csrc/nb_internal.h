@@ -336,11 +336,11 @@ std::string trace_report(nb_handle_s *h);
 // reports it for p).  Pointers the driver does not know as an allocation (module globals, host memory) pass.
 void check_extent(nb_handle_s *h, const void *p, long long lo_bytes, long long hi_bytes, const char *what);
 
-// Launches `kernel` so that it may become resident while the kernel before it on the stream still runs (programmatic
+// ahead: launches `kernel` so that it may become resident while the kernel before it on the stream still runs (programmatic
 // dependent launch): the kernel executes grid_dependency_wait() before it touches memory that an earlier kernel may
 // have written or may still read, and nothing before it but constants, weights and its own set-up.
 template <class... P, class... A>
-inline void launch_overlapped(nb_handle_s *h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+inline void launch_kernel(nb_handle_s *h, bool ahead, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -350,8 +350,12 @@ inline void launch_overlapped(nb_handle_s *h, void (*kernel)(P...), dim3 grid, d
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ahead ? 1 : 0;
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // a failure is sticky: check_launch reports it
+}
+template <class... P, class... A>
+inline void launch_overlapped(nb_handle_s *h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+    launch_kernel(h, true, kernel, grid, block, smem, args...);
 }
 
 // Appends the raw bytes of a value to a cache key.
