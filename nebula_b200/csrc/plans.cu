@@ -638,10 +638,11 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
     //    step 0 has nothing to multiply (h_{-1} = 0 and bW is already in pre); otherwise act(bW) is not zero and
     //    step 0 runs the recurrent layer on a zero state like every other step.
     // With linear gate layers on the TF32 tensor-core path, steps 1 .. T-1 run as one cooperative kernel that keeps
-    // the recurrent weights in shared memory (lstm_persistent.cu); step 0 is the cell update alone.
+    // the recurrent weights in shared memory (lstm_persistent.cu); step 0 is the cell update alone.  It stores quads, so a
+    // caller's tensors off a 16-byte boundary take the launch per step.
     const char *lp_env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
     bool persistent = tc_w && !three && linear && hr && (H % 8) == 0 && lstm_persistent_supported(h, T, B, H) &&
-                      !(lp_env && *lp_env == '0');
+                      !(((uintptr_t)out | (uintptr_t)cell) & 15) && !(lp_env && *lp_env == '0');
     if (persistent) {
         launch_lstm_cell(h, pre.p, nullptr, cell, out, hr, B, H);
         ww.ensure_split(h);

@@ -178,3 +178,27 @@ def test_small_products(handle, shape, ta, tb):
     bound = 2.0 ** -24 * ((K + 4) * 0.5 * (np.abs(a64) @ np.abs(b64)) + 4 * np.abs(Cm[:, :N]) + 4 * np.abs(want))
     assert (np.abs(got[:, :N] - want) <= bound).all()
     assert np.array_equal(got[:, N:], Cm[:, N:])
+
+
+@pytest.mark.parametrize("which", ["out", "cell", "x"])
+@pytest.mark.parametrize("H", [64, 40])
+def test_lstm_to_any_address(handle, H, which):
+    """A caller's tensors 4 bytes off a 16-byte boundary: the same results as on one (x: on the CUDA cores, so only close)."""
+    import torch
+    from nebula_b200 import api
+    T, B = 3, 5
+    g = torch.Generator(device="cuda").manual_seed(H)
+    handle.set_math("tf32")
+    plan = api.Lstm(handle, T, B, H, H, False, "linear")
+    plan.set_weights(torch.randn(8 * (H + H * H), device="cuda", generator=g) / H ** 0.5)
+    x = torch.randn(T * B * H, device="cuda", generator=g)
+    def run(off):
+        t = {k: torch.zeros(T * B * H + 4, device="cuda")[off.get(k, 0):][:T * B * H] for k in ("x", "out", "cell")}
+        t["x"].copy_(x)
+        handle.check(handle.lib.nb_lstm_forward(plan.p, t["x"].data_ptr(), t["out"].data_ptr(), t["cell"].data_ptr()))
+        handle.synchronize()
+        return t["out"].clone(), t["cell"].clone()
+    want, got = run({}), run({which: 1})
+    plan.close()
+    for a, b in zip(want, got):
+        assert torch.equal(a, b) if which != "x" else float((a - b).abs().max()) <= 1e-3 * float(a.abs().max())
