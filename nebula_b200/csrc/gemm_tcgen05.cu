@@ -1201,8 +1201,9 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
 // A convolution of one or a few small images has fewer tiles than SMs, and its tiles run their whole K alone: at about 0.15 us
 // per 32-column block (two TMA requests of one thread) the 3x3 layers of a single ResNet-50 image (8 tiles, 72 and 144
 // blocks) took 29 and 47 us.  Such layers are cut along K until they occupy the SMs, four blocks per slice at least; the
-// slices are added by splitk_reduce4_kernel (2-3 us), so layers of fewer than 32 blocks stay whole.  Layers with more
-// tiles than half the SMs are never cut: their results do not depend on the batch.
+// slices are added by splitk_reduce4_kernel (2-3 us), so layers of fewer than 32 blocks stay whole.  Tiles are counted over the
+// whole batch, so an image alone and the same image in a batch that leaves the layer whole, or cuts it into fewer slices, add
+// in different orders and may differ in the last bits.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
     const int c_blocks = (Kc + BLOCK_K - 1) / BLOCK_K, blocks = g.ksize * (g.ksize_w > 0 ? g.ksize_w : g.ksize) * c_blocks;
     if (blocks < 32 || (N % 4) != 0) return 1;

@@ -202,3 +202,29 @@ def test_lstm_to_any_address(handle, H, which):
     plan.close()
     for a, b in zip(want, got):
         assert torch.equal(a, b) if which != "x" else float((a - b).abs().max()) <= 1e-3 * float(a.abs().max())
+
+
+# (images, of them alone, C, H, F, k): a convolution cut along K for the few images and not, or otherwise, for the many
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+@pytest.mark.parametrize("case", [(64, 1, 256, 7, 96, 3), (40, 4, 512, 7, 512, 3), (30, 2, 1024, 7, 64, 1), (9, 3, 128, 14, 256, 3)], ids=str)
+def test_few_images_of_a_batch(handle, mode, case):
+    """Small batches are cut along K where large ones are not, so an image alone and in its batch add in different orders.  Both
+    are sums of the same products: they differ by at most the truncations of their accumulations, 2^-23 of sum|a||b| for each of
+    the K / 8 steps and the slices on either side (3xTF32: promoted every 12 steps, and the rounding of two operands' low terms)."""
+    from nebula_b200 import api
+    B, n, C, H, F, k = case
+    rng = np.random.default_rng(C)
+    x = rng.standard_normal((B, H, H, C), dtype=np.float32)
+    w = (rng.standard_normal((F, C, k, k)) * np.sqrt(2.0 / (C * k * k))).astype(np.float32)
+    handle.set_math(mode)
+    ys = []
+    for images in (x, x[B - n:]):
+        plan = api.Conv2d(handle, len(images), C, H, H, F, k, 1, k // 2, False, "linear", api.LAYOUT_NHWC)
+        plan.set_weights(w, np.zeros(F, np.float32))
+        ys.append(plan.forward(_t(images)).cpu().numpy().astype(np.float64)[-n:])
+        handle.synchronize()
+        plan.close()
+    xp = np.pad(np.abs(x[B - n:]).astype(np.float64), ((0, 0), (k // 2,) * 2, (k // 2,) * 2, (0, 0)))
+    size = sum(xp[:, i:i + H, j:j + H] @ np.abs(w[:, :, i, j]).T.astype(np.float64) for i in range(k) for j in range(k))
+    steps = 2 * (C * k * k / 8 + 16) if mode == "tf32" else 2 * (12 + C * k * k / 96 + 16) + 4
+    assert (np.abs(ys[0] - ys[1]) <= steps * 2.0 ** -23 * size).all()
