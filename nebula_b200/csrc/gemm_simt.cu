@@ -259,26 +259,30 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
 
 // _gemm_ with few columns of K and few tiles, where a product is a handful of dependent steps whatever its tiles: 16 x 16
 // outputs per CTA, one per thread, operands loaded straight into both tiles.  Nothing is set up per copy and thread, which is
-// what the kernel above spends such a call on (64 x 64 x 64: 4.3 us here, 6.6 there; 200 x 48 x 16: 2.0 and 3.7).
+// what the kernel above spends such a call on (64 x 64 x 64: 4.3 us here, 6.6 there; 200 x 48 x 16: 2.0 and 3.7).  It adds in
+// the same order (even and odd columns apart): the two give the same bits, and half the chain of one sum.
 __global__ void __launch_bounds__(256) gemm_small_kernel(int ta, int tb, int M, int N, int K, float alpha, const float *A, int lda,
                                                          const float *B, int ldb, float beta, float *C, int ldc) {
     __shared__ float As[16][17], Bs[16][17];
     grid_dependents_start();
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int row = blockIdx.y * 16 + ty, col = blockIdx.x * 16 + tx;
-    float acc = 0.0f;
+    float even = 0.0f, odd = 0.0f;
     for (int k0 = 0; k0 < K; k0 += 16) {
         const int ka = k0 + tx, kb = k0 + ty;
         As[ty][tx] = (row < M && ka < K) ? (ta ? A[(size_t)ka * lda + row] : A[(size_t)row * lda + ka]) : 0.0f;
         Bs[ty][tx] = (col < N && kb < K) ? (tb ? B[(size_t)col * ldb + kb] : B[(size_t)kb * ldb + col]) : 0.0f;
         __syncthreads();
 #pragma unroll
-        for (int k = 0; k < 16; k++) acc = fmaf(As[ty][k], Bs[k][tx], acc);
+        for (int k = 0; k < 16; k += 2) {
+            even = fmaf(As[ty][k], Bs[k][tx], even);
+            odd = fmaf(As[ty][k + 1], Bs[k + 1][tx], odd);
+        }
         __syncthreads();
     }
     if (row < M && col < N) {
         float *c = C + (size_t)row * ldc + col;
-        *c = alpha * acc + (beta == 0.0f ? 0.0f : beta * *c);
+        *c = alpha * (even + odd) + (beta == 0.0f ? 0.0f : beta * *c);
     }
 }
 

@@ -228,3 +228,17 @@ def test_few_images_of_a_batch(handle, mode, case):
     size = sum(xp[:, i:i + H, j:j + H] @ np.abs(w[:, :, i, j]).T.astype(np.float64) for i in range(k) for j in range(k))
     steps = 2 * (C * k * k / 8 + 16) if mode == "tf32" else 2 * (12 + C * k * k / 96 + 16) + 4
     assert (np.abs(ys[0] - ys[1]) <= steps * 2.0 ** -23 * size).all()
+
+
+def test_small_products_in_the_order_of_large_ones(handle):
+    """The first rows of a product that runs in 16 x 16 tiles and of one of more rows that does not, bit for bit."""
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(0)
+    for K in (40, 100):
+        a, b = torch.randn(2048, K, device="cuda", generator=g), torch.randn(1000, K, device="cuda", generator=g)
+        outs = []
+        for M in (64, 2048):
+            c = torch.empty(M, 1000, device="cuda")
+            handle.gemm(False, True, M, 1000, K, 1.0, a, K, b, K, 0.0, c, 1000)
+            outs.append(c[:64])
+        assert torch.equal(*outs)
