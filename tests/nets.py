@@ -18,7 +18,7 @@ def tiny_vgg(batch=4):
 
 
 def mid_vgg(batch=2):
-    """Big enough (56x56, 64/128 channels) for the 3x3 halo kernel and its fused pooling."""
+    """Big enough (56x56, 64/128 channels) for the filter-column stages and their fused pooling."""
     return vgg16(batch=batch, height=56, width=56, fc=64, classes=10, widths=(64, 128, 64, 64, 64))
 
 

@@ -1,4 +1,4 @@
-"""Calls queued behind one another, each on new inputs: every one must give what it gives when it is waited for."""
+"""Calls and passes queued behind one another, each on new inputs: every one must give what it gives when it is waited for."""
 import numpy as np
 import pytest
 
@@ -40,3 +40,29 @@ def test_gathered_convolutions(handle, mode, layout, case):
     ref = O.conv_forward(np.ascontiguousarray(nchw(xs[-1]).cpu().numpy()), w.cpu().numpy(), bias.cpu().numpy(), k, s, p, "relu", None)
     assert_close(nchw(queued[-1]).cpu().numpy(), ref, mode, f"gathered conv {case}")
     plan.close()
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3", "fp32"])
+@pytest.mark.parametrize("name", ["toy_convnet", "tiny_resnet", "mid_vgg", "tiny_lstm", "dbn", "rnn"])
+def test_passes_on_other_inputs(handle, name, mode):
+    """Passes of a network queued on three inputs in turn, the last one read: a pass that left an earlier one's output would show."""
+    import torch
+    from nebula_b200 import api, workloads
+    from tests import nets
+    wl = (workloads.dbn(batch=5, height=32, width=32) if name == "dbn" else
+          workloads.rnn2(batch=9, time_steps=5, input_size=40, hidden=72, classes=50) if name == "rnn" else getattr(nets, name)(3))
+    handle.set_math(mode)
+    net = api.Network(handle, wl.cfg)
+    net.load_weights(wl.make_weights(11))
+    xs = [torch.from_numpy(wl.make_input(s)).cuda() for s in (1, 2, 3)]
+    alone = []
+    for x in xs:
+        net.forward(x)
+        handle.synchronize()
+        alone.append(net.logits().copy())
+    for last in range(3):
+        for k in range(6):
+            net.forward(xs[(last + k + 1) % 3])
+        handle.synchronize()
+        assert (net.logits() == alone[last]).all()
+    net.close()
