@@ -17,8 +17,11 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIBDIR = PKG / "lib"
 LIB = LIBDIR / "libnebula_b200.so"
-SOURCES = ["api.cu", "network.cu", "plans.cu", "elementwise.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "static_scratch.cu", "arena.cu", "lstm_persistent.cu",
-           "recurrent_cluster.cu"]
+# (source, object name, extra flags)
+SOURCES = [(s, s, []) for s in ("api.cu", "network.cu", "plans.cu", "elementwise.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "static_scratch.cu",
+                                "arena.cu", "lstm_persistent.cu", "recurrent_cluster.cu")]
+# the CUDA-core contraction, a module per pair of copy modes (gemm_simt.cuh)
+SOURCES += [("gemm_simt_kernels.cu", f"gemm_simt_kernels_{a}{b}", [f"-DNB_SIMT_A={a}", f"-DNB_SIMT_B={b}"]) for a in range(3) for b in range(3)]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr", "-Xptxas", "-v"]
 
@@ -43,11 +46,12 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     objdir.mkdir(exist_ok=True)
     nvcc = _nvcc()
 
-    def compile_one(src: str):
-        obj = objdir / (src + ".o")
-        cmd = [nvcc, *NVCC_FLAGS, "-c", str(CSRC / src), "-o", str(obj)]
+    def compile_one(item):
+        src, name, flags = item
+        obj = objdir / (name + ".o")
+        cmd = [nvcc, *NVCC_FLAGS, *flags, "-c", str(CSRC / src), "-o", str(obj)]
         r = subprocess.run(cmd, capture_output=True, text=True)
-        (objdir / (src + ".log")).write_text(r.stdout + r.stderr)
+        (objdir / (name + ".log")).write_text(r.stdout + r.stderr)
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed on {src}:\n{r.stderr[-4000:]}")
         if verbose:
