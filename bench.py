@@ -323,13 +323,8 @@ def gpu_arm(args):
         tf32_peak = peaks["bf16_sustained"] / 2.0
         if args.math == "tf32x3":
             tf32_peak /= 3.0
-        # dominant kernel: whichever tensor-core contraction kernel took more device time in the timed region
-        kernels = {"gemm_tf32_tcgen05_kernel": ("tc_ms", "tc_flops", "tc_launches"),
-                   "conv3x3_halo_tcgen05_kernel": ("halo_ms", "halo_flops", "halo_launches")}
-        dom = max(kernels, key=lambda k: prof[kernels[k][0]])
-        other = [k for k in kernels if k != dom][0]
-        d_ms, d_fl, d_n = (prof[f] for f in kernels[dom])
-        o_ms, o_fl, o_n = (prof[f] for f in kernels[other])
+        dom = "gemm_tf32_tcgen05_kernel"
+        d_ms, d_fl, d_n = prof["tc_ms"], prof["tc_flops"], prof["tc_launches"]
         achieved = d_fl / (d_ms / 1e3) / 1e12 if d_ms > 0 else 0.0
         # dram__bytes_read + dram__bytes_write per launch of the dominant kernel: not something a run can measure on
         # itself; taken from the table of ncu captures kept with the package (null when this workload has none)
@@ -367,12 +362,6 @@ def gpu_arm(args):
                                      else "the region `value` comes from",
                          "kernel": dom,
                          "launches_per_step": d_n / K, "kernel_ms_per_step": round(d_ms / K, 4),
-                         "other_tensor_kernel": {"kernel": other, "launches_per_step": o_n / K,
-                                                 "ms_per_step": round(o_ms / K, 4),
-                                                 "achieved": round(o_fl / (o_ms / 1e3) / 1e12, 2) if o_ms > 0 else 0.0},
-                         "all_tensor_kernels": {"ms_per_step": round((d_ms + o_ms) / K, 4),
-                                                "achieved": round((d_fl + o_fl) / ((d_ms + o_ms) / 1e3) / 1e12, 2)
-                                                if d_ms + o_ms > 0 else 0.0},
                          "peak_source": f"{peaks['source']}: bf16 cuBLAS sustained {peaks['bf16_sustained']} TFLOP/s / 2 "
                                         "(dense TF32 rate is half the bf16 rate)" + (" / 3 products" if args.math == "tf32x3" else ""),
                          "other_contraction_ms_per_step": round(prof["simt_ms"] / K, 4)},
