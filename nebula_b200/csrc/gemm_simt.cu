@@ -173,6 +173,7 @@ void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
 // four transpose cases), unlike the reference's CUDA stand-in (common/gemm.cu:38-153) which ignores lda/ldb/ldc.
 void launch_sgemm(nb_handle_s *h, bool ta, bool tb, int M, int N, int K, float alpha, const float *A, int lda,
                   const float *B, int ldb, float beta, float *C, int ldc) {
+    // (the operator has refused more rows since its first kernel, whose grid they did not fit; the limit is part of it by now)
     if ((M + 15) / 16 > 65535) throw Error(NB_ERR_UNSUPPORTED, "gemm: M too large for this operator");
     if (small_gemm(ta, tb, M, N, K)) {
         gemm_small_kernel<<<dim3((N + 15) / 16, (M + 15) / 16), 256, 0, h->stream>>>(ta, tb, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
