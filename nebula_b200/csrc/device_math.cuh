@@ -133,7 +133,9 @@ __device__ __forceinline__ float4 apply_activation4_cheap(float4 x, int act) {
 }
 
 __device__ __forceinline__ float4 apply_activation4_fast(float4 x, int act) {
-    if (act == NB_ACT_RELU || act == NB_ACT_LINEAR || act == NB_ACT_LEAKY) return apply_activation4_cheap(x, act);
+    if (act == NB_ACT_RELU || act == NB_ACT_LINEAR || act == NB_ACT_LEAKY)
+        return make_float4(apply_activation_fast(x.x, act), apply_activation_fast(x.y, act), apply_activation_fast(x.z, act),
+                           apply_activation_fast(x.w, act));
     return apply_activation4_call(x, act);
 }
 
