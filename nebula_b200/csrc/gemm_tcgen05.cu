@@ -886,7 +886,7 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra) {
     key_add(k, a.act); key_add(k, a.round_out_tf32); key_add(k, a.y); key_add(k, a.ldy); key_add(k, a.y_nchw); key_add(k, a.y_pool);
     key_add(k, a.lstm_H); key_add(k, a.lstm_c_prev); key_add(k, a.lstm_c); key_add(k, a.lstm_h); key_add(k, a.lstm_h_round);
     key_add(k, a.b_static);
-    key_add(k, a.split_k); key_add(k, a.block_n_hint); key_add(k, a.algo_flops);
+    key_add(k, a.split_k); key_add(k, a.block_n_hint); key_add(k, a.k_part); key_add(k, a.algo_flops);
     return k;
 }
 
@@ -998,7 +998,8 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     // tile width in filters: widest tile that still gives every SM work
     // Promoted accumulation: always for 3xTF32 (its point is fp32-level agreement); in TF32 mode only for
     // very long contractions, where the accumulator's round-toward-zero bias (~K * 7.5e-9) nears TF32's own error.
-    const bool promote = three_pass || (long)p.kb_per_split * BLOCK_K >= 8192;   // per split when K is split
+    const bool promote = three_pass || (long)p.kb_per_split * BLOCK_K >= 8192 ||  // per split when K is split
+                         (a.k_part > 0 && a.k_part < p.kb_per_split);
     int block_n = 256;
     if (three_pass || gather || promote) block_n = 128;
     if (a.block_n_hint) block_n = std::min(block_n, a.block_n_hint);
@@ -1024,7 +1025,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     // accumulation chains of at most 512 K elements (TF32) / 12 MMAs (3xTF32) in the tensor core: every accumulating MMA
     // truncates the running sum (a shrink of about 6e-8 per step that adds up layer after layer).  A 3xTF32 K block is
     // 12 MMAs, of which only the 4 hi*hi ones go into the promoted chain (the cross terms have columns of their own)
-    p.kb_per_part = !promote ? p.kb_per_split : (three_pass ? 3 : 16);
+    p.kb_per_part = !promote ? p.kb_per_split : (three_pass ? 3 : (a.k_part > 0 ? a.k_part : 16));
     p.parts = (p.kb_per_split + p.kb_per_part - 1) / p.kb_per_part;
 
     // two K blocks per ring stage: tiles of up to 128 columns whose K slices pair up, a box of whole 8-row groups (the

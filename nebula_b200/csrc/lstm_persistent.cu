@@ -1,19 +1,34 @@
-// The recurrence of one LSTM layer as ONE cooperative kernel over all time steps (lstm_layer.cc:262-311 per step).
+// The recurrence of one LSTM layer as ONE cooperative kernel over all time steps (lstm_layer.cc:250-311 per step), TF32 mode.
 //
-// A launch per time step costs about 20 us on this part for a 64 x 4096 x 1024 product that needs 3: pipeline fill,
-// 32 small K blocks issued by single lanes, launch gaps.  Here every CTA owns 32 gate columns (8 hidden units x
-// i,f,g,o), keeps its 32 x H slice of the recurrent weights in shared memory for the whole sequence (128 KB at
-// H = 1024, loaded once by TMA) and the cell state of its units in registers.  Per step it streams h_{t-1} (rounded
-// to TF32, [B x H]) from L2 into a ring of 128-byte-swizzled K blocks with plain loads, multiplies on the tensor core
-// (tcgen05.mma kind::tf32, M = 128, N = 32, accumulator in TMEM), adds the input-side pre-activations, runs the cell
-// update and writes c_t, h_t and the rounded h_t.  A grid-wide barrier (one atomic counter, bounded spin) separates
-// the steps: step t + 1 of every CTA reads what all CTAs wrote in step t.
+// Bound by the latency of a step: a launch per step costs 12 to 20 us on this part for a 64 x 4096 x 1024 product that needs 1.
+// Clusters of four CTAs own 32 hidden units (128 gate columns) each, and each CTA of a cluster a quarter of K:
+//   * its 128 x K/4 slice of the recurrent weights stays in tensor memory for the whole sequence, as the A operand of the MMAs
+//     (M = gate columns, N = batch rows, K = 8): an MMA then reads nothing from shared memory but h, and its time falls with the
+//     batch;
+//   * per step it loads only its quarter of h_{t-1} (rounded to TF32) from L2 by TMA: 64 KB at B = 64, H = 1024;
+//   * its partial sums leave for the four CTAs over distributed shared memory (st.async onto the receiver's mbarrier): TMEM lanes
+//     32 q .. 32 q + 31 hold the eight units that CTA q finishes.  The receiver adds them in the
+//     order of K, adds the input-side pre-activations, runs the cell update and writes c_t, h_t and the rounded h_t.
+// Steps are chained through one arrival counter per K block of h (the warps of four CTAs write it): a lane per block polls its counter
+// (bounded) and issues that block's copy, so a CTA waits only for the units it reads.
+// Against one CTA per 32 columns with all of K in shared memory (M = batch rows, N = 32: 128 MMAs of 40 cycles, 256 KB of h per
+// CTA and step, one grid-wide counter): T128 B64 H1024 9.3 -> 5.4 us a step,
+// and two such layers with their projection 2963 -> 1950 us.
 //
-// h_{t-1} was written by other SMs' ordinary stores earlier in this same kernel and is read here by TMA, i.e. through
-// the async proxy: the writers release (a release-add on the barrier counter), the thread that issues the copies acquires
-// the counter itself and then issues fence.proxy.async before its first copy of the step.  (A first version read h with ld.global.cg from
-// 128 threads: correct, but 63 us per step, three times slower than a launch per step.)  The results are bit-identical
-// to the per-step path (same K order, same fp32 cell arithmetic).
+// A step is a chain of latencies (publishing 1300 cycles, polling 1000, a copy 700, MMAs 400, the exchange 700, a cell 1100; the
+// rest is waiting for the slowest of its peers), not of volume: with an eighth of h copied it takes 0.2 us less.  So the batch
+// runs as four groups of rows, each a chain of its own with its own warps, barriers and counters (one group 2082 us, two 1985,
+// four 1949), and every warp publishes by itself.
+//
+// Why a step's buffers need no release by their reader.  A CTA starts the MMAs of step t + 2 after every unit of its quarter of
+// h_{t+1} is published; each of those took the partial sums of step t + 1 of all four CTAs of its cluster, one of which read
+// the units of h_t that this CTA published after it had read its accumulators and its received sums of step t.  So two
+// accumulators, two receive buffers and two barriers per kind, by the parity of the step, are enough.
+//
+// h_{t-1} was written by other SMs' ordinary stores earlier in this same kernel and is read here by TMA, i.e. through the async
+// proxy: the writers release (a release-add on the block's counter), the lane that issues the copy acquires the counter itself
+// and then issues fence.proxy.async.  The results are bit-identical to the launch-per-step path: it sums the same quarters of K
+// and adds them in the same order (lstm_k_part), step 0 and the cell use the same formulas.
 #include <cstring>
 
 #include "tc_common.cuh"
@@ -24,22 +39,31 @@ using namespace tc;
 
 namespace {
 
-constexpr int LP_N = 32;                    // gate columns per CTA
-constexpr int LP_STAGES = 4;                // most ring stages (barrier slots)
-constexpr int LP_THREADS = 192;             // warps 0-3: epilogue; warp 4: MMA issue; warp 5: grid barrier and TMA
-constexpr int LP_W_TILE = LP_N * 128;       // one K block of the weight slice: 32 rows x 128 bytes
+constexpr int LP_SLICES = 4;                // CTAs of a cluster = slices of K
+constexpr int LP_UNITS = 32;                // hidden units of a cluster = columns of a K block of h
+constexpr int LP_CELL_WARPS = 16;           // warps 0-15: accumulators and cells of all groups of rows
+constexpr int LP_GROUPS = 4;                // groups of batch rows; each has a warp for its MMAs and one for its h_{t-1} too
+constexpr int LP_THREADS = 32 * (LP_CELL_WARPS + 2 * LP_GROUPS);
+constexpr int LP_MAX_STAGES = 16;           // of a group
+constexpr int LP_SMEM = 227 * 1024;
+constexpr int LP_TMEM = 512;
+constexpr int LP_COUNTER_STRIDE = 32;       // words: a counter per 128-byte line
+constexpr int LP_MAX_BLOCKS = 48;           // K blocks that have a counter
+constexpr int LP_BARS = 2 * LP_MAX_STAGES + 4;      // barriers of a group
 
 struct LstmPParams {
-    CUtensorMap tm_w;           // recurrent weights [4H rows][H], box {32, 32}
-    CUtensorMap tm_h;           // rounded hidden states as {32, T*B rows, H/32}, box {32, B, cbs}
-    int cbs;                    // K blocks per ring stage and TMA request (2 when B % 8 == 0 and H % 64 == 0)
-    int stages, stage_bytes;    // ring geometry: a stage holds cbs slices of B rows and the 128-row window of the last
+    CUtensorMap tm_h;           // rounded hidden states [T][B][H], box {32, Rg, 1}: rows past B arrive as zeros
+    const float *w;             // recurrent weights [4H][H], rows [unit][i,f,g,o], TF32-rounded
     const float *pre;           // [T][B][4H] input-side pre-activations (biases included), columns [unit][i,f,g,o]
-    float *hr_w;                // [T][B][H] rounded hidden states: step t writes [t]; step t + 1 reads it through tm_h
+    float *hr;                  // [T][B][H] rounded hidden states: step t writes [t]; step t + 1 reads it through tm_h
     float *cell, *out;          // [T][B][H]
     int T, B, H;
-    int t_first;                // first step this kernel runs (the steps before it are in cell/out/hr already)
-    unsigned int *sync;         // grid barrier counter, zero at launch
+    int chunk_rows;             // batch rows of a set of clusters
+    int Rg;                     // rows of a group, the MMA's N (a multiple of 16)
+    int kb_per_slice;           // K blocks per CTA (the last ones may have fewer, or none)
+    int slices;                 // CTAs of a cluster that have K blocks
+    int stages;                 // ring slots of a group, Rg x 32 floats each
+    unsigned int *sync;         // a counter per group and K block, then the exit counter; all zero between launches
     int *status;
 };
 
@@ -51,74 +75,134 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p) {
 __device__ __forceinline__ void red_release_add(unsigned int *p, unsigned int v) {
     asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void st_async_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(dst), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
+}
+// mbar_wait for data that other CTAs of the cluster stored
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int *abort_flag, int *status) {
+    const long long t0 = clock64();
+    for (;;) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+        if (*abort_flag) return false;
+        if (clock64() - t0 > WAIT_LIMIT_CYCLES) {
+            *abort_flag = 1;
+            atomicExch(status, (int)DEV_TIMEOUT);
+            return false;
+        }
+    }
+}
 
+// ITEMS: cells that a thread finishes (16 warps of 8 units x 4 rows), 1 up to 64 rows, else 2.
+template <int ITEMS>
 __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __grid_constant__ LstmPParams p) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    const int KB = p.H / BLOCK_K;                           // K blocks per step
-    uint8_t *w_smem = smem;                                  // [KB][32 rows][128 B], swizzled by TMA
-    uint8_t *a_ring = smem + (size_t)KB * LP_W_TILE;         // [LP_STAGES][128 rows][128 B]
-    const int stages = p.stages, stage_bytes = p.stage_bytes, cbs = p.cbs;
-    uint64_t *bars = (uint64_t *)(a_ring + stages * stage_bytes);
-    uint64_t *full = bars;                  // loaders -> MMA   [LP_STAGES]
-    uint64_t *empty = bars + LP_STAGES;     // MMA -> loaders   [LP_STAGES]
-    uint64_t *w_full = bars + 2 * LP_STAGES;
-    uint64_t *acc_full = w_full + 1;
-    uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    // the group of rows this warp works for: its place among the cell warps, the MMA warps, the TMA warps
+    constexpr int CW = LP_CELL_WARPS / LP_GROUPS;
+    const int grp = warp < LP_CELL_WARPS ? warp / CW : (warp - LP_CELL_WARPS) % LP_GROUPS;
+    const int stage_bytes = p.Rg * 128, stages = p.stages;
+    const int KB = (p.H + BLOCK_K - 1) / BLOCK_K;
+    const int rank = blockIdx.x % LP_SLICES, cluster = blockIdx.x / LP_SLICES % KB, chunk = blockIdx.x / LP_SLICES / KB;
+    const int row0 = chunk * p.chunk_rows + grp * p.Rg;     // the group's first row
+    const int rows = max(0, min(p.Rg, min((chunk + 1) * p.chunk_rows, p.B) - row0)), row_end = row0 + rows;
+    unsigned int *counters = p.sync + (size_t)(chunk * LP_GROUPS + grp) * KB * LP_COUNTER_STRIDE;     // of this group's rows
+    const int quads = (rows + 3) / 4;                        // groups of four batch rows
+    const int recv_floats = p.Rg * 32;                       // one CTA's partial sums of a group for this CTA's 32 gate columns
+    uint8_t *ring = smem + grp * stages * stage_bytes;       // [stages][Rg rows][128 B], 128-byte swizzle
+    float *recv = (float *)(smem + LP_GROUPS * stages * stage_bytes) + grp * 2 * LP_SLICES * recv_floats;   // [parity][source][quad][gate * 8 + unit][4 rows]
+    uint64_t *bars = (uint64_t *)(smem + LP_GROUPS * (stages * stage_bytes + 2 * LP_SLICES * recv_floats * 4));
+    uint64_t *full = bars + grp * LP_BARS;                   // TMA -> MMA
+    uint64_t *empty = full + LP_MAX_STAGES;                  // MMA -> TMA
+    uint64_t *acc_full = empty + LP_MAX_STAGES;              // MMA -> accumulator readers, by parity
+    uint64_t *recv_full = acc_full + 2;                      // partial sums of all slices have arrived, by parity
+    uint32_t *tmem_slot = (uint32_t *)(bars + LP_GROUPS * LP_BARS);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < LP_STAGES; s++) {
+    const int kb0 = rank * p.kb_per_slice, nkb = max(0, min(p.kb_per_slice, KB - kb0));
+    const int cell_warps = min(CW, p.Rg / 4);               // of a group, with rows to send or to finish
+    const uint32_t recv_bytes = (uint32_t)(p.slices * quads * 32 * 16);
+    if (warp < LP_CELL_WARPS && warp % CW == 0 && lane == 0) {
+        for (int s = 0; s < LP_MAX_STAGES; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(w_full, 1);
-        mbar_init(acc_full, 1);
-        *abort_flag = 0;
+        for (int a = 0; a < 2; a++) {
+            mbar_init(&acc_full[a], 1);
+            mbar_init(&recv_full[a], 1);
+        }
+        if (warp == 0) *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mbar_expect_tx(&recv_full[0], recv_bytes);          // a phase is armed one round ahead of its data
+        mbar_expect_tx(&recv_full[1], recv_bytes);
     }
-    if (warp == 4) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(32u)
+    if (warp == LP_CELL_WARPS) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)LP_TMEM)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // rows of the A tiles that no batch row fills: the MMA reads all 128, give them a defined value once
-    for (int i = threadIdx.x; i < stages * stage_bytes / 16; i += blockDim.x)
-        reinterpret_cast<float4 *>(a_ring)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int n0 = blockIdx.x * LP_N;                       // first gate column of this CTA
-    const unsigned int ctas = gridDim.x;
+    const uint32_t w_col = tmem_base + (uint32_t)(2 * LP_GROUPS * p.Rg), acc_col = tmem_base + (uint32_t)(2 * grp * p.Rg);
+
+    if (warp < LP_CELL_WARPS) {
+        // this CTA's slice of the weights: TMEM lane 32 q + 8 g + u holds gate g of unit 8 q + u of the cluster
+        const int unit = cluster * LP_UNITS + 8 * (warp & 3) + (lane & 7);
+        const float *src = p.w + ((long)4 * unit + (lane >> 3)) * p.H;
+        for (int i = warp >> 2; i < nkb; i += LP_CELL_WARPS / 4) {
+            const int k0 = (kb0 + i) * BLOCK_K;
+            uint32_t v[32];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {               // (H is a multiple of 4: quads lie inside the row or outside)
+                const float4 x = unit < p.H && k0 + j < p.H ? __ldg(reinterpret_cast<const float4 *>(src + k0 + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[j] = __float_as_uint(x.x); v[j + 1] = __float_as_uint(x.y); v[j + 2] = __float_as_uint(x.z); v[j + 3] = __float_as_uint(x.w);
+            }
+            tmem_st_32x32(w_col + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(i * BLOCK_K), v);
+        }
+        tmem_st_wait();
+        tc_fence_before();
+    }
+    __syncthreads();
+    // every CTA of the cluster has its barriers ready before a peer's stores arrive
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    tc_fence_after();
     bool ok = true;
 
-    if (warp == 4) {
-        // ------------------------------------------------ weights (once), then the MMAs of every step
+    if (rows == 0) {
+        // (fewer rows than groups)
+    } else if (warp >= LP_CELL_WARPS && warp < LP_CELL_WARPS + LP_GROUPS) {
+        // ------------------------------------------------ the MMAs of every step
         if (elect_one()) {
-            mbar_expect_tx(w_full, (uint32_t)(KB * LP_W_TILE));
-            for (int kb = 0; kb < KB; kb++) tma_load_3d(w_smem + kb * LP_W_TILE, &p.tm_w, w_full, kb * BLOCK_K, n0, 0);
-            ok = mbar_wait(w_full, 0, abort_flag, p.status);
-            const uint32_t idesc = p.B <= 64 ? make_idesc(64, LP_N) : make_idesc(BLOCK_M, LP_N);     // 64-row MMAs for small batches
+            const uint32_t idesc = make_idesc(BLOCK_M, p.Rg);
             int stage = 0;
             uint32_t phase = 0;
-            for (int t = p.t_first; t < p.T && ok; t++) {
-                for (int kb = 0; kb < KB; kb += cbs) {
+            for (int t = 1; t < p.T && nkb > 0 && ok; t++) {
+                const uint32_t d = acc_col + (uint32_t)((t & 1) * p.Rg);
+                for (int i = 0; i < nkb; i++) {
                     if (!(ok = mbar_wait(&full[stage], phase, abort_flag, p.status))) break;
                     tc_fence_after();
-                    for (int c = 0; c < cbs; c++) {
-                        const uint32_t a_lo = smem_desc_lo(smem_u32(a_ring + stage * stage_bytes + c * p.B * 128));
-                        const uint32_t b_lo = smem_desc_lo(smem_u32(w_smem + (kb + c) * LP_W_TILE));
+                    const uint32_t b_lo = smem_desc_lo(smem_u32(ring + stage * stage_bytes));
 #pragma unroll
-                        for (int k = 0; k < BLOCK_K / UMMA_K; k++)
-                            umma_tf32(tmem_base, smem_desc(a_lo + 2 * k), smem_desc(b_lo + 2 * k), idesc, (kb | c | k) != 0);
-                    }
+                    for (int k = 0; k < BLOCK_K / UMMA_K; k++)
+                        umma_tf32_ts(d, w_col + (uint32_t)(i * BLOCK_K + k * UMMA_K), smem_desc(b_lo + 2 * k), idesc, (i | k) != 0);
                     umma_commit(&empty[stage]);
                     if (++stage == stages) { stage = 0; phase ^= 1; }
                 }
-                if (ok) umma_commit(acc_full);
+                if (ok) umma_commit(&acc_full[t & 1]);
             }
             // the last releases of the ring must have landed before the CTA may exit
             for (int i = 0; i < stages && ok; i++) {
@@ -127,103 +211,121 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
             }
         }
         __syncwarp();
-    } else if (warp == 5) {
-        // ------------------------------------------------ h_{t-1} of every step, one K block per ring stage
-        if (elect_one()) {
-            int stage = 0;
-            uint32_t phase = 0;
-            const uint32_t tx = (uint32_t)(p.B * BLOCK_K * 4 * cbs);
-            for (int t = p.t_first; t < p.T && ok; t++) {
-                if (t > p.t_first) {
-                    // grid barrier: all CTAs have arrived with h_{t-1}.  Their stores (generic proxy) are ordered before this
-                    // acquire; the fence orders the copies below (async proxy) behind it
-                    const unsigned int target = ctas * (unsigned int)(t - p.t_first);
-                    const long long t0 = clock64();
-                    while (ld_acquire_u32(p.sync) < target) {
-                        if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
-                            *abort_flag = 1;
-                            atomicExch(p.status, (int)DEV_TIMEOUT);
-                            ok = false;
-                            break;
-                        }
+    } else if (warp >= LP_CELL_WARPS) {
+        // ------------------------------------------------ h_{t-1} of every step: lane i fetches K block i of this slice
+        int slot = lane % stages;
+        uint32_t phase = (uint32_t)(lane / stages) & 1;
+        const unsigned int *counter = counters + (size_t)(kb0 + lane) * LP_COUNTER_STRIDE;
+        const uint32_t tx = (uint32_t)stage_bytes;
+        for (int t = 1; t < p.T && ok; t++) {
+            bool done = lane >= nkb;
+            const unsigned int target = (unsigned int)(LP_SLICES * cell_warps) * (unsigned int)t;
+            const long long t0 = clock64();
+            while (ok && !__all_sync(0xffffffffu, done)) {
+                bool give_up = false;
+                if (!done) {
+                    if (ld_acquire_u32(counter) >= target && mbar_try_wait(&empty[slot], phase ^ 1)) {
+                        // the units' stores (generic proxy) are ordered before the acquire; the copy (async proxy) behind this fence
+                        asm volatile("fence.proxy.async;" ::: "memory");
+                        mbar_expect_tx(&full[slot], tx);
+                        tma_load_3d(ring + slot * stage_bytes, &p.tm_h, &full[slot], (kb0 + lane) * BLOCK_K, row0, t - 1);
+                        done = true;
+                    } else if (*abort_flag || clock64() - t0 > WAIT_LIMIT_CYCLES) {
+                        if (!*abort_flag) atomicExch(p.status, (int)DEV_TIMEOUT);
+                        *abort_flag = 1;
+                        give_up = true;
                     }
-                    if (!ok) break;
-                    asm volatile("fence.proxy.async;" ::: "memory");
                 }
-                for (int kb = 0; kb < KB; kb += cbs) {
-                    if (!(ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.status))) break;
-                    mbar_expect_tx(&full[stage], tx);
-                    tma_load_3d(a_ring + stage * stage_bytes, &p.tm_h, &full[stage], 0, (t - 1) * p.B, kb);
-                    if (++stage == stages) { stage = 0; phase ^= 1; }
-                }
+                ok = !__any_sync(0xffffffffu, give_up);
             }
+            slot += nkb;
+            while (slot >= stages) { slot -= stages; phase ^= 1; }
         }
-        __syncwarp();
-    } else {
-        // ------------------------------------------------ epilogue of every step, then the grid barrier
-        const int tid = threadIdx.x;                        // 0..127
-        // the batch row whose accumulators this thread's TMEM lane holds: lane = row for a 128-row MMA; a 64-row MMA
-        // puts 16 rows into the first 16 lanes of each 32-lane quarter
-        const int lane = tid & 31;
-        const int brow = p.B <= 64 ? (lane < 16 ? 16 * warp + lane : 1 << 20) : tid;
-        const bool row_ok = brow < p.B;
-        const int unit0 = n0 >> 2;                          // first hidden unit of this CTA (8 of them)
-        float c[8];
+    } else if (warp % CW < cell_warps) {
+        // ------------------------------------------------ accumulators to the cluster, cells, and the step's results
+        // Every warp by itself: it waits for the MMAs, sends 16 batch rows of 32 gate columns to the CTA that finishes those
+        // (TMEM lanes 32 q .. belong to warps of index q modulo 4), waits for what it was sent, finishes 8 units x 4 rows and
+        // publishes them.  A cell is a chain of some 600 cycles whatever its neighbours do, so it takes the warps, a cell per
+        // thread: four cells per thread of four warps took 2700 cycles of a step's 12 300, and their sends 1200.
+        const int q = warp & 3, gw = warp % CW;
+        const int u = lane & 7, unit = cluster * LP_UNITS + 8 * rank + u;   // the unit this thread finishes, and its row of a quad
+        const bool unit_ok = unit < p.H;
+        float c[ITEMS];
 #pragma unroll
-        for (int u = 0; u < 8; u++) c[u] = 0.0f;
-        if (row_ok && p.t_first > 0) {
-            const float *cp = p.cell + ((size_t)(p.t_first - 1) * p.B + brow) * p.H + unit0;
-            const float4 lo = *reinterpret_cast<const float4 *>(cp), hi = *reinterpret_cast<const float4 *>(cp + 4);
-            c[0] = lo.x; c[1] = lo.y; c[2] = lo.z; c[3] = lo.w; c[4] = hi.x; c[5] = hi.y; c[6] = hi.z; c[7] = hi.w;
-        }
-        uint32_t acc_phase = 0;
-        for (int t = p.t_first; t < p.T && ok; t++) {
-            // gates of this CTA's 8 units for row `tid`; threads only leave the loop together, at the votes, so that
-            // none is left alone at a barrier
+        for (int i = 0; i < ITEMS; i++) c[i] = 0.0f;
+        const uint32_t peer_recv = map_to_rank(smem_u32(recv), (uint32_t)q);
+        const uint32_t peer_bar = map_to_rank(smem_u32(recv_full), (uint32_t)q);
+        for (int t = 0; t < p.T && ok; t++) {
+            const int par = t & 1;
+            const uint32_t phase = (uint32_t)((t - 1) >> 1) & 1;            // of both barriers of this parity (t = 1, 2: the first)
             // the input-side pre-activations of this step come from DRAM: fetched while the MMAs run
-            const size_t row = (size_t)t * p.B + brow;
-            float4 z4[8];
-            if (row_ok) {
-                const float4 *zin = reinterpret_cast<const float4 *>(p.pre + row * 4 * p.H + n0);
+            float4 z[ITEMS];
 #pragma unroll
-                for (int u = 0; u < 8; u++) z4[u] = __ldg(zin + u);
+            for (int i = 0; i < ITEMS; i++) {
+                const int b = row0 + 4 * (gw + CW * i) + (lane >> 3);
+                z[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (unit_ok && b < row_end) z[i] = __ldg(reinterpret_cast<const float4 *>(p.pre + ((size_t)t * p.B + b) * 4 * p.H) + unit);
             }
-            ok = epilogue_all(mbar_wait(acc_full, acc_phase, abort_flag, p.status), 1);
-            if (!ok) break;
-            acc_phase ^= 1;
-            tc_fence_after();
-            uint32_t v[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(warp * 32) << 16), v);
-            tmem_ld_wait();
-            tc_fence_before();
-            float hn[8];
-            const size_t o = row * p.H + unit0;
-            if (row_ok) {
+            if (t > 0 && nkb > 0) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[par], phase, abort_flag, p.status));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t dst = peer_recv + (uint32_t)(((par * LP_SLICES + rank) * recv_floats + lane * 4) * 4), bar = peer_bar + 8 * par;
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const float zi = __uint_as_float(v[4 * u]) + z4[u].x, zf = __uint_as_float(v[4 * u + 1]) + z4[u].y;
-                    const float zg = __uint_as_float(v[4 * u + 2]) + z4[u].z, zo = __uint_as_float(v[4 * u + 3]) + z4[u].w;
-                    const float2 ch = lstm_cell_unit_f32_inline(zi, zf, zg, zo, c[u]);
-                    c[u] = ch.x; hn[u] = ch.y;
-                }
+                for (int i = 0; i < ITEMS; i++) {
+                    const int j0 = 4 * ((gw >> 2) + CW / 4 * i);            // the first of this warp's quads
+                    if (j0 >= quads) break;
+                    uint32_t v[16];
+                    tmem_ld_32x16(acc_col + ((uint32_t)(q * 32) << 16) + (uint32_t)(par * p.Rg + 4 * j0), v);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    *reinterpret_cast<float4 *>(p.hr_w + o + 4 * q) = make_float4(round_tf32(hn[4 * q]), round_tf32(hn[4 * q + 1]),
-                                                                                   round_tf32(hn[4 * q + 2]), round_tf32(hn[4 * q + 3]));
+                    for (int j = 0; j < 4; j++)
+                        if (j0 + j < quads) st_async_v4(dst + (uint32_t)(j0 + j) * 512, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], bar);
                 }
+                tc_fence_before();
             }
-            // ---- grid barrier, this CTA's arrival: its rounded h_t is written (the barrier orders the group's stores before
-            // the release).  What the next step does not read leaves behind it, so that the release does not wait for it
+            if (t > 0) {
+                ok = __all_sync(0xffffffffu, mbar_wait_cluster(smem_u32(&recv_full[par]), phase, abort_flag, p.status));
+                if (!ok) break;
+                if (gw == 0 && lane == 0) mbar_expect_tx(&recv_full[par], recv_bytes);      // step t + 2
+            }
+            float hn[ITEMS];
+#pragma unroll
+            for (int i = 0; i < ITEMS; i++) {
+                const int quad = gw + CW * i;
+                const size_t b = row0 + 4 * quad + (lane >> 3);
+                if (!unit_ok || b >= (size_t)row_end) continue;
+                float2 ch;
+                if (t == 0) {                   // nothing to multiply: h_{-1} = 0
+                    ch = lstm_cell_unit(z[i].x, z[i].y, z[i].z, z[i].w, 0.0f);
+                } else {
+                    const float *src = recv + par * LP_SLICES * recv_floats + quad * 128 + u * 4 + (lane >> 3);
+                    float g[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) g[k] = src[32 * k];
+                    for (int s = 1; s < p.slices; s++) {        // the slices of K in order
+                        src += recv_floats;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) g[k] += src[32 * k];
+                    }
+                    ch = lstm_cell_unit_f32_inline(g[0] + z[i].x, g[1] + z[i].y, g[2] + z[i].z, g[3] + z[i].w, c[i]);
+                }
+                c[i] = ch.x; hn[i] = ch.y;
+                p.hr[((size_t)t * p.B + b) * p.H + unit] = round_tf32(ch.y);
+            }
+            // ---- this warp's part of the block is published (and its accumulators and sums are read).  What the next step does
+            // not read leaves behind it, so that the release does not wait for it
             if (t + 1 < p.T) {
-                epilogue_bar_sync(1);
-                if (tid == 0) red_release_add(p.sync, 1u);
+                __syncwarp();
+                if (lane == 0) red_release_add(counters + (size_t)cluster * LP_COUNTER_STRIDE, 1u);
             }
-            if (row_ok) {
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    *reinterpret_cast<float4 *>(p.cell + o + 4 * q) = make_float4(c[4 * q], c[4 * q + 1], c[4 * q + 2], c[4 * q + 3]);
-                    *reinterpret_cast<float4 *>(p.out + o + 4 * q) = make_float4(hn[4 * q], hn[4 * q + 1], hn[4 * q + 2], hn[4 * q + 3]);
-                }
+            for (int i = 0; i < ITEMS; i++) {
+                const int b = row0 + 4 * (gw + CW * i) + (lane >> 3);
+                if (!unit_ok || b >= row_end) continue;
+                const size_t o = ((size_t)t * p.B + b) * p.H + unit;
+                p.cell[o] = c[i];
+                p.out[o] = hn[i];
             }
         }
         if (!ok) *abort_flag = 1;
@@ -235,10 +337,24 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
         for (int i = 0; i < 64; i++) __nanosleep(2000);     // let copies and MMAs in flight land before TMEM goes
         __syncthreads();
     }
-    if (warp == 4) {
+    if (warp == LP_CELL_WARPS) {
         __syncwarp();
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(32u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)LP_TMEM) : "memory");
+    }
+    // no CTA leaves while a peer may still store into it
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // the last CTA of the grid to get here leaves the counters as it found them (nobody polls any more)
+    if (warp == 0) {
+        const int exits = (int)gridDim.x / LP_SLICES * LP_GROUPS;
+        bool last = false;
+        if (lane == 0) {
+            __threadfence();
+            last = atomicAdd(p.sync + (size_t)exits * LP_COUNTER_STRIDE, 1u) == gridDim.x - 1;
+        }
+        if (__any_sync(0xffffffffu, last))
+            for (int i = lane; i <= exits; i += 32) p.sync[(size_t)i * LP_COUNTER_STRIDE] = 0;
     }
 }
 
@@ -248,71 +364,117 @@ struct LstmPLaunch : LaunchRecord {
     double flops;
 };
 
+const void *kernel_of(int B) { return B <= 64 ? (const void *)lstm_persistent_kernel<1> : (const void *)lstm_persistent_kernel<2>; }
+
+int rows_of(int B) { return (B + 16 * LP_GROUPS - 1) / (16 * LP_GROUPS) * 16; }       // of a group
+int smem_of(int B, int stages) {
+    return LP_GROUPS * (stages + 2 * LP_SLICES) * rows_of(B) * 128 + 1024 + 8 * LP_GROUPS * LP_BARS + 16;
+}
+int stages_of(int B) {
+    int s = LP_MAX_STAGES;
+    while (s > 1 && smem_of(B, s) > LP_SMEM) s--;
+    return s;
+}
+
 }  // namespace
 
-void lstm_persistent_prepare_device() {
-    NB_CHECK_CUDA(cudaFuncSetAttribute(lstm_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+void lstm_persistent_prepare_device(nb_handle_s *h) {
+    for (int B : {64, 128}) NB_CHECK_CUDA(cudaFuncSetAttribute(kernel_of(B), cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM));
+    // clusters of four that run at once, with a CTA per SM (the kernel takes all of tensor memory)
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(LP_SLICES);
+    cfg.blockDim = dim3(LP_THREADS);
+    cfg.dynamicSmemBytes = LP_SMEM;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = LP_SLICES; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel_of(128), &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+    h->lstm_clusters = n;
 }
 
-// Whether the recurrence of an LSTM layer can run as the persistent kernel: TF32 mode on the tensor-core path, gate
-// layers without an activation of their own, H a multiple of 32 whose weight slice and ring fit in shared memory,
-// one CTA per 32 gate columns with all of them resident at once, a batch of at most 128 rows.
+int lstm_persistent_counters() { return (LP_GROUPS * LP_MAX_BLOCKS + 1) * LP_COUNTER_STRIDE; }
+
+// K blocks of one slice of a recurrent product: the order in which TF32 LSTM steps add, in this kernel and launched step by step.
+int lstm_k_part(int H) {
+    const int KB = (H + BLOCK_K - 1) / BLOCK_K;
+    return (KB + LP_SLICES - 1) / LP_SLICES;
+}
+
+namespace {
+
+// A batch runs as equal chunks of at most 128 rows, each on a set of clusters of its own.
+int chunks_of(int B) { return (B + 127) / 128; }
+int chunk_rows_of(int B) { return (B + chunks_of(B) - 1) / chunks_of(B); }
+
+}  // namespace
+
+// Whether the recurrence of an LSTM layer can run as the persistent kernel: TF32 mode on the tensor-core path, gate layers
+// without an activation of their own, whole quads of units, weights and accumulators that fit tensor memory, all clusters
+// resident at once (up to 128 rows at H = 1024, 256 at 512, 1152 at 128).  A second launch for more rows gains little or loses:
+// H = 1024, 8 steps: B = 129 / 256 / 512: 306 / 352 / 669 us in two or four launches, 309 / 344 / 472 launched step by step.
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H) {
     if (!h->encode_tiled || h->cc_major != 10 || !h->cooperative_launch) return false;
-    if (T < 2 || B < 1 || B > 128 || (H % 32) != 0) return false;      // (a box of B rows: any B up to 128)
-    const int ctas = 4 * H / LP_N;
-    const size_t smem = (size_t)(H / BLOCK_K) * LP_W_TILE + 2 * (A_STAGE_BYTES + (size_t)B * 128) + 1024 + 256;   // two stages at least
-    return ctas <= h->sm_count && smem <= 227 * 1024;
+    if (T < 2 || B < 1 || H < 32 || (H % 4) != 0 || (B > 128 && (H % 32) != 0)) return false;
+    const long KB = (H + BLOCK_K - 1) / BLOCK_K;
+    if (lstm_k_part(H) > 32 || KB * chunks_of(B) > std::min(h->lstm_clusters, LP_MAX_BLOCKS)) return false;
+    return 2 * LP_GROUPS * rows_of(chunk_rows_of(B)) + lstm_k_part(H) * BLOCK_K <= LP_TMEM;
 }
 
-// Steps t_first .. T-1 of the recurrence (t_first >= 1: c, h and the rounded h of step t_first - 1 are in place).
-void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B,
-                     int H, int t_first) {
+// All steps of the recurrence: writes cell, out and hr.
+void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H) {
     std::string key;
     key.push_back('P');
     key_add(key, w_hi); key_add(key, pre); key_add(key, cell); key_add(key, out); key_add(key, hr);
-    key_add(key, T); key_add(key, B); key_add(key, H); key_add(key, t_first);
+    key_add(key, T); key_add(key, B); key_add(key, H);
     auto it = h->launch_cache.find(key);
     if (it == h->launch_cache.end()) {
         std::unique_ptr<LstmPLaunch> L(new LstmPLaunch());
         std::memset(&L->p, 0, sizeof L->p);
         const long long F4 = 4;
+        const int KB = (H + BLOCK_K - 1) / BLOCK_K, rows = chunk_rows_of(B), Rg = rows_of(rows);
         check_extent(h, w_hi, 0, (long long)4 * H * H * F4, "recurrent weights");
         check_extent(h, pre, 0, (long long)T * B * 4 * H * F4, "input-side pre-activations");
         check_extent(h, cell, 0, (long long)T * B * H * F4, "cell states");
         check_extent(h, out, 0, (long long)T * B * H * F4, "hidden states");
-        check_extent(h, hr, 0, (long long)T * B * H * F4, "rounded hidden states");
-        cuuint64_t dims[3] = {(cuuint64_t)H, (cuuint64_t)(4 * H), 1};
-        cuuint64_t strides[2] = {(cuuint64_t)H * 4, (cuuint64_t)H * 4 * (cuuint64_t)(4 * H)};
-        cuuint32_t bx[3] = {(cuuint32_t)BLOCK_K, (cuuint32_t)LP_N, 1};
+        // (columns past H and rows past B arrive as zeros, but are read)
+        const long long last = (long long)(chunks_of(B) - 1) * rows + LP_GROUPS * Rg;
+        check_extent(h, hr, 0, (((long long)(T - 1) * B + last) * H + KB * BLOCK_K - H) * F4, "rounded hidden states");
+        cuuint64_t dims[3] = {(cuuint64_t)H, (cuuint64_t)B, (cuuint64_t)T};
+        cuuint64_t strides[2] = {(cuuint64_t)H * 4, (cuuint64_t)H * 4 * (cuuint64_t)B};
+        cuuint32_t bx[3] = {(cuuint32_t)BLOCK_K, (cuuint32_t)Rg, 1};
         cuuint32_t es[3] = {1, 1, 1};
-        encode_tensor_map(h, &L->p.tm_w, w_hi, 3, dims, strides, bx, es);
-        // two K blocks per request when the second slice starts on the swizzle pattern's 1024-byte repeat
-        const int cbs = ((B % 8) == 0 && (H % (2 * BLOCK_K)) == 0) ? 2 : 1;
-        const int stage_bytes = (cbs - 1) * B * 128 + A_STAGE_BYTES;
-        const int w_bytes = (H / BLOCK_K) * LP_W_TILE;
-        const int stages = std::min(LP_STAGES, (227 * 1024 - 1024 - 256 - w_bytes) / stage_bytes);
-        cuuint64_t hdims[3] = {(cuuint64_t)BLOCK_K, (cuuint64_t)T * (cuuint64_t)B, (cuuint64_t)(H / BLOCK_K)};
-        cuuint64_t hstrides[2] = {(cuuint64_t)H * 4, (cuuint64_t)BLOCK_K * 4};
-        cuuint32_t hbx[3] = {(cuuint32_t)BLOCK_K, (cuuint32_t)B, (cuuint32_t)cbs};
-        cuuint32_t hes[3] = {1, 1, 1};
-        encode_tensor_map(h, &L->p.tm_h, hr, 3, hdims, hstrides, hbx, hes);
-        L->p.cbs = cbs; L->p.stages = stages; L->p.stage_bytes = stage_bytes;
-        L->p.pre = pre; L->p.hr_w = hr; L->p.cell = cell; L->p.out = out;
-        L->p.T = T; L->p.B = B; L->p.H = H; L->p.t_first = t_first;
+        encode_tensor_map(h, &L->p.tm_h, hr, 3, dims, strides, bx, es);
+        L->p.w = w_hi; L->p.pre = pre; L->p.hr = hr; L->p.cell = cell; L->p.out = out;
+        L->p.T = T; L->p.B = B; L->p.H = H; L->p.chunk_rows = rows; L->p.Rg = Rg;
+        L->p.kb_per_slice = lstm_k_part(H);
+        L->p.slices = (KB + L->p.kb_per_slice - 1) / L->p.kb_per_slice;
+        L->p.stages = stages_of(rows);
         L->p.sync = h->d_grid_sync; L->p.status = h->d_status;
-        L->grid = 4 * H / LP_N;
-        L->smem = w_bytes + stages * stage_bytes + 1024 + 256;
-        L->flops = 2.0 * (double)(T - t_first) * B * 4.0 * H * H;
+        L->grid = KB * LP_SLICES * chunks_of(B);
+        L->smem = smem_of(rows, L->p.stages);
+        L->flops = 2.0 * (double)(T - 1) * B * 4.0 * H * H;
         if (h->launch_cache.size() > 4096) h->launch_cache.clear();
         it = h->launch_cache.emplace(std::move(key), std::move(L)).first;
     }
     const LstmPLaunch &L = static_cast<const LstmPLaunch &>(*it->second);
-    NB_CHECK_CUDA(cudaMemsetAsync(h->d_grid_sync, 0, sizeof(unsigned int), h->stream));
     ProfileScope prof(h, 0, L.flops);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)L.grid);
+    cfg.blockDim = dim3(LP_THREADS);
+    cfg.dynamicSmemBytes = (size_t)L.smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = LP_SLICES; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeCooperative;
+    at[1].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
     void *args[1] = {const_cast<LstmPParams *>(&L.p)};
-    NB_CHECK_CUDA(cudaLaunchCooperativeKernel((const void *)lstm_persistent_kernel, dim3(L.grid), dim3(LP_THREADS), args, (size_t)L.smem,
-                                              h->stream));
+    NB_CHECK_CUDA(cudaLaunchKernelExC(&cfg, kernel_of(chunk_rows_of(B)), args));
     check_launch("lstm_persistent_kernel");
     count_launch(h);
     prof.finish();

@@ -62,7 +62,8 @@ struct nb_handle_s {
     int cc_major = 0;
     std::string last_error;
     int *d_status = nullptr;            // device status word (nb::DEV_*)
-    unsigned int *d_grid_sync = nullptr; // arrival counter of the persistent LSTM kernel's grid barrier
+    unsigned int *d_grid_sync = nullptr; // arrival counters of the persistent LSTM kernel (it leaves them zero)
+    int lstm_clusters = 0;              // lstm_persistent.cu: clusters of its size that the device runs at once
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
     bool recurrent_ready = false;       // recurrent_cluster.cu: limits set, clusters_at_once filled
     unsigned long long simt_ready = 0;  // gemm_simt.cu: kernels loaded and with their limits set, by variant and copy modes
@@ -217,6 +218,8 @@ struct GemmArgs {
     int split_k = 1;
     // tensor-core kernel: tile width in output columns (64, 128 or 256) instead of the built-in choice; 0 = automatic
     int block_n_hint = 0;
+    // tensor-core kernel, TF32: K blocks per partial sum (those are added in fp32 registers); 0 = built-in choice
+    int k_part = 0;
     double algo_flops = 0;          // algorithmic FLOPs of this launch for profiling (0: 2*M*N*Kc*taps)
 };
 
@@ -366,10 +369,12 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra);
 
 // Per-device set-up of the tensor-core kernels (shared-memory limits; also loads their code), once per handle.
 void gemm_tc_prepare_device();
-void lstm_persistent_prepare_device();
+void lstm_persistent_prepare_device(nb_handle_s *h);
+int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
-void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B,
-                     int H, int t_first);
+void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H);
+// K blocks of 32 per partial sum of a TF32 LSTM layer's recurrent product
+int lstm_k_part(int H);
 // what a contraction runs on: the tensor cores in TF32 or 3xTF32, or the CUDA cores
 enum GemmPath { PATH_TC = 0, PATH_TC3 = 1, PATH_SIMT = 2 };
 // The recurrence of an LSTM (gates = 4) or RNN (gates = 1) layer over all steps, exact fp32, for layers whose recurrent

@@ -557,9 +557,9 @@ void LstmPlan::set_weights(const float *stream, size_t count, int mem) {
 }
 
 // The modes that promise fp32 agreement, widths off 32 and gate layers with an activation run all steps in one kernel of exact
-// fp32 products where that is the faster way.  The layers whose batches up to 128 run on the tensor cores in one kernel
-// (lstm_persistent.cu) take the same TF32 products a launch per step beyond (bit-identical), whatever the cluster would cost; a
-// single step of linear gate layers has no product.  NEBULA_B200_LSTM_PERSISTENT=0: a launch per step in every case.
+// fp32 products where that is the faster way.  Linear layers of widths that are multiples of 32 take TF32 products at every batch,
+// whatever the cluster would cost (lstm_persistent.cu, a launch per step beyond its batches); a single step of linear gate
+// layers has no product.  NEBULA_B200_LSTM_PERSISTENT=0: a launch per step in every case.
 bool LstmPlan::one_kernel() const {
     const char *env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
     if (env && *env == '0') return false;
@@ -637,18 +637,8 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
     // 2. the recurrence: z_t = pre_t + act(h_{t-1} * W^T + bW), then the cell update.  With linear gate layers
     //    step 0 has nothing to multiply (h_{-1} = 0 and bW is already in pre); otherwise act(bW) is not zero and
     //    step 0 runs the recurrent layer on a zero state like every other step.
-    // With linear gate layers on the TF32 tensor-core path, steps 1 .. T-1 run as one cooperative kernel that keeps
-    // the recurrent weights in shared memory (lstm_persistent.cu); step 0 is the cell update alone.  It stores quads, so a
-    // caller's tensors off a 16-byte boundary take the launch per step.
-    const char *lp_env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
-    bool persistent = tc_w && !three && linear && hr && (H % 8) == 0 && lstm_persistent_supported(h, T, B, H) &&
-                      !(((uintptr_t)out | (uintptr_t)cell) & 15) && !(lp_env && *lp_env == '0');
-    if (persistent) {
-        launch_lstm_cell(h, pre.p, nullptr, cell, out, hr, B, H);
-        ww.ensure_split(h);
-        lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H, 1);
-        return;
-    }
+    // All steps in one kernel where the layer has one: exact fp32 on a cluster, or, with linear gate layers on the TF32
+    // tensor-core path, one cooperative kernel that keeps the recurrent weights in tensor memory (lstm_persistent.cu).
     if (one_kernel()) {
         RecurrentArgs r{};
         r.w = ww.exact.p; r.pre = pre.p; r.shift = linear ? nullptr : shift_w.p;
@@ -656,6 +646,12 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         r.T = T; r.B = B; r.H = H; r.gates = 4; r.act = d.activation;
         r.cell_f32 = tc_w && !three;
         recurrent_cluster(h, r);
+        return;
+    }
+    const char *lp_env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
+    if (tc_w && !three && linear && hr && lstm_persistent_supported(h, T, B, H) && !(lp_env && *lp_env == '0')) {
+        ww.ensure_split(h);
+        lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H);
         return;
     }
     for (int t = 0; t < T; t++) {
@@ -674,6 +670,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
                 a.b_static = ww.split_ready;
                 ww.ensure_split(h);
                 a.b = ww.hi.p; a.b_lo = ww.lo.p;
+                if (linear && !three && lstm_persistent_supported(h, T, B, H)) a.k_part = lstm_k_part(H);      // as the one-kernel recurrence adds
                 a.lstm_H = H; a.lstm_c_prev = c_prev; a.lstm_c = ct; a.lstm_h = ht; a.lstm_h_round = hrt;
                 gemm_tc(h, a, three);
                 continue;
