@@ -415,9 +415,10 @@ int chunk_rows_of(int B) { return (B + chunks_of(B) - 1) / chunks_of(B); }
 // without an activation of their own, whole quads of units, weights and accumulators that fit tensor memory, all clusters
 // resident at once (up to 128 rows at H = 1024, 256 at 512, 1152 at 128).  A second launch for more rows gains little or loses:
 // H = 1024, 8 steps: B = 129 / 256 / 512: 306 / 352 / 669 us in two or four launches, 309 / 344 / 472 launched step by step.
+// Two steps have one product, and the kernel's set-up costs more than its launch (T2 B64 H416, two layers: 66 and 54 us).
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H) {
     if (!h->encode_tiled || h->cc_major != 10 || !h->cooperative_launch) return false;
-    if (T < 2 || B < 1 || H < 32 || (H % 4) != 0 || (B > 128 && (H % 32) != 0)) return false;
+    if (T < 3 || B < 1 || H < 32 || (H % 4) != 0 || (B > 128 && (H % 32) != 0)) return false;
     const long KB = (H + BLOCK_K - 1) / BLOCK_K;
     if (lstm_k_part(H) > 32 || KB * chunks_of(B) > std::min(h->lstm_clusters, LP_MAX_BLOCKS)) return false;
     return 2 * LP_GROUPS * rows_of(chunk_rows_of(B)) + lstm_k_part(H) * BLOCK_K <= LP_TMEM;
