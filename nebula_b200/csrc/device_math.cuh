@@ -29,6 +29,51 @@ __device__ __forceinline__ float round_tf32(float x) {
     return __uint_as_float(r);
 }
 
+// exp in double without branches, so that several of them overlap: the argument is reduced by Cody and Waite's split of ln 2
+// to |r| <= 0.35, the exponential of r is its Taylor polynomial of degree 12 (the rest is below 2^-53 of it), and the power of
+// two is added to the exponent.  Arguments are cut to +-708, where the result is still a normal number: the callers add it to 1,
+// or compare against where exp overflows themselves.  NaN stays NaN.
+// The library's exp and division branch on their special cases, which puts the chains of a thread's values one behind the
+// other: the tanh layer of 512 x 256 x 256 took 17.4 us with them, 15.2 with these; 2^24 values by themselves 45 and 39.
+__device__ __forceinline__ double exp_for_activation(double z) {
+    z = z > 708.0 ? 708.0 : z;
+    z = z < -708.0 ? -708.0 : z;
+    const double big = 6755399441055744.0;              // 1.5 * 2^52: adding it leaves the nearest integer in the low bits
+    const double kb = fma(z, 1.4426950408889634, big), k = kb - big;
+    double r = fma(k, -0.6931471805598903, z);     // ln 2 to 42 bits: k times it is exact
+    r = fma(k, -5.497923018708371e-14, r);             // and the rest
+    double p = 1.0 / 479001600.0;
+    p = fma(p, r, 1.0 / 39916800.0);
+    p = fma(p, r, 1.0 / 3628800.0);
+    p = fma(p, r, 1.0 / 362880.0);
+    p = fma(p, r, 1.0 / 40320.0);
+    p = fma(p, r, 1.0 / 5040.0);
+    p = fma(p, r, 1.0 / 720.0);
+    p = fma(p, r, 1.0 / 120.0);
+    p = fma(p, r, 1.0 / 24.0);
+    p = fma(p, r, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1.0);
+    p = fma(p, r, 1.0);
+    return __hiloint2double(__double2hiint(p) + (__double2loint(kb) << 20), __double2loint(p));
+}
+// n / d for d in [1, 1e308): the hardware's approximation of 1 / d, one step of Newton's iteration, and one correction of the
+// quotient by its remainder.
+__device__ __forceinline__ double divide_for_activation(double n, double d) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    y = fma(y, fma(-d, y, 1.0), y);
+    const double q = n * y;
+    return fma(fma(-d, q, n), y, q);
+}
+__device__ __forceinline__ float logistic_double(float x) { return (float)divide_for_activation(1.0, 1.0 + exp_for_activation(-(double)x)); }
+__device__ __forceinline__ float loggy_double(float x) { return (float)(divide_for_activation(2.0, 1.0 + exp_for_activation(-(double)x)) - 1.0); }
+__device__ __forceinline__ float tanh_double(float x) {
+    const double z = 2.0 * (double)x, e = exp_for_activation(z);
+    const double t = divide_for_activation(e - 1.0, e + 1.0);
+    return z > 709.782712893384 ? __int_as_float(0x7fffffff) : (float)t;        // (inf - 1) / (inf + 1)
+}
+
 // The reference's CPU activations (common/activations.cc:6-91).  Its constants
 // are doubles, so each formula is evaluated in double and stored back as float,
 // which reproduces the CPU results including tanh's NaN for large inputs
@@ -39,12 +84,9 @@ __device__ __forceinline__ float apply_activation(float x, int act) {
         case NB_ACT_RELU: return x > 0.0f ? x : 0.0f;
         case NB_ACT_LEAKY: return x > 0.0f ? x : (float)(0.1 * (double)x);
         case NB_ACT_RELIE: return x > 0.0f ? x : (float)(0.01 * (double)x);
-        case NB_ACT_LOGISTIC: return (float)(1.0 / (1.0 + exp(0.0 - (double)x)));
-        case NB_ACT_LOGGY: return (float)(2.0 / (1.0 + exp(0.0 - (double)x)) - 1.0);
-        case NB_ACT_TANH: {
-            const double e = exp(2.0 * (double)x);
-            return (float)((e - 1.0) / (e + 1.0));
-        }
+        case NB_ACT_LOGISTIC: return logistic_double(x);
+        case NB_ACT_LOGGY: return loggy_double(x);
+        case NB_ACT_TANH: return tanh_double(x);
         case NB_ACT_ELU: return x > 0.0f ? x * x : (float)((double)x * (exp((double)x) - 1.0));
         case NB_ACT_HARDTAN: return (x < 1.0f && x > -1.0f) ? 1.0f : 0.0f;
         case NB_ACT_LHTAN: return (x > 0.0f && x < 1.0f) ? 1.0f : 0.0f;
@@ -66,18 +108,11 @@ __device__ __forceinline__ float apply_activation(float x, int act) {
 // instruction stream of loops that almost always run relu / leaky / linear.
 static __device__ __noinline__ float apply_activation_call(float x, int act) { return apply_activation(x, act); }
 
-// Four values at once: a double exponential is a chain of some two hundred cycles, and the four chains overlap.
+// Four values at once: a double exponential is a long chain, and the four chains overlap.
 __device__ __forceinline__ float4 apply_activation4(float4 x, int act) {
-    if (act == NB_ACT_LOGISTIC || act == NB_ACT_LOGGY || act == NB_ACT_TANH) {
-        const double m = act == NB_ACT_TANH ? 2.0 : -1.0;
-        const double e0 = exp(m * (double)x.x), e1 = exp(m * (double)x.y), e2 = exp(m * (double)x.z), e3 = exp(m * (double)x.w);
-        if (act == NB_ACT_TANH)
-            return make_float4((float)((e0 - 1.0) / (e0 + 1.0)), (float)((e1 - 1.0) / (e1 + 1.0)), (float)((e2 - 1.0) / (e2 + 1.0)),
-                               (float)((e3 - 1.0) / (e3 + 1.0)));
-        const double q0 = 1.0 + e0, q1 = 1.0 + e1, q2 = 1.0 + e2, q3 = 1.0 + e3;
-        if (act == NB_ACT_LOGISTIC) return make_float4((float)(1.0 / q0), (float)(1.0 / q1), (float)(1.0 / q2), (float)(1.0 / q3));
-        return make_float4((float)(2.0 / q0 - 1.0), (float)(2.0 / q1 - 1.0), (float)(2.0 / q2 - 1.0), (float)(2.0 / q3 - 1.0));
-    }
+    if (act == NB_ACT_LOGISTIC) return make_float4(logistic_double(x.x), logistic_double(x.y), logistic_double(x.z), logistic_double(x.w));
+    if (act == NB_ACT_LOGGY) return make_float4(loggy_double(x.x), loggy_double(x.y), loggy_double(x.z), loggy_double(x.w));
+    if (act == NB_ACT_TANH) return make_float4(tanh_double(x.x), tanh_double(x.y), tanh_double(x.z), tanh_double(x.w));
     return make_float4(apply_activation(x.x, act), apply_activation(x.y, act), apply_activation(x.z, act), apply_activation(x.w, act));
 }
 
