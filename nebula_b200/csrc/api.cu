@@ -105,7 +105,7 @@ int nb_create(int device_id, nb_handle_t *handle) {
                 h->trace_dev = (CUdeviceptr)dp;
             }
         }
-        gemm_tc_prepare_device();
+        gemm_tc_prepare_device(h);
         lstm_persistent_prepare_device(h);
         elementwise_prepare_device();
     });

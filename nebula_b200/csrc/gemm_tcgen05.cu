@@ -64,8 +64,9 @@ struct TcParams {
     // (connected layers wider than L2), the B tile (m fastest), so that the second reader finds it in L2
     int m_fastest;
     int tx_bytes_a;             // bytes one A box load delivers
-    // split-K: a tile is (m_tile, n_tile, split); split s runs K blocks [s*kb_per_split, (s+1)*kb_per_split)
-    // and stores into slab s of y (batch coordinate n + s*NB): y then holds k_splits partial tensors
+    // split-K: a tile is (m_tile, n_tile, split); split s runs K blocks [s*kb_per_split, (s+1)*kb_per_split).  In a cluster
+    // the splits of a tile are its CTAs, which finish it together; otherwise split s is stored into slab s of y (batch
+    // coordinate n + s*NB): y then holds k_splits partial tensors
     int k_splits, kb_per_split;
     // The tensor core's fp32 accumulator rounds toward zero at every K=8 step (a bias that grows with K).
     // After every kb_per_part K blocks the partial sums are promoted to registers (round-to-nearest adds)
@@ -177,10 +178,188 @@ struct Cfg {
     static_assert(LAYOUT_BYTES + 1024 <= SMEM_BYTES, "ring, staging buffers and barriers must fit");
 };
 
+// All threads of the cluster; what each wrote to its shared memory before is visible to the others behind it.
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster(uint32_t smem_addr, int rank) {
+    float4 v;
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %4, %5;\n\t"
+        "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+        : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(smem_addr), "r"(rank) : "memory");
+    return v;
+}
+
+// The epilogue warps of a CTA of a tile whose K is cut over a cluster.  Every CTA leaves its partial sums in its shared memory
+// (the ring is free: its MMAs are done); behind the cluster's barrier each takes an equal share of the tile's rows, adds the
+// partial sums over the cluster's shared memory in the order of K, and finishes them: folded batch-norm and bias, shortcut,
+// activation, rounding, 2x2/2 max-pool, rows as NHWC or NCHW.  Bound by latency: with partial tensors in HBM and a kernel behind it
+// that adds them a small layer took about 3 us more, and a tile's activations had one SM: a ResNet-50 image 466 -> 424 us, the RNN
+// (tanh layers of 512 x 256 x 256) 113 -> 102, VGG-16 b1 in 3xTF32 567 -> 535.
+template <int BLOCK_N, bool THREE, bool PROMOTE>
+__device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *smem, uint32_t tmem_base, uint64_t *acc_full, uint64_t *acc_empty,
+                                                 uint64_t *x_empty, bool cross_cols, volatile int *abort_flag) {
+    using C = Cfg<BLOCK_N, THREE, false>;
+    constexpr int CH = BLOCK_N / 64, N4 = BLOCK_N / 4;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = (warp - 2) >> 2, bar_id = 1 + grp, q = warp & 3, r = q * 32 + lane;
+    const int t = threadIdx.x - 64;                         // 0..255
+    const TileIter ti(p, blockIdx.x, gridDim.x);
+    const int S = p.k_splits, rank = ti.split, n0 = ti.n_tile * BLOCK_N;
+    const int box_rows = p.bw * p.bh * p.bn;
+    float4 *part = reinterpret_cast<float4 *>(smem);        // [rows][BLOCK_N]: 16-byte chunk c of row r at c ^ (r % 8)
+
+    // this CTA's share: rows, or pooled pixels; a thread has the same four columns in all of its items
+    const int units = p.e.pool ? box_rows / 4 : box_rows, per = (units + S - 1) / S;
+    const int u0 = rank * per, u_end = min(units, u0 + per);
+    // (NCHW output: lanes along the pixels, else along the columns)
+    const int c4 = p.e.plane ? t / (256 / N4) : t % N4, first_u = u0 + (p.e.plane ? t % (256 / N4) : t / N4), col = n0 + 4 * c4;
+    const bool col_ok = col < p.e.N;                        // (N is a multiple of 4)
+    float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (col_ok && p.e.scale) sc = __ldg(reinterpret_cast<const float4 *>(p.e.scale + col));
+    if (col_ok && p.e.shift) sh = __ldg(reinterpret_cast<const float4 *>(p.e.shift + col));
+    // row of the box -> output pixel
+    struct Pixel { int n, oh, ow; bool ok; long row; };
+    auto pixel = [&](int row) {
+        Pixel x;
+        x.ow = ti.tw * p.bw + row % p.bw; x.oh = ti.th * p.bh + row / p.bw % p.bh; x.n = ti.tn * p.bn + row / (p.bw * p.bh);
+        x.ok = x.ow < p.OW && x.oh < p.OH && x.n < p.NB;
+        x.row = ((long)x.n * p.OH + x.oh) * p.OW + x.ow;
+        return x;
+    };
+    auto residual = [&](const Pixel &x) {
+        const float *a = col < p.e.addend_cols ? addend_row(p.e, x.ok, x.row, x.n, x.oh, x.ow) : nullptr;
+        return a ? *reinterpret_cast<const float4 *>(a + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    grid_dependency_wait();
+    // (the first item's shortcut is fetched while the MMAs run)
+    float4 first_res = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p.e.addend && col_ok && first_u < u_end) first_res = residual(pixel(first_u));
+
+    bool ok = true;
+    auto keep = [&](const uint32_t (&v)[32], int chunk) {
+        if (r >= box_rows) return;
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            part[r * N4 + ((chunk * 8 + j) ^ (r & 7))] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                                    __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+    };
+    const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16);
+    if (!PROMOTE || p.parts == 1) {
+        ok = epilogue_all(mbar_wait(&acc_full[0], 0, abort_flag, p.status), bar_id);
+        if (ok) {
+            tc_fence_after();
+#pragma unroll 1
+            for (int chunk = grp; chunk < BLOCK_N / 32; chunk += 2) {
+                uint32_t v[32];
+                tmem_ld_32x32(lanes + (uint32_t)(chunk * 32), v);
+                tmem_ld_wait();
+                keep(v, chunk);
+            }
+            tc_fence_before();
+        }
+    } else if constexpr (PROMOTE) {
+        uint32_t sum[CH][32];
+        const int tile_kb = min(p.kb_per_split, p.num_k_blocks - rank * p.kb_per_split);
+        const int parts = (tile_kb + p.kb_per_part - 1) / p.kb_per_part;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        for (int i = 0; i < parts; i++) {
+            if (!(ok = epilogue_all(mbar_wait(&acc_full[acc], acc_phase, abort_flag, p.status), bar_id))) break;
+            tc_fence_after();
+#pragma unroll
+            for (int ci = 0; ci < CH; ci++) {
+                uint32_t v[32];
+                tmem_ld_32x32(lanes + (uint32_t)(acc * BLOCK_N + (grp + 2 * ci) * 32), v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; j++) sum[ci][j] = i == 0 ? v[j] : __float_as_uint(__uint_as_float(sum[ci][j]) + __uint_as_float(v[j]));
+                if (cross_cols && i == parts - 1) {         // the cross terms: complete with the last MMAs
+                    tmem_ld_32x32(lanes + (uint32_t)(2 * BLOCK_N + (grp + 2 * ci) * 32), v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; j++) sum[ci][j] = __float_as_uint(__uint_as_float(sum[ci][j]) + __uint_as_float(v[j]));
+                }
+            }
+            tc_fence_before();
+            mbar_arrive(&acc_empty[acc]);
+            if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        }
+        if (ok) {
+#pragma unroll
+            for (int ci = 0; ci < CH; ci++) keep(sum[ci], grp + 2 * ci);
+        }
+    }
+    __syncwarp();
+    cluster_barrier();
+
+    const uint32_t part32 = smem_u32(part);
+    auto value = [&](int row, const Pixel &x, bool first) {
+        const uint32_t at = part32 + (uint32_t)(row * N4 + (c4 ^ (row & 7))) * 16;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int s0 = 0; s0 < S; s0 += 8) {
+            float4 v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (s0 + i < S) v[i] = ld_cluster(at, s0 + i);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                if (s0 + i >= S) continue;
+                if (s0 + i == 0) a = v[0];
+                else { a.x += v[i].x; a.y += v[i].y; a.z += v[i].z; a.w += v[i].w; }
+            }
+        }
+        if (p.e.scale) {
+            a.x = fmaf(a.x, sc.x, sh.x); a.y = fmaf(a.y, sc.y, sh.y); a.z = fmaf(a.z, sc.z, sh.z); a.w = fmaf(a.w, sc.w, sh.w);
+        } else {
+            a.x += sh.x; a.y += sh.y; a.z += sh.z; a.w += sh.w;
+        }
+        if (p.e.addend) {
+            const float4 b = first ? first_res : residual(x);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        a = apply_activation4_fast(a, p.e.act);
+        if (p.e.round_out) { a.x = round_tf32(a.x); a.y = round_tf32(a.y); a.z = round_tf32(a.z); a.w = round_tf32(a.w); }
+        return a;
+    };
+    for (int u = first_u; u < u_end && col_ok; u += 256 / N4) {
+        float *dst;
+        float4 a;
+        if (!p.e.pool) {
+            const Pixel x = pixel(u);
+            if (!x.ok) continue;
+            a = value(u, x, u == first_u);
+            if (p.e.plane) {
+                dst = p.e.y + ((long)x.n * p.e.N + col) * p.e.plane + (x.row - (long)x.n * p.e.plane);
+                dst[0] = a.x; dst[p.e.plane] = a.y; dst[2L * p.e.plane] = a.z; dst[3L * p.e.plane] = a.w;
+                continue;
+            }
+            dst = p.e.y + x.row * p.e.ldy + col;
+        } else {
+            const int hw = p.bw >> 1, hh = p.bh >> 1;
+            const int r00 = ((u / (hw * hh)) * p.bh + 2 * (u / hw % hh)) * p.bw + 2 * (u % hw);
+            const Pixel x = pixel(r00);         // (extents and boxes are even: a window lies inside or outside)
+            if (!x.ok) continue;
+            a = make_float4(-1e8f, -1e8f, -1e8f, -1e8f);        // the reference's identity
+#pragma unroll 1
+            for (int k = 0; k < 4; k++) {
+                const float4 b = value(r00 + (k >> 1) * p.bw + (k & 1), x, false);
+                a.x = b.x > a.x ? b.x : a.x; a.y = b.y > a.y ? b.y : a.y; a.z = b.z > a.z ? b.z : a.z; a.w = b.w > a.w ? b.w : a.w;
+            }
+            dst = p.e.y + (((long)x.n * (p.OH >> 1) + (x.oh >> 1)) * (p.OW >> 1) + (x.ow >> 1)) * p.e.ldy + col;
+        }
+        if (p.e.tma_store) *reinterpret_cast<float4 *>(dst) = a;        // (16-byte aligned rows)
+        else { dst[0] = a.x; dst[1] = a.y; dst[2] = a.z; dst[3] = a.w; }
+    }
+}
+
 // ------------------------------------------------------------------- kernel
 // GATHER: warps 10-13 build the A tile (compiled apart so that the common variants, which launch ten warps, are not
 // held to the register budget of fourteen).
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
+// CLUSTER: a tile's K is cut over the k_splits CTAs of a cluster, one tile per cluster (cluster_epilogue).
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER>
 __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
     using C = Cfg<BLOCK_N, THREE, GATHER>;
@@ -371,6 +550,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         }
         }
         __syncwarp();
+        if (CLUSTER) cluster_barrier();
     } else if (warp == 1) {
         // -------------------------------------------------------- MMA issuer
         // One elected lane.  Its time per MMA is the tensor core's: about 65 cycles for a 128 x 64 x 8 TF32 MMA, 75 for
@@ -483,6 +663,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         }
         }
         __syncwarp();
+        if (CLUSTER) cluster_barrier();
+    } else if (CLUSTER && warp < 10) {
+        if constexpr (CLUSTER)
+            cluster_epilogue<BLOCK_N, THREE, PROMOTE>(p, smem, tmem_base, acc_full, acc_empty, x_empty, cross_cols, abort_flag);
     } else if (warp < 10) {
         // ---------------------------------------------------------- epilogue
         // Two groups of four warps; group g owns the 32-column slabs of parity g, its own staging
@@ -739,6 +923,8 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 if (++buf == C::A_BUFS) buf = 0;
             }
         }
+        __syncwarp();
+        if (CLUSTER) cluster_barrier();
     }
 
     // ------------------------------------------------------------- teardown
@@ -753,6 +939,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         __syncwarp();
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+    }
+    if (CLUSTER) {          // no CTA leaves while a peer reads its partial sums
+        __syncwarp();
+        cluster_barrier();
     }
 }
 
@@ -823,8 +1013,8 @@ void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const c
 
 struct Variant { const void *kernel; int smem; };      // takes a TcParams, or a TcGatherParams
 
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER>
-Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER = false>
+Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER, CLUSTER>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
 
 // index: [gather][three][promote][block_n: 0 = 64, 1 = 128, 2 = 256]; absent combinations are null
 const Variant VARIANTS[2][2][2][3] = {
@@ -838,12 +1028,20 @@ const Variant VARIANTS[2][2][2][3] = {
       {variant<64, true, true, true>(), variant<128, true, true, true>(), {nullptr, 0}}}},
 };
 
+// index: [three][promote][block_n]: K cut over clusters
+const Variant CLUSTER_VARIANTS[2][2][3] = {
+    {{variant<64, false, false, false, true>(), variant<128, false, false, false, true>(), variant<256, false, false, false, true>()},
+     {variant<64, false, true, false, true>(), variant<128, false, true, false, true>(), {nullptr, 0}}},
+    {{{nullptr, 0}, {nullptr, 0}, {nullptr, 0}},
+     {variant<64, true, true, false, true>(), variant<128, true, true, false, true>(), {nullptr, 0}}},
+};
+
 // One worked-out launch: kernel parameters (tile geometry, tensor maps), kernel variant, grid.
 struct TcLaunch : LaunchRecord {
     TcGatherParams p;       // the other variants take the TcParams it starts with
     Variant v;
     bool gather = false;
-    int grid = 1, threads = 320;
+    int grid = 1, threads = 320, cluster = 1;
     double flops = 0;
     std::string desc;       // names the launch in error messages
 };
@@ -852,12 +1050,35 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 
-void gemm_tc_prepare_device() {
+void gemm_tc_prepare_device(nb_handle_s *h) {
     for (auto &g : VARIANTS)
         for (auto &t : g)
             for (auto &pr : t)
                 for (auto &v : pr)
                     if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+    for (auto &t : CLUSTER_VARIANTS)
+        for (auto &pr : t)
+            for (auto &v : pr) {
+                if (!v.kernel) continue;
+                NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+                NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            }
+    // clusters of a CTA per SM that run at once, by size
+    for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
+        const Variant &v = CLUSTER_VARIANTS[0][0][0];
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)S);
+        cfg.blockDim = dim3(320);
+        cfg.dynamicSmemBytes = (size_t)v.smem;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, v.kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+        h->tc_clusters[S] = n;
+    }
 }
 
 void encode_tensor_map(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const cuuint64_t *dims,
@@ -886,7 +1107,7 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra) {
     key_add(k, a.act); key_add(k, a.round_out_tf32); key_add(k, a.y); key_add(k, a.ldy); key_add(k, a.y_nchw); key_add(k, a.y_pool);
     key_add(k, a.lstm_H); key_add(k, a.lstm_c_prev); key_add(k, a.lstm_c); key_add(k, a.lstm_h); key_add(k, a.lstm_h_round);
     key_add(k, a.b_static);
-    key_add(k, a.split_k); key_add(k, a.block_n_hint); key_add(k, a.k_part); key_add(k, a.algo_flops);
+    key_add(k, a.split_k); key_add(k, a.split_cluster); key_add(k, a.block_n_hint); key_add(k, a.k_part); key_add(k, a.algo_flops);
     return k;
 }
 
@@ -927,14 +1148,15 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         g.ksize = 1; g.stride = 1; g.pad = 0;
         g.sc = 1; g.sw = a.lda; g.sh = (long)a.lda * a.M; g.sn = (long)a.lda * a.M;
     }
-    // Split-K: the K blocks (taps x channel slices) are divided among `split_k` tiles that each write their
-    // own slab of y ([split][batch][OH][OW][N]); the caller adds the slabs and applies the epilogue.
+    // Split-K: the K blocks (taps x channel slices) are divided among the `split_k` CTAs of a cluster, or among tiles that each
+    // write their own slab of y ([split][batch][OH][OW][N]); the caller then adds the slabs and applies the epilogue.
     const int S = (!gather && a.split_k > 1) ? a.split_k : 1;
+    const bool cluster = S > 1 && a.split_cluster;
     const int kc = a.Kc;
     const int ksize_w = g.ksize_w > 0 ? g.ksize_w : g.ksize;
     const int taps = g.ksize * ksize_w;
     const bool pool = a.y_pool != nullptr;
-    Box box = choose_box(g.OW, g.OH, g.batch, g.stride, pool, S > 1, (double)g.sn * 4.0);
+    Box box = choose_box(g.OW, g.OH, g.batch, g.stride, pool, S > 1 && !cluster, (double)g.sn * 4.0);
     const bool col3 = a.a_is_conv && !gather && !three_pass && S == 1 && column_stages(g, kc, a.N);
     const bool pairs = !col3 && !gather && !three_pass && kc % (2 * BLOCK_K) == 0;      // K slices may be fetched in pairs
     if (col3) box = Box{16, 8, 1};
@@ -953,8 +1175,13 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     // whole pairs of K slices per split where that leaves none empty (256-wide tiles do not fetch pairs)
     if (S > 1 && p.c_blocks % 2 == 0 && (p.kb_per_split & 1) && a.block_n_hint <= 128 && (long)(S - 1) * (p.kb_per_split + 1) < p.num_k_blocks)
         p.kb_per_split++;
-    if (S > 1 && ((long)(S - 1) * p.kb_per_split >= p.num_k_blocks || a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
-        throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks and a plain epilogue");
+    if (S > 1 && (long)(S - 1) * p.kb_per_split >= p.num_k_blocks)
+        throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks");
+    if (S > 1 && !cluster && (a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
+        throw Error(NB_ERR_INVALID_ARG, "split-K into slabs needs a plain epilogue");
+    if (cluster && (S > TC_MAX_CLUSTER || (a.N % 4) != 0 || a.lstm_H ||
+                    (a.addend && (a.res_stride == 0 || (a.res_c % 4) != 0 || (a.ld_addend % 4) != 0 || !aligned16(a.addend)))))
+        throw Error(NB_ERR_INVALID_ARG, "split-K over a cluster needs quads of columns");
     p.k_splits = S;
     p.m_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
     p.e.N = a.N;
@@ -970,16 +1197,17 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.e.y = a.y; p.e.ldy = a.ldy;
     p.e.tma_store = a.y && aligned16(a.y) && (a.ldy % 4) == 0 && !a.y_nchw;
     if (a.y_nchw) {
-        if (!a.a_is_conv || gather || S > 1 || pool || a.lstm_H > 0)
+        if (!a.a_is_conv || gather || (S > 1 && !cluster) || pool || a.lstm_H > 0)
             throw Error(NB_ERR_INVALID_ARG, "NCHW output needs a whole convolution whose rows are pixels");
         p.e.plane = g.OH * g.OW;
     }
-    if (S > 1 && !p.e.tma_store) throw Error(NB_ERR_INVALID_ARG, "split-K needs a 16-byte aligned output with ldy % 4 == 0");
+    if (S > 1 && !cluster && !p.e.tma_store) throw Error(NB_ERR_INVALID_ARG, "split-K needs a 16-byte aligned output with ldy % 4 == 0");
     p.e.pool = pool ? 1 : 0;
     if (pool) {
         if (!a.a_is_conv || (g.OW & 1) || (g.OH & 1) || (a.N % 4) || !aligned16(a.y_pool) || a.addend)
             throw Error(NB_ERR_UNSUPPORTED, "fused 2x2 pooling needs even output extents and a 16-byte aligned NHWC tensor");
-        p.e.tma_store = 0;
+        p.e.tma_store = cluster;            // (there: whether rows are quads on 16-byte boundaries)
+        if (cluster) { p.e.y = a.y_pool; p.e.ldy = a.N; }
     } else if (a.lstm_H > 0) {
         if (a.a_is_conv || S > 1 || a.N != 4 * a.lstm_H || !a.lstm_c || !a.lstm_h)
             throw Error(NB_ERR_INVALID_ARG, "LSTM epilogue needs a plain [M,4H] product and c/h outputs");
@@ -1012,7 +1240,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         long best_cost = 0;
         for (int bn = widest; bn >= 64; bn /= 2) {
             if (bn > 64 && a.N <= bn / 2) continue;         // more than half of the tile would be padding
-            const long tiles = (long)p.m_tiles * S * ((a.N + bn - 1) / bn);
+            const long tiles = (long)p.m_tiles * ((a.N + bn - 1) / bn) * S;
             const long waves = (tiles + h->sm_count - 1) / h->sm_count;
             const long mma = bn == 256 ? 512 : (bn == 128 ? 256 : 192);
             const long supply = (long)(BLOCK_M + bn) * BLOCK_K * 4 / 71;
@@ -1115,7 +1343,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         check_extent(h, a.addend, 0, fl * F4, "addend");
     }
     if (a.y && !pool && !a.lstm_H)
-        check_extent(h, a.y, 0, (((long long)S * a.M - 1) * a.ldy + a.N) * F4, "output");
+        check_extent(h, a.y, 0, (((long long)(cluster ? 1 : S) * a.M - 1) * a.ldy + a.N) * F4, "output");
     if (pool) check_extent(h, a.y_pool, 0, (long long)g.batch * (g.OH / 2) * (g.OW / 2) * a.N * F4, "pooled output");
     if (a.lstm_H > 0) {
         const long long fl = (long long)a.M * a.lstm_H * F4;
@@ -1162,7 +1390,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         if (three_pass) encode(h, &p.tm_b_lo, a.b_lo, 3, dims, strides, bx, es);
     }
 
-    if (p.e.tma_store) {   // Y: dims {N, OW, OH, NB}; the same pixel box as A, 32 columns wide
+    if (p.e.tma_store && !cluster) {   // Y: dims {N, OW, OH, NB}; the same pixel box as A, 32 columns wide
         cuuint64_t dims[4] = {(cuuint64_t)a.N, (cuuint64_t)g.OW, (cuuint64_t)g.OH, (cuuint64_t)g.batch * (cuuint64_t)S};
         cuuint64_t strides[3] = {(cuuint64_t)a.ldy * 4, (cuuint64_t)a.ldy * 4 * (cuuint64_t)g.OW,
                                  (cuuint64_t)a.ldy * 4 * (cuuint64_t)g.OW * (cuuint64_t)g.OH};
@@ -1171,7 +1399,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         encode(h, &p.tm_y, a.y, 4, dims, strides, bx, es);
     }
 
-    if (pool) {          // pooled Y: dims {N, OW/2, OH/2, NB}
+    if (pool && !cluster) {          // pooled Y: dims {N, OW/2, OH/2, NB}
         cuuint64_t dims[4] = {(cuuint64_t)a.N, (cuuint64_t)(g.OW / 2), (cuuint64_t)(g.OH / 2), (cuuint64_t)g.batch};
         cuuint64_t strides[3] = {(cuuint64_t)a.N * 4, (cuuint64_t)a.N * 4 * (cuuint64_t)(g.OW / 2),
                                  (cuuint64_t)a.N * 4 * (cuuint64_t)(g.OW / 2) * (cuuint64_t)(g.OH / 2)};
@@ -1180,10 +1408,12 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         encode(h, &p.tm_yp, a.y_pool, 4, dims, strides, bx, es);
     }
 
-    L->v = VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][block_n == 256 ? 2 : (block_n == 128 ? 1 : 0)];
+    const int width = block_n == 256 ? 2 : (block_n == 128 ? 1 : 0);
+    L->v = cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
+    L->cluster = cluster ? S : 1;
     if (!L->v.kernel) throw Error(NB_ERR_UNSUPPORTED, "no tensor-core kernel variant for this tile width");
     const int tiles = p.m_tiles * p.n_tiles * p.k_splits;
-    L->grid = std::max(1, std::min(tiles, h->sm_count));
+    L->grid = cluster ? tiles : std::max(1, std::min(tiles, h->sm_count));
     L->threads = (three_pass || gather) ? 448 : 320;
     L->gather = gather;
     L->flops = a.algo_flops > 0 ? a.algo_flops : 2.0 * (double)a.M * a.N * a.Kc * taps;
@@ -1191,7 +1421,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
               std::to_string(taps) + " stride=" + std::to_string(g.stride) + " out=" + std::to_string(g.OW) + "x" +
               std::to_string(g.OH) + "x" + std::to_string(g.batch) + " box=" + std::to_string(box.bw) + "x" +
               std::to_string(box.bh) + "x" + std::to_string(box.bn) + " block_n=" + std::to_string(block_n) +
-              " splits=" + std::to_string(S) + (p.col3 ? (p.halves == 2 ? " col3x2" : " col3") : "") + (p.cbs == 2 ? " cbs2" : "") + (gather ? " gather" : "") +
+              " splits=" + std::to_string(S) + (cluster ? "c" : "") + (p.col3 ? (p.halves == 2 ? " col3x2" : " col3") : "") + (p.cbs == 2 ? " cbs2" : "") + (gather ? " gather" : "") +
               (three_pass ? " 3xtf32" : "") +
               (pool ? " pool" : "") + (a.addend ? " addend" : "") + (a.lstm_H ? " lstm" : "") + "]";
     return L;
@@ -1216,6 +1446,42 @@ int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
     int per = (blocks + S - 1) / S;
     if (c_blocks % 2 == 0) per += per & 1;      // whole pairs of slices: two-block ring stages stay possible
     return (blocks + per - 1) / per;
+}
+
+// The time of a contraction whose tiles are cut over clusters of S CTAs, all clusters resident at once, in units of a 64-wide
+// TF32 K block (0.225 us); S = 1: whole, in waves.  Negative: it does not run that way.  Of a cluster each CTA adds S partial
+// sums of 1/S of its tile, so the exchange costs most for the smallest and the largest, and a large cluster waits for that many
+// SMs of one part of the device.  3x3 layers of one image (28 x 28 x 128, 14 x 14 x 256, 7 x 7 x 512), us: whole 13.1 / 21.0 /
+// 37.7, S = 2: 11.1 / 15.0 / 22.4, 4: 7.6 / 9.8 / 13.6, 6: 7.6 / 7.9 / 11.1, 9: 7.9 / 7.9 / 9.3; the weight of S is a ResNet-50 image's
+// (0.5: 435 us, 1: 427, 1.5: 424, 2: 425).  128-wide tiles were never better in TF32.  A 3xTF32 block takes half as long again, a
+// 128-wide one a third more, and its exchange four times as long (3xTF32, 19 x 19 x 100 at 20 images: whole 25 us, two halves of K
+// 30; 14 x 14 x 512 at 8: 64 and 50).
+double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, int S, int bn, bool three_pass, int act) {
+    const long tiles = m_tiles * ((N + bn - 1) / bn);
+    const double block = (three_pass ? 1.5 : 1.0) * (bn == 64 ? 1.0 : 1.33);
+    const double heavy = act == NB_ACT_RELU || act == NB_ACT_LEAKY || act == NB_ACT_LINEAR ? 0.0 : 24.0 * bn / 64;     // the double formulas
+    if (S == 1) return (double)((tiles + h->sm_count - 1) / h->sm_count) * (blocks * block + heavy);
+    const int per = (blocks + S - 1) / S;
+    if (tiles > h->tc_clusters[S] || (long)(S - 1) * per >= blocks) return -1;
+    return per * block + heavy / S + 1.5 * S + 26.0 * (bn / 64) * (bn / 64) / (S * S);
+}
+
+// The tile width and cluster size of a convolution.  In TF32 only where its 64-wide tiles leave half of the SMs idle, as above.
+TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool) {
+    TcSplit best{1, 0};
+    const int c_blocks = (Kc + BLOCK_K - 1) / BLOCK_K, blocks = g.ksize * (g.ksize_w > 0 ? g.ksize_w : g.ksize) * c_blocks;
+    if ((N % 4) != 0) return best;
+    const Box box = choose_box(g.OW, g.OH, g.batch, g.stride, pool, false, (double)g.C * g.H * g.W * 4.0);
+    const long m_tiles = (long)((g.OW + box.bw - 1) / box.bw) * ((g.OH + box.bh - 1) / box.bh) * ((g.batch + box.bn - 1) / box.bn);
+    if (!three_pass && 2 * m_tiles * ((N + 63) / 64) > h->sm_count) return best;
+    double best_cost = tc_cluster_cost(h, m_tiles, N, blocks, 1, 64, three_pass, act);
+    if (three_pass && N > 64) best_cost = std::min(best_cost, tc_cluster_cost(h, m_tiles, N, blocks, 1, 128, true, act));
+    for (int bn = 64; bn <= (three_pass && N > 64 ? 128 : 64); bn *= 2)
+        for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
+            const double cost = tc_cluster_cost(h, m_tiles, N, blocks, S, bn, three_pass, act);
+            if (cost >= 0 && cost < best_cost) { best_cost = cost; best = TcSplit{S, bn}; }
+        }
+    return best;
 }
 
 // A lane of the epilogue owns a pixel, so in NCHW a warp's stores of a column are as contiguous as its box's pixels.  Boxes
@@ -1245,15 +1511,17 @@ void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass) {
     cfg.blockDim = dim3((unsigned)L.threads);
     cfg.dynamicSmemBytes = (size_t)L.v.smem;
     cfg.stream = h->stream;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)L.cluster; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
     // The gather variants are not launched ahead.  Launched ahead, every second of two queued calls (30 channels, 3x3, 8
     // images of 33 x 33: 9 K blocks, 69 CTAs) left about ten CTAs whose accumulators never completed, so that the wait for them
     // ran out and the output kept the call's before; alone the same call is right.  They are the only launches with more than
     // 4096 bytes of parameters (TcGatherParams: 4160), the one thing that sets them apart; the cause is not proven.
-    cfg.numAttrs = L.gather ? 0 : 1;
+    cfg.numAttrs = L.gather ? 0 : (L.cluster > 1 ? 2 : 1);
     void *args[1] = {const_cast<TcGatherParams *>(&L.p)};
     (void)cudaLaunchKernelExC(&cfg, L.v.kernel, args);
     try {

@@ -65,6 +65,7 @@ struct nb_handle_s {
     unsigned int *d_grid_sync = nullptr; // arrival counters of the persistent LSTM kernel (it leaves them zero)
     int lstm_clusters = 0;              // lstm_persistent.cu: clusters of its size that the device runs at once
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
+    int tc_clusters[17] = {0};          // gemm_tcgen05.cu: the same for its kernel
     bool recurrent_ready = false;       // recurrent_cluster.cu: limits set, clusters_at_once filled
     unsigned long long simt_ready = 0;  // gemm_simt.cu: kernels loaded and with their limits set, by variant and copy modes
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
@@ -215,7 +216,10 @@ struct GemmArgs {
     // contract K in `split_k` slices of ceil(K blocks / split_k) 32-wide blocks (the last may be
     // shorter, none empty); slice s writes y + s*M*ldy
     // (y must hold split_k * M * ldy floats; the caller reduces the slices and applies the epilogue)
+    // split_cluster: the slices are the CTAs of a cluster (up to TC_MAX_CLUSTER), which add them and run the
+    // whole epilogue themselves
     int split_k = 1;
+    bool split_cluster = false;
     // tensor-core kernel: tile width in output columns (64, 128 or 256) instead of the built-in choice; 0 = automatic
     int block_n_hint = 0;
     // tensor-core kernel, TF32: K blocks per partial sum (those are added in fp32 registers); 0 = built-in choice
@@ -229,6 +233,12 @@ bool gemm_tc_supported(const nb_handle_s *h, const GemmArgs &a);
 void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
 // How many K slices (GemmArgs::split_k) an NHWC convolution should be cut into on the tensor cores; 1: none.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
+// How many CTAs of a cluster (GemmArgs::split_k; 1: no cluster) the K of an NHWC convolution's tiles should be cut over on the
+// tensor cores, and the tile width.
+struct TcSplit { int S, block_n; };
+TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool);
+constexpr int TC_MAX_CLUSTER = 16;
+double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, int S, int bn, bool three_pass, int act);
 // Is an NCHW output (GemmArgs::y_nchw) the faster way for this convolution, against a layout pass behind it?
 bool conv_tc_writes_nchw(const GemmArgs &a, bool three_pass);
 // CUDA-core fp32 path: any extents, strides and alignments.
@@ -368,7 +378,7 @@ inline void key_add(std::string &k, const T &v) { k.append(reinterpret_cast<cons
 std::string gemm_args_key(const GemmArgs &a, char tag, int extra);
 
 // Per-device set-up of the tensor-core kernels (shared-memory limits; also loads their code), once per handle.
-void gemm_tc_prepare_device();
+void gemm_tc_prepare_device(nb_handle_s *h);
 void lstm_persistent_prepare_device(nb_handle_s *h);
 int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);

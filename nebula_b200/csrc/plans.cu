@@ -74,6 +74,9 @@ ConvPlan::ConvPlan(nb_handle_s *hh, const nb_conv2d_desc_t &desc) : nb_plan_s(NB
     // NEBULA_B200_ROW_WINDOWS=0 (read when the plan is created) sends these layers through the in-kernel gather instead
     const char *rw_env = std::getenv("NEBULA_B200_ROW_WINDOWS");
     tc_split = conv_tc_split(h, conv_args(nullptr, true).g, d.channels, d.filters);
+    for (int three = 0; three < 2; three++)
+        for (int pool = 0; pool < 2; pool++)
+            tc_cluster[three][pool] = conv_tc_cluster(h, conv_args(nullptr, true).g, d.channels, d.filters, d.activation, three, pool);
     rowwin_ok = !(rw_env && *rw_env == '0') && d.channels <= 4 && rw_inner <= 256 && d.stride <= 8 && h->encode_tiled &&
                 h->cc_major == 10;
 }
@@ -135,10 +138,14 @@ bool ConvPlan::can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const {
            (conn_c % 4) == 0 && (d.filters % 4) == 0;
 }
 
-int ConvPlan::splits(const ForwardOpts &o) const {
-    if (path(o) == PATH_SIMT || o.addend) return 1;
-    if (o.residual && ((o.res_c % 4) != 0 || ((uintptr_t)o.residual & 15))) return 1;     // (the reduction reads it in quads)
-    return tc_split;
+// K over clusters, whose CTAs run the whole epilogue.  A call on a caller's NHWC tensor, which takes a pass in front, keeps the
+// product and the addition of its slices as two kernels: the launches of such a call are relied on.
+TcSplit ConvPlan::splits(const ForwardOpts &o, bool *clusters) const {
+    const GemmPath pth = path(o);
+    *clusters = !(o.x_nhwc && (o.x_foreign || (pth == PATH_TC && !o.x_rounded)));
+    if (pth == PATH_SIMT || o.addend) return TcSplit{1, 0};
+    if (o.residual && ((o.res_c % 4) != 0 || ((uintptr_t)o.residual & 15))) return TcSplit{1, 0};     // (read in quads there)
+    return *clusters ? tc_cluster[pth == PATH_TC3][o.pool_out != nullptr] : TcSplit{tc_split, 0};
 }
 
 // The TMA-fed tensor-core routes write NCHW themselves where their pixel boxes suit it; the others (CUDA cores, in-kernel
@@ -146,7 +153,12 @@ int ConvPlan::splits(const ForwardOpts &o) const {
 bool ConvPlan::writes_nchw(const ForwardOpts &o) {
     if (o.y_nhwc || h->math_mode == NB_MATH_FP32) return false;
     const bool simt = path(o) == PATH_SIMT, three = h->math_mode == NB_MATH_TF32X3;
-    if (simt ? !rowwin_ok : splits(o) > 1) return false;
+    bool clusters;
+    if (simt) {
+        if (!rowwin_ok) return false;
+    } else if (splits(o, &clusters).S > 1) {
+        return clusters;                // (they have small outputs)
+    }
     if (nchw_direct[three] < 0)
         nchw_direct[three] = conv_tc_writes_nchw(simt ? rowwin_args(nullptr, nullptr, false) : conv_args(nullptr, true), three);
     return nchw_direct[three] > 0;
@@ -195,8 +207,9 @@ size_t ConvPlan::reserve(const ForwardOpts &o) {
     } else {
         const bool need_round = (pth == PATH_TC) && !o.x_rounded;
         if (!o.x_nhwc || need_round || o.x_foreign) x_scratch.reserve(xin);
-        const int S = splits(o);
-        if (S > 1) split_ws.reserve((size_t)S * yout);
+        bool clusters;
+        const int S = splits(o, &clusters).S;
+        if (S > 1 && !clusters) split_ws.reserve((size_t)S * yout);
     }
     return workspace_bytes();
 }
@@ -315,9 +328,14 @@ void ConvPlan::forward(const float *x, float *y, const ForwardOpts &o) {
         w.ensure_split(h);
         a.b = w.hi.p;
         a.b_lo = w.lo.p;
-        int S = splits(o);
-        if (o.residual && ((uintptr_t)y & 15)) S = 1;       // (the reduction writes a folded shortcut's sums in quads)
-        if (S > 1) {
+        bool clusters;
+        const TcSplit split = splits(o, &clusters);
+        int S = split.S;
+        if (!clusters && o.residual && ((uintptr_t)y & 15)) S = 1;       // (the reduction writes a folded shortcut's sums in quads)
+        if (S > 1 && clusters) {
+            a.split_k = S; a.split_cluster = true; a.block_n_hint = split.block_n;
+            gemm_tc(h, a, pth == PATH_TC3);
+        } else if (S > 1) {
             GemmArgs sa = a;
             sa.split_k = S;
             sa.scale = sa.shift = sa.addend = nullptr; sa.res_stride = 0; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;
@@ -420,6 +438,34 @@ void FcPlan::split_choice(GemmPath pth, bool has_addend, int rows, int *S_out, i
     *S_out = S; *block_n_out = block_n;
 }
 
+// The same over clusters, which run the whole epilogue.  Clusters do not fill the SMs (132 CTAs of fours, 120 of eights, 112 of
+// sixteens of 148), so weights that take long to stream go to slabs on all of them; the others take the width and size with the
+// shortest run, as convolutions do (conv_tc_cluster).  In TF32 from 2048 columns on that depends on K, N and the device only.
+void FcPlan::cluster_choice(GemmPath pth, int rows, int *S_out, int *block_n_out) const {
+    const int kblocks = (d.inputs + 31) / 32;
+    const long m_tiles = d.inputs >= 2048 ? 1 : (rows + 127L) / 128;
+    *S_out = 1; *block_n_out = 0;
+    if (2 * m_tiles * ((d.outputs + 63) / 64) > h->sm_count) return;
+    double best = tc_cluster_cost(h, m_tiles, d.outputs, kblocks, 1, 64, pth == PATH_TC3, d.activation);
+    for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
+        const double cost = tc_cluster_cost(h, m_tiles, d.outputs, kblocks, S, 64, pth == PATH_TC3, d.activation);
+        if (cost >= 0 && cost < best) { best = cost; *S_out = S; *block_n_out = 64; }
+    }
+}
+
+// (3xTF32 on a caller's tensor keeps the product and the addition of its slices as two kernels: the launches of such a call are
+// relied on)
+bool FcPlan::splits(GemmPath pth, const ForwardOpts &o, int rows, int *S, int *block_n) const {
+    split_choice(pth, o.addend != nullptr, rows, S, block_n);
+    if (pth == PATH_SIMT || o.addend || (d.outputs % 4) != 0 || (pth == PATH_TC3 && (o.x_foreign || (*S == 1 && d.inputs >= 2048)))) return false;
+    if ((size_t)d.inputs * d.outputs > ((size_t)6 << 20)) return false;
+    int s, bn;
+    cluster_choice(pth, rows, &s, &bn);
+    if (s == 1) return false;
+    *S = s; *block_n = bn;
+    return true;
+}
+
 size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
     const int M = rows > 0 ? rows : d.batch;
     const GemmPath pth = path();
@@ -430,8 +476,8 @@ size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
         gemm_simt_load(h, a);
     }
     int S, bn;
-    split_choice(pth, o.addend != nullptr, M, &S, &bn);
-    if (S > 1) split_ws.reserve((size_t)S * M * d.outputs);
+    const bool clusters = splits(pth, o, M, &S, &bn);
+    if (S > 1 && !clusters) split_ws.reserve((size_t)S * M * d.outputs);
     return workspace_bytes();
 }
 
@@ -469,8 +515,11 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
     w.ensure_split(h);
     a.b = w.hi.p; a.b_lo = w.lo.p;
     int S, block_n;
-    split_choice(pth, o.addend != nullptr, M, &S, &block_n);
-    if (S > 1) {
+    const bool clusters = splits(pth, o, M, &S, &block_n);
+    if (S > 1 && clusters) {
+        a.split_k = S; a.split_cluster = true; a.block_n_hint = block_n;
+        gemm_tc(h, a, pth == PATH_TC3);
+    } else if (S > 1) {
         GemmArgs sa = a;
         sa.split_k = S; sa.block_n_hint = block_n;
         sa.scale = nullptr; sa.shift = nullptr; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;

@@ -77,7 +77,9 @@ struct ConvPlan : nb_plan_s {
     DeviceBuffer x_rowwin;
     DeviceBuffer scale, shift;
     bool has_scale = false, ready = false;
-    int tc_split = 1;           // K slices on the tensor cores: a search over pixel boxes, so done once
+    // K slices on the tensor cores, a search over pixel boxes, so done once: into slabs, and over clusters [3xTF32][pooled output]
+    int tc_split = 1;
+    TcSplit tc_cluster[2][2];
     int nchw_direct[2] = {-1, -1};      // TF32, 3xTF32: does the epilogue write NCHW?  (-1: not asked yet)
     DeviceBuffer x_scratch, y_scratch, split_ws;
     ConvPlan(nb_handle_s *h, const nb_conv2d_desc_t &desc);
@@ -92,7 +94,7 @@ struct ConvPlan : nb_plan_s {
     GemmArgs conv_args(const float *x, bool nhwc) const;
     GemmArgs rowwin_args(const float *xw, const float *weights, bool cuda_cores) const;
     // K slices of the tensor-core path with these options (1: none)
-    int splits(const ForwardOpts &o) const;
+    TcSplit splits(const ForwardOpts &o, bool *clusters) const;
     bool writes_nchw(const ForwardOpts &o);
     // can the following 2x2 stride-2 max-pool be done in this layer's epilogue?
     bool can_fuse_pool() const;
@@ -114,6 +116,8 @@ struct FcPlan : nb_plan_s {
     size_t workspace_bytes() const override { return (x_scratch.n + split_ws.n) * sizeof(float); }
     // split-K choice for `rows` input rows: number of K slices (1: none) and the tile width that goes with it
     void split_choice(GemmPath pth, bool has_addend, int rows, int *S, int *block_n) const;
+    void cluster_choice(GemmPath pth, int rows, int *S_out, int *block_n_out) const;
+    bool splits(GemmPath pth, const ForwardOpts &o, int rows, int *S, int *block_n) const;      // true: over clusters
     void output_dims(int dims[3]) const override { dims[0] = d.outputs; dims[1] = 1; dims[2] = 1; }
     GemmPath path() const;
 };

@@ -1,0 +1,75 @@
+"""Contractions whose K is cut over a cluster, at the edges: boxes of few and ragged rows, columns off the tile width, a last
+slice that is shorter, shares that leave CTAs without rows, NCHW and NHWC rows, the shortcut and the pool folded in.  NCHW
+layers on their own, networks for what only they fold, against the CPU oracle."""
+import numpy as np
+import pytest
+
+from tests.util import assert_close, logit_err, NET_TOL
+
+pytestmark = pytest.mark.gpu
+
+
+def _t(a):
+    import torch
+    return torch.from_numpy(np.ascontiguousarray(a, dtype=np.float32)).cuda()
+
+
+# (B, C, H, W, F, k, stride, pad)
+CONVS = [(1, 512, 7, 7, 512, 3, 1, 1), (1, 256, 1, 1, 64, 1, 1, 0), (2, 132, 9, 7, 36, 3, 1, 1), (3, 96, 13, 5, 68, 5, 2, 2),
+         (1, 128, 28, 28, 128, 3, 1, 1), (5, 2048, 3, 3, 60, 1, 1, 0), (7, 64, 11, 11, 260, 3, 2, 0), (40, 256, 2, 2, 132, 2, 1, 0)]
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+@pytest.mark.parametrize("case", CONVS, ids=lambda c: "x".join(map(str, c)))
+def test_nchw_convolution(handle, mode, case):
+    from nebula_b200 import api
+    from oracle import oracle as O
+    B, C, H, W, F, k, s, p = case
+    rng = np.random.default_rng(C + F)
+    x = rng.standard_normal((B, C, H, W), dtype=np.float32)
+    w = (rng.standard_normal((F, C, k, k)) * np.sqrt(2.0 / (C * k * k))).astype(np.float32)
+    b = (0.1 * rng.standard_normal(F)).astype(np.float32)
+    bn = ((rng.random(F) + 0.5).astype(np.float32), (0.1 * rng.standard_normal(F)).astype(np.float32), (rng.random(F) + 0.5).astype(np.float32))
+    handle.set_math(mode)
+    plan = api.Conv2d(handle, B, C, H, W, F, k, s, p, True, "leaky")
+    plan.set_weights(w, b, bn)
+    xd = _t(x)
+    y = plan.forward(xd)
+    again = plan.forward(xd)            # (queued behind it)
+    handle.synchronize()
+    plan.close()
+    assert_close(y.cpu().numpy(), O.conv_forward(x, w, b, k, s, p, "leaky", bn), mode, f"{case}")
+    assert (y == again).all()
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+@pytest.mark.parametrize("batch", [1, 3])
+@pytest.mark.parametrize("size", [20, 14])
+def test_network_of_small_layers(handle, mode, batch, size):
+    """Pool and shortcut folded in, connected layers of several depths behind."""
+    import torch
+    from nebula_b200 import api
+    from nebula_b200.workloads import NetBuilder
+    from oracle import oracle as O
+    b = NetBuilder("n", batch, channels=64, height=size, width=size, bias_init="bias_n01")
+    b.conv(128, 3, 1, 1, "relu", bn=True)
+    b.conv(128, 3, 1, 1, "relu")
+    b.maxpool(2, 2, 0)
+    b.conv(256, 1, 1, 0, "leaky")
+    b.conv(256, 3, 1, 1, "linear", bn=True)
+    b.shortcut(2, "relu")
+    b.connected(300, "tanh")
+    b.connected(100, "logistic")
+    b.connected(12, "linear")
+    wl = b.build("normal")
+    w, x = wl.make_weights(3), wl.make_input(4)
+    ref = O.forward_network(wl.cfg, w, x, keep_all=True)
+    handle.set_math(mode)
+    net = api.Network(handle, wl.cfg)
+    net.load_weights(w)
+    net.forward(torch.from_numpy(x).cuda())
+    handle.synchronize()
+    got = net.logits()
+    net.close()
+    # TF32: six layers of 2^-12 per operand, few samples: the limit of the suite's small networks (tests/util.py)
+    assert logit_err(got, ref[-1], batch) <= (2.6e-3 if mode == "tf32" else NET_TOL[mode])
