@@ -398,6 +398,7 @@ struct RecurrentArgs {
     int T, B, H, gates, act;
     int cell_f32;               // LSTM: gate activations in fp32 instead of the double formulas
     int round_out;              // RNN: store TF32-rounded values
+    bool by_layer;              // the order of additions must not depend on the batch
 };
 // step_path: what a launch per step would run on
 bool recurrent_cluster_pays(nb_handle_s *h, int gates, int H, int B, int T, bool linear, GemmPath step_path);

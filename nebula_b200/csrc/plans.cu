@@ -694,6 +694,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         r.cell = cell; r.out = out; r.out_round = hr;
         r.T = T; r.B = B; r.H = H; r.gates = 4; r.act = d.activation;
         r.cell_f32 = tc_w && !three;
+        r.by_layer = !tc_w && B <= 256;
         recurrent_cluster(h, r);
         return;
     }
@@ -816,6 +817,7 @@ void RnnPlan::forward(const float *x, float *out, bool x_rounded, bool round_out
         r.T = T; r.B = B; r.H = d.hidden; r.gates = 1; r.act = d.activation;
         const bool out_tc = out_gate->path() == PATH_TC;
         r.round_out = out_tc;
+        r.by_layer = hid_gate->path() == PATH_SIMT && B <= 256;
         recurrent_cluster(h, r);
         ForwardOpts q;
         q.x_rounded = out_tc; q.round_out = round_out;
