@@ -63,15 +63,24 @@ bool small_gemm(bool ta, bool tb, int M, int N, int K) {
     return (tiles - 230) * 1.2e-4 * K <= gain_us;
 }
 
-// rate of a tile shape relative to the largest (fewer outputs per operand read, shorter runs between barriers)
-const double RATE[] = {1.0, 0.85, 0.7, 0.6};
+// Cycles of an SM that runs `on_sm` CTAs of tile shape i over K columns each: the share of the FMA rate that the shape reaches
+// (fewer outputs per operand read, longer runs between barriers), and its start and stores.  The 64 x 128 tile alone on an SM
+// lacks a second CTA to run behind its barriers, the more the shorter its copies.  Fitted to AlexNet's layers at 4 and 16 images and
+// to products of 64 to 2048 rows and K of 60 to 4000.
+double tile_cost(int i, const SimtVariant &v, long on_sm, int K, bool quads) {
+    static const double rate[] = {0.50, 0.41, 0.36, 0.33}, fixed[] = {4000, 1300, 200, 400};
+    double r = rate[i];
+    if (i == 0 && on_sm == 1) r = quads ? 0.47 : 0.30;
+    return on_sm * ((double)v.bm * v.bn * K / 128 / r + fixed[i]);
+}
 
-// Ranges of K: none shorter than 256 columns, and only as many as it takes to occupy the SMs with 64 x 64 tiles of
-// one image (one row of a connected layer, all rows of _gemm_).
-int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks) {
+// Ranges of K: none shorter than `least` columns, and only as many as it takes to occupy the SMs `times` over with 64 x 64 tiles of
+// one image (one row of a connected layer, all rows of _gemm_).  _gemm_: 256 x 1024 x 1024 two ranges 29 us, eight 23.  A layer's
+// S counts one image alone, so its batches fill the SMs anyway (64 -> 64 3x3 at 56 x 56, 16 images: whole 123 us, two ranges 137).
+int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks, int least, int times) {
     const long tiles = ((unit_rows + 63) / 64) * ((N + 63) / 64);
     int S = 1;
-    while (S < 8 && tiles * S < h->sm_count && k_blocks / (2 * S) >= 256 / BK) S *= 2;
+    while (S < 8 && tiles * S < (long)times * h->sm_count && k_blocks / (2 * S) >= least / BK) S *= 2;
     return S;
 }
 
@@ -79,14 +88,15 @@ int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks) {
 // None is loaded with the handle (all of them took 19 ms of a process's first one, while a handle uses a few at most): a plan
 // asks for its own when it reserves its scratch (gemm_simt_load); a kernel first met by a launch, captured ones included, is
 // loaded there.
-const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int S, int amode, int bmode) {
+const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, int S, int amode, int bmode) {
     const SimtVariant *all = variants(amode, bmode);
     int best = 0;
     double best_cost = 0;
     for (int i = 0; i < SIMT_VARIANTS; i++) {
         const SimtVariant &v = all[i];
         const long ctas = ((M + v.bm - 1L) / v.bm) * ((N + v.bn - 1L) / v.bn) * S;
-        const double cost = (double)((ctas + h->sm_count - 1) / h->sm_count) * v.bm * v.bn / RATE[i];
+        const long on_sm = (ctas + h->sm_count - 1) / h->sm_count;
+        const double cost = tile_cost(i, v, on_sm, K / S, amode == VEC_K && bmode == VEC_K);
         if (i == 0 || cost < best_cost) { best_cost = cost; best = i; }
     }
     const SimtVariant &v = all[best];
@@ -101,7 +111,7 @@ const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int S, int amode
 }
 
 void launch(nb_handle_s *h, SimtParams &p, int amode, int bmode, int S) {
-    const SimtVariant &v = ready_variant(h, p.M, p.N, S, amode, bmode);
+    const SimtVariant &v = ready_variant(h, p.M, p.N, p.k_blocks * BK, S, amode, bmode);
     p.n_tiles = (p.N + v.bn - 1) / v.bn;
     p.kb_per_split = (p.k_blocks + S - 1) / S;
     cudaLaunchConfig_t cfg = {};
@@ -151,14 +161,14 @@ static void simt_params(const nb_handle_s *h, const GemmArgs &a, SimtParams *out
     // channel (NCHW) is read with lanes along the pixels
     *amode = p.g.sc == 1 ? (a.Kc % 4 == 0 && vec_ok(p.a, p.g.sn, p.g.sh, p.g.sw) ? VEC_K : ONE_K) : ONE_ROW;
     *bmode = a.Kc % 4 == 0 && vec_ok(p.b, a.ldb, p.b_tap, 0) ? VEC_K : ONE_K;
-    *S = split_of(h, a.a_is_conv ? (long)p.g.OH * p.g.OW : 1, a.N, p.k_blocks);
+    *S = split_of(h, a.a_is_conv ? (long)p.g.OH * p.g.OW : 1, a.N, p.k_blocks, 256, 1);
 }
 
 void gemm_simt_load(nb_handle_s *h, const GemmArgs &a) {
     SimtParams p{};
     int amode, bmode, S;
     simt_params(h, a, &p, &amode, &bmode, &S);
-    ready_variant(h, p.M, p.N, S, amode, bmode);
+    ready_variant(h, p.M, p.N, p.k_blocks * BK, S, amode, bmode);
 }
 
 void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
@@ -195,7 +205,7 @@ void launch_sgemm(nb_handle_s *h, bool ta, bool tb, int M, int N, int K, float a
     p.y = C; p.ldy = ldc;
     const int amode = ta ? ONE_ROW : (K % 4 == 0 && vec_ok(A, lda, 0, 0) ? VEC_K : ONE_K);
     const int bmode = !tb ? ONE_ROW : (K % 4 == 0 && vec_ok(B, ldb, 0, 0) ? VEC_K : ONE_K);
-    launch(h, p, amode, bmode, split_of(h, M, N, p.k_blocks));
+    launch(h, p, amode, bmode, split_of(h, M, N, p.k_blocks, 128, 2));
 }
 
 void gemm(nb_handle_s *h, const GemmArgs &a) {

@@ -10,6 +10,8 @@
 //   * Both operands lie in shared memory with K contiguous (rows of 16 floats, stride 20: eight rows of a 128-bit
 //     read fall into 32 different banks), so the copies are cp.async straight from global memory in the operands'
 //     own order (16 bytes each where alignment allows, else 4) and nothing is transposed by the threads.
+//   * Copies advance their addresses from block to block; what depends on the filter tap is worked out when a tap begins (per copy
+//     and block it was four tenths of all instructions, many of them on the FMA pipe).
 //   * A thread owns RM x RN outputs and multiplies with packed fma.rn.f32x2 along K: a 128-bit read delivers two
 //     packed pairs, the accumulator pair holds the even and the odd columns' sums.  At 8 x 8 outputs a k-quad is 16
 //     reads for 128 packed FMAs; the read port is idle three quarters of the time.
@@ -72,6 +74,8 @@ struct TileMap {
     static constexpr int TOTAL = ROWS * PER_ROW;
     static constexpr int COPIES = (TOTAL + THREADS - 1) / THREADS;
     static constexpr int ROW_SLOTS = MODE == ONE_ROW ? 1 : COPIES;      // different rows a thread touches
+    // copy i lies this many floats behind copy 0 in shared memory
+    static constexpr int STEP = MODE == ONE_ROW ? THREADS / ROWS : THREADS / PER_ROW * LDK;
     __device__ static bool active(int tid, int i) { return TOTAL % THREADS == 0 || tid + i * THREADS < TOTAL; }
     __device__ static int row(int tid, int i) {
         if (MODE == ONE_ROW) return tid % ROWS;         // THREADS is a multiple of ROWS
@@ -120,8 +124,8 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
     const int n0 = (int)(blockIdx.x % p.n_tiles) * BN;
     const int kb0 = blockIdx.z * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
 
-    // the rows this thread copies: A's pixel origin, B's row offset (-1: outside)
-    long a_base[MA::ROW_SLOTS], b_base[MB::ROW_SLOTS];
+    // the rows this thread copies: A's pixel origins (-1: outside), B's first row
+    long a_base[MA::ROW_SLOTS];
     int a_h[MA::ROW_SLOTS], a_w[MA::ROW_SLOTS];
 #pragma unroll
     for (int i = 0; i < MA::ROW_SLOTS; i++) {
@@ -135,13 +139,10 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
             a_w[i] = (rem - oh * p.g.OW) * p.g.stride - (p.g.pad_w >= 0 ? p.g.pad_w : p.g.pad);
         }
     }
-#pragma unroll
-    for (int i = 0; i < MB::ROW_SLOTS; i++) {
-        const int n = n0 + MB::row(tid, i);
-        b_base[i] = MB::active(tid, i) && n < p.N ? (long)n * p.b_row : -1;
-    }
+    const long b_base = (long)(n0 + MB::row(tid, 0)) * p.b_row;
 
-    // the K block the next copy fetches
+    // The K block the next copies fetch, and where each of them reads: the address arithmetic of a tap (64-bit products, which
+    // run on the FMA pipe) is done when the tap begins; from block to block a copy's address only advances.
     int c0 = 0, kh = 0, kw = 0;
     long b_tap = 0;
     if (kb0) {
@@ -150,35 +151,60 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
         kh = tap / p.ksize_w; kw = tap - kh * p.ksize_w;
         b_tap = (long)tap * p.b_tap;
     }
+    // (B's rows lie a constant distance apart, and so do the columns of a ONE_ROW thread: one address for all of its copies)
+    const float *a_src[MA::ROW_SLOTS], *b_src;
+    unsigned a_in = 0, b_in = 0;            // row slots that lie inside
+    auto begin_tap = [&]() {
+        a_in = 0;
+#pragma unroll
+        for (int s = 0; s < MA::ROW_SLOTS; s++) {
+            const int ih = a_h[s] + kh, iw = a_w[s] + kw;
+            const bool in = a_base[s] >= 0 && ih >= 0 && ih < p.g.H && iw >= 0 && iw < p.g.W;
+            a_src[s] = in ? p.a + a_base[s] + (long)ih * p.g.sh + (long)iw * p.g.sw + (long)(c0 + MA::col(tid, s)) * p.g.sc : p.a;
+            a_in |= (in ? 1u : 0u) << s;
+        }
+        b_src = p.b + b_tap + b_base + (long)(c0 + MB::col(tid, 0)) * p.b_col;
+    };
+#pragma unroll
+    for (int s = 0; s < MB::ROW_SLOTS; s++) b_in |= (MB::active(tid, s) && n0 + MB::row(tid, s) < p.N ? 1u : 0u) << s;
+    begin_tap();
+    const long a_step = AMODE == ONE_ROW ? BK * p.g.sc : BK, b_step = BMODE == ONE_ROW ? BK * p.b_col : BK;
+    const long a_next = AMODE == ONE_ROW ? T::THREADS / BM * p.g.sc : 0;        // from one copy of a slot to the next
+    const long b_next = BMODE == ONE_ROW ? T::THREADS / BN * p.b_col : T::THREADS / MB::PER_ROW * p.b_row;
+    const bool whole = p.Kc % BK == 0;      // no block has columns past the last
+    const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint32_t a_dst = smem32 + (uint32_t)(MA::row(tid, 0) * LDK + MA::col(tid, 0)) * 4;
+    const uint32_t b_dst = smem32 + (uint32_t)((BM + MB::row(tid, 0)) * LDK + MB::col(tid, 0)) * 4;
     auto fetch = [&](int slot) {
-        float *as = smem + slot * T::STAGE_FLOATS, *bs = as + BM * LDK;
-        const uint32_t as32 = (uint32_t)__cvta_generic_to_shared(as), bs32 = (uint32_t)__cvta_generic_to_shared(bs);
+        const uint32_t at = (uint32_t)(slot * T::STAGE_FLOATS * 4);
+        const float *src = a_src[0];
 #pragma unroll
         for (int i = 0; i < MA::COPIES; i++) {
             if (!MA::active(tid, i)) continue;
             const int s = AMODE == ONE_ROW ? 0 : i;
-            const int ih = a_h[s] + kh, iw = a_w[s] + kw, c = c0 + MA::col(tid, i);
-            const bool in = a_base[s] >= 0 && ih >= 0 && ih < p.g.H && iw >= 0 && iw < p.g.W && c < p.Kc;
-            const float *src = in ? p.a + a_base[s] + (long)ih * p.g.sh + (long)iw * p.g.sw + (long)c * p.g.sc : p.a;
-            const uint32_t dst = as32 + (uint32_t)(MA::row(tid, i) * LDK + MA::col(tid, i)) * 4;
-            if (AMODE == VEC_K) cp_async16(dst, src, in);
-            else cp_async4(dst, src, in);
+            const bool in = (a_in >> s & 1) && (whole || c0 + MA::col(tid, i) < p.Kc);
+            if (AMODE != ONE_ROW) src = a_src[s];
+            if (AMODE == VEC_K) cp_async16(a_dst + at + i * MA::STEP * 4, in ? src : p.a, in);
+            else cp_async4(a_dst + at + i * MA::STEP * 4, in ? src : p.a, in);
+            if (AMODE == ONE_ROW) src += a_next;
         }
+#pragma unroll
+        for (int s = 0; s < MA::ROW_SLOTS; s++) a_src[s] += a_step;
+        src = b_src;
 #pragma unroll
         for (int i = 0; i < MB::COPIES; i++) {
             if (!MB::active(tid, i)) continue;
-            const int s = BMODE == ONE_ROW ? 0 : i;
-            const int c = c0 + MB::col(tid, i);
-            const bool in = b_base[s] >= 0 && c < p.Kc;
-            const float *src = in ? p.b + b_tap + b_base[s] + (long)c * p.b_col : p.b;
-            const uint32_t dst = bs32 + (uint32_t)(MB::row(tid, i) * LDK + MB::col(tid, i)) * 4;
-            if (BMODE == VEC_K) cp_async16(dst, src, in);
-            else cp_async4(dst, src, in);
+            const bool in = (b_in >> (BMODE == ONE_ROW ? 0 : i) & 1) && (whole || c0 + MB::col(tid, i) < p.Kc);
+            if (BMODE == VEC_K) cp_async16(b_dst + at + i * MB::STEP * 4, in ? src : p.b, in);
+            else cp_async4(b_dst + at + i * MB::STEP * 4, in ? src : p.b, in);
+            src += b_next;
         }
+        b_src += b_step;
         c0 += BK;
         if (c0 >= p.Kc) {
             c0 = 0; b_tap += p.b_tap;
             if (++kw == p.ksize_w) { kw = 0; kh++; }
+            begin_tap();
         }
     };
 
@@ -262,7 +288,8 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
 
 typedef void (*SimtKernel)(const SimtParams);
 struct SimtVariant { SimtKernel kernel; int bm, bn, threads, smem; };
-// 8 x 8, 8 x 4 and 4 x 4 outputs per thread; the last for few rows
+// 8 x 8 (two CTAs per SM: one of 128 x 128 with a barrier for all of the SM's warps took twice as long on AlexNet's third and
+// fourth layers, 82 -> 44 us and 115 -> 60), 8 x 4 and 4 x 4 outputs per thread; the last for few rows
 constexpr int SIMT_VARIANTS = 4;
 
 template <int AMODE, int BMODE, int BM, int BN, int RM, int RN, int STAGES>

@@ -6,7 +6,7 @@ namespace nb {
 template <>
 const SimtVariant *simt_variants<NB_SIMT_A, NB_SIMT_B>() {
     static const SimtVariant v[SIMT_VARIANTS] = {
-        simt_variant<NB_SIMT_A, NB_SIMT_B, 128, 128, 8, 8, 3>(), simt_variant<NB_SIMT_A, NB_SIMT_B, 64, 64, 8, 4, 4>(),
+        simt_variant<NB_SIMT_A, NB_SIMT_B, 64, 128, 8, 8, 4>(), simt_variant<NB_SIMT_A, NB_SIMT_B, 64, 64, 8, 4, 4>(),
         simt_variant<NB_SIMT_A, NB_SIMT_B, 32, 64, 4, 4, 4>(), simt_variant<NB_SIMT_A, NB_SIMT_B, 16, 128, 4, 4, 4>()};
     return v;
 }
