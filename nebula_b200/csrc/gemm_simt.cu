@@ -23,6 +23,93 @@ const SimtVariant *variants(int amode, int bmode) {
     return table[amode][bmode]();
 }
 
+// A product of at most eight rows: the weights stream once from HBM, and a tile of 16 rows would spend its FMAs on rows that are not
+// there (AlexNet's connected layers at 4 images, 9216 -> 4096 and 4096 -> 4096: 79 and 38 us in 16 x 128 tiles, 38 and 19 here, 0.9
+// of the copy rate being 26 and 11).  A thread owns an output column of all MR rows; 64 columns of weights at a time come through a
+// ring of shared memory by 16-byte cp.async (rows of 64 floats, stride 68: a 128-bit read of eight rows falls into 32 banks), the
+// rows of A beside them, read as broadcasts.  Ranges of K, packed FMAs along K and their order are the tiles' above, so that a
+// row alone and in a batch that runs there gives the same bits.
+constexpr int ROWS_BN = 64, ROWS_BK = 64, ROWS_LD = ROWS_BK + 4, ROWS_STAGES = 5;
+constexpr int rows_smem(int MR) { return ROWS_STAGES * (ROWS_BN * ROWS_LD + MR * ROWS_BK) * 4; }
+
+template <int MR>
+__global__ void __launch_bounds__(ROWS_BN) gemm_rows_kernel(const SimtParams p) {
+    constexpr int STAGE = ROWS_BN * ROWS_LD + MR * ROWS_BK;     // floats
+    extern __shared__ __align__(16) float smem[];
+    grid_dependents_start();
+    const int tid = threadIdx.x, n0 = blockIdx.x * ROWS_BN;
+    const int k0 = blockIdx.z * p.kb_per_split * BK, k1 = min(k0 + p.kb_per_split * BK, p.Kc);
+    const int blocks = max(0, (k1 - k0 + ROWS_BK - 1) / ROWS_BK);
+    const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
+    const int quad = tid & 15, row = tid >> 4;                  // of the first copy: 16 lanes copy a row, 4 rows at a time
+    const float *src = p.b + (long)(n0 + row) * p.b_row + k0 + 4 * quad;
+    auto fetch = [&](int block, int slot) {
+        const uint32_t at = smem32 + (uint32_t)(slot * STAGE * 4);
+        const bool in_k = k0 + block * ROWS_BK + 4 * quad < k1;
+#pragma unroll
+        for (int i = 0; i < ROWS_BN / 4; i++) {
+            const bool in = in_k && n0 + row + 4 * i < p.N;
+            cp_async16(at + (uint32_t)((row + 4 * i) * ROWS_LD + 4 * quad) * 4, in ? src + (long)block * ROWS_BK + (long)(4 * i) * p.b_row : p.b, in);
+        }
+#pragma unroll
+        for (int i = 0; i < (MR * 16 + ROWS_BN - 1) / ROWS_BN; i++) {
+            const int m = row + 4 * i;
+            if (m >= MR) break;
+            const bool in = in_k && m < p.M;
+            cp_async16(at + (uint32_t)(ROWS_BN * ROWS_LD + m * ROWS_BK + 4 * quad) * 4, in ? p.a + (long)m * p.g.sw + k0 + block * ROWS_BK + 4 * quad : p.a, in);
+        }
+    };
+    unsigned long long acc[MR];
+#pragma unroll
+    for (int m = 0; m < MR; m++) acc[m] = 0ull;
+#pragma unroll
+    for (int s = 0; s < ROWS_STAGES - 1; s++) {
+        if (s < blocks) fetch(s, s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    int slot = 0;
+    for (int block = 0; block < blocks; block++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_STAGES - 2) : "memory");
+        __syncthreads();                // this block has arrived, and the slot fetched into next is no longer read
+        if (block + ROWS_STAGES - 1 < blocks) fetch(block + ROWS_STAGES - 1, slot == 0 ? ROWS_STAGES - 1 : slot - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const float *bs = smem + slot * STAGE + tid * ROWS_LD, *as = smem + slot * STAGE + ROWS_BN * ROWS_LD;
+#pragma unroll
+        for (int q = 0; q < ROWS_BK / 4; q++) {
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(bs + 4 * q);
+#pragma unroll
+            for (int m = 0; m < MR; m++) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(as + m * ROWS_BK + 4 * q);
+                ffma2(acc[m], a.x, b.x);
+                ffma2(acc[m], a.y, b.y);
+            }
+        }
+        if (++slot == ROWS_STAGES) slot = 0;
+    }
+    auto sum = [](unsigned long long v) { return __uint_as_float((unsigned)v) + __uint_as_float((unsigned)(v >> 32)); };
+    const int S = gridDim.z, n = n0 + tid;
+    if (S == 1) {
+#pragma unroll
+        for (int m = 0; m < MR; m++)
+            if (m < p.M && n < p.N) store_out(p, m, n, sum(acc[m]));
+        return;
+    }
+    // the cluster's partial sums: each CTA adds and writes its share
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < MR; m++) smem[m * ROWS_BN + tid] = sum(acc[m]);
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    for (int e = blockIdx.z * ROWS_BN + tid; e < MR * ROWS_BN; e += S * ROWS_BN) {
+        const int m = e / ROWS_BN, c = n0 + e % ROWS_BN;
+        if (m >= p.M || c >= p.N) continue;
+        float x = cluster.map_shared_rank(smem, 0)[e];
+        for (int q = 1; q < S; q++) x += cluster.map_shared_rank(smem, q)[e];
+        store_out(p, m, c, x);
+    }
+    cluster.sync();                     // no CTA may exit while another still reads its partial sums
+}
+
 // _gemm_ with few columns of K and few tiles, where a product is a handful of dependent steps whatever its tiles: 16 x 16
 // outputs per CTA, one per thread, operands loaded straight into both tiles.  Nothing is set up per copy and thread, which is
 // what the kernel above spends such a call on (64 x 64 x 64: 4.3 us here, 6.6 there; 200 x 48 x 16: 2.0 and 3.7).  It adds in
@@ -88,11 +175,16 @@ int split_of(const nb_handle_s *h, long unit_rows, int N, int k_blocks, int leas
 // None is loaded with the handle (all of them took 19 ms of a process's first one, while a handle uses a few at most): a plan
 // asks for its own when it reserves its scratch (gemm_simt_load); a kernel first met by a launch, captured ones included, is
 // loaded there.
-const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, int S, int amode, int bmode) {
-    const SimtVariant *all = variants(amode, bmode);
-    int best = 0;
+constexpr int ROWS_MAX = 8;
+const SimtVariant ROWS_VARIANTS[4] = {{gemm_rows_kernel<1>, 1, ROWS_BN, ROWS_BN, rows_smem(1)}, {gemm_rows_kernel<2>, 2, ROWS_BN, ROWS_BN, rows_smem(2)},
+                                      {gemm_rows_kernel<4>, 4, ROWS_BN, ROWS_BN, rows_smem(4)}, {gemm_rows_kernel<8>, 8, ROWS_BN, ROWS_BN, rows_smem(8)}};
+
+const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, bool plain, int S, int amode, int bmode) {
+    const bool rows = plain && M <= ROWS_MAX && amode == VEC_K && bmode == VEC_K;
+    const SimtVariant *all = rows ? ROWS_VARIANTS : variants(amode, bmode);
+    int best = rows ? (M > 4 ? 3 : (M > 2 ? 2 : (int)M - 1)) : 0;
     double best_cost = 0;
-    for (int i = 0; i < SIMT_VARIANTS; i++) {
+    for (int i = 0; i < SIMT_VARIANTS && !rows; i++) {
         const SimtVariant &v = all[i];
         const long ctas = ((M + v.bm - 1L) / v.bm) * ((N + v.bn - 1L) / v.bn) * S;
         const long on_sm = (ctas + h->sm_count - 1) / h->sm_count;
@@ -100,7 +192,7 @@ const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, int S, in
         if (i == 0 || cost < best_cost) { best_cost = cost; best = i; }
     }
     const SimtVariant &v = all[best];
-    const unsigned long long bit = 1ull << (9 * best + 3 * amode + bmode);
+    const unsigned long long bit = 1ull << (rows ? 9 * SIMT_VARIANTS + best : 9 * best + 3 * amode + bmode);
     if (!(h->simt_ready & bit)) {
         cudaFuncAttributes fa;          // (loads the code)
         if (v.smem > 48 * 1024) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
@@ -110,8 +202,13 @@ const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, int S, in
     return v;
 }
 
+// A is a matrix: one image of height 1, a 1x1 filter.
+bool plain_rows(const SimtParams &p) {
+    return p.g.H == 1 && p.g.ksize == 1 && p.ksize_w == 1 && p.g.stride == 1 && p.g.pad == 0 && p.g.pad_w <= 0 && p.g.OW == p.M;
+}
+
 void launch(nb_handle_s *h, SimtParams &p, int amode, int bmode, int S) {
-    const SimtVariant &v = ready_variant(h, p.M, p.N, p.k_blocks * BK, S, amode, bmode);
+    const SimtVariant &v = ready_variant(h, p.M, p.N, p.k_blocks * BK, plain_rows(p), S, amode, bmode);
     p.n_tiles = (p.N + v.bn - 1) / v.bn;
     p.kb_per_split = (p.k_blocks + S - 1) / S;
     cudaLaunchConfig_t cfg = {};
@@ -168,7 +265,7 @@ void gemm_simt_load(nb_handle_s *h, const GemmArgs &a) {
     SimtParams p{};
     int amode, bmode, S;
     simt_params(h, a, &p, &amode, &bmode, &S);
-    ready_variant(h, p.M, p.N, p.k_blocks * BK, S, amode, bmode);
+    ready_variant(h, p.M, p.N, p.k_blocks * BK, plain_rows(p), S, amode, bmode);
 }
 
 void gemm_simt(nb_handle_s *h, const GemmArgs &a) {
