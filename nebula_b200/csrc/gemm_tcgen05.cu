@@ -173,9 +173,9 @@ struct Cfg {
     static constexpr int TMEM_COLS = 2 * BLOCK_N;
     static constexpr int OUT_STAGE_BYTES = BLOCK_M * 32 * 4;     // one 128 x 32 output slab
     static constexpr int LAYOUT_BYTES = STAGES * STAGE_BYTES + 2 * OUT_STAGE_BYTES + 256 /*barriers*/;
-    // all of the 227 KB a CTA may have: what the layout and its alignment leave over holds the epilogue's scale/shift values
+    // all of the 227 KB a CTA may have: what the layout leaves over holds the epilogue's scale/shift values
     static constexpr int SMEM_BYTES = 227 * 1024;
-    static_assert(LAYOUT_BYTES + 1024 <= SMEM_BYTES, "ring, staging buffers and barriers must fit");
+    static_assert(LAYOUT_BYTES + (THREE ? 0 : 2 * BLOCK_N * 4) <= SMEM_BYTES, "ring, staging buffers, barriers and scale/shift values must fit");
 };
 
 // All threads of the cluster; what each wrote to its shared memory before is visible to the others behind it.
@@ -359,13 +359,13 @@ __device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *sme
 // GATHER: warps 10-13 build the A tile (compiled apart so that the common variants, which launch ten warps, are not
 // held to the register budget of fourteen).
 // CLUSTER: a tile's K is cut over the k_splits CTAs of a cluster, one tile per cluster (cluster_epilogue).
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER>
+// LEAN: only what epilogue_lean does.
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER, bool LEAN>
 __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
     using C = Cfg<BLOCK_N, THREE, GATHER>;
     constexpr int STAGES = C::STAGES;                   // barrier slots; the ring uses the first p.stages of them
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    extern __shared__ __align__(1024) uint8_t smem[];
     // per stage: [A | B], 3xTF32 [A | B | B_lo] (gathered: [A | B | A_lo | B_lo]), or [A0 | A1 | B0 | B1] with two K blocks per stage
     const int cbs = THREE ? 1 : p.cbs;
     const int stages = p.stages;
@@ -390,11 +390,9 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
     uint64_t *x_empty = acc_empty + 2;        // epilogue -> MMA: the cross terms have been read (where there is one set)
     uint32_t *tmem_slot = (uint32_t *)(x_empty + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
-    // per epilogue group: scale [BLOCK_N / 2] then shift [BLOCK_N / 2] of the columns of its slabs, if the alignment of
-    // the dynamic shared memory left room behind the barriers (it does when the base is 1024-byte aligned already)
+    // per epilogue group: scale [BLOCK_N / 2] then shift [BLOCK_N / 2] of the columns of its slabs
     float *aff_base = (float *)((uint8_t *)bars + 256);
-    const bool aff_smem = !THREE && !PROMOTE && p.e.shift != nullptr && p.e.lstm_H == 0 &&
-                          smem_raw + C::SMEM_BYTES >= (uint8_t *)(aff_base + 2 * BLOCK_N);
+    const bool aff_smem = LEAN || (!THREE && !PROMOTE && p.e.shift != nullptr && p.e.lstm_H == 0);
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -753,9 +751,13 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                         if (PROMOTE) {}         // (those variants have no registers to spare for it)
                         else if (chunk + 2 < BLOCK_N / 32 && col0 + 64 < p.e.N) next = taddr + 64;
                         else if (hf + 1 < halves) next = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * acc_cols + (hf + 1) * BLOCK_N + grp * 32);
-                        epilogue_chunk<THREE>(p.e, &p.tm_y, &p.tm_yp, v, col0, hrow, hbox, slab, bar_id, store_thread, t, stores_in_flight,
-                                              [&] { if (next) { tmem_ld_32x32(next, v); loaded = true; } },
-                                              aff_smem ? aff_base + grp * BLOCK_N + (chunk >> 1) * 32 : nullptr, BLOCK_N / 2);
+                        const float *aff = aff_smem ? aff_base + grp * BLOCK_N + (chunk >> 1) * 32 : nullptr;
+                        auto staged = [&] { if (next) { tmem_ld_32x32(next, v); loaded = true; } };
+                        if constexpr (LEAN)
+                            epilogue_lean(p.e, &p.tm_y, v, col0, hrow, hbox, slab, bar_id, store_thread, stores_in_flight, staged, aff, BLOCK_N / 2);
+                        else
+                            epilogue_chunk<THREE>(p.e, &p.tm_y, &p.tm_yp, v, col0, hrow, hbox, slab, bar_id, store_thread, t, stores_in_flight, staged,
+                                                  aff, BLOCK_N / 2);
                         slab = slab == slab0 ? slab1 : slab0;
                     }
                 }
@@ -1013,8 +1015,8 @@ void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const c
 
 struct Variant { const void *kernel; int smem; };      // takes a TcParams, or a TcGatherParams
 
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER = false>
-Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER, CLUSTER>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER = false, bool LEAN = false>
+Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER, CLUSTER, LEAN>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
 
 // index: [gather][three][promote][block_n: 0 = 64, 1 = 128, 2 = 256]; absent combinations are null
 const Variant VARIANTS[2][2][2][3] = {
@@ -1036,6 +1038,10 @@ const Variant CLUSTER_VARIANTS[2][2][3] = {
      {variant<64, true, true, false, true>(), variant<128, true, true, false, true>(), {nullptr, 0}}},
 };
 
+// index: [block_n]: the plain epilogue by itself
+const Variant LEAN_VARIANTS[3] = {variant<64, false, false, false, false, true>(), variant<128, false, false, false, false, true>(),
+                                  variant<256, false, false, false, false, true>()};
+
 // One worked-out launch: kernel parameters (tile geometry, tensor maps), kernel variant, grid.
 struct TcLaunch : LaunchRecord {
     TcGatherParams p;       // the other variants take the TcParams it starts with
@@ -1056,6 +1062,7 @@ void gemm_tc_prepare_device(nb_handle_s *h) {
             for (auto &pr : t)
                 for (auto &v : pr)
                     if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+    for (auto &v : LEAN_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     for (auto &t : CLUSTER_VARIANTS)
         for (auto &pr : t)
             for (auto &v : pr) {
@@ -1409,7 +1416,10 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     }
 
     const int width = block_n == 256 ? 2 : (block_n == 128 ? 1 : 0);
-    L->v = cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
+    const bool lean = !three_pass && !promote && !gather && !cluster && p.e.tma_store && p.e.shift &&
+                      (a.act == NB_ACT_RELU || a.act == NB_ACT_LEAKY || a.act == NB_ACT_LINEAR) &&
+                      (!a.addend || (p.e.addend_vec && p.e.addend_cols % 4 == 0 && !p.e.addend_post));
+    L->v = lean ? LEAN_VARIANTS[width] : cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
     L->cluster = cluster ? S : 1;
     if (!L->v.kernel) throw Error(NB_ERR_UNSUPPORTED, "no tensor-core kernel variant for this tile width");
     const int tiles = p.m_tiles * p.n_tiles * p.k_splits;

@@ -332,6 +332,71 @@ static __device__ __noinline__ void activate_slab(float *x, int act) {
     }
 }
 
+// The same for what most layers are: scale/shift from shared memory (`aff`: 32 scale values, 1 where the layer has none, and
+// `aff_shift` floats further the shift values), an addend of whole quads added before the activation or none, relu, leaky or linear,
+// a TMA store.  In a kernel of its own, without the other modes' code between its instructions.
+template <class Staged>
+__device__ __forceinline__ void epilogue_lean(const EpiParams &e, const CUtensorMap *tm_y, uint32_t (&v)[32], int col0, const EpiRow &rw, const EpiBox &bx,
+                                              float4 *slab, int bar_id, bool store_thread, int stores_in_flight, Staged &&staged, const float *aff,
+                                              int aff_shift) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        const float4 sc = lds128(aff + j), sh = lds128(aff + aff_shift + j);
+        v[j] = __float_as_uint(fmaf(__uint_as_float(v[j]), sc.x, sh.x));
+        v[j + 1] = __float_as_uint(fmaf(__uint_as_float(v[j + 1]), sc.y, sh.y));
+        v[j + 2] = __float_as_uint(fmaf(__uint_as_float(v[j + 2]), sc.z, sh.z));
+        v[j + 3] = __float_as_uint(fmaf(__uint_as_float(v[j + 3]), sc.w, sh.w));
+    }
+    if (rw.arow) {
+        const float *arow = rw.arow + col0;
+        auto add = [&](int j) {
+            const float4 ad = *reinterpret_cast<const float4 *>(arow + j);
+            v[j] = __float_as_uint(__uint_as_float(v[j]) + ad.x);
+            v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + ad.y);
+            v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + ad.z);
+            v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + ad.w);
+        };
+        if (col0 + 32 <= e.addend_cols) {       // (without a branch between them the eight loads overlap)
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) add(j);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                if (col0 + j < e.addend_cols) add(j);
+        }
+    }
+    if (e.act == NB_ACT_RELU) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
+    } else if (e.act == NB_ACT_LEAKY) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) {
+            const float x = __uint_as_float(v[j]);
+            v[j] = __float_as_uint(x > 0.0f ? x : (float)(0.1 * (double)x));
+        }
+    }
+    if (e.round_out) {
+#pragma unroll
+        for (int j = 0; j < 32; j++) v[j] = __float_as_uint(round_tf32(__uint_as_float(v[j])));
+    }
+    if (store_thread) {             // the group's previous store must have finished reading the staging buffer
+        if (stores_in_flight) tma_store_wait_read<1>();
+        else tma_store_wait_read<0>();
+    }
+    epilogue_bar_sync(bar_id);
+#pragma unroll
+    for (int j = 0; j < 8; j++)     // 16-byte chunk j of row r lives at chunk j ^ (r % 8)
+        slab[rw.srow * 8 + (j ^ (rw.srow & 7))] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                             __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+    staged();
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    epilogue_bar_sync(bar_id);
+    if (store_thread) {
+        tma_store_4d(tm_y, slab, col0, bx.ow0, bx.oh0, bx.n0);
+        tma_store_commit();
+    }
+}
+
 // One 128-row x 32-column slab of accumulators (already in registers): folded batch-norm
 // scale/shift + bias, optional addend, activation, optional TF32 rounding, then either a swizzled
 // staging slab that leaves by TMA (optionally 2x2/2 max-pooled first) or plain global stores.
