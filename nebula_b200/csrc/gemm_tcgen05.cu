@@ -44,6 +44,7 @@ using namespace tc;
 
 namespace {
 
+constexpr int RESIDUAL_OFFSET = 128 * 1024;     // of the shortcut's slab buffers (64 KB at most, in front of the staging buffers)
 constexpr int GATHER_MAX_K = 384;      // largest k*k*C (rounded up to 32) the gather table in the kernel parameters holds
 
 struct TcParams {
@@ -112,6 +113,11 @@ struct TcGatherParams : TcParams {
 };
 template <bool GATHER> struct ParamsOf { typedef TcParams type; };
 template <> struct ParamsOf<true> { typedef TcGatherParams type; };
+
+// in = false: nothing is read and the destination becomes zero
+__device__ __forceinline__ void cp_async16(uint32_t dst, const float *src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+}
 
 // The digits (split, n_tile, tw, th, tn) of a CTA's current tile.  Decoding a tile index costs seven integer
 // divisions (over a thousand cycles of dependent instructions on a role's critical path), so the index is decoded
@@ -360,7 +366,11 @@ __device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *sme
 // held to the register budget of fourteen).
 // CLUSTER: a tile's K is cut over the k_splits CTAs of a cluster, one tile per cluster (cluster_epilogue).
 // LEAN: only what epilogue_lean does.
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER, bool LEAN>
+// RESIDUAL: a folded shortcut besides, its slabs through shared memory by cp.async in coalesced rows, a tile ahead of their use: read
+// by the lanes that add them, each its own row, they kept 32 KB per SM in flight, and a slab took an epilogue group 3300 to
+// 4800 cycles where one without a shortcut takes 1500.  ResNet-50 b64 2234 -> 2042 us (expansions of 14 x 14 planes 41 -> 31 us, 28 x 28
+// 67 -> 48, 56 x 56 112 -> 89); one K block per stage, for with two the 128 KB of ring hold two stages (2300 us).
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER, bool LEAN, bool RESIDUAL>
 __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
     using C = Cfg<BLOCK_N, THREE, GATHER>;
@@ -689,13 +699,37 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         uint32_t acc_phase = 0;
         bool ok = true;
         TileIter ti(p, blockIdx.x, gridDim.x);
+        // RESIDUAL: slab buffers of 32 rows per warp (one per slab of a tile) behind the shorter ring, and the tile the next copies are for
+        [[maybe_unused]] TileIter ahead = ti;
+        [[maybe_unused]] int ahead_tile = blockIdx.x;
+        [[maybe_unused]] const uint32_t res_buf = smem_u32(smem) + RESIDUAL_OFFSET + (uint32_t)ew * (CH * 4096);
+        [[maybe_unused]] auto fetch_residual = [&](int ci) {        // slab ci of tile `ahead`
+            if (ahead_tile >= total_tiles) return;
+            const int w = ahead.tw * p.bw + rw, h = ahead.th * p.bh + rh, n = ahead.tn * p.bn + rn;
+            const int ih = h * p.e.res_stride, iw = w * p.e.res_stride;
+            const bool in = rn < p.bn && w < p.OW && h < p.OH && n < p.NB && h < p.e.res_h && w < p.e.res_w && ih < p.e.res_h && iw < p.e.res_w;
+            const int pixel = in ? (n * p.e.res_h + ih) * p.e.res_w + iw : -1;      // this lane's row
+            const int col = ahead.n_tile * BLOCK_N + (grp + 2 * ci) * 32 + 4 * (lane & 7);
+#pragma unroll
+            for (int i = 0; i < 8; i++) {               // eight lanes a row, four rows at a time
+                const int row = 4 * i + (lane >> 3), px = __shfl_sync(0xffffffffu, pixel, row);
+                const bool ok = px >= 0 && col < p.e.addend_cols;
+                cp_async16(res_buf + (uint32_t)(ci * 4096 + row * 128 + ((lane & 7) ^ (row & 7)) * 16),
+                           ok ? p.e.addend + (long)px * p.e.ld_addend + col : p.e.addend, ok);
+            }
+        };
         grid_dependency_wait();                 // (addends, cell states; the outputs may still be read)
+        if constexpr (RESIDUAL) {
+#pragma unroll
+            for (int ci = 0; ci < CH; ci++) fetch_residual(ci);
+            ahead.next(p); ahead_tile += gridDim.x;
+        }
         for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ti.next(p)) {
             const int split = ti.split, n_tile = ti.n_tile, tw = ti.tw, th = ti.th, tn = ti.tn;
             const int ow = tw * p.bw + rw, oh = th * p.bh * halves + rh, n = tn * p.bn + rn;
             const bool row_ok = (rn < p.bn) && ow < p.OW && oh < p.OH && n < p.NB;
             const long row = ((long)n * p.OH + oh) * p.OW + ow;
-            const EpiRow erow{r, row, row_ok, addend_row(p.e, row_ok, row, n, oh, ow)};
+            const EpiRow erow{r, row, row_ok, RESIDUAL ? nullptr : addend_row(p.e, row_ok, row, n, oh, ow)};
             const EpiBox ebox{p.bw, p.bh, p.bn, tw * p.bw, th * p.bh * halves, tn * p.bn + split * p.NB};
             if (aff_smem && n_tile != aff_tile) {
                 // this group's scale/shift values for the tile column (its slabs are chunks grp, grp + 2, ...)
@@ -726,6 +760,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                 tc_fence_after();
                 uint32_t v[32];
                 bool loaded = false;            // v holds a tcgen05.ld issued while the previous slab was being stored
+                if constexpr (RESIDUAL) {
+                    asm volatile("cp.async.wait_all;" ::: "memory");        // this tile's slabs, under way since the tile before
+                    __syncwarp();
+                }
 #pragma unroll 1
                 for (int hf = 0; hf < halves; hf++) {
                     // the second half of a two-box tile: the same raster p.bh image rows further down
@@ -741,7 +779,10 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
 #pragma unroll 1
                     for (int chunk = grp; chunk < BLOCK_N / 32; chunk += 2) {
                         const int col0 = n_tile * BLOCK_N + chunk * 32;
-                        if (col0 >= p.e.N) break;         // uniform across the group
+                        if (col0 >= p.e.N) {              // uniform across the group
+                            if constexpr (RESIDUAL) { fetch_residual(chunk >> 1); continue; }
+                            break;
+                        }
                         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * acc_cols + hf * BLOCK_N + chunk * 32);
                         if (!loaded) tmem_ld_32x32(taddr, v);
                         tmem_ld_wait();
@@ -753,14 +794,34 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
                         else if (hf + 1 < halves) next = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * acc_cols + (hf + 1) * BLOCK_N + grp * 32);
                         const float *aff = aff_smem ? aff_base + grp * BLOCK_N + (chunk >> 1) * 32 : nullptr;
                         auto staged = [&] { if (next) { tmem_ld_32x32(next, v); loaded = true; } };
-                        if constexpr (LEAN)
-                            epilogue_lean(p.e, &p.tm_y, v, col0, hrow, hbox, slab, bar_id, store_thread, stores_in_flight, staged, aff, BLOCK_N / 2);
+                        if constexpr (RESIDUAL) {
+                            epilogue_lean(p.e, &p.tm_y, v, col0, hrow, hbox, slab, bar_id, store_thread, stores_in_flight, staged, aff, BLOCK_N / 2,
+                                          [&](uint32_t (&x)[32]) {
+                                if (col0 < p.e.addend_cols) {
+#pragma unroll
+                                    for (int j = 0; j < 8; j++) {
+                                        float4 a;
+                                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w)
+                                                     : "r"(res_buf + (uint32_t)((chunk >> 1) * 4096 + lane * 128 + (j ^ (lane & 7)) * 16)));
+                                        x[4 * j] = __float_as_uint(__uint_as_float(x[4 * j]) + a.x);
+                                        x[4 * j + 1] = __float_as_uint(__uint_as_float(x[4 * j + 1]) + a.y);
+                                        x[4 * j + 2] = __float_as_uint(__uint_as_float(x[4 * j + 2]) + a.z);
+                                        x[4 * j + 3] = __float_as_uint(__uint_as_float(x[4 * j + 3]) + a.w);
+                                    }
+                                }
+                                __syncwarp();               // the buffer has been read
+                                fetch_residual(chunk >> 1);
+                            });
+                        } else if constexpr (LEAN)
+                            epilogue_lean(p.e, &p.tm_y, v, col0, hrow, hbox, slab, bar_id, store_thread, stores_in_flight, staged, aff, BLOCK_N / 2,
+                                          [&](uint32_t (&x)[32]) { if (hrow.arow) add_quads(p.e, x, hrow.arow, col0); });
                         else
                             epilogue_chunk<THREE>(p.e, &p.tm_y, &p.tm_yp, v, col0, hrow, hbox, slab, bar_id, store_thread, t, stores_in_flight, staged,
                                                   aff, BLOCK_N / 2);
                         slab = slab == slab0 ? slab1 : slab0;
                     }
                 }
+                if constexpr (RESIDUAL) { ahead.next(p); ahead_tile += gridDim.x; }
                 tc_fence_before();
                 mbar_arrive(&acc_empty[acc]);
                 if (++acc == 2) { acc = 0; acc_phase ^= 1; }
@@ -814,6 +875,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
             }
         }
         if (store_thread) tma_store_wait_all();     // staged tiles must have left shared memory
+        if constexpr (RESIDUAL) asm volatile("cp.async.wait_all;" ::: "memory");
     } else if constexpr (GATHER) {
         // ------------------------------------------------- in-kernel patch gather
         // One thread per tile row (output pixel): 32 columns (kh,kw,c) of this K block are read
@@ -1015,8 +1077,8 @@ void encode(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const c
 
 struct Variant { const void *kernel; int smem; };      // takes a TcParams, or a TcGatherParams
 
-template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER = false, bool LEAN = false>
-Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER, CLUSTER, LEAN>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
+template <int BLOCK_N, bool THREE, bool PROMOTE, bool GATHER, bool CLUSTER = false, bool LEAN = false, bool RESIDUAL = false>
+Variant variant() { return {(const void *)gemm_tf32_tcgen05_kernel<BLOCK_N, THREE, PROMOTE, GATHER, CLUSTER, LEAN, RESIDUAL>, Cfg<BLOCK_N, THREE, GATHER>::SMEM_BYTES}; }
 
 // index: [gather][three][promote][block_n: 0 = 64, 1 = 128, 2 = 256]; absent combinations are null
 const Variant VARIANTS[2][2][2][3] = {
@@ -1038,6 +1100,8 @@ const Variant CLUSTER_VARIANTS[2][2][3] = {
      {variant<64, true, true, false, true>(), variant<128, true, true, false, true>(), {nullptr, 0}}},
 };
 
+// index: [block_n]: a folded shortcut through shared memory
+const Variant RESIDUAL_VARIANTS[2] = {variant<64, false, false, false, false, true, true>(), variant<128, false, false, false, false, true, true>()};
 // index: [block_n]: the plain epilogue by itself
 const Variant LEAN_VARIANTS[3] = {variant<64, false, false, false, false, true>(), variant<128, false, false, false, false, true>(),
                                   variant<256, false, false, false, false, true>()};
@@ -1062,6 +1126,7 @@ void gemm_tc_prepare_device(nb_handle_s *h) {
             for (auto &pr : t)
                 for (auto &v : pr)
                     if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+    for (auto &v : RESIDUAL_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     for (auto &v : LEAN_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     for (auto &t : CLUSTER_VARIANTS)
         for (auto &pr : t)
@@ -1255,6 +1320,12 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
             if (best_cost == 0 || cost < best_cost) { best_cost = cost; block_n = bn; }
         }
     }
+    // a shortcut's slabs through shared memory: 1x1 layers of several tiles per SM.  (A single tile per SM has nothing to fetch ahead of,
+    // and its short ring takes one K block per stage: ResNet-50 b1 412 us without, 423 with.)
+    const bool residual = a.addend && a.res_stride > 0 && !a.addend_after_act && !cluster && !promote && !gather && !col3 && p.e.addend_vec &&
+                          p.e.addend_cols % 4 == 0 && !a.block_n_hint && taps == 1 && p.e.tma_store && a.shift &&
+                          (a.act == NB_ACT_RELU || a.act == NB_ACT_LEAKY || a.act == NB_ACT_LINEAR) && kc <= 512 && (long)p.m_tiles * ((a.N + 127) / 128) > h->sm_count;
+    if (residual) block_n = std::min(block_n, 128);
     p.n_tiles = (a.N + block_n - 1) / block_n;
     p.m_fastest = (!a.a_is_conv && !gather && (size_t)a.N * a.Kc * 4 > ((size_t)48 << 20)) ? 1 : 0;
     // accumulation chains of at most 512 K elements (TF32) / 12 MMAs (3xTF32) in the tensor core: every accumulating MMA
@@ -1280,7 +1351,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         p.tx_bytes_a = BLOCK_K * 4 * box.bw * box.bh * box.bn;
     }
     const int box_rows = box.bw * box.bh * box.bn;
-    p.cbs = (pairs && !promote && (S == 1 || p.kb_per_split % 2 == 0) && block_n <= 128 &&
+    p.cbs = (pairs && !promote && !residual && (S == 1 || p.kb_per_split % 2 == 0) && block_n <= 128 &&
              (box_rows == BLOCK_M ? a.a_is_conv : alone && box_rows % 8 == 0)) ? 2 : 1;
     p.a_slice_bytes = box_rows * 128;
     p.a_region = A_STAGE_BYTES + (p.cbs - 1) * p.a_slice_bytes;
@@ -1290,11 +1361,11 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         const int ring = std::min(8, (196 * 1024) / stage1) * stage1;       // bytes the variant's ring holds
         p.a_box_bytes = BLOCK_K * 4 * box.bw * (box.bh * halves + 2);
         p.stage_bytes = p.col3 ? p.a_box_bytes + 3 * b_stage : (p.cbs == 2 ? p.a_region + 2 * b_stage : stage1);
-        p.stages = std::min(8, ring / p.stage_bytes);
+        p.stages = std::min(8, (residual ? RESIDUAL_OFFSET : ring) / p.stage_bytes);
         // a second staging buffer per epilogue group in what the ring leaves unused; a one-column filter (row windows:
         // one stage per tile, bound by its epilogue) gives up its third stage for it
         if (p.col3 && ksize_w == 1 && p.stages > 2) p.stages = 2;
-        const int ring_cap = std::min(8, (196 * 1024) / stage1) * stage1;
+        const int ring_cap = residual ? 0 : std::min(8, (196 * 1024) / stage1) * stage1;
         const int used = p.stages * p.stage_bytes;
         p.slab2_offset = (!three_pass && !promote && !gather && ring_cap - used >= 2 * BLOCK_M * 32 * 4) ? used : 0;
     }
@@ -1419,7 +1490,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     const bool lean = !three_pass && !promote && !gather && !cluster && p.e.tma_store && p.e.shift &&
                       (a.act == NB_ACT_RELU || a.act == NB_ACT_LEAKY || a.act == NB_ACT_LINEAR) &&
                       (!a.addend || (p.e.addend_vec && p.e.addend_cols % 4 == 0 && !p.e.addend_post));
-    L->v = lean ? LEAN_VARIANTS[width] : cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
+    L->v = residual ? RESIDUAL_VARIANTS[width] : lean ? LEAN_VARIANTS[width] : cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
     L->cluster = cluster ? S : 1;
     if (!L->v.kernel) throw Error(NB_ERR_UNSUPPORTED, "no tensor-core kernel variant for this tile width");
     const int tiles = p.m_tiles * p.n_tiles * p.k_splits;

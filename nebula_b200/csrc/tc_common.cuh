@@ -332,13 +332,32 @@ static __device__ __noinline__ void activate_slab(float *x, int act) {
     }
 }
 
+// Adds a row's quads of the slab at col0 to its values.
+__device__ __forceinline__ void add_quads(const EpiParams &e, uint32_t (&v)[32], const float *row, int col0) {
+    const float *arow = row + col0;
+    auto add = [&](int j) {
+        const float4 ad = *reinterpret_cast<const float4 *>(arow + j);
+        v[j] = __float_as_uint(__uint_as_float(v[j]) + ad.x);
+        v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + ad.y);
+        v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + ad.z);
+        v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + ad.w);
+    };
+    if (col0 + 32 <= e.addend_cols) {       // (without a branch between them the eight loads overlap)
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) add(j);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4)
+            if (col0 + j < e.addend_cols) add(j);
+    }
+}
+
 // The same for what most layers are: scale/shift from shared memory (`aff`: 32 scale values, 1 where the layer has none, and
-// `aff_shift` floats further the shift values), an addend of whole quads added before the activation or none, relu, leaky or linear,
-// a TMA store.  In a kernel of its own, without the other modes' code between its instructions.
-template <class Staged>
+// `aff_shift` floats further the shift values), what `add(v)` adds before the activation, relu, leaky or linear, a TMA store.  In a kernel of its own, without the other modes' code between its instructions.
+template <class Staged, class Add>
 __device__ __forceinline__ void epilogue_lean(const EpiParams &e, const CUtensorMap *tm_y, uint32_t (&v)[32], int col0, const EpiRow &rw, const EpiBox &bx,
                                               float4 *slab, int bar_id, bool store_thread, int stores_in_flight, Staged &&staged, const float *aff,
-                                              int aff_shift) {
+                                              int aff_shift, Add &&add) {
 #pragma unroll
     for (int j = 0; j < 32; j += 4) {
         const float4 sc = lds128(aff + j), sh = lds128(aff + aff_shift + j);
@@ -347,24 +366,7 @@ __device__ __forceinline__ void epilogue_lean(const EpiParams &e, const CUtensor
         v[j + 2] = __float_as_uint(fmaf(__uint_as_float(v[j + 2]), sc.z, sh.z));
         v[j + 3] = __float_as_uint(fmaf(__uint_as_float(v[j + 3]), sc.w, sh.w));
     }
-    if (rw.arow) {
-        const float *arow = rw.arow + col0;
-        auto add = [&](int j) {
-            const float4 ad = *reinterpret_cast<const float4 *>(arow + j);
-            v[j] = __float_as_uint(__uint_as_float(v[j]) + ad.x);
-            v[j + 1] = __float_as_uint(__uint_as_float(v[j + 1]) + ad.y);
-            v[j + 2] = __float_as_uint(__uint_as_float(v[j + 2]) + ad.z);
-            v[j + 3] = __float_as_uint(__uint_as_float(v[j + 3]) + ad.w);
-        };
-        if (col0 + 32 <= e.addend_cols) {       // (without a branch between them the eight loads overlap)
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) add(j);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                if (col0 + j < e.addend_cols) add(j);
-        }
-    }
+    add(v);
     if (e.act == NB_ACT_RELU) {
 #pragma unroll
         for (int j = 0; j < 32; j++) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
