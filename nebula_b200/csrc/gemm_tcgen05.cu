@@ -1555,7 +1555,8 @@ TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, 
     const Box box = choose_box(g.OW, g.OH, g.batch, g.stride, pool, false, (double)g.C * g.H * g.W * 4.0);
     const long m_tiles = (long)((g.OW + box.bw - 1) / box.bw) * ((g.OH + box.bh - 1) / box.bh) * ((g.batch + box.bn - 1) / box.bn);
     if (!three_pass && 2 * m_tiles * ((N + 63) / 64) > h->sm_count) return best;
-    double best_cost = tc_cluster_cost(h, m_tiles, N, blocks, 1, 64, three_pass, act);
+    // (filter-column stages fetch a block in less: 56 x 56 x 64 whole 7.8 us, in clusters 8 to 9.6)
+    double best_cost = tc_cluster_cost(h, m_tiles, N, blocks, 1, 64, three_pass, act) * (!three_pass && column_stages(g, Kc, N) ? 0.6 : 1.0);
     if (three_pass && N > 64) best_cost = std::min(best_cost, tc_cluster_cost(h, m_tiles, N, blocks, 1, 128, true, act));
     for (int bn = 64; bn <= (three_pass && N > 64 ? 128 : 64); bn *= 2)
         for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
