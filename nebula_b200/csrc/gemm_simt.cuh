@@ -20,7 +20,8 @@
 //     rank order and writes it.  No workspace, no second launch, no atomics.  In layers S depends on N, K and the pixels of
 //     ONE image, never on the batch, so a batch and its slices add in the same order; in _gemm_ it depends on M as well.
 // Measured against the 64 x 64 tile with scalar loads and two barriers per 16 columns (and a 16 x 16 tile for _gemm_)
-// before it: AlexNet b4 in fp32 2938 -> 642 us, 256 x 1024 x 1024 _gemm_ + bias + relu 183 -> 30 us.
+// before it: AlexNet b4 in fp32 2938 -> 454 us (its connected layers by gemm_rows_kernel), 256 x 1024 x 1024 _gemm_ + bias + relu
+// 183 -> 27 us.
 //
 // This header: the kernel and what launches must know of it.  gemm_simt_kernels.cu compiles it once per pair of copy modes (a
 // module each: the first kernel of all 36 in one took 15 ms to load), gemm_simt.cu chooses and launches.
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
 #pragma unroll
     for (int s = 0; s < MB::ROW_SLOTS; s++) b_in |= (MB::active(tid, s) && n0 + MB::row(tid, s) < p.N ? 1u : 0u) << s;
     begin_tap();
+    grid_dependency_wait();
     const long a_step = AMODE == ONE_ROW ? BK * p.g.sc : BK, b_step = BMODE == ONE_ROW ? BK * p.b_col : BK;
     const long a_next = AMODE == ONE_ROW ? T::THREADS / BM * p.g.sc : 0;        // from one copy of a slot to the next
     const long b_next = BMODE == ONE_ROW ? T::THREADS / BN * p.b_col : T::THREADS / MB::PER_ROW * p.b_row;

@@ -222,7 +222,7 @@ __device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *sme
     const int u0 = rank * per, u_end = min(units, u0 + per);
     // (NCHW output: lanes along the pixels, else along the columns)
     const int c4 = p.e.plane ? t / (256 / N4) : t % N4, first_u = u0 + (p.e.plane ? t % (256 / N4) : t / N4), col = n0 + 4 * c4;
-    const bool col_ok = col < p.e.N;                        // (N is a multiple of 4)
+    const bool col_ok = col < p.e.N;                        // (convolutions: whole quads)
     float4 sc = make_float4(1.f, 1.f, 1.f, 1.f), sh = make_float4(0.f, 0.f, 0.f, 0.f);
     if (col_ok && p.e.scale) sc = __ldg(reinterpret_cast<const float4 *>(p.e.scale + col));
     if (col_ok && p.e.shift) sh = __ldg(reinterpret_cast<const float4 *>(p.e.shift + col));
@@ -357,7 +357,12 @@ __device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *sme
             dst = p.e.y + (((long)x.n * (p.OH >> 1) + (x.oh >> 1)) * (p.OW >> 1) + (x.ow >> 1)) * p.e.ldy + col;
         }
         if (p.e.tma_store) *reinterpret_cast<float4 *>(dst) = a;        // (16-byte aligned rows)
-        else { dst[0] = a.x; dst[1] = a.y; dst[2] = a.z; dst[3] = a.w; }
+        else {
+            dst[0] = a.x;
+            if (col + 1 < p.e.N) dst[1] = a.y;
+            if (col + 2 < p.e.N) dst[2] = a.z;
+            if (col + 3 < p.e.N) dst[3] = a.w;
+        }
     }
 }
 
@@ -1251,9 +1256,9 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks");
     if (S > 1 && !cluster && (a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
         throw Error(NB_ERR_INVALID_ARG, "split-K into slabs needs a plain epilogue");
-    if (cluster && (S > TC_MAX_CLUSTER || (a.N % 4) != 0 || a.lstm_H ||
-                    (a.addend && (a.res_stride == 0 || (a.res_c % 4) != 0 || (a.ld_addend % 4) != 0 || !aligned16(a.addend)))))
-        throw Error(NB_ERR_INVALID_ARG, "split-K over a cluster needs quads of columns");
+    if (cluster && (S > TC_MAX_CLUSTER || (a.a_is_conv && (a.N % 4) != 0) || a.lstm_H ||
+                    (a.addend && (!a.a_is_conv || a.res_stride == 0 || (a.res_c % 4) != 0 || (a.ld_addend % 4) != 0 || !aligned16(a.addend)))))
+        throw Error(NB_ERR_INVALID_ARG, "split-K over a cluster needs a convolution's columns, and a shortcut's, in quads");
     p.k_splits = S;
     p.m_tiles = p.tiles_w * p.tiles_h * p.tiles_n;
     p.e.N = a.N;

@@ -73,3 +73,54 @@ def test_network_of_small_layers(handle, mode, batch, size):
     net.close()
     # TF32: six layers of 2^-12 per operand, few samples: the limit of the suite's small networks (tests/util.py)
     assert logit_err(got, ref[-1], batch) <= (2.6e-3 if mode == "tf32" else NET_TOL[mode])
+
+
+@pytest.mark.parametrize("mode", ["tf32", "tf32x3"])
+@pytest.mark.parametrize("rows,inputs,outputs", [(32, 500, 30), (1, 1000, 1), (5, 516, 62), (130, 2052, 67), (33, 4096, 5), (64, 300, 129)])
+def test_connected_with_ragged_outputs(handle, mode, rows, inputs, outputs):
+    import torch
+    from nebula_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(inputs + outputs)
+    w, bias = torch.randn(outputs, inputs, device="cuda", generator=g) * inputs ** -0.5, torch.randn(outputs, device="cuda", generator=g)
+    x = torch.randn(rows, inputs, device="cuda", generator=g)
+    handle.set_math(mode)
+    plan = api.Connected(handle, rows, inputs, outputs, False, "logistic")
+    plan.set_weights(w, bias)
+    y = torch.full((rows * outputs + 64,), 7.0, device="cuda")
+    handle.check(handle.lib.nb_fc_forward(plan.p, x.data_ptr(), y.data_ptr()))
+    handle.synchronize()
+    plan.close()
+    z = x.double() @ w.double().T + bias.double()
+    # TF32 rounds each operand by 2^-11 at most; 3xTF32 drops products of 2^-22 and adds in fp32, as TF32 does; the logistic's
+    # slope is 1/4 at most and its own rounding a few ulp
+    unit = 2.0 ** -10 if mode == "tf32" else 2.0 ** -21
+    bound = 0.25 * ((unit + inputs * 2.0 ** -24) * (x.double().abs() @ w.double().abs().T) + 2.0 ** -23 * z.abs()) + 2.0 ** -22
+    assert bool(((y[:rows * outputs].view(rows, outputs).double() - torch.sigmoid(z)).abs() <= bound).all())
+    assert bool((y[rows * outputs:] == 7.0).all())
+
+
+@pytest.mark.parametrize("rows,K,N", [(32, 30, 62), (3, 30, 62), (20, 7, 5), (8, 64, 64)])
+def test_few_cuda_core_ctas_behind_a_tensor_core_layer(handle, rows, K, N):
+    """Launched ahead of the layer in front, the product must still read what that layer wrote."""
+    import torch
+    from nebula_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(K)
+    handle.set_math("tf32")
+    front = api.Connected(handle, rows, 4096, K, False, "linear")
+    front.set_weights(torch.randn(K, 4096, device="cuda", generator=g), torch.zeros(K, device="cuda"))
+    w = torch.randn(N, K, device="cuda", generator=g)
+    xs = [torch.randn(rows, 4096, device="cuda", generator=g) for _ in range(5)]
+    mid, out = torch.empty(rows, K, device="cuda"), torch.empty(5, rows, N, device="cuda")
+    torch.cuda.synchronize()
+    for i, x in enumerate(xs):
+        handle.check(handle.lib.nb_fc_forward(front.p, x.data_ptr(), mid.data_ptr()))
+        handle.gemm(False, True, rows, N, K, 1.0, mid, K, w, K, 0.0, out[i], N)
+    handle.synchronize()
+    for i, x in enumerate(xs):
+        m = front.forward(x)
+        handle.synchronize()
+        z = torch.empty(rows, N, device="cuda")
+        handle.gemm(False, True, rows, N, K, 1.0, m.reshape(rows, K), K, w, K, 0.0, z, N)
+        handle.synchronize()
+        assert torch.equal(z, out[i])
+    front.close()
