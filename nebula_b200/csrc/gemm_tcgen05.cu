@@ -1336,7 +1336,8 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     // accumulation chains of at most 512 K elements (TF32) / 12 MMAs (3xTF32) in the tensor core: every accumulating MMA
     // truncates the running sum (a shrink of about 6e-8 per step that adds up layer after layer).  A 3xTF32 K block is
     // 12 MMAs, of which only the 4 hi*hi ones go into the promoted chain (the cross terms have columns of their own)
-    p.kb_per_part = !promote ? p.kb_per_split : (three_pass ? 3 : (a.k_part > 0 ? a.k_part : 16));
+    // (a slice of two or three blocks is cut once more: in a single part its cross terms would go into the chain, 24 to 36 MMAs)
+    p.kb_per_part = !promote ? p.kb_per_split : (three_pass ? (S > 1 && p.kb_per_split <= 3 ? (p.kb_per_split + 1) / 2 : 3) : (a.k_part > 0 ? a.k_part : 16));
     p.parts = (p.kb_per_split + p.kb_per_part - 1) / p.kb_per_part;
 
     // two K blocks per ring stage: tiles of up to 128 columns whose K slices pair up, a box of whole 8-row groups (the

@@ -124,3 +124,23 @@ def test_few_cuda_core_ctas_behind_a_tensor_core_layer(handle, rows, K, N):
         handle.synchronize()
         assert torch.equal(z, out[i])
     front.close()
+
+
+@pytest.mark.parametrize("C,F,size", [(128, 64, 5), (192, 128, 7), (256, 64, 7), (384, 96, 5), (512, 512, 7), (768, 64, 9)])
+def test_short_slices_keep_the_cross_terms_apart(handle, C, F, size):
+    """3xTF32 on positive operands, where the tensor core's truncation of the running sum shows as a shrink: a part of at most three
+    K blocks adds twelve products to a chain that grows linearly and loses at most an ulp (2^-23) at each: 12 / 2 ulp.  With the
+    cross terms in the same chain a slice of two or three blocks has 24 or 36 (384 channels: 8.3e-7, 2.1e-7 with them apart)."""
+    import torch
+    from nebula_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(C)
+    w, x = torch.rand(F, C, 1, 1, device="cuda", generator=g), torch.rand(1, C, size, size, device="cuda", generator=g)
+    handle.set_math("tf32x3")
+    plan = api.Conv2d(handle, 1, C, size, size, F, 1, 1, 0, False, "linear")
+    plan.set_weights(w, torch.zeros(F, device="cuda"))
+    y = plan.forward(x)
+    handle.synchronize()
+    plan.close()
+    want = torch.einsum("fc,chw->fhw", w.double().reshape(F, C), x.double()[0])
+    shrink = ((y.double().reshape(want.shape) - want) / want).mean().item()
+    assert abs(shrink) <= 6 * 2.0 ** -23
