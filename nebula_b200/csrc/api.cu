@@ -106,7 +106,6 @@ int nb_create(int device_id, nb_handle_t *handle) {
             }
         }
         gemm_tc_prepare_device(h);
-        lstm_persistent_prepare_device(h);
         elementwise_prepare_device();
     });
     if (rc != NB_OK) {

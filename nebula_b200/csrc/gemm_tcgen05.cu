@@ -1133,29 +1133,36 @@ void gemm_tc_prepare_device(nb_handle_s *h) {
                     if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     for (auto &v : RESIDUAL_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
     for (auto &v : LEAN_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
-    for (auto &t : CLUSTER_VARIANTS)
-        for (auto &pr : t)
-            for (auto &v : pr) {
-                if (!v.kernel) continue;
-                NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
-                NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            }
-    // clusters of a CTA per SM that run at once, by size
-    for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
-        const Variant &v = CLUSTER_VARIANTS[0][0][0];
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)S);
-        cfg.blockDim = dim3(320);
-        cfg.dynamicSmemBytes = (size_t)v.smem;
-        cudaLaunchAttribute at;
-        at.id = cudaLaunchAttributeClusterDimension;
-        at.val.clusterDim.x = (unsigned)S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, v.kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
-        h->tc_clusters[S] = n;
+}
+
+// Clusters of `size` CTAs, one per SM, that run at once.  The cluster kernels are loaded by the first layer that they are a
+// candidate for, and the device is asked about the sizes that a layer could take, so a handle that has none pays for none.
+static int clusters_at_once(const nb_handle_s *h, int size) {
+    if (!h->tc_clusters_ready) {
+        for (auto &t : CLUSTER_VARIANTS)
+            for (auto &pr : t)
+                for (auto &v : pr) {
+                    if (!v.kernel) continue;
+                    NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+                    NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+                }
+        std::fill(std::begin(h->tc_clusters), std::end(h->tc_clusters), -1);
+        h->tc_clusters_ready = true;
     }
+    int &n = h->tc_clusters[size];
+    if (n >= 0) return n;
+    const Variant &v = CLUSTER_VARIANTS[0][0][0];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)size);
+    cfg.blockDim = dim3(320);
+    cfg.dynamicSmemBytes = (size_t)v.smem;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)size; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, v.kernel, &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
+    return n;
 }
 
 void encode_tensor_map(nb_handle_s *h, CUtensorMap *tm, const void *base, int rank, const cuuint64_t *dims,
@@ -1549,7 +1556,7 @@ double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, in
     const double heavy = act == NB_ACT_RELU || act == NB_ACT_LEAKY || act == NB_ACT_LINEAR ? 0.0 : 24.0 * bn / 64;     // the double formulas
     if (S == 1) return (double)((tiles + h->sm_count - 1) / h->sm_count) * (blocks * block + heavy);
     const int per = (blocks + S - 1) / S;
-    if (tiles > h->tc_clusters[S] || (long)(S - 1) * per >= blocks) return -1;
+    if ((long)(S - 1) * per >= blocks || tiles * S > h->sm_count || tiles > clusters_at_once(h, S)) return -1;
     return per * block + heavy / S + 1.5 * S + 26.0 * (bn / 64) * (bn / 64) / (S * S);
 }
 

@@ -349,7 +349,9 @@ int stages_of(int B) {
 
 }  // namespace
 
-void lstm_persistent_prepare_device(nb_handle_s *h) {
+// Limits set, and clusters counted, when the first layer asks.
+static int clusters_at_once(const nb_handle_s *h) {
+    if (h->lstm_clusters >= 0) return h->lstm_clusters;
     for (int B : {64, 128}) NB_CHECK_CUDA(cudaFuncSetAttribute(kernel_of(B), cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM));
     // clusters of four that run at once, with a CTA per SM (the kernel takes all of tensor memory)
     cudaLaunchConfig_t cfg = {};
@@ -363,7 +365,7 @@ void lstm_persistent_prepare_device(nb_handle_s *h) {
     cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel_of(128), &cfg) != cudaSuccess) { (void)cudaGetLastError(); n = 0; }
-    h->lstm_clusters = n;
+    return h->lstm_clusters = n;
 }
 
 int lstm_persistent_counters() { return (LP_GROUPS * LP_MAX_BLOCKS + 1) * LP_COUNTER_STRIDE; }
@@ -391,7 +393,7 @@ bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H) {
     if (!h->encode_tiled || h->cc_major != 10 || !h->cooperative_launch) return false;
     if (T < 3 || B < 1 || H < 32 || (H % 4) != 0 || (B > 128 && (H % 32) != 0)) return false;
     const long KB = (H + BLOCK_K - 1) / BLOCK_K;
-    if (lstm_k_part(H) > 32 || KB * chunks_of(B) > std::min(h->lstm_clusters, LP_MAX_BLOCKS)) return false;
+    if (lstm_k_part(H) > 32 || KB * chunks_of(B) > std::min(clusters_at_once(h), LP_MAX_BLOCKS)) return false;
     return 2 * LP_GROUPS * rows_of(chunk_rows_of(B)) + lstm_k_part(H) * BLOCK_K <= LP_TMEM;
 }
 

@@ -63,9 +63,10 @@ struct nb_handle_s {
     std::string last_error;
     int *d_status = nullptr;            // device status word (nb::DEV_*)
     unsigned int *d_grid_sync = nullptr; // arrival counters of the persistent LSTM kernel (it leaves them zero)
-    int lstm_clusters = 0;              // lstm_persistent.cu: clusters of its size that the device runs at once
+    mutable int lstm_clusters = -1;     // lstm_persistent.cu: clusters of its size that the device runs at once (-1: not asked yet)
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
-    int tc_clusters[17] = {0};          // gemm_tcgen05.cu: the same for its kernel
+    mutable int tc_clusters[17] = {0};  // gemm_tcgen05.cu: the same for its kernel, once tc_clusters_ready (-1: not asked yet)
+    mutable bool tc_clusters_ready = false;
     bool recurrent_ready = false;       // recurrent_cluster.cu: limits set, clusters_at_once filled
     unsigned long long simt_ready = 0;  // gemm_simt.cu: kernels loaded and with their limits set, by variant and copy modes
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
@@ -379,7 +380,6 @@ std::string gemm_args_key(const GemmArgs &a, char tag, int extra);
 
 // Per-device set-up of the tensor-core kernels (shared-memory limits; also loads their code), once per handle.
 void gemm_tc_prepare_device(nb_handle_s *h);
-void lstm_persistent_prepare_device(nb_handle_s *h);
 int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H);

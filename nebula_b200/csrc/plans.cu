@@ -627,6 +627,7 @@ size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, boo
     const bool tc_u = tcm && (in % 4) == 0 && in >= 32;
     const bool tc_w = tcm && (H % 4) == 0 && H >= 32;
     const bool three = h->math_mode == NB_MATH_TF32X3;
+    if (tc_w && !three) (void)lstm_persistent_supported(h, T, B, H);        // (loads that kernel)
     pre.reserve(rows * 4 * H);
     if (!tc_w) z.reserve((size_t)B * 4 * H);
     GemmArgs a;
