@@ -24,6 +24,8 @@
 // h_{t+1} is published; each of those took the partial sums of step t + 1 of all four CTAs of its cluster, one of which read
 // the units of h_t that this CTA published after it had read its accumulators and its received sums of step t.  So two
 // accumulators, two receive buffers and two barriers per kind, by the parity of the step, are enough.
+// That says nothing about the slots of the ring that h arrives in, which are released by the MMAs that read them: a block's counter
+// belongs to another cluster, and may show h_t before this CTA has multiplied its blocks of h_{t-1}.
 //
 // h_{t-1} was written by other SMs' ordinary stores earlier in this same kernel and is read here by TMA, i.e. through the async
 // proxy: the writers release (a release-add on the block's counter), the lane that issues the copy acquires the counter itself
@@ -188,14 +190,20 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
         uint32_t phase = (uint32_t)(lane / stages) & 1;
         const unsigned int *counter = counters + (size_t)(kb0 + lane) * LP_COUNTER_STRIDE;
         const uint32_t tx = (uint32_t)stage_bytes;
+        // A slot's uses are issued in their order.  The use before this lane's belongs to an earlier step, all of whose copies are under
+        // way, or to lane - stages (slices of more blocks than slots).  Once it is under way, the slot's barrier is in the phase that
+        // ends with its release or in the next; tested earlier, it can be one phase further back, whose predecessor has the parity
+        // waited for, and the copy would land on a tile that the MMAs have yet to read.
+        const unsigned before = lane < stages ? 0 : 1u << (lane - stages);
         for (int t = 1; t < p.T && ok; t++) {
             bool done = lane >= nkb;
             const unsigned int target = (unsigned int)(LP_SLICES * cell_warps) * (unsigned int)t;
             const long long t0 = clock64();
-            while (ok && !__all_sync(0xffffffffu, done)) {
+            unsigned issued;                                // lanes whose copy of this step is under way
+            while (ok && (issued = __ballot_sync(0xffffffffu, done)) != 0xffffffffu) {
                 bool give_up = false;
                 if (!done) {
-                    if (ld_acquire_u32(counter) >= target && mbar_try_wait(&empty[slot], phase ^ 1)) {
+                    if ((issued & before) == before && ld_acquire_u32(counter) >= target && mbar_try_wait(&empty[slot], phase ^ 1)) {
                         // the units' stores (generic proxy) are ordered before the acquire; the copy (async proxy) behind this fence
                         asm volatile("fence.proxy.async;" ::: "memory");
                         mbar_expect_tx(&full[slot], tx);

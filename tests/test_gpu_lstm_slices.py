@@ -41,3 +41,29 @@ def test_lstm_in_slices_of_k(handle, case, monkeypatch):
     assert_close(runs[0][0].cpu().numpy(), ref, "tf32", f"{case}")
     for out, cell in runs[1:]:
         assert torch.equal(out, runs[0][0]) and torch.equal(cell, runs[0][1])
+
+
+@pytest.mark.parametrize("B", [65, 100, 128])
+@pytest.mark.parametrize("H", [772, 900, 1024])
+def test_slices_of_more_blocks_than_the_ring_has_slots(handle, H, B, monkeypatch):
+    """65 rows and more leave six slots to a group of rows, a slice of these widths has seven or eight blocks: two copies of a step
+    share a slot.  Many steps, several times, bit for bit what a launch per step gives."""
+    import torch
+    from nebula_b200 import api
+    T = 64
+    g = torch.Generator(device="cuda").manual_seed(H + B)
+    handle.set_math("tf32")
+    plan = api.Lstm(handle, T, B, 32, H, False, "linear")
+    plan.set_weights((torch.rand(8 * H + 4 * H * H + 4 * H * 32, device="cuda", generator=g) * 2 - 1) / H ** 0.5)
+    x = torch.randn(T, B, 32, device="cuda", generator=g)
+    monkeypatch.setenv("NEBULA_B200_LSTM_PERSISTENT", "0")
+    n0 = handle.launch_count()
+    want = plan.forward(x)
+    per_step = handle.launch_count() - n0
+    monkeypatch.setenv("NEBULA_B200_LSTM_PERSISTENT", "1")
+    n0 = handle.launch_count()
+    got = [plan.forward(x) for _ in range(4)]
+    assert handle.launch_count() - n0 == 4 * (per_step - T + 1), "all steps in one launch"
+    handle.synchronize()
+    plan.close()
+    assert bool(want.abs().amax() > 0) and all(torch.equal(y, want) for y in got)
