@@ -378,7 +378,7 @@ static int clusters_at_once(const nb_handle_s *h) {
 
 int lstm_persistent_counters() { return (LP_GROUPS * LP_MAX_BLOCKS + 1) * LP_COUNTER_STRIDE; }
 
-// K blocks of one slice of a recurrent product: the order in which TF32 LSTM steps add, in this kernel and launched step by step.
+// K blocks of one slice of a recurrent product.
 int lstm_k_part(int H) {
     const int KB = (H + BLOCK_K - 1) / BLOCK_K;
     return (KB + LP_SLICES - 1) / LP_SLICES;
@@ -404,6 +404,11 @@ bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H) {
     if (lstm_k_part(H) > 32 || KB * chunks_of(B) > std::min(clusters_at_once(h), LP_MAX_BLOCKS)) return false;
     return 2 * LP_GROUPS * rows_of(chunk_rows_of(B)) + lstm_k_part(H) * BLOCK_K <= LP_TMEM;
 }
+
+// The order of additions is the width's: the batches and sequences that a launch per step takes add the slices that this kernel would
+// add, so that a batch and its slices give the same bits.  Against K whole, H = 1024, a step takes 19.4 -> 19.5 us at 256 rows, 25.9 ->
+// 27.2 at 512; H = 416 at 1000 rows 20.5 -> 21.9.
+bool lstm_in_slices(const nb_handle_s *h, int H) { return lstm_persistent_supported(h, 3, 1, H); }
 
 // All steps of the recurrence: writes cell, out and hr.
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H) {

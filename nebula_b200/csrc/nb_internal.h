@@ -383,7 +383,9 @@ void gemm_tc_prepare_device(nb_handle_s *h);
 int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H);
-// K blocks of 32 per partial sum of a TF32 LSTM layer's recurrent product
+// Are the recurrent products of TF32 LSTM layers of this width added in slices of K, at every batch and number of steps, and of
+// how many K blocks of 32?
+bool lstm_in_slices(const nb_handle_s *h, int H);
 int lstm_k_part(int H);
 // what a contraction runs on: the tensor cores in TF32 or 3xTF32, or the CUDA cores
 enum GemmPath { PATH_TC = 0, PATH_TC3 = 1, PATH_SIMT = 2 };

@@ -608,8 +608,8 @@ void LstmPlan::set_weights(const float *stream, size_t count, int mem) {
 
 // The modes that promise fp32 agreement, widths off 32 and gate layers with an activation run all steps in one kernel of exact
 // fp32 products where that is the faster way.  Linear layers of widths that are multiples of 32 take TF32 products at every batch,
-// whatever the cluster would cost (lstm_persistent.cu, a launch per step beyond its batches); a single step of linear gate
-// layers has no product.  NEBULA_B200_LSTM_PERSISTENT=0: a launch per step in every case.
+// whatever the cluster would cost (lstm_persistent.cu, a launch per step beyond its batches, which adds in the same order); a single
+// step of linear gate layers has no product.  NEBULA_B200_LSTM_PERSISTENT=0: a launch per step in every case.
 bool LstmPlan::one_kernel() const {
     const char *env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
     if (env && *env == '0') return false;
@@ -627,7 +627,7 @@ size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, boo
     const bool tc_u = tcm && (in % 4) == 0 && in >= 32;
     const bool tc_w = tcm && (H % 4) == 0 && H >= 32;
     const bool three = h->math_mode == NB_MATH_TF32X3;
-    if (tc_w && !three) (void)lstm_persistent_supported(h, T, B, H);        // (loads that kernel)
+    if (tc_w && !three && d.activation == NB_ACT_LINEAR) (void)lstm_in_slices(h, H);        // (loads the kernel)
     pre.reserve(rows * 4 * H);
     if (!tc_w) z.reserve((size_t)B * 4 * H);
     GemmArgs a;
@@ -722,7 +722,7 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
                 a.b_static = ww.split_ready;
                 ww.ensure_split(h);
                 a.b = ww.hi.p; a.b_lo = ww.lo.p;
-                if (linear && !three && lstm_persistent_supported(h, T, B, H)) a.k_part = lstm_k_part(H);      // as the one-kernel recurrence adds
+                if (linear && !three && lstm_in_slices(h, H)) a.k_part = lstm_k_part(H);      // as the one-kernel recurrence adds
                 a.lstm_H = H; a.lstm_c_prev = c_prev; a.lstm_c = ct; a.lstm_h = ht; a.lstm_h_round = hrt;
                 gemm_tc(h, a, three);
                 continue;

@@ -67,3 +67,25 @@ def test_slices_of_more_blocks_than_the_ring_has_slots(handle, H, B, monkeypatch
     handle.synchronize()
     plan.close()
     assert bool(want.abs().amax() > 0) and all(torch.equal(y, want) for y in got)
+
+
+@pytest.mark.parametrize("H", [96, 500, 1024, 1056])
+def test_the_width_decides_the_order_of_additions(handle, H):
+    """A batch that runs a launch per step, its slices in one launch, and its first two steps by themselves: the same bits."""
+    import torch
+    from nebula_b200 import api
+    T, B = 4, 300
+    g = torch.Generator(device="cuda").manual_seed(H)
+    w = (torch.rand(8 * H + 4 * H * H + 4 * H * 64, device="cuda", generator=g) * 2 - 1) / H ** 0.5
+    x = torch.randn(T, B, 64, device="cuda", generator=g)
+    handle.set_math("tf32")
+    def run(steps, lo, hi):
+        plan = api.Lstm(handle, steps, hi - lo, 64, H, False, "linear")
+        plan.set_weights(w)
+        y = plan.forward(x[:steps, lo:hi].contiguous())
+        handle.synchronize()
+        plan.close()
+        return y
+    want = run(T, 0, B)
+    assert torch.equal(want, torch.cat([run(T, lo, hi) for lo, hi in ((0, 1), (1, 65), (65, 170), (170, 300))], 1))
+    assert torch.equal(want[:2, :64], run(2, 0, 64))
