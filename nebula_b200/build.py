@@ -19,7 +19,7 @@ LIBDIR = PKG / "lib"
 LIB = LIBDIR / "libnebula_b200.so"
 # (source, object name, extra flags)
 SOURCES = [(s, s, []) for s in ("api.cu", "network.cu", "plans.cu", "elementwise.cu", "gemm_simt.cu", "gemm_tcgen05.cu", "static_scratch.cu",
-                                "arena.cu", "lstm_persistent.cu", "recurrent_cluster.cu")]
+                                "arena.cu", "lstm_persistent.cu", "lstm_wide.cu", "recurrent_cluster.cu")]
 # the CUDA-core contraction, a module per pair of copy modes (gemm_simt.cuh)
 SOURCES += [("gemm_simt_kernels.cu", f"gemm_simt_kernels_{a}{b}", [f"-DNB_SIMT_A={a}", f"-DNB_SIMT_B={b}"]) for a in range(3) for b in range(3)]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",

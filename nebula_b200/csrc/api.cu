@@ -74,8 +74,8 @@ int nb_create(int device_id, nb_handle_t *handle) {
                                                 std::to_string(prop.major) + std::to_string(prop.minor));
         NB_CHECK_CUDA(cudaMalloc((void **)&h->d_status, sizeof(int)));
         NB_CHECK_CUDA(cudaMemset(h->d_status, 0, sizeof(int)));
-        NB_CHECK_CUDA(cudaMalloc((void **)&h->d_grid_sync, lstm_persistent_counters() * sizeof(unsigned int)));
-        NB_CHECK_CUDA(cudaMemset(h->d_grid_sync, 0, lstm_persistent_counters() * sizeof(unsigned int)));
+        NB_CHECK_CUDA(cudaMalloc((void **)&h->d_grid_sync, (lstm_persistent_counters() + 1) * sizeof(unsigned int)));
+        NB_CHECK_CUDA(cudaMemset(h->d_grid_sync, 0, (lstm_persistent_counters() + 1) * sizeof(unsigned int)));
         int coop = 0;
         NB_CHECK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_id));
         h->cooperative_launch = coop != 0;

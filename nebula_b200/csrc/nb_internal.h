@@ -62,7 +62,8 @@ struct nb_handle_s {
     int cc_major = 0;
     std::string last_error;
     int *d_status = nullptr;            // device status word (nb::DEV_*)
-    unsigned int *d_grid_sync = nullptr; // arrival counters of the persistent LSTM kernel (it leaves them zero)
+    unsigned int *d_grid_sync = nullptr; // arrival counters of lstm_persistent.cu (it leaves them zero), behind them that of lstm_wide.cu
+    mutable bool lstm_wide_ready = false; // lstm_wide.cu: its kernel is loaded, with its limit set
     mutable int lstm_clusters = -1;     // lstm_persistent.cu: clusters of its size that the device runs at once (-1: not asked yet)
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
     mutable int tc_clusters[17] = {0};  // gemm_tcgen05.cu: the same for its kernel, once tc_clusters_ready (-1: not asked yet)
@@ -383,6 +384,9 @@ void gemm_tc_prepare_device(nb_handle_s *h);
 int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H);
+bool lstm_wide_supported(const nb_handle_s *h, int T, int B, int H);
+void lstm_wide(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H, int kb_per_part,
+               int t_first);
 // Are the recurrent products of TF32 LSTM layers of this width added in slices of K, at every batch and number of steps, and of
 // how many K blocks of 32?
 bool lstm_in_slices(const nb_handle_s *h, int H);

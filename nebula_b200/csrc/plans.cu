@@ -627,7 +627,10 @@ size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, boo
     const bool tc_u = tcm && (in % 4) == 0 && in >= 32;
     const bool tc_w = tcm && (H % 4) == 0 && H >= 32;
     const bool three = h->math_mode == NB_MATH_TF32X3;
-    if (tc_w && !three && d.activation == NB_ACT_LINEAR) (void)lstm_in_slices(h, H);        // (loads the kernel)
+    if (tc_w && !three && d.activation == NB_ACT_LINEAR) {      // (loads the kernels)
+        (void)lstm_in_slices(h, H);
+        if (!lstm_persistent_supported(h, T, B, H)) (void)lstm_wide_supported(h, T, B, H);
+    }
     pre.reserve(rows * 4 * H);
     if (!tc_w) z.reserve((size_t)B * 4 * H);
     GemmArgs a;
@@ -701,9 +704,17 @@ void LstmPlan::forward(const float *x, float *out, float *cell, bool x_rounded, 
         return;
     }
     const char *lp_env = std::getenv("NEBULA_B200_LSTM_PERSISTENT");
-    if (tc_w && !three && linear && hr && lstm_persistent_supported(h, T, B, H) && !(lp_env && *lp_env == '0')) {
+    const bool tf32_steps = tc_w && !three && linear && hr && !(lp_env && *lp_env == '0');
+    if (tf32_steps && lstm_persistent_supported(h, T, B, H)) {
         ww.ensure_split(h);
         lstm_persistent(h, ww.hi.p, pre.p, cell, out, hr, T, B, H);
+        return;
+    }
+    // (it stores quads)
+    if (tf32_steps && !(((uintptr_t)out | (uintptr_t)cell) & 15) && lstm_wide_supported(h, T, B, H)) {
+        launch_lstm_cell(h, pre.p, nullptr, cell, out, hr, B, H);
+        ww.ensure_split(h);
+        lstm_wide(h, ww.hi.p, pre.p, cell, out, hr, T, B, H, lstm_in_slices(h, H) ? lstm_k_part(H) : H / 32, 1);
         return;
     }
     for (int t = 0; t < T; t++) {

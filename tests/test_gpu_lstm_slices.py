@@ -1,7 +1,6 @@
-"""The TF32 LSTM recurrence in one kernel (lstm_persistent.cu) at the edges of its tiles: widths off its 32-unit blocks and
-with empty slices of K, batches around the MMA's 16 columns, its groups of rows and
-the 128 rows of a chunk, three steps and more.  Against the CPU
-oracle, and bit for bit against a launch per step, which adds the same slices of K in the same order."""
+"""The TF32 LSTM recurrence in one kernel (lstm_persistent.cu; lstm_wide.cu for what does not fit that) at the edges of its tiles:
+widths off its 32-unit blocks and with empty slices of K, batches around the MMA's 16 columns, its groups of rows and the 128 rows
+of a chunk.  Against the CPU oracle, and bit for bit against a launch per step, which adds the same slices of K in the same order."""
 import numpy as np
 import pytest
 
@@ -12,7 +11,13 @@ pytestmark = pytest.mark.gpu
 # (T, B, inputs, H)
 CASES = [(3, 1, 32, 32), (3, 15, 36, 64), (4, 16, 32, 96), (3, 17, 40, 452), (5, 64, 32, 512), (3, 65, 64, 500), (3, 128, 32, 1020),
          (6, 3, 32, 1024), (3, 127, 32, 288), (3, 33, 32, 1184),
-         (3, 129, 32, 512), (3, 200, 32, 576), (3, 251, 32, 64), (4, 1000, 32, 32)]
+         (3, 129, 32, 512), (3, 200, 32, 576), (3, 251, 32, 64), (4, 1000, 32, 32),
+         (3, 65, 32, 1056), (5, 128, 32, 1056), (6, 1, 32, 1088), (9, 64, 64, 1088), (3, 100, 32, 1152), (12, 128, 32, 1184), (3, 20, 32, 1216),
+         (2, 64, 32, 256), (2, 128, 32, 1056), (2, 65, 32, 416), (2, 20, 32, 1184)]
+# launches fewer than a launch per step: step 0 is a kernel of its own in front of lstm_wide.cu
+WIDE = {(3, 33, 32, 1184), (3, 65, 32, 1056), (5, 128, 32, 1056), (6, 1, 32, 1088), (9, 64, 64, 1088), (3, 100, 32, 1152), (12, 128, 32, 1184),
+        (2, 64, 32, 256), (2, 128, 32, 1056), (2, 65, 32, 416)}
+PER_STEP = {(3, 200, 32, 576), (3, 20, 32, 1216), (2, 20, 32, 1184)}       # (more clusters, or weights, than the device holds)
 
 
 @pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(map(str, c)))
@@ -31,13 +36,16 @@ def test_lstm_in_slices_of_k(handle, case, monkeypatch):
     plan = api.Lstm(handle, T, B, inp, H, False, "linear")
     plan.set_weights(w)
     xd = torch.from_numpy(x).cuda()
-    runs = []
+    runs, launches = [], []
     for env in ("1", "0", "1"):                 # (the kernel leaves its counters ready for the next launch)
         monkeypatch.setenv("NEBULA_B200_LSTM_PERSISTENT", env)
+        n0 = handle.launch_count()
         out, cell = plan.forward(xd, want_cell=True)
+        launches.append(handle.launch_count() - n0)
         runs.append((out.clone(), cell.clone()))
     handle.synchronize()
     plan.close()
+    assert launches[1] - launches[0] == (0 if case in PER_STEP else T - 2 if case in WIDE else T - 1)
     assert_close(runs[0][0].cpu().numpy(), ref, "tf32", f"{case}")
     for out, cell in runs[1:]:
         assert torch.equal(out, runs[0][0]) and torch.equal(cell, runs[0][1])
