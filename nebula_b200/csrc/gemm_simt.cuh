@@ -10,8 +10,8 @@
 //   * Both operands lie in shared memory with K contiguous (rows of 16 floats, stride 20: eight rows of a 128-bit
 //     read fall into 32 different banks), so the copies are cp.async straight from global memory in the operands'
 //     own order (16 bytes each where alignment allows, else 4) and nothing is transposed by the threads.
-//   * Copies advance their addresses from block to block; what depends on the filter tap is worked out when a tap begins (per copy
-//     and block it was four tenths of all instructions, many of them on the FMA pipe).
+//   * Copies advance their addresses from block to block and from tap to tap; a tap begins with a comparison per row (64-bit
+//     products per copy and block were four tenths of all instructions, many of them on the FMA pipe).
 //   * A thread owns RM x RN outputs and multiplies with packed fma.rn.f32x2 along K: a 128-bit read delivers two
 //     packed pairs, the accumulator pair holds the even and the odd columns' sums.  At 8 x 8 outputs a k-quad is 16
 //     reads for 128 packed FMAs; the read port is idle three quarters of the time.
@@ -125,25 +125,7 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
     const int n0 = (int)(blockIdx.x % p.n_tiles) * BN;
     const int kb0 = blockIdx.z * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
 
-    // the rows this thread copies: A's pixel origins (-1: outside), B's first row
-    long a_base[MA::ROW_SLOTS];
-    int a_h[MA::ROW_SLOTS], a_w[MA::ROW_SLOTS];
-#pragma unroll
-    for (int i = 0; i < MA::ROW_SLOTS; i++) {
-        const long m = m0 + MA::row(tid, i);
-        a_base[i] = -1; a_h[i] = a_w[i] = 0;
-        if (MA::active(tid, i) && m < p.M) {
-            const int per = p.g.OH * p.g.OW;            // a row index fits 31 bits
-            const int n = (int)m / per, rem = (int)m - n * per, oh = rem / p.g.OW;
-            a_base[i] = (long)n * p.g.sn;
-            a_h[i] = oh * p.g.stride - p.g.pad;
-            a_w[i] = (rem - oh * p.g.OW) * p.g.stride - (p.g.pad_w >= 0 ? p.g.pad_w : p.g.pad);
-        }
-    }
-    const long b_base = (long)(n0 + MB::row(tid, 0)) * p.b_row;
-
-    // The K block the next copies fetch, and where each of them reads: the address arithmetic of a tap (64-bit products, which
-    // run on the FMA pipe) is done when the tap begins; from block to block a copy's address only advances.
+    // the K block the next copies fetch
     int c0 = 0, kh = 0, kw = 0;
     long b_tap = 0;
     if (kb0) {
@@ -152,19 +134,30 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
         kh = tap / p.ksize_w; kw = tap - kh * p.ksize_w;
         b_tap = (long)tap * p.b_tap;
     }
-    // (B's rows lie a constant distance apart, and so do the columns of a ONE_ROW thread: one address for all of its copies)
-    const float *a_src[MA::ROW_SLOTS], *b_src;
+    // Where the copies read: an address only advances, by the same distance for all rows, from block to block and from tap to tap
+    // (outside of the operand it is not used).  B's rows lie a constant distance apart, and so do the columns of a ONE_ROW thread:
+    // one address for all of its copies.
+    const float *a_src[MA::ROW_SLOTS], *b_src = p.b + b_tap + (long)(n0 + MB::row(tid, 0)) * p.b_row + (long)(c0 + MB::col(tid, 0)) * p.b_col;
+    int a_h[MA::ROW_SLOTS], a_w[MA::ROW_SLOTS];         // the pixels' origins
+#pragma unroll
+    for (int i = 0; i < MA::ROW_SLOTS; i++) {
+        const long m = m0 + MA::row(tid, i);
+        a_h[i] = a_w[i] = -(1 << 30);                   // (no row: outside at every tap)
+        a_src[i] = p.a;
+        if (MA::active(tid, i) && m < p.M) {
+            const int per = p.g.OH * p.g.OW;            // a row index fits 31 bits
+            const int n = (int)m / per, rem = (int)m - n * per, oh = rem / p.g.OW;
+            a_h[i] = oh * p.g.stride - p.g.pad;
+            a_w[i] = (rem - oh * p.g.OW) * p.g.stride - (p.g.pad_w >= 0 ? p.g.pad_w : p.g.pad);
+            a_src[i] += (long)n * p.g.sn + (long)(a_h[i] + kh) * p.g.sh + (long)(a_w[i] + kw) * p.g.sw + (long)(c0 + MA::col(tid, i)) * p.g.sc;
+        }
+    }
     unsigned a_in = 0, b_in = 0;            // row slots that lie inside
     auto begin_tap = [&]() {
         a_in = 0;
 #pragma unroll
-        for (int s = 0; s < MA::ROW_SLOTS; s++) {
-            const int ih = a_h[s] + kh, iw = a_w[s] + kw;
-            const bool in = a_base[s] >= 0 && ih >= 0 && ih < p.g.H && iw >= 0 && iw < p.g.W;
-            a_src[s] = in ? p.a + a_base[s] + (long)ih * p.g.sh + (long)iw * p.g.sw + (long)(c0 + MA::col(tid, s)) * p.g.sc : p.a;
-            a_in |= (in ? 1u : 0u) << s;
-        }
-        b_src = p.b + b_tap + b_base + (long)(c0 + MB::col(tid, 0)) * p.b_col;
+        for (int s = 0; s < MA::ROW_SLOTS; s++)
+            a_in |= ((unsigned)(a_h[s] + kh) < (unsigned)p.g.H && (unsigned)(a_w[s] + kw) < (unsigned)p.g.W ? 1u : 0u) << s;
     };
 #pragma unroll
     for (int s = 0; s < MB::ROW_SLOTS; s++) b_in |= (MB::active(tid, s) && n0 + MB::row(tid, s) < p.N ? 1u : 0u) << s;
@@ -173,6 +166,8 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
     const long a_step = AMODE == ONE_ROW ? BK * p.g.sc : BK, b_step = BMODE == ONE_ROW ? BK * p.b_col : BK;
     const long a_next = AMODE == ONE_ROW ? T::THREADS / BM * p.g.sc : 0;        // from one copy of a slot to the next
     const long b_next = BMODE == ONE_ROW ? T::THREADS / BN * p.b_col : T::THREADS / MB::PER_ROW * p.b_row;
+    // from behind a tap's last block to the next tap's first, in the same row of the filter, and what a new row adds
+    const long a_tap = p.g.sw - p.c_blocks * a_step, a_row = p.g.sh - p.ksize_w * p.g.sw, b_tap_step = p.b_tap - p.c_blocks * b_step;
     const bool whole = p.Kc % BK == 0;      // no block has columns past the last
     const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t a_dst = smem32 + (uint32_t)(MA::row(tid, 0) * LDK + MA::col(tid, 0)) * 4;
@@ -204,8 +199,12 @@ __global__ void __launch_bounds__((BM / RM) * (BN / RN)) gemm_fp32_simt_kernel(c
         b_src += b_step;
         c0 += BK;
         if (c0 >= p.Kc) {
-            c0 = 0; b_tap += p.b_tap;
-            if (++kw == p.ksize_w) { kw = 0; kh++; }
+            c0 = 0;
+            long next = a_tap;
+            if (++kw == p.ksize_w) { kw = 0; kh++; next += a_row; }
+#pragma unroll
+            for (int s = 0; s < MA::ROW_SLOTS; s++) a_src[s] += next;
+            b_src += b_tap_step;
             begin_tap();
         }
     };
