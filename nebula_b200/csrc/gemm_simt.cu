@@ -153,11 +153,12 @@ bool small_gemm(bool ta, bool tb, int M, int N, int K) {
 // Cycles of an SM that runs `on_sm` CTAs of tile shape i over K columns each: the share of the FMA rate that the shape reaches
 // (fewer outputs per operand read, longer runs between barriers), and its start and stores.  The 64 x 128 tile alone on an SM
 // lacks a second CTA to run behind its barriers, the more the shorter its copies.  Fitted to AlexNet's layers at 4 and 16 images and
-// to products of 64 to 2048 rows and K of 60 to 4000.
+// to products of 64 to 2048 rows and K of 60 to 4000; that tile's rate alone with whole quads to 880 layers and products timed with every
+// shape (968 x 89 x 2352 takes 27 us in 64 x 64 tiles, 41 in the 64 x 128 that a rate of 0.47 chose; 2873 x 348 x 96 14 and 25).
 double tile_cost(int i, const SimtVariant &v, long on_sm, int K, bool quads) {
     static const double rate[] = {0.50, 0.41, 0.36, 0.33}, fixed[] = {4000, 1300, 200, 400};
     double r = rate[i];
-    if (i == 0 && on_sm == 1) r = quads ? 0.47 : 0.30;
+    if (i == 0 && on_sm == 1) r = quads ? 0.38 : 0.30;
     return on_sm * ((double)v.bm * v.bn * K / 128 / r + fixed[i]);
 }
 
