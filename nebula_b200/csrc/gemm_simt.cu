@@ -219,10 +219,14 @@ void launch(nb_handle_s *h, SimtParams &p, int amode, int bmode, int S) {
     cfg.stream = h->stream;
     // Not launched ahead of the kernel in front: several of these CTAs fit an SM, and those that became resident early
     // would crowd the SMs which that kernel leaves free (AlexNet b4 fp32: 650 us in order, 764 us ahead).
-    // A few CTAs crowd nobody: 32 x 30 x 62 at the end of the deep belief network 10.5 -> 6.7 us.
+    // A few CTAs with little to do crowd nobody: 32 x 30 x 62 at the end of the deep belief network 10.5 -> 6.7 us, four layers of
+    // 300 at 16 rows 61 -> 56.  With much to do they spend it on the SMs they crowded (24 CTAs of 15 552 columns of K each: 491 us in
+    // order, about 680 ahead), and behind a layer of many rows, which is long itself, the line is lower (659 x 312 -> 10 and the three
+    // layers in front 75.6 us ahead, 70.9 in order).
+    const bool ahead = (long)cfg.gridDim.x * S <= h->sm_count / 4 && p.kb_per_split * BK <= (p.M <= 128 ? 512 : 256);
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = (long)cfg.gridDim.x * S <= h->sm_count / 4 ? 1 : 0;
+    at[0].val.programmaticStreamSerializationAllowed = ahead ? 1 : 0;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = 1; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = (unsigned)S;
     cfg.attrs = at;
