@@ -1221,6 +1221,12 @@ bool gemm_tc_supported(const nb_handle_s *h, const GemmArgs &a) {
     return true;
 }
 
+int tc_blocks_per_split(int c_blocks, int blocks, int S, int block_n) {
+    const int per = (blocks + S - 1) / S;
+    // whole pairs of K slices per split where that leaves none empty (256-wide tiles do not fetch pairs)
+    return per + (S > 1 && c_blocks % 2 == 0 && (per & 1) && block_n <= 128 && (long)(S - 1) * (per + 1) < blocks ? 1 : 0);
+}
+
 namespace {
 
 // Works out one launch: tiling, kernel variant, tensor maps; checks that every operand's extent lies inside the
@@ -1266,10 +1272,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     p.ksize_w = ksize_w; p.stride = g.stride; p.pad_h = g.pad; p.pad_w = g.pad_w >= 0 ? g.pad_w : g.pad;
     p.c_blocks = (kc + BLOCK_K - 1) / BLOCK_K;
     p.num_k_blocks = taps * p.c_blocks;
-    p.kb_per_split = (p.num_k_blocks + S - 1) / S;
-    // whole pairs of K slices per split where that leaves none empty (256-wide tiles do not fetch pairs)
-    if (S > 1 && p.c_blocks % 2 == 0 && (p.kb_per_split & 1) && a.block_n_hint <= 128 && (long)(S - 1) * (p.kb_per_split + 1) < p.num_k_blocks)
-        p.kb_per_split++;
+    p.kb_per_split = tc_blocks_per_split(p.c_blocks, p.num_k_blocks, S, a.block_n_hint);
     if (S > 1 && (long)(S - 1) * p.kb_per_split >= p.num_k_blocks)
         throw Error(NB_ERR_INVALID_ARG, "split-K needs non-empty splits of ceil(K blocks / splits) blocks");
     if (S > 1 && !cluster && (a.y_pool || a.addend || a.scale || a.shift || a.act != NB_ACT_LINEAR))
@@ -1571,8 +1574,19 @@ double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, in
     return per * block + heavy / S + 1.5 * S + 26.0 * (bn / 64) * (bn / 64) / (S * S);
 }
 
+// The time of the same cut into S slabs, by tiles in waves, and of the kernel that adds M rows of them (another 30 units behind the
+// product, 8 bytes per partial sum at 5 TB/s).  Clusters give one layer 16 times as many SMs as it has tiles at most, slabs all of
+// them: 10 x 42568 -> 28, a cluster of 16 31.6 us, 32 slabs 27.3; 55060 -> 80 35.2 and 23.5; 3xTF32, 7x7, 176 -> 32 at 5 images of 34 x 34,
+// two CTAs 72 and three slabs 52.  But 6068 -> 12 at 3 rows 9.6 and 11.2, 10132 -> 392 at 105 rows 18.7 and 22.4.
+double tc_slab_cost(const nb_handle_s *h, long m_tiles, long M, int N, int blocks, int S, int bn, bool three_pass) {
+    const double block = (three_pass ? 1.5 : 1.0) * (m_tiles == 1 ? (bn == 64 ? 1.0 : (bn == 128 ? 1.1 : 1.3)) : (bn == 64 ? 1.0 : 1.33));
+    const long tiles = m_tiles * ((N + bn - 1) / bn) * S;
+    return (double)((tiles + h->sm_count - 1) / h->sm_count) * ((blocks + S - 1) / S) * block + 38.0 + 7.1e-6 * S * M * N;
+}
+
 // The tile width and cluster size of a convolution.  In TF32 only where its 64-wide tiles leave half of the SMs idle, as above.
-TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool) {
+// Of `slabs` (conv_tc_split) instead where those take less time, with a layout pass behind them if the output is NCHW: TcSplit{slabs, 0}.
+TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool, int slabs, bool nchw) {
     TcSplit best{1, 0};
     const int c_blocks = (Kc + BLOCK_K - 1) / BLOCK_K, blocks = g.ksize * (g.ksize_w > 0 ? g.ksize_w : g.ksize) * c_blocks;
     if ((N % 4) != 0) return best;
@@ -1587,6 +1601,9 @@ TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, 
             const double cost = tc_cluster_cost(h, m_tiles, N, blocks, S, bn, three_pass, act);
             if (cost >= 0 && cost < best_cost) { best_cost = cost; best = TcSplit{S, bn}; }
         }
+    const long rows = (long)g.batch * g.OH * g.OW;
+    if (best.S > 1 && slabs > 1 && tc_slab_cost(h, m_tiles, rows, N, blocks, slabs, 64, three_pass) + (nchw ? 12.0 + 7.1e-6 * rows * N : 0.0) < best_cost)
+        return TcSplit{slabs, 0};
     return best;
 }
 

@@ -236,11 +236,14 @@ void gemm_tc(nb_handle_s *h, const GemmArgs &a, bool three_pass);
 // How many K slices (GemmArgs::split_k) an NHWC convolution should be cut into on the tensor cores; 1: none.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N);
 // How many CTAs of a cluster (GemmArgs::split_k; 1: no cluster) the K of an NHWC convolution's tiles should be cut over on the
-// tensor cores, and the tile width.
+// tensor cores, and the tile width (0: S is a number of slabs).
 struct TcSplit { int S, block_n; };
-TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool);
+TcSplit conv_tc_cluster(const nb_handle_s *h, const ConvGeom &g, int Kc, int N, int act, bool three_pass, bool pool, int slabs, bool nchw);
 constexpr int TC_MAX_CLUSTER = 16;
 double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, int S, int bn, bool three_pass, int act);
+double tc_slab_cost(const nb_handle_s *h, long m_tiles, long M, int N, int blocks, int S, int bn, bool three_pass);
+// K blocks of 32 in each of S slices (the last may be shorter), with tiles of block_n columns
+int tc_blocks_per_split(int c_blocks, int blocks, int S, int block_n);
 // Is an NCHW output (GemmArgs::y_nchw) the faster way for this convolution, against a layout pass behind it?
 bool conv_tc_writes_nchw(const GemmArgs &a, bool three_pass);
 // CUDA-core fp32 path: any extents, strides and alignments.

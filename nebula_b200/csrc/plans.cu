@@ -74,9 +74,6 @@ ConvPlan::ConvPlan(nb_handle_s *hh, const nb_conv2d_desc_t &desc) : nb_plan_s(NB
     // NEBULA_B200_ROW_WINDOWS=0 (read when the plan is created) sends these layers through the in-kernel gather instead
     const char *rw_env = std::getenv("NEBULA_B200_ROW_WINDOWS");
     tc_split = conv_tc_split(h, conv_args(nullptr, true).g, d.channels, d.filters);
-    for (int three = 0; three < 2; three++)
-        for (int pool = 0; pool < 2; pool++)
-            tc_cluster[three][pool] = conv_tc_cluster(h, conv_args(nullptr, true).g, d.channels, d.filters, d.activation, three, pool);
     rowwin_ok = !(rw_env && *rw_env == '0') && d.channels <= 4 && rw_inner <= 256 && d.stride <= 8 && h->encode_tiled &&
                 h->cc_major == 10;
 }
@@ -145,7 +142,12 @@ TcSplit ConvPlan::splits(const ForwardOpts &o, bool *clusters) const {
     *clusters = !(o.x_nhwc && (o.x_foreign || (pth == PATH_TC && !o.x_rounded)));
     if (pth == PATH_SIMT || o.addend) return TcSplit{1, 0};
     if (o.residual && ((o.res_c % 4) != 0 || ((uintptr_t)o.residual & 15))) return TcSplit{1, 0};     // (read in quads there)
-    return *clusters ? tc_cluster[pth == PATH_TC3][o.pool_out != nullptr] : TcSplit{tc_split, 0};
+    if (!*clusters) return TcSplit{tc_split, 0};
+    TcSplit &t = tc_cluster[pth == PATH_TC3][o.pool_out != nullptr][!o.y_nhwc];
+    if (t.S == 0)
+        t = conv_tc_cluster(h, conv_args(nullptr, true).g, d.channels, d.filters, d.activation, pth == PATH_TC3, o.pool_out != nullptr, tc_split, !o.y_nhwc);
+    *clusters = t.S == 1 || t.block_n > 0;
+    return t;
 }
 
 // The TMA-fed tensor-core routes write NCHW themselves where their pixel boxes suit it; the others (CUDA cores, in-kernel
@@ -439,32 +441,57 @@ void FcPlan::split_choice(GemmPath pth, bool has_addend, int rows, int *S_out, i
 }
 
 // The same over clusters, which run the whole epilogue.  Clusters do not fill the SMs (132 CTAs of fours, 120 of eights, 112 of
-// sixteens of 148), so weights that take long to stream go to slabs on all of them; the others take the width and size with the
-// shortest run, as convolutions do (conv_tc_cluster).  In TF32 from 2048 columns on that depends on K, N and the device only.
-// Any number of outputs: the rows of a ragged one are stored value by value (32 x 500 -> 30, logistic: 17.4 us whole, 6.2 here).
-void FcPlan::cluster_choice(GemmPath pth, int rows, int *S_out, int *block_n_out) const {
-    const int kblocks = (d.inputs + 31) / 32;
-    const long m_tiles = d.inputs >= 2048 ? 1 : (rows + 127L) / 128;
-    *S_out = 1; *block_n_out = 0;
-    if (2 * m_tiles * ((d.outputs + 63) / 64) > h->sm_count) return;
-    double best = tc_cluster_cost(h, m_tiles, d.outputs, kblocks, 1, 64, pth == PATH_TC3, d.activation);
-    for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
-        const double cost = tc_cluster_cost(h, m_tiles, d.outputs, kblocks, S, 64, pth == PATH_TC3, d.activation);
-        if (cost >= 0 && cost < best) { best = cost; *S_out = S; *block_n_out = 64; }
-    }
-}
-
+// sixteens of 148), so weights that take long to stream go to slabs on all of them, and so do few columns of long K (tc_slab_cost);
+// the others take the size with the shortest run, as convolutions do (conv_tc_cluster).  Any number of outputs: the rows of a
+// ragged one are stored value by value (32 x 500 -> 30, logistic: 17.4 us whole, 6.2 here).
+// In TF32 below 512 and from 2048 inputs on, the layer and the device alone decide in which slices a layer of clusters adds (below 512,
+// where many rows are as usual as few, the size that suits one, two and four rows of tiles); of more tiles than are resident at once the
+// same slices are slabs, or partial sums of whole tiles (442 x 5916 -> 408: as clusters one behind the other 54.3 us, as slabs 25;
+// 1362 x 7408 -> 120 59 and 31).  Between them, and in 3xTF32, the rows count.
 // (3xTF32 on a caller's tensor keeps the product and the addition of its slices as two kernels: the launches of such a call are
 // relied on)
-bool FcPlan::splits(GemmPath pth, const ForwardOpts &o, int rows, int *S, int *block_n) const {
-    split_choice(pth, o.addend != nullptr, rows, S, block_n);
-    if (pth == PATH_SIMT || o.addend || (pth == PATH_TC3 && (o.x_foreign || (*S == 1 && d.inputs >= 2048)))) return false;
-    if ((size_t)d.inputs * d.outputs > ((size_t)6 << 20)) return false;
-    int s, bn;
-    cluster_choice(pth, rows, &s, &bn);
-    if (s == 1) return false;
-    *S = s; *block_n = bn;
-    return true;
+FcPlan::Split FcPlan::splits(GemmPath pth, const ForwardOpts &o, int rows) const {
+    Split slabs{1, 0, 0, false};
+    split_choice(pth, o.addend != nullptr, rows, &slabs.S, &slabs.block_n);
+    const bool three = pth == PATH_TC3;
+    if (pth == PATH_SIMT || o.addend || (three && (o.x_foreign || (slabs.S == 1 && d.inputs >= 2048)))) return slabs;
+    if ((size_t)d.inputs * d.outputs > ((size_t)6 << 20)) return slabs;
+    const int kblocks = (d.inputs + 31) / 32, N = d.outputs;
+    const bool by_layer = !three && (d.inputs < 512 || d.inputs >= 2048);
+    const long row_tiles = (rows + 127L) / 128, m_tiles = by_layer ? 1 : row_tiles;
+    if (2 * m_tiles * ((N + 63) / 64) > h->sm_count) return slabs;
+    auto cluster_cost = [&](long m, int S) { return tc_cluster_cost(h, m, N, kblocks, S, 64, three, d.activation); };
+    auto cost_of = [&](int S) {
+        double cost = cluster_cost(m_tiles, S);
+        if (!by_layer || d.inputs >= 2048 || cost < 0) return cost;
+        cost *= 2;
+        for (int m = 2; m <= 4; m += 2) {
+            const double whole = cluster_cost(m, 1), cut = S > 1 ? cluster_cost(m, S) : whole;
+            cost += cut >= 0 ? std::min(cut, whole) : whole;
+        }
+        return cost;
+    };
+    Split best{1, 0, 0, false};
+    double best_cost = cost_of(1);
+    for (int S = 2; S <= TC_MAX_CLUSTER; S++) {
+        const double cost = cost_of(S);
+        if (cost >= 0 && cost < best_cost) { best_cost = cost; best = Split{S, 64, 0, true}; }
+    }
+    if (best.S == 1) return slabs;
+    if (slabs.S > 1 && tc_slab_cost(h, m_tiles, by_layer ? 64 : rows, N, kblocks, slabs.S, slabs.block_n, three) < cluster_cost(m_tiles, best.S)) return slabs;
+    if (!by_layer || row_tiles == 1) return best;
+
+    const int per = tc_blocks_per_split(kblocks, kblocks, best.S, 64);
+    best_cost = cluster_cost(row_tiles, best.S);
+    Split run = best;
+    for (int w = 64; w <= (N > 64 ? 128 : 64); w *= 2) {
+        // (slices of 256 K blocks and more are partial sums themselves)
+        const double whole = tc_cluster_cost(h, row_tiles, N, kblocks, 1, w, false, d.activation);
+        if (per < 256 && (best_cost < 0 || whole < best_cost)) { best_cost = whole; run = Split{1, w, per, false}; }
+        const double cut = tc_slab_cost(h, row_tiles, rows, N, kblocks, best.S, w, false);
+        if ((N % 4) == 0 && (best_cost < 0 || cut < best_cost)) { best_cost = cut; run = Split{best.S, w, 0, false}; }
+    }
+    return run;
 }
 
 size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
@@ -476,9 +503,8 @@ size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
         a.lda = a.ldb = a.Kc = d.inputs; a.M = M; a.N = d.outputs;
         gemm_simt_load(h, a);
     }
-    int S, bn;
-    const bool clusters = splits(pth, o, M, &S, &bn);
-    if (S > 1 && !clusters) split_ws.reserve((size_t)S * M * d.outputs);
+    const Split split = splits(pth, o, M);
+    if (split.S > 1 && !split.cluster) split_ws.reserve((size_t)split.S * M * d.outputs);
     return workspace_bytes();
 }
 
@@ -515,14 +541,15 @@ void FcPlan::forward(const float *x, float *y, const ForwardOpts &o, int rows) {
     a.b_static = w.split_ready;
     w.ensure_split(h);
     a.b = w.hi.p; a.b_lo = w.lo.p;
-    int S, block_n;
-    const bool clusters = splits(pth, o, M, &S, &block_n);
-    if (S > 1 && clusters) {
-        a.split_k = S; a.split_cluster = true; a.block_n_hint = block_n;
+    const Split split = splits(pth, o, M);
+    const int S = split.S;
+    a.k_part = split.k_part; a.block_n_hint = split.block_n;
+    if (S > 1 && split.cluster) {
+        a.split_k = S; a.split_cluster = true;
         gemm_tc(h, a, pth == PATH_TC3);
     } else if (S > 1) {
         GemmArgs sa = a;
-        sa.split_k = S; sa.block_n_hint = block_n;
+        sa.split_k = S;
         sa.scale = nullptr; sa.shift = nullptr; sa.act = NB_ACT_LINEAR; sa.round_out_tf32 = false;
         sa.y = split_ws.p; sa.ldy = d.outputs;
         sa.algo_flops = 2.0 * (double)M * d.outputs * d.inputs;

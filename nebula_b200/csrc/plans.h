@@ -77,9 +77,10 @@ struct ConvPlan : nb_plan_s {
     DeviceBuffer x_rowwin;
     DeviceBuffer scale, shift;
     bool has_scale = false, ready = false;
-    // K slices on the tensor cores, a search over pixel boxes, so done once: into slabs, and over clusters [3xTF32][pooled output]
+    // K slices on the tensor cores, a search over pixel boxes, so done once: into slabs, and over clusters when a call first asks
+    // (it loads their kernels) [3xTF32][pooled output][NCHW output]
     int tc_split = 1;
-    TcSplit tc_cluster[2][2];
+    mutable TcSplit tc_cluster[2][2][2] = {};
     int nchw_direct[2] = {-1, -1};      // TF32, 3xTF32: does the epilogue write NCHW?  (-1: not asked yet)
     DeviceBuffer x_scratch, y_scratch, split_ws;
     ConvPlan(nb_handle_s *h, const nb_conv2d_desc_t &desc);
@@ -116,8 +117,9 @@ struct FcPlan : nb_plan_s {
     size_t workspace_bytes() const override { return (x_scratch.n + split_ws.n) * sizeof(float); }
     // split-K choice for `rows` input rows: number of K slices (1: none) and the tile width that goes with it
     void split_choice(GemmPath pth, bool has_addend, int rows, int *S, int *block_n) const;
-    void cluster_choice(GemmPath pth, int rows, int *S_out, int *block_n_out) const;
-    bool splits(GemmPath pth, const ForwardOpts &o, int rows, int *S, int *block_n) const;      // true: over clusters
+    // how K is cut for `rows` input rows, and into partial sums of how many K blocks where it runs whole (0: as it comes)
+    struct Split { int S, block_n, k_part; bool cluster; };
+    Split splits(GemmPath pth, const ForwardOpts &o, int rows) const;
     void output_dims(int dims[3]) const override { dims[0] = d.outputs; dims[1] = 1; dims[2] = 1; }
     GemmPath path() const;
 };
