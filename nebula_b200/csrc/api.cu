@@ -105,7 +105,7 @@ int nb_create(int device_id, nb_handle_t *handle) {
                 h->trace_dev = (CUdeviceptr)dp;
             }
         }
-        gemm_tc_prepare_device(h);
+        gemm_tc_prepare_device();
         elementwise_prepare_device();
     });
     if (rc != NB_OK) {

@@ -798,7 +798,7 @@ void launch_shortcut(nb_handle_s *h, const nb_shortcut_desc_t &d, const float *p
     const bool small = total < (1ull << 32);
     const bool aligned = ((((uintptr_t)prev) | ((uintptr_t)conn) | ((uintptr_t)y)) & 15) == 0;
     const int plane = d.out_height * d.out_width;
-    const bool cheap = d.activation == NB_ACT_RELU || d.activation == NB_ACT_LEAKY || d.activation == NB_ACT_LINEAR;
+    const bool cheap = cheap_activation(d.activation);
     if (d.layout == NB_LAYOUT_NHWC && (d.conn_channels % 4) == 0 && (d.out_channels % 4) == 0 && aligned) {
         const auto kernel = cheap ? (small ? shortcut_nhwc4_kernel<unsigned, true> : shortcut_nhwc4_kernel<size_t, true>)
                                   : (small ? shortcut_nhwc4_kernel<unsigned, false> : shortcut_nhwc4_kernel<size_t, false>);

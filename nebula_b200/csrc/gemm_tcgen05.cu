@@ -1136,14 +1136,27 @@ inline bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 
-void gemm_tc_prepare_device(nb_handle_s *h) {
-    for (auto &g : VARIANTS)
-        for (auto &t : g)
+void gemm_tc_prepare_device() {
+    for (auto &t : VARIANTS[0])
+        for (auto &pr : t)
+            for (auto &v : pr)
+                if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+}
+
+void gemm_tc_load(const nb_handle_s *h, unsigned groups) {
+    groups &= ~h->tc_loaded;
+    auto load = [](const Variant &v) {
+        if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+    };
+    if (groups & TC_GATHER)
+        for (auto &t : VARIANTS[1])
             for (auto &pr : t)
-                for (auto &v : pr)
-                    if (v.kernel) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
-    for (auto &v : RESIDUAL_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
-    for (auto &v : LEAN_VARIANTS) NB_CHECK_CUDA(cudaFuncSetAttribute(v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem));
+                for (auto &v : pr) load(v);
+    if (groups & TC_LEAN)
+        for (auto &v : LEAN_VARIANTS) load(v);
+    if (groups & TC_RESIDUAL)
+        for (auto &v : RESIDUAL_VARIANTS) load(v);
+    h->tc_loaded |= groups;
 }
 
 // Clusters of `size` CTAs, one per SM, that run at once.  The cluster kernels are loaded by the first layer that they are a
@@ -1350,7 +1363,7 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
     // and its short ring takes one K block per stage: ResNet-50 b1 412 us without, 423 with.)
     const bool residual = a.addend && a.res_stride > 0 && !a.addend_after_act && !cluster && !promote && !gather && !col3 && p.e.addend_vec &&
                           p.e.addend_cols % 4 == 0 && !a.block_n_hint && taps == 1 && p.e.tma_store && a.shift &&
-                          (a.act == NB_ACT_RELU || a.act == NB_ACT_LEAKY || a.act == NB_ACT_LINEAR) && kc <= 512 && (long)p.m_tiles * ((a.N + 127) / 128) > h->sm_count;
+                          cheap_activation(a.act) && kc <= 512 && (long)p.m_tiles * ((a.N + 127) / 128) > h->sm_count;
     if (residual) block_n = std::min(block_n, 128);
     p.n_tiles = (a.N + block_n - 1) / block_n;
     p.m_fastest = (!a.a_is_conv && !gather && (size_t)a.N * a.Kc * 4 > ((size_t)48 << 20)) ? 1 : 0;
@@ -1515,9 +1528,10 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
 
     const int width = block_n == 256 ? 2 : (block_n == 128 ? 1 : 0);
     const bool lean = !three_pass && !promote && !gather && !cluster && p.e.tma_store && p.e.shift &&
-                      (a.act == NB_ACT_RELU || a.act == NB_ACT_LEAKY || a.act == NB_ACT_LINEAR) &&
+                      cheap_activation(a.act) &&
                       (!a.addend || (p.e.addend_vec && p.e.addend_cols % 4 == 0 && !p.e.addend_post));
     L->v = residual ? RESIDUAL_VARIANTS[width] : lean ? LEAN_VARIANTS[width] : cluster ? CLUSTER_VARIANTS[three_pass ? 1 : 0][promote ? 1 : 0][width] : VARIANTS[gather ? 1 : 0][three_pass ? 1 : 0][promote ? 1 : 0][width];
+    gemm_tc_load(h, residual ? TC_RESIDUAL : lean ? TC_LEAN : gather ? TC_GATHER : 0);
     L->cluster = cluster ? S : 1;
     if (!L->v.kernel) throw Error(NB_ERR_UNSUPPORTED, "no tensor-core kernel variant for this tile width");
     const int tiles = p.m_tiles * p.n_tiles * p.k_splits;
@@ -1567,7 +1581,7 @@ int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
 double tc_cluster_cost(const nb_handle_s *h, long m_tiles, int N, int blocks, int S, int bn, bool three_pass, int act) {
     const long tiles = m_tiles * ((N + bn - 1) / bn);
     const double block = (three_pass ? 1.5 : 1.0) * (bn == 64 ? 1.0 : 1.33);
-    const double heavy = act == NB_ACT_RELU || act == NB_ACT_LEAKY || act == NB_ACT_LINEAR ? 0.0 : 24.0 * bn / 64;     // the double formulas
+    const double heavy = cheap_activation(act) ? 0.0 : 24.0 * bn / 64;     // the double formulas
     if (S == 1) return (double)((tiles + h->sm_count - 1) / h->sm_count) * (blocks * block + heavy);
     const int per = (blocks + S - 1) / S;
     if ((long)(S - 1) * per >= blocks || tiles * S > h->sm_count || tiles > clusters_at_once(h, S)) return -1;

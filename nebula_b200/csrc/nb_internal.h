@@ -68,6 +68,7 @@ struct nb_handle_s {
     int clusters_at_once[17] = {0};     // by size (2, 4, 8, 16): clusters of one CTA per SM that the device runs at once
     mutable int tc_clusters[17] = {0};  // gemm_tcgen05.cu: the same for its kernel, once tc_clusters_ready (-1: not asked yet)
     mutable bool tc_clusters_ready = false;
+    mutable unsigned tc_loaded = 0;     // gemm_tcgen05.cu: groups of kernels that are loaded (gemm_tc_load)
     bool recurrent_ready = false;       // recurrent_cluster.cu: limits set, clusters_at_once filled
     unsigned long long simt_ready = 0;  // gemm_simt.cu: kernels loaded and with their limits set, by variant and copy modes
     bool cooperative_launch = false;    // the device co-schedules the CTAs of a cooperative launch
@@ -382,8 +383,13 @@ inline void key_add(std::string &k, const T &v) { k.append(reinterpret_cast<cons
 // Every field of a GemmArgs that decides a launch's parameters.
 std::string gemm_args_key(const GemmArgs &a, char tag, int extra);
 
-// Per-device set-up of the tensor-core kernels (shared-memory limits; also loads their code), once per handle.
-void gemm_tc_prepare_device(nb_handle_s *h);
+// Per-device set-up of the plain tensor-core kernels (shared-memory limits; also loads their code), once per handle.
+void gemm_tc_prepare_device();
+// The same for the others, which a plan asks for when it reserves its scratch, or else its first launch, captured ones included:
+// a process's first handle takes a third less time without them.
+enum : unsigned { TC_GATHER = 1, TC_LEAN = 2, TC_RESIDUAL = 4 };
+void gemm_tc_load(const nb_handle_s *h, unsigned groups);
+inline bool cheap_activation(int act) { return act == NB_ACT_RELU || act == NB_ACT_LEAKY || act == NB_ACT_LINEAR; }
 int lstm_persistent_counters();         // words of nb_handle_s::d_grid_sync
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H);
 void lstm_persistent(nb_handle_s *h, const float *w_hi, const float *pre, float *cell, float *out, float *hr, int T, int B, int H);

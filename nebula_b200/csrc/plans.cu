@@ -202,13 +202,15 @@ size_t ConvPlan::reserve(const ForwardOpts &o) {
     if (pth == PATH_SIMT && rowwin_ok) {
         x_rowwin.reserve((size_t)d.batch * d.height * rw_wp * 4);
         if (!tc_mode) gemm_simt_load(h, rowwin_args(nullptr, nullptr, true));
+        else if (h->math_mode == NB_MATH_TF32 && cheap_activation(d.activation)) gemm_tc_load(h, TC_LEAN);
     } else if (pth == PATH_SIMT && pack_ok && tc_mode && h->encode_tiled) {
-        // the kernel gathers x in place
+        gemm_tc_load(h, TC_GATHER);     // the kernel gathers x in place
     } else if (pth == PATH_SIMT) {
         gemm_simt_load(h, conv_args(nullptr, o.x_nhwc));
     } else {
         const bool need_round = (pth == PATH_TC) && !o.x_rounded;
         if (!o.x_nhwc || need_round || o.x_foreign) x_scratch.reserve(xin);
+        if (pth == PATH_TC && cheap_activation(o.residual ? o.res_act : d.activation)) gemm_tc_load(h, o.residual ? TC_LEAN | TC_RESIDUAL : TC_LEAN);
         bool clusters;
         const int S = splits(o, &clusters).S;
         if (S > 1 && !clusters) split_ws.reserve((size_t)S * yout);
@@ -503,6 +505,7 @@ size_t FcPlan::reserve(const ForwardOpts &o, int rows) {
         a.lda = a.ldb = a.Kc = d.inputs; a.M = M; a.N = d.outputs;
         gemm_simt_load(h, a);
     }
+    if (pth == PATH_TC && cheap_activation(d.activation)) gemm_tc_load(h, TC_LEAN);
     const Split split = splits(pth, o, M);
     if (split.S > 1 && !split.cluster) split_ws.reserve((size_t)split.S * M * d.outputs);
     return workspace_bytes();
@@ -654,6 +657,7 @@ size_t LstmPlan::reserve(bool own_cell, bool x_rounded, bool have_out_round, boo
     const bool tc_u = tcm && (in % 4) == 0 && in >= 32;
     const bool tc_w = tcm && (H % 4) == 0 && H >= 32;
     const bool three = h->math_mode == NB_MATH_TF32X3;
+    if (tc_u && !three && d.activation == NB_ACT_LINEAR) gemm_tc_load(h, TC_LEAN);
     if (tc_w && !three && d.activation == NB_ACT_LINEAR) {      // (loads the kernels)
         (void)lstm_in_slices(h, H);
         if (!lstm_persistent_supported(h, T, B, H)) (void)lstm_wide_supported(h, T, B, H);
