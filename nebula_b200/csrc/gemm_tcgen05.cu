@@ -206,7 +206,7 @@ __device__ __forceinline__ float4 ld_cluster(uint32_t smem_addr, int rank) {
 // (tanh layers of 512 x 256 x 256) 113 -> 102, VGG-16 b1 in 3xTF32 567 -> 535.
 template <int BLOCK_N, bool THREE, bool PROMOTE>
 __device__ __forceinline__ void cluster_epilogue(const TcParams &p, uint8_t *smem, uint32_t tmem_base, uint64_t *acc_full, uint64_t *acc_empty,
-                                                 uint64_t *x_empty, bool cross_cols, volatile int *abort_flag) {
+                                                 bool cross_cols, volatile int *abort_flag) {
     using C = Cfg<BLOCK_N, THREE, false>;
     constexpr int CH = BLOCK_N / 64, N4 = BLOCK_N / 4;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -690,7 +690,7 @@ gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type
         if (CLUSTER) cluster_barrier();
     } else if (CLUSTER && warp < 10) {
         if constexpr (CLUSTER)
-            cluster_epilogue<BLOCK_N, THREE, PROMOTE>(p, smem, tmem_base, acc_full, acc_empty, x_empty, cross_cols, abort_flag);
+            cluster_epilogue<BLOCK_N, THREE, PROMOTE>(p, smem, tmem_base, acc_full, acc_empty, cross_cols, abort_flag);
     } else if (warp < 10) {
         // ---------------------------------------------------------- epilogue
         // Two groups of four warps; group g owns the 32-column slabs of parity g, its own staging
@@ -1108,10 +1108,9 @@ const Variant VARIANTS[2][2][2][3] = {
       {variant<64, true, true, true>(), variant<128, true, true, true>(), {nullptr, 0}}}},
 };
 
-// index: [three][promote][block_n]: K cut over clusters
+// index: [three][promote][block_n]: K cut over clusters (in TF32 no wider tile was ever the better one)
 const Variant CLUSTER_VARIANTS[2][2][3] = {
-    {{variant<64, false, false, false, true>(), variant<128, false, false, false, true>(), variant<256, false, false, false, true>()},
-     {variant<64, false, true, false, true>(), variant<128, false, true, false, true>(), {nullptr, 0}}},
+    {{variant<64, false, false, false, true>(), {nullptr, 0}, {nullptr, 0}}, {variant<64, false, true, false, true>(), {nullptr, 0}, {nullptr, 0}}},
     {{{nullptr, 0}, {nullptr, 0}, {nullptr, 0}},
      {variant<64, true, true, false, true>(), variant<128, true, true, false, true>(), {nullptr, 0}}},
 };
@@ -1360,7 +1359,8 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
         }
     }
     // a shortcut's slabs through shared memory: 1x1 layers of several tiles per SM.  (A single tile per SM has nothing to fetch ahead of,
-    // and its short ring takes one K block per stage: ResNet-50 b1 412 us without, 423 with.)
+    // and its short ring takes one K block per stage: ResNet-50 b1 412 us without, 423 with.  That ring costs more the longer K is: 640 ->
+    // 1024 at 64 images of 14 x 14 62.3 us through shared memory and 59.5 from memory, 1024 -> 1024 89 and 76; 512 -> 1024 53 both.)
     const bool residual = a.addend && a.res_stride > 0 && !a.addend_after_act && !cluster && !promote && !gather && !col3 && p.e.addend_vec &&
                           p.e.addend_cols % 4 == 0 && !a.block_n_hint && taps == 1 && p.e.tma_store && a.shift &&
                           cheap_activation(a.act) && kc <= 512 && (long)p.m_tiles * ((a.N + 127) / 128) > h->sm_count;
