@@ -30,7 +30,7 @@ __device__ __forceinline__ float round_tf32(float x) {
 }
 
 // exp in double without branches, so that several of them overlap: the argument is reduced by Cody and Waite's split of ln 2
-// to |r| <= 0.35, the exponential of r is its Taylor polynomial of degree 12 (the rest is below 2^-53 of it), and the power of
+// to |r| <= 0.35, the exponential of r is its Taylor polynomial of degree 12 (the rest is at most 2.1 * 2^-53 of it), and the power of
 // two is added to the exponent.  Arguments are cut to +-708, where the result is still a normal number: the callers add it to 1,
 // or compare against where exp overflows themselves.  NaN stays NaN.
 // The library's exp and division branch on their special cases, which puts the chains of a thread's values one behind the

@@ -394,7 +394,7 @@ int chunk_rows_of(int B) { return (B + chunks_of(B) - 1) / chunks_of(B); }
 
 // Whether the recurrence of an LSTM layer can run as the persistent kernel: TF32 mode on the tensor-core path, gate layers
 // without an activation of their own, whole quads of units, weights and accumulators that fit tensor memory, all clusters
-// resident at once (up to 128 rows at H = 1024, 256 at 512, 1152 at 128).  A second launch for more rows gains little or loses:
+// resident at once (up to 128 rows at H = 1024, 256 at 512, 1024 at 128).  A second launch for more rows gains little or loses:
 // H = 1024, 8 steps: B = 129 / 256 / 512: 306 / 352 / 669 us in two or four launches, 309 / 344 / 472 launched step by step.
 // Two steps have one product, and the kernel's set-up costs more than its launch (T2 B64 H416, two layers: 66 and 54 us).
 bool lstm_persistent_supported(const nb_handle_s *h, int T, int B, int H) {
