@@ -380,12 +380,13 @@ __global__ void __launch_bounds__((THREE || GATHER) ? 448 : 320, 1)
 gemm_tf32_tcgen05_kernel(const __grid_constant__ typename ParamsOf<GATHER>::type p) {
     using C = Cfg<BLOCK_N, THREE, GATHER>;
     constexpr int STAGES = C::STAGES;                   // barrier slots; the ring uses the first p.stages of them
-    // The swizzle pattern repeats every 1024 bytes.  The compiler makes faster code where it does not see that the ring begins at such
-    // an address (7x7, 88 -> 40 at 9 images of 78 x 78 124 and 115 us, VGG-16 b8 in 3xTF32 1546 and 1525, ResNet-50 b64 2017 and 2004),
-    // and for the plain variants where it does not see either that it is shared memory (1x1, 3 -> 257 at 25 of 68 x 73 75 and 70).
+    // The swizzle pattern repeats every 1024 bytes.  The compiler makes faster code of the variants where it does not see that the ring
+    // begins at such an address (7x7, 88 -> 40 at 9 images of 78 x 78 124 and 115 us, VGG-16 b8 in 3xTF32 1546 and 1525, ResNet-50 b64 2017
+    // and 2004, the deep belief network 128.3 and 126.2; but 1x1, 3 -> 257 at 25 of 68 x 73 72 and 75), and of the plain 64-wide one where it
+    // does not see either that it is shared memory (1x1, 128 -> 24 at 50 of 62 x 62 75 and 72).
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = smem_raw;
-    if constexpr (!THREE && !PROMOTE && !GATHER && !CLUSTER && !LEAN) {
+    if constexpr (BLOCK_N == 64 && !THREE && !PROMOTE && !GATHER && !CLUSTER && !LEAN) {
         asm volatile("" : "+l"(smem));
     } else {
         uint32_t offset = 0;
@@ -1553,8 +1554,9 @@ std::unique_ptr<TcLaunch> build_launch(nb_handle_s *h, const GemmArgs &a, bool t
 
 // A convolution of one or a few small images has fewer tiles than SMs, and its tiles run their whole K alone: at about 0.15 us
 // per 32-column block (two TMA requests of one thread) the 3x3 layers of a single ResNet-50 image (8 tiles, 72 and 144
-// blocks) took 29 and 47 us.  Such layers are cut along K until they occupy the SMs, four blocks per slice at least; the
-// slices are added by splitk_reduce4_kernel (2-3 us), so layers of fewer than 32 blocks stay whole.  Tiles are counted over the
+// blocks) took 29 and 47 us.  Into slabs (a caller's NHWC tensor, and where tc_slab_cost is below the clusters' cost) such layers are
+// cut until they occupy the SMs, four blocks per slice at least; the slices are added by splitk_reduce4_kernel (2-3 us), so layers of
+// fewer than 32 blocks stay whole.  Tiles are counted over the
 // whole batch, so an image alone and the same image in a batch that leaves the layer whole, or cuts it into fewer slices, add
 // in different orders and may differ in the last bits.
 int conv_tc_split(const nb_handle_s *h, const ConvGeom &g, int Kc, int N) {
