@@ -136,7 +136,7 @@ bool ConvPlan::can_fuse_shortcut(int conn_c, int conn_h, int conn_w) const {
 }
 
 // K over clusters, whose CTAs run the whole epilogue.  A call on a caller's NHWC tensor, which takes a pass in front, keeps the
-// product and the addition of its slices as two kernels: the launches of such a call are relied on.
+// product and the addition of its slices as two kernels: its launch count is relied on (tests/test_gpu_split.py), at 2 to 3 us a call.
 TcSplit ConvPlan::splits(const ForwardOpts &o, bool *clusters) const {
     const GemmPath pth = path(o);
     *clusters = !(o.x_nhwc && (o.x_foreign || (pth == PATH_TC && !o.x_rounded)));
@@ -450,8 +450,8 @@ void FcPlan::split_choice(GemmPath pth, bool has_addend, int rows, int *S_out, i
 // where many rows are as usual as few, the size that suits one, two and four rows of tiles); of more tiles than are resident at once the
 // same slices are slabs, or partial sums of whole tiles (442 x 5916 -> 408: as clusters one behind the other 54.3 us, as slabs 25;
 // 1362 x 7408 -> 120 59 and 31).  Between them, and in 3xTF32, the rows count.
-// (3xTF32 on a caller's tensor keeps the product and the addition of its slices as two kernels: the launches of such a call are
-// relied on)
+// (3xTF32 on a caller's tensor keeps the product and the addition of its slices as two kernels: its launch count is relied on,
+// tests/test_gpu_ranges.py)
 FcPlan::Split FcPlan::splits(GemmPath pth, const ForwardOpts &o, int rows) const {
     Split slabs{1, 0, 0, false};
     split_choice(pth, o.addend != nullptr, rows, &slabs.S, &slabs.block_n);
