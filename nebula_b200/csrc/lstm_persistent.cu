@@ -199,11 +199,12 @@ __global__ void __launch_bounds__(LP_THREADS, 1) lstm_persistent_kernel(const __
             bool done = lane >= nkb;
             const unsigned int target = (unsigned int)(LP_SLICES * cell_warps) * (unsigned int)t;
             const long long t0 = clock64();
-            unsigned issued;                                // lanes whose copy of this step is under way
-            while (ok && (issued = __ballot_sync(0xffffffffu, done)) != 0xffffffffu) {
+            while (ok && !__all_sync(0xffffffffu, done)) {
+                // lanes whose copy of this step is under way (asked only where two copies of a step share a slot: 20 ns a step)
+                const unsigned issued = nkb > stages ? __ballot_sync(0xffffffffu, done) : 0xffffffffu;
                 bool give_up = false;
                 if (!done) {
-                    if ((issued & before) == before && ld_acquire_u32(counter) >= target && mbar_try_wait(&empty[slot], phase ^ 1)) {
+                    if (ld_acquire_u32(counter) >= target && (issued & before) == before && mbar_try_wait(&empty[slot], phase ^ 1)) {
                         // the units' stores (generic proxy) are ordered before the acquire; the copy (async proxy) behind this fence
                         asm volatile("fence.proxy.async;" ::: "memory");
                         mbar_expect_tx(&full[slot], tx);
