@@ -268,11 +268,12 @@ struct LstmWLaunch : LaunchRecord {
 // activation of their own, H a multiple of 32 whose weight slice and two ring stages fit in shared memory, one CTA per 32 gate
 // columns with all of them resident at once, a batch of at most 128 rows.  Two steps have one product, for which the set-up pays with
 // many rows and weights only (us, here and per step: 20 rows, H = 256 21.0 / 20.0, 768 24.9 / 24.0, 1184 29.3 / 28.9; 64 rows, H = 64
-// 27.3 / 26.2, 256 19.6 / 21.1, 768 23.3 / 25.9, 1024 25.2 / 28.9; 128 rows, H = 256 20.6 / 22.7, 1024 29.3 / 31.1).
+// 27.3 / 26.2, 256 19.6 / 21.1, 768 23.3 / 25.9, 1024 25.2 / 28.9; 128 rows, H = 256 20.6 / 22.7, 1024 29.3 / 31.1; 48 rows, H = 768
+// 24.7 / 27.1, 1024 26.5 / 29.4, 1184 30.7 / 29.9).
 bool lstm_wide_supported(const nb_handle_s *h, int T, int B, int H) {
     if (!h->encode_tiled || h->cc_major != 10 || !h->cooperative_launch) return false;
     if (T < 2 || B < 1 || B > 128 || (H % 32) != 0) return false;      // (a box of B rows: any B up to 128)
-    if (T == 2 && (B < 64 || H < 256)) return false;
+    if (T == 2 && (B < 40 || H < 256 || (B < 64 && (H < 768 || H > 1056)))) return false;
     const int ctas = 4 * H / LW_N;
     const size_t smem = (size_t)(H / BLOCK_K) * LW_W_TILE + 2 * (A_STAGE_BYTES + (size_t)B * 128) + 1024 + 256;   // two stages at least
     if (ctas > h->sm_count || smem > 227 * 1024) return false;

@@ -97,3 +97,22 @@ def test_the_width_decides_the_order_of_additions(handle, H):
     want = run(T, 0, B)
     assert torch.equal(want, torch.cat([run(T, lo, hi) for lo, hi in ((0, 1), (1, 65), (65, 170), (170, 300))], 1))
     assert torch.equal(want[:2, :64], run(2, 0, 64))
+
+
+@pytest.mark.parametrize("B,H", [(40, 768), (48, 1024), (63, 1056)])
+def test_two_steps_of_fewer_rows(handle, B, H, monkeypatch):
+    """From 40 rows on, two steps of wide layers are one launch behind step 0 too: bit for bit the launch per step."""
+    import torch
+    from nebula_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(H)
+    handle.set_math("tf32")
+    plan = api.Lstm(handle, 2, B, 32, H, False, "linear")
+    plan.set_weights((torch.rand(8 * H + 4 * H * H + 4 * H * 32, device="cuda", generator=g) * 2 - 1) / H ** 0.5)
+    x = torch.randn(2, B, 32, device="cuda", generator=g)
+    got = []
+    for env in ("0", "1"):
+        monkeypatch.setenv("NEBULA_B200_LSTM_PERSISTENT", env)
+        got.append(plan.forward(x))
+    handle.synchronize()
+    plan.close()
+    assert bool(got[0].abs().amax() > 0) and torch.equal(got[0], got[1])
