@@ -155,12 +155,14 @@ bool small_gemm(bool ta, bool tb, int M, int N, int K) {
 // lacks a second CTA to run behind its barriers, the more the shorter its copies.  Fitted to AlexNet's layers at 4 and 16 images and
 // to products of 64 to 2048 rows and K of 60 to 4000; that tile's rate alone with whole quads to 880 layers and products timed with every
 // shape (968 x 89 x 2352 takes 27 us in 64 x 64 tiles, 41 in the 64 x 128 that a rate of 0.47 chose; 2873 x 348 x 96 14 and 25), and its
-// rate where A's rows come value by value, for which it lacks the registers (2508 x 74 -> 1344 48 and 68 us).
-double tile_cost(int i, const SimtVariant &v, long on_sm, int K, bool quads, bool single_a) {
+// rate where A's rows come value by value, for which it lacks the registers (2508 x 74 -> 1344 48 and 68 us).  With ten blocks of K or
+// fewer its start and its 64 stores per thread are most of it (5x5, 3 -> 384 at 9 images of 51 x 51, tanh, 195 us, 123 in 32 x 64; 3x3, 8 ->
+// 352 at 10 of 58 x 58 59 and 43).
+double tile_cost(int i, const SimtVariant &v, long on_sm, int K, bool quads, bool single_a, bool split) {
     static const double rate[] = {0.50, 0.41, 0.36, 0.33}, fixed[] = {4000, 1300, 200, 400};
     double r = i == 0 && single_a ? 0.44 : rate[i];
     if (i == 0 && on_sm == 1) r = quads ? 0.38 : 0.30;
-    return on_sm * ((double)v.bm * v.bn * K / 128 / r + fixed[i]);
+    return on_sm * ((double)v.bm * v.bn * K / 128 / r + (i == 0 && !split && K <= 160 ? 12000 : fixed[i]));
 }
 
 // Ranges of K: none shorter than `least` columns, and only as many as it takes to occupy the SMs `times` over with 64 x 64 tiles of
@@ -190,7 +192,7 @@ const SimtVariant &ready_variant(nb_handle_s *h, long M, int N, int K, bool plai
         const SimtVariant &v = all[i];
         const long ctas = ((M + v.bm - 1L) / v.bm) * ((N + v.bn - 1L) / v.bn) * S;
         const long on_sm = (ctas + h->sm_count - 1) / h->sm_count;
-        const double cost = tile_cost(i, v, on_sm, K / S, amode == VEC_K && bmode == VEC_K, amode == ONE_K);
+        const double cost = tile_cost(i, v, on_sm, K / S, amode == VEC_K && bmode == VEC_K, amode == ONE_K, S > 1);
         if (i == 0 || cost < best_cost) { best_cost = cost; best = i; }
     }
     const SimtVariant &v = all[best];
